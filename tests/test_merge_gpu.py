@@ -163,3 +163,26 @@ def test_merge_stage_fixture_of_the_prefill_forward(heads, kv_heads, dim, chunk,
     finally:
         diagnostic.MERGE_HOOK = None
     assert seen == {"inputs": ["mapping", "remote_lse", "remote_out", "self_lse", "self_out"], "outputs": ["mixed_lse", "output"]}
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 64), (torch.float32, 40), (torch.float16, 256)])
+@pytest.mark.parametrize("kmax", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("rows", [33, 18943, 18944 + 45])
+def test_list_lengths_and_rows_per_warp(rows, kmax, dtype, D):
+    """Every list length the row kernel is compiled for and the one past it, with row counts below and above the one from
+    which a warp takes 32 rows (32 x 148 x 4), against the same formula in FP64.  FP32 sums of at most 33 terms: 33 x 2^-24
+    relative to the largest term, far inside 1e-5; the 16-bit outputs are rounded once (half an ulp: 2^-9, 2^-12)."""
+    from moba_opt.ops.merge_cuda import merge_forward_cuda
+    g = torch.Generator().manual_seed(rows + kmax)
+    keep = torch.cat([(torch.rand(rows, generator=g) < 0.6).nonzero()[:, 0] for _ in range(kmax)])
+    mp = keep[torch.randperm(keep.numel(), generator=g)].cuda()
+    so, sl = torch.randn(rows, 1, D, generator=g).to("cuda", dtype), torch.randn(rows, 1, generator=g).cuda() * 3
+    ro, rl = torch.randn(mp.numel(), 1, D, generator=g).to("cuda", dtype), torch.randn(mp.numel(), generator=g).cuda() * 3
+    out, lse = merge_forward_cuda(so, sl, ro, rl, mp, kmax=kmax)
+    w_self, w = sl.double()[:, 0].exp(), rl.double().exp()
+    z = w_self.clone().index_add_(0, mp, w)
+    acc = (w_self[:, None] * so.double()[:, 0]).index_add_(0, mp, w[:, None] * ro.double()[:, 0])
+    want = acc / z[:, None]
+    tol = {torch.float32: 1e-5, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    torch.testing.assert_close(out.double()[:, 0], want, atol=1e-5, rtol=tol)
+    torch.testing.assert_close(lse.double()[:, 0], z.log(), atol=1e-5, rtol=1e-5)
