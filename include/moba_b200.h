@@ -275,6 +275,17 @@ int moba_argmax_bf16(const void* logits, int n, void* workspace, size_t workspac
 int moba_decode_linear(const void* x, const void* h_in, const void* delta, const void* norm_weight, float eps, void* h_out,
                        const void* weight, const void* bias, int k, int n, int epilogue, void* y, void* stream);
 
+/* NaN/Inf check of up to three 16-bit tensors of a call (the eager cache operations refuse such inputs before they touch the
+ * cache: src/moba_opt/kv_cache.py:97-121 of the reference, torch.isfinite(t).all() per tensor) in one launch.
+ * flags [count] int32, zero on entry, in memory both sides can reach (pinned host memory or device memory); flags[i]
+ * becomes 1 when tensor i holds a value that is not finite, and may be read once the stream has passed this point. */
+typedef struct moba_finite_input {
+  const void* data;             /* [tokens, heads, dim], last dimension contiguous, any alignment */
+  int64_t tokens, stride_t, stride_h; /* element strides of token and head */
+  int32_t heads, reserved0;
+} moba_finite_input;
+int moba_check_finite(const moba_finite_input* inputs, int count, int dim, int fp16, int32_t* flags, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -44,6 +44,12 @@ class CacheDesc(ctypes.Structure):
                 + [(n, ctypes.c_void_p) for n in ("k_cache", "v_cache", "table", "lengths", "means")])
 
 
+class FiniteInput(ctypes.Structure):
+    """Mirror of moba_finite_input in include/moba_b200.h."""
+    _fields_ = [("data", ctypes.c_void_p), ("tokens", ctypes.c_int64), ("stride_t", ctypes.c_int64), ("stride_h", ctypes.c_int64),
+                ("heads", ctypes.c_int32), ("reserved0", ctypes.c_int32)]
+
+
 _P, _VP, _I, _SZ = ctypes.POINTER(CacheDesc), ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
 # entry point -> (result type, argument types); every decode entry point of include/moba_b200.h is bound from this table
 _DECODE_ABI = {
@@ -57,6 +63,7 @@ _DECODE_ABI = {
     "moba_decode_union_capacity": (_I, [_I, _I, _I, _I]),
     "moba_decode_route": (_I, [_P, _VP, _VP, _VP, _I, _I, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP]),
     "moba_decode_attend_workspace_bytes": (_SZ, [_P, _I, _I, _I]),
+    "moba_check_finite": (_I, [ctypes.POINTER(FiniteInput), _I, _I, _I, _VP, _VP]),
     "moba_decode_attend": (_I, [_P, _VP, _VP, _VP, _I, _I, _VP, _I, _VP, _VP, _VP, _I, _VP, _SZ, _VP, _VP, _VP, _VP]),
 }
 
@@ -146,11 +153,10 @@ class CacheLife(enum.Enum):
 
 @dataclass(frozen=True)
 class TensorRule:
-    """What a q / k / v argument has to satisfy; `check` raises ValueError with the reference's wording."""
+    """What a q / k / v argument has to satisfy besides being finite; `check` raises ValueError with the reference's wording."""
     name: str
     heads: object = None        # exact head count, or None
     tokens: object = None       # exact token count, or None
-    finite: bool = True
 
     def check(self, cache, t):
         n = self.name
@@ -168,8 +174,34 @@ class TensorRule:
             raise ValueError(f"{n} KV head count differs from cache")
         if self.tokens is not None and t.shape[0] != self.tokens:
             raise ValueError(f"{n} token count differs")
-        if self.finite and not bool(torch.isfinite(t).all()):      # reads a flag back: the host waits for the stream
-            raise ValueError(f"{n} contains NaN/Inf")
+
+
+class FiniteCheck:
+    """NaN/Inf check of the q, k, v of a call: one launch over all of them that writes into pinned words, one wait for
+    the stream.  The owner serialises calls (the cache's lock)."""
+
+    def __init__(self, lib, device):
+        self._lib, self._device = lib, device
+        self._words = torch.zeros(3, dtype=torch.int32, pin_memory=True)
+        self._flags = self._words.numpy()
+
+    def require(self, named):
+        """`named`: up to three (name, [N,H,D] 16-bit tensor of the cache's device); raises ValueError for the first that
+        is not finite."""
+        if not named:
+            return
+        args = (FiniteInput * 3)()
+        for a, (_, t) in zip(args, named):
+            a.data, a.tokens, a.heads = t.data_ptr(), t.shape[0], t.shape[1]
+            a.stride_t, a.stride_h = t.stride(0), t.stride(1)
+        self._flags[:] = 0
+        stream = torch.cuda.current_stream(self._device)
+        _ext.check(self._lib.moba_check_finite(args, len(named), named[0][1].shape[2], 1 if named[0][1].dtype == torch.float16 else 0,
+                                               self._words.data_ptr(), stream.cuda_stream), "moba_check_finite")
+        stream.synchronize()
+        for flag, (name, _) in zip(self._flags.tolist(), named):
+            if flag:
+                raise ValueError(f"{name} contains NaN/Inf")
 
 
 class HostStaging:
@@ -254,6 +286,7 @@ class PagedKVCache:
             self._candidate_count = 0
             self._status = _status_word(self.device)
             self._staging = HostStaging(self.device)
+            self._finite = FiniteCheck(self._lib, self.device)
             self._attend_buffers = {}         # (rows, Hq, slots, umax) -> union lists + split-K workspace, kept between calls
 
     # ------------------------------------------------------------------ views of the CPU layout
@@ -322,10 +355,19 @@ class PagedKVCache:
         return PreparedDecode(self, sequence_ids, num_q_heads, topk=topk, mode=mode, check_finite=check_finite,
                               stable_routes=stable_routes)
 
-    def _checked_kv(self, k, v, check_finite=True):
+    def _check_inputs(self, check_finite, **tensors):
+        """The contracts of the tensors given, in the order given; a tensor's NaN/Inf fault comes before the faults of the
+        tensors after it, as when they are checked one after the other."""
         check_finite = check_finite and self.check_finite
-        TensorRule("k", heads=self.num_kv_heads, finite=check_finite).check(self, k)
-        TensorRule("v", heads=self.num_kv_heads, tokens=k.shape[0], finite=check_finite).check(self, v)
+        tokens, seen = None, []
+        try:
+            for name, t in tensors.items():
+                TensorRule(name, heads=None if name == "q" else self.num_kv_heads, tokens=tokens).check(self, t)
+                tokens = t.shape[0]
+                seen.append((name, t))
+        finally:
+            if check_finite:
+                self._finite.require(seen)
 
     def _store(self, k, v, ids, counts, extra=()):
         """Plans the append on the CPU, sends the changed table entries, the new lengths, the segment description and
@@ -356,7 +398,7 @@ class PagedKVCache:
     def append(self, k, v, *, sequence_ids, cu_seqlens=None):
         with self._lock, torch.cuda.device(self.device):
             self._guard()
-            self._checked_kv(k, v)
+            self._check_inputs(True, k=k, v=v)
             self._refuse_pool_aliases(k, v)
             ids, counts = self._segments(k.shape[0], sequence_ids, cu_seqlens)
             _, starts, _ = self._store(k, v, ids, counts)
@@ -370,7 +412,7 @@ class PagedKVCache:
         before (as `prepare_decode` offers for decode steps)."""
         with self._lock, torch.cuda.device(self.device):
             self._guard()
-            self._checked_kv(k, v, check_finite)
+            self._check_inputs(check_finite, k=k, v=v)
             self._refuse_pool_aliases(k, v)
             ids, counts = self._segments(k.shape[0], sequence_ids, cu_seqlens)
             plan, _, _ = self._store(k, v, ids, counts)
@@ -378,7 +420,7 @@ class PagedKVCache:
 
     # ------------------------------------------------------------------ attend
     def _query_rows(self, q, sequence_ids, positions):
-        TensorRule("q", finite=self.check_finite).check(self, q)
+        self._check_inputs(True, q=q)
         if q.shape[1] % self.num_kv_heads:
             raise ValueError("Hq must be a multiple of Hkv")
         ids = self._layout.validate_ids(_ints(sequence_ids, "sequence_ids"))
@@ -454,8 +496,7 @@ class PagedKVCache:
         with self._lock, torch.cuda.device(self.device):
             self._guard()
             dense = wants_dense(mode, topk)
-            self._checked_kv(k, v)
-            TensorRule("q", tokens=k.shape[0], finite=self.check_finite).check(self, q)
+            self._check_inputs(True, k=k, v=v, q=q)
             self._refuse_pool_aliases(q, k, v)
             if q.shape[1] % self.num_kv_heads:
                 raise ValueError("Hq must be a multiple of Hkv")

@@ -114,7 +114,6 @@ class PreparedDecode:
             self._device_index = dev.index
             self._pool_storage = frozenset(_storage_address(t) for t in (cache.k_cache, cache.v_cache))
             self._input_storage = frozenset(_storage_address(t) for t in (self.q, self.k, self.v))
-            self._step_pairs = ((self.q, "q"), (self.k, "k"), (self.v, "v"))
             self._umax = lib.moba_decode_union_capacity(h, hk, self.remote, self.width)
             self._u_chunk = new((b, hk, self._umax), torch.int32)
             self._u_mask = new((b, hk, self._umax), torch.int32)
@@ -157,8 +156,8 @@ class PreparedDecode:
 
     def _accept(self, tensor, target, name):
         """The caller's tensor for the fixed buffer `target`: same shape, device, dtype, contiguous, no gradient, no
-        overlap with the cache pools or with another of the plan's input buffers, finite unless the plan skips that.
-        The buffer itself passes all but the last by construction."""
+        overlap with the cache pools or with another of the plan's input buffers.  The buffer itself passes by
+        construction."""
         if tensor is not target:
             if not isinstance(tensor, torch.Tensor) or tensor.shape != target.shape:
                 raise ValueError(f"{name} must have fixed shape {tuple(target.shape)}")
@@ -171,8 +170,18 @@ class PreparedDecode:
                 raise ValueError("append inputs must not alias KV cache storage; clone first")
             if where in self._input_storage:
                 raise ValueError("input aliases another prepared workspace; clone first")
-        if self.check_finite and not bool(torch.isfinite(tensor).all()):
-            raise ValueError(f"{name} contains NaN/Inf")
+
+    def _accept_all(self, inputs):
+        """`_accept` for every (tensor, target, name) and, unless the plan skips that, the NaN/Inf check of all of them in
+        one launch; a tensor's NaN/Inf fault comes before the faults of the tensors after it."""
+        seen = []
+        try:
+            for tensor, target, name in inputs:
+                self._accept(tensor, target, name)
+                seen.append((name, tensor))
+        finally:
+            if self.check_finite:
+                self.cache._finite.require(seen)
 
     # ------------------------------------------------------------------ driver interface
     def _stream(self):
@@ -274,7 +283,7 @@ class PreparedDecode:
     def attend(self, q, *, use_graph=False):
         with self.cache._lock, torch.cuda.device(self._device_index):
             self._usable()
-            self._accept(q, self.q, "q")
+            self._accept_all(((q, self.q, "q"),))
             pos = tuple(self._state.lengths[s] - 1 for s in self.ids)
             if min(pos) < 0:
                 raise ValueError("query positions must refer to cached tokens")
@@ -291,8 +300,7 @@ class PreparedDecode:
         with self.cache._lock, torch.cuda.device(self._device_index):
             self._usable()
             pairs = ((q, self.q), (k, self.k), (v, self.v))
-            for (tensor, target), (_, name) in zip(pairs, self._step_pairs):
-                self._accept(tensor, target, name)
+            self._accept_all(((q, self.q, "q"), (k, self.k, "k"), (v, self.v, "v")))
             if use_graph and "step" not in self._graphs:
                 raise ValueError("capture('step') first")
             plan = self._state.plan()

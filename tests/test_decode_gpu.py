@@ -391,3 +391,30 @@ def test_cache_contract_violations(kwargs):
     cfg.update(kwargs)
     with pytest.raises(ValueError):
         PagedKVCache(**cfg)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("layout", ["whole", "fused", "odd"])
+def test_one_finite_check_for_all_inputs(dtype, layout):
+    """First and last element of each tensor, NaN and both infinities; the largest finite values pass.  `fused`: views of
+    one projection's output (16-byte aligned rows); `odd`: rows that start on 2-byte boundaries, read element by element."""
+    from moba_opt import PagedKVCache
+    tokens, hq, hk, d = 37, 6, 2, 24
+    cache = PagedKVCache(1, 64, hk, d, dtype=dtype)
+    if layout == "whole":
+        q, k, v = (torch.full((tokens, h, d), torch.finfo(dtype).max, device="cuda", dtype=dtype) for h in (hq, hk, hk))
+    else:
+        pad = 0 if layout == "fused" else 1
+        qkv = torch.full((tokens, hq + 2 * hk, d + pad), torch.finfo(dtype).min, device="cuda", dtype=dtype)[..., pad:]
+        q, k, v = qkv[:, :hq], qkv[:, hq:hq + hk], qkv[:, hq + hk:]
+    named = [("k", k), ("v", v), ("q", q)]
+    cache._finite.require(named)
+    for name, t in named:
+        for at in ((0, 0, 0), (tokens - 1, t.shape[1] - 1, d - 1), (tokens // 2, 0, 11)):
+            for bad in (float("nan"), float("inf"), float("-inf")):
+                keep = t[at].clone()
+                t[at] = bad
+                with pytest.raises(ValueError, match=f"{name} contains NaN/Inf"):
+                    cache._finite.require(named)
+                t[at] = keep
+    cache._finite.require(named)
