@@ -557,22 +557,16 @@ struct AttendArgs {
   float* lse;
   unsigned* status;
   float scale_log2;
+  int rowgs, spc, min_stages;  // streamed variant: (row, kv head) pairs, stages of a whole chunk, least stages per CTA
 };
 
 constexpr int kHeadBlock = 16;    // query heads of a group processed together (MMA M dimension)
 constexpr int kStageTokens = 64;  // tokens per pipeline stage: 16 per warp
-// Two 32 KB stages (D <= 128) and 160 registers let three CTAs share an SM; measured faster than three
-// stages with two CTAs when the grid fills the GPU.  A grid of at most one CTA per SM (a batch of one or two
-// requests) is bound by latency instead: each stage then costs one trip to memory and one dependent chain of
-// math, so that case runs two teams of four warps, each with a ring of its own over half of the part's stages,
-// which together have up to a whole 512-token part in flight.
-#ifndef MOBA_DEC_STAGES
-#define MOBA_DEC_STAGES 2
-#endif
-#ifndef MOBA_DEC_MINBLOCKS
-#define MOBA_DEC_MINBLOCKS 3
-#endif
-constexpr int kStages = MOBA_DEC_STAGES;  // cp.async stages in flight per CTA, throughput variant
+// A grid of at most one CTA per SM (a batch of one or two requests) is bound by latency: each stage then costs one
+// trip to memory and one dependent chain of math, so that case runs two teams of four warps, each with a ring of its own
+// over half of the part's stages, which together have up to a whole 512-token part in flight.  Everything larger is
+// streamed (decode_attend_stream_kernel).
+constexpr int stream_stages(int dp) { return dp <= 64 ? 4 : 2; }  // streamed variant: 64 KB of ring per CTA at D = 64 and 128, three CTAs per SM
 constexpr int deep_stages(int dp) { return dp <= 64 ? 4 : dp <= 128 ? 2 : 3; }  // latency variant, per team (two teams up to D = 128)
 
 // Shared-memory K/V stage: row = one token, DP bf16 values; the 16-byte units of a row are
@@ -693,7 +687,7 @@ __device__ __noinline__ float4 merge_tail_acc(const MergeTail& t, long long hbas
 // own; the latency variant runs two teams, each on half of the part's stages, because with one warp per scheduler
 // nothing hides the dependent chain of a stage (ldmatrix, mma, shuffles, exp2, mma).
 template <int DP, int NS, int TEAMS, bool F16>
-__global__ void __launch_bounds__(128 * TEAMS, (TEAMS == 1 && DP <= 128 ? MOBA_DEC_MINBLOCKS : 1)) decode_attend_kernel(AttendArgs a) {
+__global__ void __launch_bounds__(128 * TEAMS, 1) decode_attend_kernel(AttendArgs a) {
   constexpr int NT = 128 * TEAMS, NW = 4 * TEAMS;  // threads and warps of the CTA
   constexpr int KSTEPS = DP / 16;
   constexpr int DT = DP / 8;  // 8-column output tiles
@@ -1029,6 +1023,343 @@ __global__ void __launch_bounds__(128 * TEAMS, (TEAMS == 1 && DP <= 128 ? MOBA_D
   if (tid == 0) a.counters[rowg] = 0;  // ready for the next launch (graph replay included)
 }
 
+// ---- streamed variant -------------------------------------------------------------------------------------------
+// Bound by HBM; what kept it from there was the division of the work.  One CTA per (union chunk, part) left 256 KB to a
+// CTA at D = 128, which starts with four dependent trips to memory and ends with a partial and a ticket, the last wave of CTAs was
+// partly empty, and the merge of a long context had a partial per chunk.  Here the stages (64 tokens) of every (row, kv head) pair - of its
+// union of chunks, or of its whole context in dense mode - laid end to end are one list, and each of the CTAs that fit the
+// GPU at once takes an equal, consecutive share of it.  Eight requests of 16K-32K tokens, dense, 28/4 heads, D = 128:
+// 98.7 -> 78 us (4.1 -> 5.1 TB/s), step 111 -> 88 us; 64 requests of 4K-64K, routed, 12/2 heads, D = 128: step 264 -> 239 us.
+// A share may begin and end anywhere; what a CTA holds of one pair is a segment, with one partial per head in slot
+// (CTA + pair), which no other segment has, and the slots of a pair are consecutive.  The division depends on the
+// positions alone, so a result is bit-repeatable.
+struct StreamShare {
+  int total, ctas, base, rem;
+  __device__ __forceinline__ StreamShare(int stages, int grid, int least) : total(stages) {
+    ctas = min(grid, max(1, stages / least));
+    base = total / ctas;
+    rem = total - base * ctas;
+  }
+  __device__ __forceinline__ int first(int cta) const { return cta * base + min(cta, rem); }
+  __device__ __forceinline__ int owner(int stage) const {
+    const int wide = rem * (base + 1);  // stages of the CTAs that take one more than the others
+    return stage < wide ? stage / (base + 1) : rem + (stage - wide) / base;
+  }
+};
+
+template <int DP, int NS, bool F16>
+__global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_kernel(AttendArgs a) {
+  constexpr int KSTEPS = DP / 16;
+  constexpr int DT = DP / 8;
+  constexpr int STAGE_BYTES = 2 * kStageTokens * DP * 2;
+  constexpr int META = 2 * NS;  // slots of s_nv / s_mask: a slot is rewritten NS stages ahead, while its ring neighbours are read
+  extern __shared__ __align__(128) uint8_t s_pipe[];
+  __shared__ long long s_rowbase[NS][kStageTokens];
+  __shared__ int s_nv[META];
+  __shared__ unsigned s_mask[META];
+  __shared__ int s_sum[4], s_first, s_first_at, s_last;
+  __shared__ float s_big[32], s_inv[32];
+  dependents_may_start();
+  wait_for_predecessor();  // routes, positions, the appended row
+  const CacheView& cv = a.cv;
+  const int D = cv.D, G = a.Hq / cv.Hkv;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int qr = lane >> 2, qc = lane & 3;
+  const bool dense = a.selected == nullptr;
+  auto stages_of = [&](int rowg, int& visible) {
+    const int row = rowg / cv.Hkv;
+    const int pos = a.positions[row];
+    const int listed = dense ? 1 : a.u_count[rowg];
+    visible = min(pos + 1, cv.lengths[a.ids[row]]);
+    const int own = dense ? visible : visible - pos / cv.C * cv.C;
+    return (listed - 1) * a.spc + max(0, (own + kStageTokens - 1) / kStageTokens);
+  };
+  // this CTA's share: every thread sums a run of pairs, the sums are scanned, the thread that holds the share's first stage finds its pair
+  const int per = (a.rowgs + 127) >> 7;
+  const int p0 = min(a.rowgs, tid * per), p1 = min(a.rowgs, p0 + per);
+  int mine = 0, visible;
+#pragma unroll 4
+  for (int p = p0; p < p1; ++p) mine += stages_of(p, visible);
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int n = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += n;
+  }
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  int before = incl - mine;
+  for (int w = 0; w < warp; ++w) before += s_sum[w];
+  const StreamShare share(s_sum[0] + s_sum[1] + s_sum[2] + s_sum[3], gridDim.x, a.min_stages);
+  if ((int)blockIdx.x >= share.ctas) return;
+  int at = share.first(blockIdx.x);
+  const int end = share.first(blockIdx.x + 1);
+  if (at >= end) return;
+  if (at >= before && at < before + mine) {
+    int p = p0, start = before;
+    for (;; ++p) {
+      const int n = stages_of(p, visible);
+      if (at < start + n) break;
+      start += n;
+    }
+    s_first = p; s_first_at = start;
+  }
+  __syncthreads();
+  int rowg = s_first, start = s_first_at;
+
+  for (; at < end; ++rowg) {
+    const int pair_stages = stages_of(rowg, visible);
+    if (pair_stages == 0) continue;
+    const int j0 = at - start, ntiles = min(pair_stages, end - start) - j0;  // this segment: stages [j0, j0 + ntiles) of the pair
+    const int row = rowg / cv.Hkv, g = rowg - row * cv.Hkv;
+    const int sid = a.ids[row];
+    const int slot = blockIdx.x + rowg;
+    const unsigned all_heads = G >= 32 ? 0xFFFFFFFFu : ((1u << G) - 1u);
+    const int span = dense ? kStageTokens : cv.C;  // tokens of a list entry; dense: the context is a list of stages
+
+    for (int hb = 0; hb < G; hb += kHeadBlock) {
+      // the next stage to look up: entry of the list, stage inside the entry
+      int look_u = j0 / a.spc, look_off = j0 - look_u * a.spc;
+      int look_chunk = dense ? look_u : a.u_chunk[(long long)rowg * a.umax + look_u];
+      unsigned look_mask = dense ? all_heads : a.u_mask[(long long)rowg * a.umax + look_u];
+      bool look_bad = false;
+      int look_nv = 0;
+      unsigned look_heads = 0;
+      // row base of this thread's token of the stage, and the stage's token count and heads
+      auto lookup = [&]() {
+        const int t0 = look_chunk * span + look_off * kStageTokens, t = t0 + tid;
+        const int limit = min((look_chunk + 1) * span, visible);
+        const int pg = t / cv.page;
+        look_nv = limit - t0;
+        look_heads = look_mask;
+        const long long base = attend_row_base(cv, sid, g, pg, t - pg * cv.page, t < limit, look_bad);
+        if (++look_off == a.spc) {
+          look_off = 0; ++look_u;
+          if (dense) look_chunk = look_u;
+          else if (look_u < a.umax) {
+            look_chunk = a.u_chunk[(long long)rowg * a.umax + look_u];
+            look_mask = a.u_mask[(long long)rowg * a.umax + look_u];
+          }
+        }
+        return base;
+      };
+      long long first_base[NS];
+      int first_nv[NS];
+      unsigned first_heads[NS];
+      if (tid < kStageTokens) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          first_base[s] = s < ntiles ? lookup() : -1;
+          first_nv[s] = look_nv; first_heads[s] = look_heads;
+        }
+      }
+      uint32_t qf[KSTEPS][4];
+      {
+        const bool r0 = hb + qr < G, r1 = hb + qr + 8 < G;
+        const __nv_bfloat16* q0 = a.q + ((long long)row * a.Hq + g * G + hb + qr) * D;
+        const __nv_bfloat16* q1 = q0 + 8 * D;
+#pragma unroll
+        for (int ks = 0; ks < KSTEPS; ++ks) {
+          const int c0 = ks * 16 + qc * 2, c1 = c0 + 8;
+          qf[ks][0] = (r0 && c0 < D) ? *reinterpret_cast<const uint32_t*>(q0 + c0) : 0u;
+          qf[ks][1] = (r1 && c0 < D) ? *reinterpret_cast<const uint32_t*>(q1 + c0) : 0u;
+          qf[ks][2] = (r0 && c1 < D) ? *reinterpret_cast<const uint32_t*>(q0 + c1) : 0u;
+          qf[ks][3] = (r1 && c1 < D) ? *reinterpret_cast<const uint32_t*>(q1 + c1) : 0u;
+        }
+      }
+      float o[DT][4];
+#pragma unroll
+      for (int dt = 0; dt < DT; ++dt) { o[dt][0] = o[dt][1] = o[dt][2] = o[dt][3] = 0.f; }
+      float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+
+      __syncthreads();  // the previous head block or segment is done with shared memory
+      if (tid < kStageTokens) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          s_rowbase[s][tid] = first_base[s];
+          if (tid == 0) { s_nv[s] = first_nv[s]; s_mask[s] = first_heads[s]; }
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int s = 0; s < NS - 1; ++s) {
+        if (s < ntiles) attend_load_stage<DP>(cv, s_pipe + s * STAGE_BYTES, s_rowbase[s], tid);
+        cp_async_commit();
+      }
+      for (int i = 0; i < ntiles; ++i) {
+        cp_async_wait<NS - 2>();
+        __syncthreads();  // tile i has landed; every warp finished tile i-1, whose buffer is refilled next
+        const int nx = i + NS - 1;
+        if (nx < ntiles) attend_load_stage<DP>(cv, s_pipe + (nx % NS) * STAGE_BYTES, s_rowbase[nx % NS], tid);
+        cp_async_commit();
+        // look up the rows of tile nx+1 now, publish them after this tile's math (ring slot i % NS is free)
+        long long next_base = -1;
+        const bool more = tid < kStageTokens && nx + 1 < ntiles;
+        if (more) next_base = lookup();
+        const int tok0 = warp * 16;
+        const int nvalid = s_nv[i % META] - tok0;
+        const unsigned heads = s_mask[i % META] >> hb;
+        if (nvalid > 0 && (heads & 0xFFFFu)) {  // warp-uniform
+          const bool on0 = (heads >> qr) & 1u, on1 = (heads >> (qr + 8)) & 1u;
+          const uint32_t kbase = smem_u32(s_pipe + (i % NS) * STAGE_BYTES);
+          const uint32_t vbase = kbase + kStageTokens * DP * 2;
+          float sc[2][4];
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) { sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f; }
+#pragma unroll
+          for (int ks = 0; ks < KSTEPS; ++ks) {
+            uint32_t b[4];
+            const int mat = lane >> 3, r = lane & 7;
+            ldmatrix_x4(kbase + kv_unit_offset<DP>(tok0 + (mat >> 1) * 8 + r, ks * 2 + (mat & 1)), b);
+            mma_16816<F16>(sc[0], qf[ks], b[0], b[1]);
+            mma_16816<F16>(sc[1], qf[ks], b[2], b[3]);
+          }
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int col = nt * 8 + qc * 2 + (e & 1);
+              sc[nt][e] = col < nvalid && (e < 2 ? on0 : on1) ? sc[nt][e] * a.scale_log2 : -INFINITY;
+            }
+          }
+          float mx0 = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
+          float mx1 = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
+          mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 1));
+          mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 2));
+          mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 1));
+          mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 2));
+          const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);
+          // a head that has attended nothing so far keeps -inf; its exponentials are taken against 0 and are 0
+          const float b0 = n0 == -INFINITY ? 0.f : n0, b1 = n1 == -INFINITY ? 0.f : n1;
+          const float al0 = m0 == n0 ? 1.f : dec_exp2(m0 - b0), al1 = m1 == n1 ? 1.f : dec_exp2(m1 - b1);
+          m0 = n0; m1 = n1;
+          uint32_t pf[4];
+          {
+            const float p00 = dec_exp2(sc[0][0] - b0), p01 = dec_exp2(sc[0][1] - b0), p02 = dec_exp2(sc[0][2] - b1), p03 = dec_exp2(sc[0][3] - b1);
+            const float p10 = dec_exp2(sc[1][0] - b0), p11 = dec_exp2(sc[1][1] - b0), p12 = dec_exp2(sc[1][2] - b1), p13 = dec_exp2(sc[1][3] - b1);
+            l0 = l0 * al0 + (p00 + p01) + (p10 + p11);
+            l1 = l1 * al1 + (p02 + p03) + (p12 + p13);
+            pf[0] = pack16<F16>(p00, p01); pf[1] = pack16<F16>(p02, p03);
+            pf[2] = pack16<F16>(p10, p11); pf[3] = pack16<F16>(p12, p13);
+          }
+          const bool rescale = __any_sync(0xFFFFFFFFu, al0 != 1.f || al1 != 1.f);
+#pragma unroll
+          for (int dp = 0; dp < DT / 2; ++dp) {
+            uint32_t b[4];
+            const int mat = lane >> 3, r = lane & 7;
+            ldmatrix_x4_trans(vbase + kv_unit_offset<DP>(tok0 + (mat & 1) * 8 + r, dp * 2 + (mat >> 1)), b);
+#pragma unroll
+            for (int h2 = 0; h2 < 2; ++h2) {
+              float (&acc)[4] = o[dp * 2 + h2];
+              if (rescale) { acc[0] *= al0; acc[1] *= al0; acc[2] *= al1; acc[3] *= al1; }
+              mma_16816<F16>(acc, pf, b[h2 * 2], b[h2 * 2 + 1]);
+            }
+          }
+        }
+        if (more) {
+          s_rowbase[i % NS][tid] = next_base;
+          if (tid == 0) { s_nv[(nx + 1) % META] = look_nv; s_mask[(nx + 1) % META] = look_heads; }
+        }
+      }
+      if (look_bad) atomicOr(a.status, kErrBadIndex);
+      // combine the warps, then write one partial per head of the block
+      cp_async_wait<0>();
+      l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 1); l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 2);
+      l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 1); l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 2);
+      __syncthreads();
+      float* s_o = reinterpret_cast<float*>(s_pipe);  // [4 warps][16 rows][DP]
+      float* s_ml = s_o + 4 * 16 * DP;                  // [4 warps][16 rows][2]
+#pragma unroll
+      for (int dt = 0; dt < DT; ++dt) {
+        float* w0 = s_o + ((size_t)warp * 16 + qr) * DP + dt * 8 + qc * 2;
+        float* w1 = w0 + 8 * DP;
+        w0[0] = o[dt][0]; w0[1] = o[dt][1]; w1[0] = o[dt][2]; w1[1] = o[dt][3];
+      }
+      if (qc == 0) {
+        s_ml[((size_t)warp * 16 + qr) * 2] = m0; s_ml[((size_t)warp * 16 + qr) * 2 + 1] = l0;
+        s_ml[((size_t)warp * 16 + qr + 8) * 2] = m1; s_ml[((size_t)warp * 16 + qr + 8) * 2 + 1] = l1;
+      }
+      __syncthreads();
+      const int nh = min(kHeadBlock, G - hb), d2n = D >> 1;
+      for (int item = tid; item < nh * d2n; item += 128) {
+        const int hh = item / d2n, d = (item - hh * d2n) * 2;
+        const long long pidx = (long long)slot * G + hb + hh;
+        float mw[4], big = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) { mw[w] = s_ml[((size_t)w * 16 + hh) * 2]; big = fmaxf(big, mw[w]); }
+        float lsum = 0.f, v0 = 0.f, v1 = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const float wgt = mw[w] == -INFINITY ? 0.f : dec_exp2(mw[w] - big);  // a warp that saw no token of the head adds nothing
+          lsum += s_ml[((size_t)w * 16 + hh) * 2 + 1] * wgt;
+          const float2 x = *reinterpret_cast<const float2*>(s_o + ((size_t)w * 16 + hh) * DP + d);
+          v0 += x.x * wgt; v1 += x.y * wgt;
+        }
+        *reinterpret_cast<float2*>(a.pacc + pidx * D + d) = make_float2(v0, v1);
+        if (d == 0) { a.pm[pidx] = big; a.pl[pidx] = lsum; }
+      }
+    }
+
+    // ticket: the CTA that finishes a pair last merges its partials (slots c0 + rowg .. c1 + rowg, in this order)
+    const int c0 = share.owner(start), np = share.owner(start + pair_stages - 1) - c0 + 1;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = np == 1 || atomicAdd(&a.counters[rowg], 1) == np - 1;
+    __syncthreads();
+    at = start + j0 + ntiles;
+    start += pair_stages;
+    if (!s_last) continue;
+    __threadfence();
+    const long long first = (long long)(c0 + rowg) * G;  // [np][G] maxima and denominators, [np][G][D] sums
+    float* s_w = reinterpret_cast<float*>(s_pipe);          // [G][np] weights, where they fit
+    const bool kept = (size_t)np * G * 4 <= (size_t)NS * STAGE_BYTES;
+    for (int hl = warp; hl < G; hl += 4) {
+      float big = -INFINITY, lsum = 0.f;
+      for (int j = lane; j < np; j += 32) big = fmaxf(big, __ldcg(a.pm + first + (long long)j * G + hl));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xFFFFFFFFu, big, o));
+      for (int j = lane; j < np; j += 32) {
+        const float m = __ldcg(a.pm + first + (long long)j * G + hl);
+        const float w = m == -INFINITY ? 0.f : dec_exp2(m - big);
+        lsum = fmaf(__ldcg(a.pl + first + (long long)j * G + hl), w, lsum);
+        if (kept) s_w[hl * np + j] = w;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xFFFFFFFFu, lsum, o);
+      if (lane == 0) {
+        s_big[hl] = big;
+        s_inv[hl] = 1.f / lsum;
+        a.lse[(long long)row * a.Hq + g * G + hl] = (big + log2f(lsum)) * 0.6931471805599453f;
+      }
+    }
+    __syncthreads();
+    const int d4n = D >> 2;
+#pragma unroll 1
+    for (int item = tid; item < G * d4n; item += 128) {
+      const int hl = item / d4n, d = (item - hl * d4n) * 4;
+      const float* src = a.pacc + (first + hl) * D + d;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (kept) {
+#pragma unroll 8
+        for (int j = 0; j < np; ++j) merge_add(v, __ldcg(reinterpret_cast<const float4*>(src + (long long)j * G * D)), s_w[hl * np + j]);
+      } else {
+        const float big = s_big[hl];
+        for (int j = 0; j < np; ++j) {
+          const float m = __ldcg(a.pm + first + (long long)j * G + hl);
+          merge_add(v, __ldcg(reinterpret_cast<const float4*>(src + (long long)j * G * D)), m == -INFINITY ? 0.f : dec_exp2(m - big));
+        }
+      }
+      const float inv = s_inv[hl];
+      uint2 pk;
+      pk.x = pack16<F16>(v.x * inv, v.y * inv);
+      pk.y = pack16<F16>(v.z * inv, v.w * inv);
+      *reinterpret_cast<uint2*>(a.out + ((long long)row * a.Hq + g * G + hl) * D + d) = pk;
+    }
+    if (tid == 0 && np > 1) a.counters[rowg] = 0;  // ready for the next launch (graph replay included)
+    __syncthreads();  // s_w, s_last
+  }
+}
+
 }  // namespace moba
 
 using namespace moba;
@@ -1179,10 +1510,23 @@ static int attend_parts(const moba_cache_desc* c) {
   return (c->chunk_size + part_tokens - 1) / part_tokens;
 }
 
+// A share below four stages would be mostly its start and its partials (2, 4, 8 and 16 within 1 % at the sizes above).
+constexpr int kStreamLeast = 4;
+constexpr int kStreamCtas = 3 * 148;  // streamed variant: what a B200 holds at once (one per SM above head dimension 128)
+
+// Partials of a launch: a slot per (head, list entry, part), or, streamed, per head of a group and segment.
+static size_t attend_partials(const moba_cache_desc* c, int rows, int hq, int slots) {
+  const size_t fixed = (size_t)rows * hq * slots * attend_parts(c);
+  const size_t streamed = ((size_t)kStreamCtas + (size_t)rows * c->hkv) * (hq / c->hkv);
+  return fixed > streamed ? fixed : streamed;
+}
+static size_t attend_workspace(const moba_cache_desc* c, int rows, int hq, size_t partials) {
+  return align256((size_t)rows * c->hkv * 4) + 2 * align256(partials * 4) + align256(partials * c->dim * 4);
+}
+
 extern "C" size_t moba_decode_attend_workspace_bytes(const moba_cache_desc* c, int rows, int hq, int slots) {
   if (validate_cache(c) != MOBA_OK || rows < 1 || hq < 1 || slots < 1) return 0;
-  const size_t n = (size_t)rows * hq * slots * attend_parts(c);
-  return align256((size_t)rows * c->hkv * 4) + 2 * align256(n * 4) + align256(n * c->dim * 4);
+  return attend_workspace(c, rows, hq, attend_partials(c, rows, hq, slots));
 }
 
 extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const int32_t* ids, const int32_t* positions,
@@ -1205,7 +1549,7 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   a.Hq = hq; a.ns = slots; a.umax = selected ? umax : slots;
   a.parts = attend_parts(c);
   a.part_tokens = attend_part_tokens(c);
-  const size_t n = (size_t)rows * hq * slots * a.parts;
+  const size_t n = attend_partials(c, rows, hq, slots);
   char* p = static_cast<char*>(workspace);
   a.counters = reinterpret_cast<int*>(p); p += align256((size_t)rows * c->hkv * 4);
   a.pm = reinterpret_cast<float*>(p); p += align256(n * 4);
@@ -1218,36 +1562,37 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   const int dp = c->dim <= 32 ? 32 : c->dim <= 64 ? 64 : c->dim <= 128 ? 128 : 256;
   const dim3 grid(a.umax, a.parts, rows * c->hkv);
   const bool deep = (long long)grid.x * grid.y * grid.z <= decode_sm_count();
-  const int teams = deep && dp <= 128 ? 2 : 1;
-  const int stages = deep ? deep_stages(dp) : kStages;  // per team
-  const size_t red_bytes = (size_t)4 * teams * 16 * (dp + 2) * 4;
-  const size_t pipe_bytes = (size_t)teams * stages * 2 * kStageTokens * dp * 2;
-  const size_t smem = red_bytes > pipe_bytes ? red_bytes : pipe_bytes;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaSuccess;
   const bool half = (c->flags & MOBA_CACHE_FP16) != 0;
+  a.rowgs = rows * c->hkv;
+  a.spc = selected ? (c->chunk_size + kStageTokens - 1) / kStageTokens : 1;
+  a.min_stages = kStreamLeast;
   prof_begin(kProfDecodeAttend, st);
-#define MOBA_LAUNCH_ATTEND_F(L, NS, T, F)                                                                               \
-  do {                                                                                                                  \
-    e = cudaFuncSetAttribute(decode_attend_kernel<L, NS, T, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (e == cudaSuccess) e = launch_dependent(8u, decode_attend_kernel<L, NS, T, F>, grid, dim3(128 * T), smem, st, a); \
+#define MOBA_LAUNCH_ATTEND(KERNEL, GRID, THREADS, SMEM)                                                       \
+  do {                                                                                                        \
+    e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM));               \
+    if (e == cudaSuccess) e = launch_dependent(8u, KERNEL, GRID, dim3(THREADS), (size_t)(SMEM), st, a);       \
   } while (0)
-#define MOBA_LAUNCH_ATTEND_NS(L, NS, T)             \
-  do {                                              \
-    if (half) MOBA_LAUNCH_ATTEND_F(L, NS, T, true); \
-    else MOBA_LAUNCH_ATTEND_F(L, NS, T, false);     \
+#define MOBA_LAUNCH_ATTEND_DP(L)                                                                              \
+  do {                                                                                                        \
+    if (deep) {                                                                                               \
+      constexpr int T = L <= 128 ? 2 : 1, NS = deep_stages(L);                                                \
+      constexpr size_t pipe = (size_t)T * NS * 2 * kStageTokens * L * 2, red = (size_t)4 * T * 16 * (L + 2) * 4; \
+      const auto kernel = half ? decode_attend_kernel<L, NS, T, true> : decode_attend_kernel<L, NS, T, false>; \
+      MOBA_LAUNCH_ATTEND(kernel, grid, 128 * T, pipe > red ? pipe : red);                                     \
+    } else {                                                                                                  \
+      constexpr int NS = stream_stages(L);                                                                    \
+      constexpr size_t pipe = (size_t)NS * 2 * kStageTokens * L * 2, red = (size_t)4 * 16 * (L + 2) * 4;      \
+      const auto kernel = half ? decode_attend_stream_kernel<L, NS, true> : decode_attend_stream_kernel<L, NS, false>; \
+      MOBA_LAUNCH_ATTEND(kernel, dim3(L <= 128 ? kStreamCtas : kStreamCtas / 3), 128, pipe > red ? pipe : red); \
+    }                                                                                                         \
   } while (0)
-#define MOBA_LAUNCH_ATTEND(L)                                                                                      \
-  do {                                                                                                             \
-    if (deep) MOBA_LAUNCH_ATTEND_NS(L, deep_stages(L), (L <= 128 ? 2 : 1));                                        \
-    else MOBA_LAUNCH_ATTEND_NS(L, kStages, 1);                                                                     \
-  } while (0)
-  if (dp == 32) MOBA_LAUNCH_ATTEND(32);
-  else if (dp == 64) MOBA_LAUNCH_ATTEND(64);
-  else if (dp == 128) MOBA_LAUNCH_ATTEND(128);
-  else MOBA_LAUNCH_ATTEND(256);
-#undef MOBA_LAUNCH_ATTEND_NS
-#undef MOBA_LAUNCH_ATTEND_F
+  if (dp == 32) MOBA_LAUNCH_ATTEND_DP(32);
+  else if (dp == 64) MOBA_LAUNCH_ATTEND_DP(64);
+  else if (dp == 128) MOBA_LAUNCH_ATTEND_DP(128);
+  else MOBA_LAUNCH_ATTEND_DP(256);
+#undef MOBA_LAUNCH_ATTEND_DP
 #undef MOBA_LAUNCH_ATTEND
   prof_end(kProfDecodeAttend, st);
   if (e != cudaSuccess) return MOBA_ERR_CUDA;

@@ -418,3 +418,29 @@ def test_one_finite_check_for_all_inputs(dtype, layout):
                     cache._finite.require(named)
                 t[at] = keep
     cache._finite.require(named)
+
+
+@pytest.mark.parametrize("mode", ["moba", "dense"])
+@pytest.mark.parametrize("hq,hkv,dim,chunk,page,dtype", [
+    (4, 2, 64, 100, 7, torch.bfloat16),      # the last stage of a chunk is part of one
+    (6, 1, 32, 64, 16, torch.float16),       # a stage is a chunk
+    (40, 2, 96, 130, 48, torch.bfloat16),    # two head blocks per pair, padded head dimension
+    (5, 5, 128, 192, 16, torch.float16),
+    (2, 1, 256, 70, 3, torch.bfloat16),      # one CTA per SM
+])
+def test_streamed_attend_divides_uneven_work(mode, hq, hkv, dim, chunk, page, dtype):
+    """Grids above one CTA per SM take shares of one list of stages: contexts from one token to many chunks, shares that
+    begin and end inside a chunk, several requests in a share and several shares in a request, repeatable bits."""
+    from moba_opt import PagedKVCache
+    lens = [1, 63, 64, 65, 900, 2, chunk, chunk + 1, 700, 1, 333, 1024, 5, 640, 129, 77, 2 * chunk, 511]
+    cache = PagedKVCache(len(lens), 1024, hkv, dim, page_size=page, chunk_size=chunk, dtype=dtype)
+    cu = np.concatenate(([0], np.cumsum(lens))).tolist()
+    k, v = rand((cu[-1], hkv, dim), 71, dtype), rand((cu[-1], hkv, dim), 72, dtype)
+    cache.append_prefill(k, v, sequence_ids=list(range(len(lens))), cu_seqlens=cu)
+    ids = list(range(len(lens))) + [4, 11, 11, 8]                      # several queries of a request, some not at its end
+    positions = [n - 1 for n in lens] + [450, 1000, 63, 0]
+    q = rand((len(ids), hq, dim), 73, dtype)
+    result = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
+    check(cache, result, q)
+    again = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
+    assert torch.equal(result.output, again.output) and torch.equal(result.lse, again.lse)
