@@ -90,6 +90,7 @@ struct FwdItem {
   int kblock0;          // packed key block holding the chunk's first keys
   int key_begin, key_end;
   int g, h;             // kv head; SELF: query head
+  int live;             // 0 behind the CTA's last item (the other fields then hold nothing)
 };
 
 template <bool SELF>
@@ -159,7 +160,8 @@ __device__ __forceinline__ long long fwd_item_index(int k) {
   return (long long)k * G + ((k & 1) ? (G - 1 - blockIdx.x) : blockIdx.x);
 }
 
-constexpr int kFwdThreads = 384;  // warps 10 and 11 only complete the third warpgroup (register hand-over works per warpgroup)
+constexpr int kFwdThreads = 384;  // warp 11 only completes the third warpgroup (register hand-over works per warpgroup)
+constexpr int kFwdItems = 4;      // decoded work items ahead of their users
 
 template <int DPAD>
 struct FwdCfg {
@@ -182,6 +184,8 @@ struct FwdSmem {
   uint64_t q_full[2][2], q_free[2][2];  // [lane][buffer]
   uint64_t s_full[2], s_free[2], p_ready[2], o_full[2], o_free[2];
   uint64_t kv_full[4], kv_free[4];
+  uint64_t item_full[kFwdItems], item_free[kFwdItems];
+  FwdItem item[kFwdItems];
   uint32_t tmem_slot;
 };
 static_assert(sizeof(FwdSmem) <= 1024, "control block must fit its reservation");
@@ -214,6 +218,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(FwdArgs a) {
       mbar_init(&cb.o_free[l], 4);
     }
     for (int s = 0; s < 4; ++s) { mbar_init(&cb.kv_full[s], 1); mbar_init(&cb.kv_free[s], 1); }
+    for (int s = 0; s < kFwdItems; ++s) { mbar_init(&cb.item_full[s], 1); mbar_init(&cb.item_free[s], 10); }  // 8 softmax warps, MMA, producer
     mbar_fence_init();
   }
   if (warp == 0) tmem_alloc(&cb.tmem_slot, Cfg::TMEM_COLS);
@@ -223,16 +228,46 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(FwdArgs a) {
   const uint32_t tmem = cb.tmem_slot;
   bool alive = true;
 
+  // Item k of the CTA as warp 10 left it; false behind the last one.  All lanes of a warp (the producer: its one thread)
+  // read what they need through `use` before the slot is handed back.  A wait that ran out ends the role's walk: what
+  // the slot holds then is not known to be an item.
+  auto with_item = [&](int k, auto use, bool whole_warp) {
+    const int s = k % kFwdItems;
+    if (alive) alive = mbar_wait(&cb.item_full[s], (k / kFwdItems) & 1, a.status);
+    if (whole_warp) alive = __all_sync(0xFFFFFFFFu, alive);  // the lanes leave together
+    if (!alive || !cb.item[s].live) return false;
+    use(cb.item[s]);
+    return true;
+  };
+
   // The softmax warpgroups keep a whole row of S in registers; the third warpgroup gives them its share.
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-  if (warp == 9) {
+  if (warp == 10) {
+    // ================================================================== item decoder (one thread)
+    // Finding an item's expert is two binary searches, some twenty dependent loads.  Done by every role for itself at the
+    // start of an item, they stood between the items of both lanes at once; here they run items ahead.  Remote
+    // pass: 883 -> 696 us at four key tiles an item (32768 tokens, chunk 512, D = 128), 1995 -> 1748 us at sixteen
+    // (65536 tokens, chunk 2048, D = 64).
+    if (lane_id == 0) {
+      FwdItem it;
+      for (int k = 0;; ++k) {
+        const int s = k % kFwdItems;
+        it.live = fwd_decode_item<SELF>(a, fwd_item_index(k), it) ? 1 : 0;
+        if (k >= kFwdItems && !mbar_wait(&cb.item_free[s], ((k / kFwdItems) - 1) & 1, a.status)) break;
+        cb.item[s] = it;
+        mbar_arrive(&cb.item_full[s]);
+        if (!it.live) break;
+      }
+    }
+  } else if (warp == 9) {
     // ================================================================== producer (one thread)
     if (lane_id == 0) {
       int use[2] = {0, 0};  // items each lane took part in so far
       int kvt = 0;          // K/V tiles fetched so far
       FwdItem it;
-      for (int k = 0; fwd_decode_item<SELF>(a, fwd_item_index(k), it); ++k) {
+      for (int k = 0; with_item(k, [&](const FwdItem& x) { it = x; }, false); ++k) {
+        mbar_arrive(&cb.item_free[k % kFwdItems]);
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
           if (it.n[l] == 0) continue;
@@ -301,10 +336,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(FwdArgs a) {
       ++ts[l];
     };
 
-    FwdItem cur, nxt;
-    bool has = fwd_decode_item<SELF>(a, fwd_item_index(0), cur);
+    struct { int n[2]; } cur, nxt;  // all the schedule needs of an item
+    auto fetch = [&](int k, auto& to) {
+      const bool got = with_item(k, [&](const FwdItem& x) { to.n[0] = x.n[0]; to.n[1] = x.n[1]; }, true);
+      __syncwarp();
+      if (got && leader) mbar_arrive(&cb.item_free[k % kFwdItems]);
+      return got;
+    };
+    bool has = fetch(0, cur);
     for (int k = 0; has; ++k) {
-      const bool has_next = fwd_decode_item<SELF>(a, fwd_item_index(k + 1), nxt);
+      const bool has_next = fetch(k + 1, nxt);
       const int n = max(cur.n[0], cur.n[1]);
       bool pre_next[2] = {false, false};
 #pragma unroll
@@ -373,24 +414,20 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(FwdArgs a) {
     const uint32_t tO = tmem + lane_off + Cfg::COL_O + l * DPAD;
     const uint32_t tP = tmem + lane_off + Cfg::COL_P + l * Cfg::P_STRIDE;
     int tc = 0;  // tiles this lane has processed
-    FwdItem it;
-    for (int k = 0; fwd_decode_item<SELF>(a, fwd_item_index(k), it); ++k) {
-      const int n = it.n[l];
+    int n, rows, first, key_begin, chunk_end, head;
+    for (int k = 0; with_item(k, [&](const FwdItem& x) {
+           n = x.n[l]; rows = x.rows[l]; first = x.first[l]; key_begin = x.key_begin; chunk_end = x.key_end; head = x.h;
+         }, true); ++k) {
+      __syncwarp();
+      if (lane_id == 0) mbar_arrive(&cb.item_free[k % kFwdItems]);
       if (n == 0) continue;
-      int row_id = -1;  // SELF: t*Hq+h of this thread's row; REMOTE: slot id
-      const int tok = it.first[l] + row;
-      if (row < it.rows[l]) {
-        if (SELF) {
-          row_id = tok * pv.Hq + it.h;
-        } else {
-          row_id = a.rowlist[it.first[l] + row];
-          if (row_id < 0 || row_id / pv.R >= pv.T * pv.Hq) { atomicOr(a.status, kErrBadIndex); row_id = -1; }
-        }
-      }
-      const int key_end = SELF ? it.first[l] + it.rows[l] : it.key_end;  // causal: nothing past the tile's last token
+      int row_id = -1;  // SELF: t*Hq+h of this thread's row; REMOTE: slot id, looked at in the epilogue
+      const int tok = first + row;
+      if (row < rows) row_id = SELF ? tok * pv.Hq + head : a.rowlist[first + row];
+      const int key_end = SELF ? first + rows : chunk_end;  // causal: nothing past the tile's last token
       float m_used = 0.f, l_run = 0.f;
       for (int j = 0; j < n; ++j, ++tc) {
-        const int k0 = it.key_begin + j * kTile;
+        const int k0 = key_begin + j * kTile;
         int klimit = key_end - k0;                     // keys of the tile that exist
         if (SELF) klimit = min(klimit, tok - k0 + 1);  // causal inside the own chunk
         const bool need_mask = __any_sync(0xFFFFFFFFu, klimit < kTile);
@@ -505,8 +542,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(FwdArgs a) {
       tc_fence_before_sync();
       __syncwarp();
       if (lane_id == 0) mbar_arrive(&cb.o_free[l]);
-      if (row_id < 0 || !alive) continue;
+      if (row >= rows || !alive) continue;
       if (!SELF) {
+        if (row_id < 0 || row_id / pv.R >= pv.T * pv.Hq) { atomicOr(a.status, kErrBadIndex); continue; }
         const float inv = 1.f / l_run;
         __nv_bfloat16* dst = a.part_o + (long long)row_id * D;
 #pragma unroll
