@@ -6,6 +6,7 @@ cu_seqlens (cached per batch shape), buffer allocation through torch, and three 
 (route, forward, backward) on the current stream.  Routing, expert packing, attention, the LSE merge
 and the gradients all run in the sm_100a kernels of libmoba_b200.so; there is no other code path.
 """
+import contextlib
 import ctypes
 from collections import OrderedDict
 
@@ -80,6 +81,20 @@ class PrefillPlan:
         self.filtered = np.asarray(filtered, dtype=np.int64)
         self.chunk_to_batch = np.asarray(chunk_seq, dtype=np.int64)
         self.cu_chunk = np.asarray(chunk_start, dtype=np.int64)
+        self._calls = {}
+
+    def call(self, q, k, v, remote_k, flags=0):
+        """Descriptor and buffer sizes for inputs of these shapes and strides.  A descriptor has some forty fields, and
+        filling it through ctypes and asking the library four sizes took a third of the host time of a small call, so the last
+        few are kept: they depend on shapes, strides, the format and the plan's own arrays alone, never on an input's address."""
+        key = (q.shape, k.shape, q.stride(), k.stride(), v.stride(), q.dtype, remote_k, flags)
+        found = self._calls.get(key)
+        if found is None:
+            found = PrefillCall(self.desc(q, k, v, remote_k, flags))
+            for old in list(self._calls)[:-7]:       # eight at most
+                self._calls.pop(old, None)
+            self._calls[key] = found
+        return found
 
     def desc(self, q, k, v, remote_k, flags=0):
         d = _ext.PrefillDesc()
@@ -97,6 +112,19 @@ class PrefillPlan:
                      "qtile_local", "self_pairs", "kv_order"):
             setattr(d, name, getattr(self, name).data_ptr())
         return d
+
+
+class PrefillCall:
+    """A filled descriptor, a reference to it as the entry points take it, and the bytes each of them wants."""
+    __slots__ = ("desc", "ref", "state_bytes", "route_bytes", "fwd_bytes", "bwd_bytes")
+
+    def __init__(self, desc):
+        lib = _ext.lib()
+        self.desc, self.ref = desc, ctypes.byref(desc)
+        self.state_bytes = lib.moba_prefill_route_state_bytes(self.ref)
+        self.route_bytes = lib.moba_prefill_route_scratch_bytes(self.ref)
+        self.fwd_bytes = lib.moba_prefill_fwd_scratch_bytes(self.ref)
+        self.bwd_bytes = lib.moba_prefill_bwd_scratch_bytes(self.ref)
 
 
 def get_plan(cu, chunk_size, device):
@@ -141,21 +169,39 @@ def _aligned(t):
     return t
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    if _raw_stream is None or device.index is None:
+        return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(_raw_stream(device.index))
+
+
+def _current(device):
+    """Makes `device` the current one for a `with` block; nothing to do, and nothing to pay for, when it is already."""
+    return _SAME_DEVICE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _bytes(n, device):
+    return torch.empty(n, dtype=torch.uint8, device=device)
 
 
 def route(q, k, plan, remote_k, flags=0):
     """Runs the routing kernels; returns the opaque route-state tensor (uint8)."""
-    lib = _ext.lib()
-    d = plan.desc(q, k, k, remote_k, flags)
-    state = torch.empty(lib.moba_prefill_route_state_bytes(ctypes.byref(d)), dtype=torch.uint8, device=q.device)
-    nbytes = lib.moba_prefill_route_scratch_bytes(ctypes.byref(d))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
-    with _ext.nvtx("moba.route"):
-        _ext.check(lib.moba_prefill_route(ctypes.byref(d), q.data_ptr(), k.data_ptr(), state.data_ptr(),
-                                          scratch.data_ptr(), nbytes, _stream(q.device)), "moba_prefill_route")
+    call = plan.call(q, k, k, remote_k, flags)
+    state = _bytes(call.state_bytes, q.device)
+    _route(call, q, k, state, _bytes(call.route_bytes, q.device), call.route_bytes, _stream(q.device))
     return state
+
+
+def _route(call, q, k, state, scratch, nbytes, stream):
+    with _ext.nvtx("moba.route"):
+        _ext.check(_ext.lib().moba_prefill_route(call.ref, q.data_ptr(), k.data_ptr(), state.data_ptr(), scratch.data_ptr(), nbytes,
+                                                 stream), "moba_prefill_route")
 
 
 def selected_table(state, total, hq, remote_k):
@@ -169,45 +215,42 @@ class _MobaPrefill(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, plan, remote_k, flags, bwd_flags):
-        lib = _ext.lib()
         q, k, v = _aligned(q), _aligned(k), _aligned(v)
-        with torch.cuda.device(q.device):
-            state = route(q, k, plan, remote_k, flags)
+        device = q.device
+        with _current(device):
+            call = plan.call(q, k, v, remote_k, flags | bwd_flags)
+            stream = _stream(device)
+            state = _bytes(call.state_bytes, device)
+            nbytes = max(call.route_bytes, call.fwd_bytes)
+            scratch = _bytes(nbytes, device)       # routing is done with it when the forward starts
+            _route(call, q, k, state, scratch, nbytes, stream)
             if ROUTE_HOOK is not None and remote_k > 0:
                 _fire_hook(plan, state, q.shape[0], q.shape[1], remote_k)
-            d = plan.desc(q, k, v, remote_k)
-            nbytes = lib.moba_prefill_fwd_scratch_bytes(ctypes.byref(d))
-            scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
-            out = torch.empty((q.shape[0], q.shape[1], q.shape[2]), dtype=q.dtype, device=q.device)
-            lse = torch.empty((q.shape[0], q.shape[1]), dtype=torch.float32, device=q.device)
+            out = torch.empty(q.shape, dtype=q.dtype, device=device)
+            lse = torch.empty(q.shape[:2], dtype=torch.float32, device=device)
             with _ext.nvtx("moba.forward"):
-                _ext.check(lib.moba_prefill_fwd(ctypes.byref(d), q.data_ptr(), k.data_ptr(), v.data_ptr(),
-                                                state.data_ptr(), scratch.data_ptr(), nbytes,
-                                                out.data_ptr(), lse.data_ptr(), _status_word(q.device).data_ptr(),
-                                                _stream(q.device)), "moba_prefill_fwd")
+                _ext.check(_ext.lib().moba_prefill_fwd(call.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), state.data_ptr(),
+                                                       scratch.data_ptr(), nbytes, out.data_ptr(), lse.data_ptr(),
+                                                       _status_word(device).data_ptr(), stream), "moba_prefill_fwd")
         ctx.save_for_backward(q, k, v, out, lse, state)
-        ctx.plan, ctx.remote_k, ctx.bwd_flags = plan, remote_k, bwd_flags
+        ctx.plan, ctx.remote_k, ctx.flags = plan, remote_k, flags | bwd_flags
         ctx.mark_non_differentiable(lse)
         return out, lse
 
     @staticmethod
     def backward(ctx, d_out, _d_lse):
-        lib = _ext.lib()
         q, k, v, out, lse, state = ctx.saved_tensors
-        plan, remote_k = ctx.plan, ctx.remote_k
         d_out = d_out.contiguous()
-        with torch.cuda.device(q.device):
-            d = plan.desc(q, k, v, remote_k, ctx.bwd_flags)
-            nbytes = lib.moba_prefill_bwd_scratch_bytes(ctypes.byref(d))
-            scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
-            dq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-            dk = torch.empty(k.shape, dtype=k.dtype, device=q.device)
-            dv = torch.empty(v.shape, dtype=v.dtype, device=q.device)
+        device = q.device
+        with _current(device):
+            call = ctx.plan.call(q, k, v, ctx.remote_k, ctx.flags)
+            scratch = _bytes(call.bwd_bytes, device)
+            dq, dk, dv = (torch.empty(t.shape, dtype=t.dtype, device=device) for t in (q, k, v))
             with _ext.nvtx("moba.backward"):
-                _ext.check(lib.moba_prefill_bwd(ctypes.byref(d), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                                lse.data_ptr(), d_out.data_ptr(), state.data_ptr(),
-                                                scratch.data_ptr(), nbytes, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                                                _status_word(q.device).data_ptr(), _stream(q.device)), "moba_prefill_bwd")
+                _ext.check(_ext.lib().moba_prefill_bwd(call.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                                                       lse.data_ptr(), d_out.data_ptr(), state.data_ptr(), scratch.data_ptr(),
+                                                       call.bwd_bytes, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                                       _status_word(device).data_ptr(), _stream(device)), "moba_prefill_bwd")
         return dq, dk, dv, None, None, None, None
 
 
