@@ -180,9 +180,8 @@ class FiniteCheck:
     """NaN/Inf check of the q, k, v of a call: one launch over all of them that writes into pinned words, one wait for
     the stream.  The owner serialises calls (the cache's lock)."""
 
-    def __init__(self, lib, device):
-        self._lib, self._device = lib, device
-        self._words = torch.zeros(3, dtype=torch.int32, pin_memory=True)
+    def __init__(self, lib, device, words):
+        self._lib, self._device, self._words = lib, device, words    # at least three pinned int32
         self._flags = self._words.numpy()
 
     def require(self, named):
@@ -211,7 +210,9 @@ class HostStaging:
 
     def __init__(self, device, slots=4, words=4096):
         self.device = device
-        self._pinned = [torch.empty(words, dtype=torch.int32, pin_memory=True) for _ in range(slots)]
+        block = torch.zeros(slots * words + 4, dtype=torch.int32, pin_memory=True)   # one allocation: pinning is slow
+        self._pinned = list(block[:slots * words].split(words))
+        self.spare = block[slots * words:]         # for whoever needs a word both sides can reach (FiniteCheck)
         self._busy = [None] * slots
         self._next = 0
 
@@ -286,7 +287,7 @@ class PagedKVCache:
             self._candidate_count = 0
             self._status = _status_word(self.device)
             self._staging = HostStaging(self.device)
-            self._finite = FiniteCheck(self._lib, self.device)
+            self._finite = FiniteCheck(self._lib, self.device, self._staging.spare)
             self._attend_buffers = {}         # (rows, Hq, slots, umax) -> union lists + split-K workspace, kept between calls
 
     # ------------------------------------------------------------------ views of the CPU layout
