@@ -41,4 +41,24 @@ inline cudaError_t launch_dependent(unsigned kind, void (*kernel)(KArgs...), dim
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// The same for a grid of clusters of `cluster` CTAs along x.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent_cluster(unsigned kind, void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster, size_t smem,
+                                            cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (dependent_launch_mask() & kind) ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 }  // namespace moba

@@ -264,4 +264,26 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 // Waits until the calling thread's bulk groups have read their shared-memory sources / have completed.
 __device__ __forceinline__ void bulk_wait_group_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_group() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// ---- thread-block clusters: a barrier over all threads of the cluster's CTAs (release, acquire) and loads from the shared
+// memory of another CTA of the cluster, addressed by this CTA's own address of the same variable
+__device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_smem(const void* own, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(own)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float peer_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 peer_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 }  // namespace moba

@@ -444,3 +444,26 @@ def test_streamed_attend_divides_uneven_work(mode, hq, hkv, dim, chunk, page, dt
     check(cache, result, q)
     again = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
     assert torch.equal(result.output, again.output) and torch.equal(result.lse, again.lse)
+
+
+@pytest.mark.parametrize("mode", ["moba", "dense"])
+@pytest.mark.parametrize("lens,hq,hkv,dim,chunk,page,dtype", [
+    ((1,), 4, 1, 64, 100, 7, torch.bfloat16),             # fewer stages than CTAs in the cluster
+    ((1000,), 14, 2, 64, 100, 16, torch.bfloat16),        # the last stage of a chunk is part of one
+    ((63, 64, 65), 32, 1, 32, 64, 16, torch.float16),     # two head blocks, a stage is a chunk
+    ((640, 5, 129, 333), 6, 3, 96, 130, 48, torch.bfloat16),   # twelve pairs: clusters of eight
+    ((511, 700), 5, 5, 128, 192, 16, torch.float16),
+    ((900, 71), 2, 1, 256, 70, 3, torch.bfloat16),        # one team per CTA
+])
+def test_cluster_attend_divides_a_request(lens, mode, hq, hkv, dim, chunk, page, dtype):
+    """Small batches: the stages of a (request, kv head) pair over the CTAs of a cluster, repeatable bits."""
+    from moba_opt import PagedKVCache
+    cache = PagedKVCache(len(lens), max(lens) + 8, hkv, dim, page_size=page, chunk_size=chunk, dtype=dtype)
+    cu = np.concatenate(([0], np.cumsum(lens))).tolist()
+    k, v = rand((cu[-1], hkv, dim), 81, dtype), rand((cu[-1], hkv, dim), 82, dtype)
+    cache.append_prefill(k, v, sequence_ids=list(range(len(lens))), cu_seqlens=cu)
+    q = rand((len(lens), hq, dim), 83, dtype)
+    result = cache.attend(q, sequence_ids=list(range(len(lens))), topk=4, mode=mode)
+    check(cache, result, q)
+    again = cache.attend(q, sequence_ids=list(range(len(lens))), topk=4, mode=mode)
+    assert torch.equal(result.output, again.output) and torch.equal(result.lse, again.lse)
