@@ -90,7 +90,11 @@ struct WsSmem {
 };
 static_assert(sizeof(WsSmem) <= 8192, "control block must fit its reservation");
 
-template <bool F16>
+// SPLIT > 1: a key block's query tiles are divided over the CTAs of a cluster (blockIdx.x % SPLIT), each with dK and dV of
+// its own; at the end CTA 0 adds the others' sums, read from their shared memory in rank order, to its own.  A batch
+// with few key blocks otherwise lasts as long as its earliest chunk, which most later rows attend, while most SMs are idle.
+// 6131 tokens in three sequences, 8/2 heads, D = 64, 100 key blocks: 124 -> 71 us.
+template <bool F16, int SPLIT>
 __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
   constexpr int DPAD = 64;
   constexpr int TILE_BYTES = kTile * DPAD * 2;
@@ -111,7 +115,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
   const PrefillView& pv = a.pv;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = pv.D;
-  const int kblock = a.kv_order[blockIdx.x];
+  const int part = SPLIT > 1 ? blockIdx.x % SPLIT : 0;
+  const int kblock = a.kv_order[blockIdx.x / SPLIT];
   const int g = blockIdx.y;
   const int c = pv.qtile_chunk[kblock];
   const int k0 = pv.qtile_tok0[kblock];
@@ -126,7 +131,10 @@ __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
     remote_rows = a.seg_base[c * pv.Hq + (g + 1) * pv.G] - remote_begin;
   }
   const int n_remote = (remote_rows + kTile - 1) / kTile;
-  const int n_iter = pv.G * n_self + n_remote;
+  // this CTA's tiles: it0, it0 + 1, ..., n_iter of them (CTA 0 always has one)
+  const int n_all = pv.G * n_self + n_remote;
+  const int it0 = (n_all * part + SPLIT - 1) / SPLIT;
+  const int n_iter = (n_all * (part + 1) + SPLIT - 1) / SPLIT - it0;
 
   if ((smem_u32(smem) & 1023u) != 0) {
     if (tid == 0) atomicOr(a.status, kErrBadIndex);
@@ -216,7 +224,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
       // One thread asks the copy engine for the packed tiles: 16 KB of Q, 16 KB of dO and three 512-byte
       // metadata rows per tile, all contiguous in global memory, completion counted on the slot's barrier.
       if (lane == 0) {
-        {  // stationary K and V images of the key block
+        if (n_iter > 0) {  // stationary K and V images of the key block
           const size_t kvoff = ((size_t)kblock * pv.Hkv + g) * TILE_BYTES;
           mbar_arrive_expect_tx(&cb.kv_ready, 2 * TILE_BYTES);
           bulk_load(sK, reinterpret_cast<const uint8_t*>(a.kpack) + kvoff, TILE_BYTES, &cb.kv_ready);
@@ -227,15 +235,16 @@ __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
         for (int j = 0; j < n_iter; ++j) {
           const int b = j % kWsRing;
           long long tile;
-          if (j < n_remote) {
+          const int ja = it0 + j;
+          if (ja < n_remote) {
             // The key blocks of a chunk walk the same expert list at the same time, each a couple of tiles
             // apart: a tile fetched by one of them is still in the L2 cache for the others, the dQ rows
             // they all add into stay there too, and no two of them add into the same rows at once.
-            int jr = j + (kb * 2) % n_remote;
+            int jr = ja + (kb * 2) % n_remote;
             if (jr >= n_remote) jr -= n_remote;
             tile = remote_tile0 + jr;
           } else {
-            const int s = j - n_remote;
+            const int s = ja - n_remote;
             const int hl = s / n_self, i = kb + (s - hl * n_self);
             tile = (long long)(kblock - kb + i) * pv.Hq + g * pv.G + hl;  // query tiles of a chunk are consecutive
           }
@@ -351,7 +360,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
       const int ms = it % kWsRing;
       // queries below qmin are masked for this key: all of them for a key that does not exist, the
       // earlier ones on the causal diagonal (tile of the key block itself)
-      const bool diag = it >= n_remote && ((it - n_remote) % n_self) == 0;
+      const bool diag = it0 + it >= n_remote && ((it0 + it - n_remote) % n_self) == 0;
       const int qmin = r >= nkeys ? kTile : (diag ? r : 0);
       const bool unmasked = __all_sync(0xFFFFFFFFu, qmin <= half * 64);
       alive = warp_wait(&cb.qdo_full[ms], (it / kWsRing) & 1, a.status, alive);  // the tile's metadata is in the slot
@@ -424,14 +433,46 @@ __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
     if (n_iter > 0) {
       alive = warp_wait(&cb.dq_done, (n_iter - 1) & 1, a.status, alive);
       tc_fence_after_sync();
-      // dK (warps 0-3) and dV (warps 4-7) of the key block: thread = key row
+    }
+    // dK (warps 0-3) and dV (warps 4-7) of the key block: thread = key row
+    const uint32_t tacc = tlane + (half == 0 ? COL_DK : COL_DV);
+    if (SPLIT > 1 && part > 0) {
+      // The ring is dead: every product that read it has completed.  16-byte units of a row lie 128 rows apart, so that
+      // the lanes of a warp touch consecutive units, here and when CTA 0 reads them.
+      float4* mine = reinterpret_cast<float4*>(sQ) + half * 16 * kTile + r;
+#pragma unroll
+      for (int pc = 0; pc < 2; ++pc) {
+        uint32_t v[32];
+        tmem_ld32(tacc + pc * 32, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          mine[(pc * 8 + u) * kTile] = n_iter > 0 ? make_float4(__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1]), __uint_as_float(v[4 * u + 2]),
+                                                                __uint_as_float(v[4 * u + 3]))
+                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      cluster_barrier();
+    } else {
+      if (SPLIT > 1) cluster_barrier();
       const bool ok = r < nkeys && alive;
       __nv_bfloat16* dst = (half == 0 ? a.dk : a.dv) + ((long long)(k0 + r) * pv.Hkv + g) * D;
 #pragma unroll
       for (int pc = 0; pc < 2; ++pc) {
         uint32_t v[32];
-        tmem_ld32(tlane + (half == 0 ? COL_DK : COL_DV) + pc * 32, v);
+        tmem_ld32(tacc + pc * 32, v);
         tmem_ld_wait();
+#pragma unroll
+        for (int other = 1; other < SPLIT; ++other) {
+          const uint32_t from = peer_smem(sQ, other) + (uint32_t)((half * 16 + pc * 8) * kTile + r) * 16u;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const float4 x = peer_f32x4(from + u * kTile * 16);
+            v[4 * u] = __float_as_uint(__uint_as_float(v[4 * u]) + x.x);
+            v[4 * u + 1] = __float_as_uint(__uint_as_float(v[4 * u + 1]) + x.y);
+            v[4 * u + 2] = __float_as_uint(__uint_as_float(v[4 * u + 2]) + x.z);
+            v[4 * u + 3] = __float_as_uint(__uint_as_float(v[4 * u + 3]) + x.w);
+          }
+        }
         if (ok) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8)
@@ -445,18 +486,32 @@ __global__ void __launch_bounds__(kWsThreads, 1) attn_bwd_ws_kernel(BwdArgs a) {
       }
     }
   }
+  if (SPLIT > 1) {
+    if (warp >= 8) cluster_barrier();  // the compute warps passed it above
+    cluster_barrier();                 // no CTA leaves while CTA 0 may still read its sums
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, TMEM_COLS);
 }
 
-cudaError_t launch_bwd_ws(const BwdArgs& a, cudaStream_t st) {
+template <int SPLIT>
+static cudaError_t launch_bwd_ws_as(const BwdArgs& a, cudaStream_t st) {
   const size_t smem = 8192 + (size_t)kTile * 64 * 2 * (1 + 2 * kWsRing) + (size_t)kTile * kStageRow + (size_t)kTile * kTile * 2;
-  const auto kernel = a.pv.fp16 ? attn_bwd_ws_kernel<true> : attn_bwd_ws_kernel<false>;
+  const auto kernel = a.pv.fp16 ? attn_bwd_ws_kernel<true, SPLIT> : attn_bwd_ws_kernel<false, SPLIT>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kernel<<<dim3(a.pv.n_qtiles, a.pv.Hkv), kWsThreads, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_clusters(kernel, dim3(a.pv.n_qtiles * SPLIT, a.pv.Hkv), dim3(kWsThreads), SPLIT, smem, st, a);
+}
+
+cudaError_t launch_bwd_ws(const BwdArgs& a, cudaStream_t st) {
+  // A key block per SM or fewer leaves SMs without work, and up to two per SM the earliest chunks, attended by several times
+  // the rows of an average one, still set the time; beyond that the blocks, heaviest first, even out by themselves.  Whole
+  // training pass, 8681 tokens, 6/1 heads, D = 64, 68 blocks: 380 -> 240 us; 1647 tokens, D = 128, 26 blocks: host-bound either way.
+  const long long blocks = (long long)a.pv.n_qtiles * a.pv.Hkv;
+  if (blocks <= kSplit4Blocks) return launch_bwd_ws_as<4>(a, st);
+  if (blocks <= kSplit2Blocks) return launch_bwd_ws_as<2>(a, st);
+  return launch_bwd_ws_as<1>(a, st);
 }
 
 }  // namespace moba

@@ -34,7 +34,8 @@ static_assert(sizeof(Smem128) <= 4096, "control block must fit its reservation")
 
 }  // namespace
 
-template <bool F16>
+// SPLIT > 1: the query tiles of a key block over the CTAs of a cluster, as in prefill_attn_bwd_ws.cu.
+template <bool F16, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) {
   constexpr int DPAD = 128;
   constexpr int KV_BYTES = kTile * DPAD * 2;      // 32 KB: two 64-column panels of 128 rows
@@ -55,7 +56,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
   const PrefillView& pv = a.pv;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = pv.D;
-  const int kblock = a.kv_order[blockIdx.x];
+  const int part = SPLIT > 1 ? blockIdx.x % SPLIT : 0;
+  const int kblock = a.kv_order[blockIdx.x / SPLIT];
   const int g = blockIdx.y;
   const int c = pv.qtile_chunk[kblock];
   const int k0 = pv.qtile_tok0[kblock];
@@ -67,8 +69,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
   int remote_rows = 0;
   if (pv.R > 0) remote_rows = a.seg_base[c * pv.Hq + (g + 1) * pv.G] - a.seg_base[c * pv.Hq + g * pv.G];
   const int n_remote = (remote_rows + kTile - 1) / kTile;
-  const int n_tiles = pv.G * n_self + n_remote;
-  const int n_iter = 2 * n_tiles;  // two 64-row steps per query tile
+  // this CTA's query tiles start at jt0 (CTA 0 always has one), two 64-row steps each
+  const int n_all = pv.G * n_self + n_remote;
+  const int jt0 = (n_all * part + SPLIT - 1) / SPLIT;
+  const int n_iter = 2 * ((n_all * (part + 1) + SPLIT - 1) / SPLIT - jt0);
 
   if ((smem_u32(smem) & 1023u) != 0) {
     if (tid == 0) atomicOr(a.status, kErrBadIndex);
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
     if (warp == 9) {
       // ================================================================== producer
       if (lane == 0) {
-        {  // stationary K and V images of the key block
+        if (n_iter > 0) {  // stationary K and V images of the key block
           const size_t kvoff = ((size_t)kblock * pv.Hkv + g) * KV_BYTES;
           mbar_arrive_expect_tx(&cb.kv_ready, 2 * KV_BYTES);
           bulk_load(sK, reinterpret_cast<const uint8_t*>(a.kpack) + kvoff, KV_BYTES, &cb.kv_ready);
@@ -181,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
         const long long self_tiles = (long long)pv.n_qtiles * pv.Hq;
         const long long remote_tile0 = pv.R > 0 ? self_tiles + a.tile_base[c * pv.Hkv + g] : 0;
         for (int j = 0; j < n_iter; ++j) {
-          const int b = j % kRing, jt = j >> 1, sub = j & 1;
+          const int b = j % kRing, jt = jt0 + (j >> 1), sub = j & 1;
           long long tile;
           if (jt < n_remote) {
             // the key blocks of a chunk walk the same expert list at the same time, a couple of tiles apart
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
       warp_arrive(&cb.ka_ready);
     }
     for (int it = 0; it < n_iter; ++it) {
-      const int ms = it % kRing, jt = it >> 1, sub = it & 1;
+      const int ms = it % kRing, jt = jt0 + (it >> 1), sub = it & 1;
       // queries below qmin (index inside the 128-row tile) are masked for this key
       const bool diag = jt >= n_remote && ((jt - n_remote) % n_self) == 0;
       const int qmin = r >= nkeys ? kTile : (diag ? r : 0);
@@ -382,14 +386,46 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
     if (n_iter > 0) {
       alive = warp_wait(&cb.dq_done, (n_iter - 1) & 1, a.status, alive);
       tc_fence_after_sync();
-      // dK (warps 0-3) and dV (warps 4-7) of the key block: thread = key row
+    }
+    // dK (warps 0-3) and dV (warps 4-7) of the key block: thread = key row
+    const uint32_t tacc = tlane + (half == 0 ? COL_DK : COL_DV);
+    if (SPLIT > 1 && part > 0) {
+      // The K and V images and the ring are dead: every product that read them has completed.  16-byte units of a row lie
+      // 128 rows apart, so that the lanes of a warp touch consecutive units, here and when CTA 0 reads them.
+      float4* mine = reinterpret_cast<float4*>(sK) + half * 32 * kTile + r;
+#pragma unroll
+      for (int pc = 0; pc < 4; ++pc) {
+        uint32_t v[32];
+        tmem_ld32(tacc + pc * 32, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          mine[(pc * 8 + u) * kTile] = n_iter > 0 ? make_float4(__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1]), __uint_as_float(v[4 * u + 2]),
+                                                                __uint_as_float(v[4 * u + 3]))
+                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      cluster_barrier();
+    } else {
+      if (SPLIT > 1) cluster_barrier();
       const bool ok = r < nkeys && alive;
       __nv_bfloat16* dst = (half == 0 ? a.dk : a.dv) + ((long long)(k0 + r) * pv.Hkv + g) * D;
 #pragma unroll
       for (int pc = 0; pc < 4; ++pc) {
         uint32_t v[32];
-        tmem_ld32(tlane + (half == 0 ? COL_DK : COL_DV) + pc * 32, v);
+        tmem_ld32(tacc + pc * 32, v);
         tmem_ld_wait();
+#pragma unroll
+        for (int other = 1; other < SPLIT; ++other) {
+          const uint32_t from = peer_smem(sK, other) + (uint32_t)((half * 32 + pc * 8) * kTile + r) * 16u;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const float4 x = peer_f32x4(from + u * kTile * 16);
+            v[4 * u] = __float_as_uint(__uint_as_float(v[4 * u]) + x.x);
+            v[4 * u + 1] = __float_as_uint(__uint_as_float(v[4 * u + 1]) + x.y);
+            v[4 * u + 2] = __float_as_uint(__uint_as_float(v[4 * u + 2]) + x.z);
+            v[4 * u + 3] = __float_as_uint(__uint_as_float(v[4 * u + 3]) + x.w);
+          }
+        }
         if (ok) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8)
@@ -403,18 +439,29 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
       }
     }
   }
+  if (SPLIT > 1) {
+    if (warp >= 8) cluster_barrier();  // the compute warps passed it above
+    cluster_barrier();                 // no CTA leaves while CTA 0 may still read its sums
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, TMEM_COLS);
 }
 
-cudaError_t launch_bwd_ws128(const BwdArgs& a, cudaStream_t st) {
+template <int SPLIT>
+static cudaError_t launch_bwd_ws128_as(const BwdArgs& a, cudaStream_t st) {
   const size_t smem = 4096 + 2 * (size_t)kTile * 128 * 2 + (size_t)kRing * 2 * kQRows * 128 * 2 + (size_t)kTile * kQRows * 2 + (size_t)kQRows * 128 * 4;
-  const auto kernel = a.pv.fp16 ? attn_bwd_ws128_kernel<true> : attn_bwd_ws128_kernel<false>;
+  const auto kernel = a.pv.fp16 ? attn_bwd_ws128_kernel<true, SPLIT> : attn_bwd_ws128_kernel<false, SPLIT>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kernel<<<dim3(a.pv.n_qtiles, a.pv.Hkv), kThreads, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_clusters(kernel, dim3(a.pv.n_qtiles * SPLIT, a.pv.Hkv), dim3(kThreads), SPLIT, smem, st, a);
+}
+
+cudaError_t launch_bwd_ws128(const BwdArgs& a, cudaStream_t st) {
+  const long long blocks = (long long)a.pv.n_qtiles * a.pv.Hkv;
+  if (blocks <= kSplit4Blocks) return launch_bwd_ws128_as<4>(a, st);
+  if (blocks <= kSplit2Blocks) return launch_bwd_ws128_as<2>(a, st);
+  return launch_bwd_ws128_as<1>(a, st);
 }
 
 }  // namespace moba

@@ -61,6 +61,24 @@ __device__ __forceinline__ bool bwd_elect_one() {
   return pred != 0;
 }
 
+// A launch whose CTAs form clusters of `cluster` along x.
+template <typename Kernel>
+inline cudaError_t launch_clusters(Kernel kernel, dim3 grid, dim3 block, unsigned cluster, size_t smem, cudaStream_t st, const BwdArgs& a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+constexpr int kSplit4Blocks = 74, kSplit2Blocks = 296;
 cudaError_t launch_bwd_ws128(const BwdArgs& a, cudaStream_t st);  // 64 < head_dim <= 128
 cudaError_t launch_bwd_ws(const BwdArgs& a, cudaStream_t st);
 // Packs dO, LSE and delta of every query tile (rows as listed in a.rowpack).

@@ -214,6 +214,34 @@ def test_gradients_against_oracle_on_seeded_inputs(lens, hq, hkv, dim, chunk, to
         _check_close(key, torch_to_f64(got), ref[key])
 
 
+@pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk", [
+    ((7,), 1, 1, 64, 64, 3),             # one query tile for a cluster of four
+    ((40, 130), 1, 1, 128, 64, 2),
+    ((129, 257), 3, 1, 128, 128, 3),     # shares of unequal size
+    ((1100, 1200), 8, 8, 64, 200, 3),    # clusters of two
+    ((1250,), 10, 10, 96, 256, 3),
+])
+def test_backward_divided_over_a_cluster(lens, hq, hkv, dim, chunk, topk):
+    """Few key blocks: the query tiles of a block over the CTAs of a cluster; dK and dV stay bit-repeatable."""
+    rng = torch.Generator().manual_seed(99)
+    total = sum(lens)
+    q, k, v = [torch.randn(total, h, dim, generator=rng).bfloat16() for h in (hq, hkv, hkv)]
+    do = torch.randn(total, hq, dim, generator=rng).bfloat16()
+    cu = cu_from_lens(lens)
+    out, lse, captured, grads = _run(q, k, v, cu, chunk, topk, d_out=do)
+    qf, kf, vf, dof = (torch_to_f64(t) for t in (q, k, v, do))
+    if max(lens) <= chunk:
+        sel = mo.dense_sel(cu, chunk, hq)
+    else:
+        r = mo.route_prefill(qf, kf, cu, chunk, topk)
+        sel = mo.sel_from_selected(captured["selected"].numpy(), r["filtered"], r["sel"].shape[-1])
+    ref = mo.attention_fixed_route(qf, kf, vf, cu, sel, chunk, d_out=dof)
+    for key, got in zip(("dq", "dk", "dv"), grads):
+        _check_close(key, torch_to_f64(got), ref[key])
+    _, _, _, again = _run(q, k, v, cu, chunk, topk, d_out=do)
+    assert torch.equal(grads[1], again[1]) and torch.equal(grads[2], again[2])
+
+
 @pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk", [((1500, 800), 4, 2, 64, 256, 3), ((1024,), 8, 2, 128, 128, 5)])
 def test_deterministic_backward_is_bit_repeatable(lens, hq, hkv, dim, chunk, topk):
     """deterministic_backward=True (the counterpart of deterministic=True in the reference's two backward calls,
