@@ -161,14 +161,16 @@ __device__ __forceinline__ long long fwd_item_index(int k) {
 }
 
 constexpr int kFwdThreads = 384;  // warp 11 only completes the third warpgroup (register hand-over works per warpgroup)
+constexpr int kEpiBlock = 32 * 128;  // bytes: 32 rows x 64 columns of 16-bit values
 constexpr int kFwdItems = 4;      // decoded work items ahead of their users
 
-template <int DPAD>
+template <int DPAD, bool SELF>
 struct FwdCfg {
   static constexpr int TILE_BYTES = kTile * DPAD * 2;
   static constexpr int QBUFS = DPAD <= 64 ? 2 : 1;   // query tile buffers per lane
   static constexpr int STAGES = DPAD <= 64 ? 4 : 2;  // K/V ring depth (a stage = K tile + V tile)
-  static constexpr int SMEM = 1024 + 2 * QBUFS * TILE_BYTES + STAGES * 2 * TILE_BYTES;
+  // the remote pass stages the rows it writes, a block per softmax warp (see store_rows64)
+  static constexpr int SMEM = 1024 + 2 * QBUFS * TILE_BYTES + STAGES * 2 * TILE_BYTES + (SELF ? 0 : 8 * kEpiBlock);
   static constexpr uint32_t TMEM_COLS = 512;
   // Tensor memory: S0 0-127, S1 128-255, O0/O1 from 256.  With D <= 64 P has columns of its own (384-511),
   // so the next S of a lane can be computed while its softmax still runs; with D = 128 all 512 columns are
@@ -190,9 +192,40 @@ struct FwdSmem {
 };
 static_assert(sizeof(FwdSmem) <= 1024, "control block must fit its reservation");
 
+// The remote pass writes whole rows, one per thread, to scattered slots.  Stored straight from the thread that holds the row,
+// a 16-byte access of a warp touches 32 lines, and the load/store pipe serves one line a cycle: 8 to 16 such accesses a
+// row, at four key tiles an item a fifth of the pass.  So rows pass through a block of shared memory per warp, from which eight
+// lanes write a row's 128 bytes: four lines an access.  Remote pass at D = 128: 710 -> 583 us (32768 tokens, chunk 512), 8500 ->
+// 8277 us (131072 tokens, chunk 4096); at D = 64 2617 -> 2428 us (4 x 32768 tokens, chunk 2048).  The self pass merges partial
+// rows in the same one-row-per-thread form and was no faster either way (997 us as it is, 1003 staged): its items wait
+// for the last product, not for the pipe.
+// Offset of 16-byte unit u of row r in a block; the swizzle keeps both views free of bank conflicts.
+__device__ __forceinline__ uint32_t stage_unit(int r, int u) { return (uint32_t)(r * 128 + ((u ^ (r & 7)) << 4)); }
+
+// Writes 64 columns of every row of the warp: `values` of the thread's row, to base + id * D for id >= 0, columns < D - col0.
+template <bool F16>
+__device__ __forceinline__ void store_rows64(uint8_t* block, const float* values, float factor, __nv_bfloat16* base, int id, int D, int col0) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    *reinterpret_cast<uint4*>(block + stage_unit(lane, u)) =
+        make_uint4(pack16<F16>(values[u * 8] * factor, values[u * 8 + 1] * factor), pack16<F16>(values[u * 8 + 2] * factor, values[u * 8 + 3] * factor),
+                   pack16<F16>(values[u * 8 + 4] * factor, values[u * 8 + 5] * factor), pack16<F16>(values[u * 8 + 6] * factor, values[u * 8 + 7] * factor));
+  __syncwarp();
+  const int u = lane & 7;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3);
+    const int to = __shfl_sync(0xFFFFFFFFu, id, r);
+    const uint4 w = *reinterpret_cast<const uint4*>(block + stage_unit(r, u));
+    if (to >= 0 && col0 + u * 8 < D) *reinterpret_cast<uint4*>(base + (long long)to * D + col0 + u * 8) = w;
+  }
+  __syncwarp();  // the block may be written again
+}
+
 template <int DPAD, bool SELF, bool F16>
 __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(FwdArgs a) {
-  using Cfg = FwdCfg<DPAD>;
+  using Cfg = FwdCfg<DPAD, SELF>;
   constexpr int TILE_BYTES = Cfg::TILE_BYTES, QBUFS = Cfg::QBUFS, STAGES = Cfg::STAGES;
   constexpr int UPR = DPAD / 8;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -542,20 +575,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(FwdArgs a) {
       tc_fence_before_sync();
       __syncwarp();
       if (lane_id == 0) mbar_arrive(&cb.o_free[l]);
-      if (row >= rows || !alive) continue;
       if (!SELF) {
-        if (row_id < 0 || row_id / pv.R >= pv.T * pv.Hq) { atomicOr(a.status, kErrBadIndex); continue; }
+        if (row < rows && (row_id < 0 || row_id / pv.R >= pv.T * pv.Hq)) { atomicOr(a.status, kErrBadIndex); row_id = -1; }
+        const int to = alive ? row_id : -1;
         const float inv = 1.f / l_run;
-        __nv_bfloat16* dst = a.part_o + (long long)row_id * D;
+        uint8_t* block = sKV + STAGES * 2 * TILE_BYTES + warp * kEpiBlock;
 #pragma unroll
-        for (int u = 0; u < UPR; ++u) {
-          if (u * 8 < D)
-            *reinterpret_cast<uint4*>(dst + u * 8) =
-                make_uint4(pack16<F16>(o_acc[u * 8] * inv, o_acc[u * 8 + 1] * inv), pack16<F16>(o_acc[u * 8 + 2] * inv, o_acc[u * 8 + 3] * inv),
-                           pack16<F16>(o_acc[u * 8 + 4] * inv, o_acc[u * 8 + 5] * inv), pack16<F16>(o_acc[u * 8 + 6] * inv, o_acc[u * 8 + 7] * inv));
-        }
-        a.part_lse[row_id] = m_used + log2f(l_run);
-      } else {
+        for (int hf = 0; hf < DPAD / 64; ++hf) store_rows64<F16>(block, o_acc + hf * 64, inv, a.part_o, to, D, hf * 64);
+        if (to >= 0) a.part_lse[to] = m_used + log2f(l_run);
+      } else if (row < rows && alive) {
         // global-softmax merge of the self branch with the row's remote partials (fixed slot order).  The loads are
         // issued in batches that do not depend on each other - the selection and the partial LSEs of four slots, then
         // the partial output rows of two slots - so that a row costs a few trips to memory, not three per slot.
@@ -645,7 +673,7 @@ static int sm_count() {
 
 template <int DPAD, bool SELF, bool F16>
 static cudaError_t launch_fwd_as(const FwdArgs& a, long long items, cudaStream_t st) {
-  const int smem = FwdCfg<DPAD>::SMEM;
+  const int smem = FwdCfg<DPAD, SELF>::SMEM;
   cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<DPAD, SELF, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const int sms = sm_count();
