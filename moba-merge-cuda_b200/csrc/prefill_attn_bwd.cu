@@ -2,7 +2,7 @@
 // held fixed, as OptMixedAttention.backward of the reference (src/moba_opt/mixed_attention.py:141-225) obtains from
 // two FlashAttention backward calls on the global O and LSE.
 //
-// Launch sequence: dq_acc = 0, delta = rowsum(dO * O), pack dO / LSE / delta per query tile, the KV-stationary main
+// Launch sequence: delta = rowsum(dO * O) and dq_acc = 0, pack dO / LSE / delta per query tile, the KV-stationary main
 // kernel (prefill_attn_bwd_ws.cu for head_dim <= 64, prefill_attn_bwd_ws128.cu above that: dK and dV of a key block
 // accumulate in tensor memory and are written once, dQ of every tile is added into the FP32 buffer row by row with bulk
 // reductions of the copy engine), dq = dq_acc rounded to the input format.  With MOBA_BWD_DETERMINISTIC the accumulator
@@ -13,15 +13,19 @@
 namespace moba {
 
 // delta[row] = sum_d dO[row,d] * O[row,d].  LPR lanes share a (token, head) row, 16 bytes of it each, so
-// every lane of a warp has work at any head dimension (LPR = 4, 8, 16 or 32: smallest power of two >= D/8).
+// every lane of a warp has work at any head dimension (LPR = 4, 8, 16 or 32: smallest power of two >= D/8).  The lanes
+// also clear their 16-byte units of the row's dQ accumulator (acc_units of them per row), which saves a launch and runs
+// the writes beside the reads: 165 -> 135 us at 131072 tokens, 14 heads, D = 64.
 template <int LPR>
 __global__ void __launch_bounds__(256) bwd_delta_kernel(const __nv_bfloat16* __restrict__ out,
                                                         const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
-                                                        long long rows, int D, bool f16) {
+                                                        uint4* __restrict__ acc, int acc_units, long long rows, int D, bool f16) {
   constexpr int RPW = 32 / LPR;  // rows per warp
   const int lane = threadIdx.x & 31, sub = lane % LPR;
   const long long row = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * RPW + lane / LPR;
   float s = 0.f;
+  if (row < rows)
+    for (int u = sub; u < acc_units; u += LPR) acc[row * acc_units + u] = make_uint4(0u, 0u, 0u, 0u);
   if (row < rows && sub * 8 < D) {
     const uint4 a = *reinterpret_cast<const uint4*>(out + row * D + sub * 8);
     const uint4 b = *reinterpret_cast<const uint4*>(dout + row * D + sub * 8);
@@ -94,16 +98,17 @@ extern "C" int moba_prefill_bwd(const moba_prefill_desc* d, const void* q, const
   float* dq_acc = reinterpret_cast<float*>(static_cast<char*>(scratch) + align256((size_t)rows * 4));
   const bool fixed = (d->flags & MOBA_BWD_DETERMINISTIC) != 0;
   const size_t acc_bytes = (size_t)rows * d->dim * (fixed ? 8 : 4);
-  if (cudaMemsetAsync(dq_acc, 0, acc_bytes, st) != cudaSuccess) return MOBA_ERR_CUDA;
   {
     const __nv_bfloat16* o16 = static_cast<const __nv_bfloat16*>(out);
     const __nv_bfloat16* do16 = static_cast<const __nv_bfloat16*>(dout);
     const int units = d->dim / 8;
+    uint4* acc = reinterpret_cast<uint4*>(dq_acc);
+    const int au = d->dim * (fixed ? 8 : 4) / 16;
     const bool f16 = (d->flags & MOBA_INPUT_FP16) != 0;
-    if (units <= 4) bwd_delta_kernel<4><<<(unsigned)((rows + 63) / 64), 256, 0, st>>>(o16, do16, delta, rows, d->dim, f16);
-    else if (units <= 8) bwd_delta_kernel<8><<<(unsigned)((rows + 31) / 32), 256, 0, st>>>(o16, do16, delta, rows, d->dim, f16);
-    else if (units <= 16) bwd_delta_kernel<16><<<(unsigned)((rows + 15) / 16), 256, 0, st>>>(o16, do16, delta, rows, d->dim, f16);
-    else bwd_delta_kernel<32><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(o16, do16, delta, rows, d->dim, f16);
+    if (units <= 4) bwd_delta_kernel<4><<<(unsigned)((rows + 63) / 64), 256, 0, st>>>(o16, do16, delta, acc, au, rows, d->dim, f16);
+    else if (units <= 8) bwd_delta_kernel<8><<<(unsigned)((rows + 31) / 32), 256, 0, st>>>(o16, do16, delta, acc, au, rows, d->dim, f16);
+    else if (units <= 16) bwd_delta_kernel<16><<<(unsigned)((rows + 15) / 16), 256, 0, st>>>(o16, do16, delta, acc, au, rows, d->dim, f16);
+    else bwd_delta_kernel<32><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(o16, do16, delta, acc, au, rows, d->dim, f16);
   }
   BwdArgs a;
   a.pv = make_view(*d);
