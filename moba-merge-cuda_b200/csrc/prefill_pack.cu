@@ -7,11 +7,10 @@
 
 namespace moba {
 
-// One CTA per (key block, kv head): rows are the block's tokens, missing tokens and head-dim padding are zero.
-__global__ void __launch_bounds__(128) pack_kv_kernel(PrefillView pv, const __nv_bfloat16* __restrict__ k,
-                                                      const __nv_bfloat16* __restrict__ v, uint8_t* __restrict__ kpack,
-                                                      uint8_t* __restrict__ vpack, int dpad) {
-  const int blk = blockIdx.x, g = blockIdx.y, tid = threadIdx.x;
+// A (key block, kv head): rows are the block's tokens, missing tokens and head-dim padding are zero.
+__device__ __forceinline__ void pack_kv(const PrefillView& pv, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
+                                        uint8_t* __restrict__ kpack, uint8_t* __restrict__ vpack, int dpad, int blk, int g) {
+  const int tid = threadIdx.x;
   const int c = pv.qtile_chunk[blk];
   const int k0 = pv.qtile_tok0[blk];
   const int nkeys = min(kTile, pv.chunk_start[c + 1] - k0);
@@ -32,14 +31,21 @@ __global__ void __launch_bounds__(128) pack_kv_kernel(PrefillView pv, const __nv
   }
 }
 
-// One CTA per query tile (own-chunk tiles first, then the expert tiles in list order).
-__global__ void __launch_bounds__(128) pack_q_kernel(PrefillView pv, const __nv_bfloat16* __restrict__ q,
-                                                     const int* __restrict__ rowlist, const int* __restrict__ seg_base,
-                                                     const int* __restrict__ tile_base, uint8_t* __restrict__ qpack,
-                                                     int* __restrict__ rowpack, int dpad, unsigned* status) {
+// One CTA per (key block, kv head), then one per query tile (own-chunk tiles first, then the expert tiles in list order):
+// one launch, since at a few thousand tokens a launch and its gap cost as much as the K and V blocks themselves.
+__global__ void __launch_bounds__(128) pack_kernel(PrefillView pv, const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                                                   const __nv_bfloat16* __restrict__ v, const int* __restrict__ rowlist,
+                                                   const int* __restrict__ seg_base, const int* __restrict__ tile_base,
+                                                   uint8_t* __restrict__ kpack, uint8_t* __restrict__ vpack, uint8_t* __restrict__ qpack,
+                                                   int* __restrict__ rowpack, int dpad, unsigned* status) {
   __shared__ int s_th[kTile];
   const int tid = threadIdx.x;
-  const long long tile = blockIdx.x;
+  const int n_kv = pv.n_qtiles * pv.Hkv;
+  if ((int)blockIdx.x < n_kv) {
+    pack_kv(pv, k, v, kpack, vpack, dpad, blockIdx.x / pv.Hkv, blockIdx.x % pv.Hkv);
+    return;
+  }
+  const long long tile = (long long)blockIdx.x - n_kv;
   const long long n_self = (long long)pv.n_qtiles * pv.Hq;
   int th = -1;
   if (tile < n_self) {
@@ -87,10 +93,6 @@ cudaError_t launch_prefill_pack(const moba_prefill_desc& d, const void* q, const
   const PrefillView pv = make_view(d);
   const PackState ps = carve_pack_state(d, route_state);
   const int dpad = pack_dpad(d);
-  pack_kv_kernel<<<dim3(d.num_qtiles, d.hkv), 128, 0, st>>>(pv, static_cast<const __nv_bfloat16*>(k),
-                                                            static_cast<const __nv_bfloat16*>(v),
-                                                            reinterpret_cast<uint8_t*>(ps.kpack),
-                                                            reinterpret_cast<uint8_t*>(ps.vpack), dpad);
   const int* rowlist = nullptr;
   const int* seg_base = nullptr;
   const int* tile_base = nullptr;
@@ -99,8 +101,10 @@ cudaError_t launch_prefill_pack(const moba_prefill_desc& d, const void* q, const
     rowlist = rs.rowlist; seg_base = rs.seg_base; tile_base = rs.tile_base;
   }
   const long long tiles = d.remote_k > 0 ? pack_q_tiles(d) : (long long)d.num_qtiles * d.hq;
-  pack_q_kernel<<<(unsigned)tiles, 128, 0, st>>>(pv, static_cast<const __nv_bfloat16*>(q), rowlist, seg_base, tile_base,
-                                                 reinterpret_cast<uint8_t*>(ps.qpack), ps.rowpack, dpad, status);
+  pack_kernel<<<(unsigned)((long long)d.num_qtiles * d.hkv + tiles), 128, 0, st>>>(
+      pv, static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), rowlist, seg_base,
+      tile_base, reinterpret_cast<uint8_t*>(ps.kpack), reinterpret_cast<uint8_t*>(ps.vpack), reinterpret_cast<uint8_t*>(ps.qpack), ps.rowpack,
+      dpad, status);
   return cudaGetLastError();
 }
 
