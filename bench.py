@@ -892,7 +892,7 @@ def run_ours(args):
                              ms_per_step=None if ms_e2e is None else ms_e2e / e2e_steps, steps=e2e_steps,
                              mode="host copies on their own streams, double-buffered across steps", numa_node=numa_node,
                              numa_h2d_gbs=numa_rates),
-                    gpu_launches=13 * args.steps,  # route 5, pack 2, forward 2, backward 4 (memsets not counted)
+                    gpu_launches=11 * args.steps,  # route 4, pack 1, forward 2, backward 4 (memsets not counted)
                     roofline=dict(bound="tensor", kernel=bwd_kernel, achieved=achieved, peak=pk["tflops"],
                                   unit="TFLOP/s", frac=achieved / pk["tflops"], peak_source=pk["source"] + " (sustained bf16)",
                                   traffic=traffic, traffic_source=traffic_source,

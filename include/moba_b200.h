@@ -182,6 +182,11 @@ int moba_decode_means(const moba_cache_desc* c, const int32_t* seqs, const int32
  * into.  Means are bit-identical to moba_decode_means. */
 int moba_prefill_to_cache(const moba_cache_desc* c, const void* k, const void* v, const int32_t* seqs, const int32_t* start,
                           const int32_t* cu_seqlens, int num_seqs, int max_chunks_touched, unsigned* status, void* stream);
+/* The same for k and v whose tokens and heads lie `stride` elements apart (views of a fused projection); strides are
+ * multiples of 8 elements and the base pointers 16-byte aligned. */
+int moba_prefill_to_cache_strided(const moba_cache_desc* cache, const void* k, int64_t k_stride_t, int64_t k_stride_h, const void* v,
+                                  int64_t v_stride_t, int64_t v_stride_h, const int32_t* seqs, const int32_t* start,
+                                  const int32_t* cu_seqlens, int num_seqs, int max_chunks_touched, unsigned* status, void* stream);
 
 /* Copies a step's q, k, v into the fixed buffers a captured step reads (prepared_decode.py:150-176 of the reference
  * does three tensor copies), as one launch.  Sizes in bytes, multiples of 16, pointers 16-byte aligned

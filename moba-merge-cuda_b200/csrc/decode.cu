@@ -198,8 +198,11 @@ __global__ void __launch_bounds__(256) decode_means_kernel(CacheView cv, const i
 // touched, kv head, sequence) stores the chunk's new K and V rows into their pages and adds the K rows up as it
 // goes (rows of the chunk that were cached before are read back), instead of an append launch over per-token
 // (sequence, position) arrays built on the host followed by a second pass over K for the means.
+// K and V may be views with token and head strides (of a fused q/k/v projection): copying them first cost 42 us of
+// the 104 us that a 65536-token prompt's hand-off took.
+struct AppendStrides { long long k_t, k_h, v_t, v_h; };  // elements
 __global__ void __launch_bounds__(256) prefill_to_cache_kernel(CacheView cv, const __nv_bfloat16* __restrict__ k,
-                                                               const __nv_bfloat16* __restrict__ v, const int* __restrict__ seqs,
+                                                               const __nv_bfloat16* __restrict__ v, AppendStrides st, const int* __restrict__ seqs,
                                                                const int* __restrict__ start, const int* __restrict__ cu,
                                                                unsigned* status) {
   extern __shared__ float s_part[];
@@ -236,9 +239,9 @@ __global__ void __launch_bounds__(256) prefill_to_cache_kernel(CacheView cv, con
         kr[j] = vr[j] = make_uint4(0u, 0u, 0u, 0u);
         if (dst[j] < 0) continue;
         if (fresh[j]) {
-          const long long src = (((long long)src0 + (lo + w0 + j * rpi - first)) * cv.Hkv + g) * cv.D + u * 8;
-          kr[j] = *reinterpret_cast<const uint4*>(k + src);
-          vr[j] = *reinterpret_cast<const uint4*>(v + src);
+          const long long token = (long long)src0 + (lo + w0 + j * rpi - first);
+          kr[j] = *reinterpret_cast<const uint4*>(k + token * st.k_t + g * st.k_h + u * 8);
+          vr[j] = *reinterpret_cast<const uint4*>(v + token * st.v_t + g * st.v_h + u * 8);
         } else {
           kr[j] = *reinterpret_cast<const uint4*>(cv.kc + dst[j]);
         }
@@ -1170,18 +1173,28 @@ extern "C" int moba_decode_means(const moba_cache_desc* c, const int32_t* seqs, 
   return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;
 }
 
-extern "C" int moba_prefill_to_cache(const moba_cache_desc* c, const void* k, const void* v, const int32_t* seqs, const int32_t* start,
-                                     const int32_t* cu_seqlens, int num_seqs, int max_chunks_touched, unsigned* status,
-                                     void* stream) {
+extern "C" int moba_prefill_to_cache_strided(const moba_cache_desc* c, const void* k, int64_t k_stride_t, int64_t k_stride_h, const void* v,
+                                             int64_t v_stride_t, int64_t v_stride_h, const int32_t* seqs, const int32_t* start,
+                                             const int32_t* cu_seqlens, int num_seqs, int max_chunks_touched, unsigned* status,
+                                             void* stream) {
   int rc = validate_cache(c);
   if (rc != MOBA_OK) return rc;
+  if ((k_stride_t | k_stride_h | v_stride_t | v_stride_h) & 7) return MOBA_ERR_UNSUPPORTED;  // 16-byte loads
+  if (((uintptr_t)k | (uintptr_t)v) & 15) return MOBA_ERR_UNSUPPORTED;
   if (!k || !v || !seqs || !start || !cu_seqlens || num_seqs < 1 || num_seqs > 65535 || max_chunks_touched < 1)
     return MOBA_ERR_INVALID;
   const int rpi = 256 / (c->dim / 8);
   prefill_to_cache_kernel<<<dim3(max_chunks_touched, c->hkv, num_seqs), 256, (size_t)rpi * c->dim * 4, (cudaStream_t)stream>>>(
-      make_cache_view(*c), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), seqs, start, cu_seqlens,
-      status);
+      make_cache_view(*c), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
+      AppendStrides{k_stride_t, k_stride_h, v_stride_t, v_stride_h}, seqs, start, cu_seqlens, status);
   return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;
+}
+
+extern "C" int moba_prefill_to_cache(const moba_cache_desc* c, const void* k, const void* v, const int32_t* seqs, const int32_t* start,
+                                     const int32_t* cu_seqlens, int num_seqs, int max_chunks_touched, unsigned* status, void* stream) {
+  if (!c) return MOBA_ERR_INVALID;
+  const int64_t head = c->dim, token = (int64_t)c->hkv * c->dim;
+  return moba_prefill_to_cache_strided(c, k, token, head, v, token, head, seqs, start, cu_seqlens, num_seqs, max_chunks_touched, status, stream);
 }
 
 extern "C" int moba_decode_stage_inputs(void* q_dst, const void* q_src, size_t q_bytes, void* k_dst, const void* k_src, size_t k_bytes,

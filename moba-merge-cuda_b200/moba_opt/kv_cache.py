@@ -50,7 +50,7 @@ class FiniteInput(ctypes.Structure):
                 ("heads", ctypes.c_int32), ("reserved0", ctypes.c_int32)]
 
 
-_P, _VP, _I, _SZ = ctypes.POINTER(CacheDesc), ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
+_P, _VP, _I, _I64, _SZ = ctypes.POINTER(CacheDesc), ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_size_t
 # entry point -> (result type, argument types); every decode entry point of include/moba_b200.h is bound from this table
 _DECODE_ABI = {
     "moba_cache_update": (_I, [_P, _VP, _I, _VP, _VP, _I, _I, _VP]),
@@ -60,6 +60,7 @@ _DECODE_ABI = {
     "moba_decode_step_begin": (_I, [_P, _VP, _VP, _VP, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP]),
     "moba_decode_stage_inputs": (_I, [_VP, _VP, _SZ, _VP, _VP, _SZ, _VP, _VP, _SZ, _VP]),
     "moba_prefill_to_cache": (_I, [_P, _VP, _VP, _VP, _VP, _VP, _I, _I, _VP, _VP]),
+    "moba_prefill_to_cache_strided": (_I, [_P, _VP, _I64, _I64, _VP, _I64, _I64, _VP, _VP, _VP, _I, _I, _VP, _VP]),
     "moba_decode_union_capacity": (_I, [_I, _I, _I, _I]),
     "moba_decode_route": (_I, [_P, _VP, _VP, _VP, _I, _I, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP]),
     "moba_decode_attend_workspace_bytes": (_SZ, [_P, _I, _I, _I]),
@@ -79,6 +80,12 @@ def decode_library():
             fn.restype, fn.argtypes = restype, argtypes
         lib._decode_abi_bound = True
     return lib
+
+
+def _rows_of_16_bytes(t):
+    """`t` itself where the append kernel can read its rows in place (16-byte aligned, any token and head stride that keeps
+    them so), a contiguous copy otherwise."""
+    return t.clone(memory_format=torch.contiguous_format) if t.stride(0) % 8 or t.stride(1) % 8 or t.data_ptr() % 16 else t
 
 
 # ----------------------------------------------------------------------------------------- small contracts
@@ -388,9 +395,9 @@ class PagedKVCache:
                      d_ids.data_ptr(), d_lengths.data_ptr(), len(ids), 0)
         c = self.chunk_size
         touched = max((first + n - 1) // c - first // c + 1 for first, n in zip(starts, counts))
-        k, v = k.contiguous(), v.contiguous()
-        self._launch("moba_prefill_to_cache", ctypes.byref(desc), k.data_ptr(), v.data_ptr(), d_ids.data_ptr(), d_starts.data_ptr(),
-                     d_cu.data_ptr(), len(ids), touched, self._status.data_ptr())
+        k, v = _rows_of_16_bytes(k), _rows_of_16_bytes(v)
+        self._launch("moba_prefill_to_cache_strided", ctypes.byref(desc), k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0),
+                     v.stride(1), d_ids.data_ptr(), d_starts.data_ptr(), d_cu.data_ptr(), len(ids), touched, self._status.data_ptr())
         lay.commit(plan)
         self._candidate_count = self._routable(plan.lengths)
         return plan, starts, sent[5:]

@@ -467,3 +467,28 @@ def test_cluster_attend_divides_a_request(lens, mode, hq, hkv, dim, chunk, page,
     check(cache, result, q)
     again = cache.attend(q, sequence_ids=list(range(len(lens))), topk=4, mode=mode)
     assert torch.equal(result.output, again.output) and torch.equal(result.lse, again.lse)
+
+
+@pytest.mark.parametrize("layout", ["fused", "heads_first", "expanded", "unaligned"])
+def test_append_reads_strided_views(layout):
+    """Views of a fused projection, a transposed layout, one head for all and rows off the 16-byte grid give the cache that
+    contiguous tensors give: pages and chunk means bit for bit."""
+    from moba_opt import PagedKVCache
+    tokens, hkv, dim = 300, 2, 40
+    if layout == "fused":
+        qkv = rand((tokens, 3 * hkv, dim), 91)
+        k, v = qkv[:, hkv:2 * hkv], qkv[:, 2 * hkv:]
+    elif layout == "heads_first":
+        k, v = (rand((hkv, tokens, dim), s).transpose(0, 1) for s in (92, 93))
+    elif layout == "expanded":
+        k, v = (rand((tokens, 1, dim), s).expand(tokens, hkv, dim) for s in (94, 95))
+    else:
+        k, v = (rand((tokens * hkv * dim + 1,), s)[1:].view(tokens, hkv, dim) for s in (96, 97))
+    caches = [PagedKVCache(2, 512, hkv, dim, page_size=7, chunk_size=64) for _ in range(2)]
+    for cache, (kk, vv) in zip(caches, ((k, v), (k.clone(memory_format=torch.contiguous_format), v.clone(memory_format=torch.contiguous_format)))):
+        cache.append(kk, vv, sequence_ids=[0, 1], cu_seqlens=[0, 130, tokens])
+    for sid in range(2):
+        assert_payload(caches[0], sid, *caches[1].materialize(sid))
+        closed = caches[0].lengths[sid] // 64
+        assert torch.equal(caches[0]._means[sid, :closed], caches[1]._means[sid, :closed])
+    assert_payload(caches[0], 0, k[:130], v[:130])
