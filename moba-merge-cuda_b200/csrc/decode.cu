@@ -9,9 +9,11 @@
 //
 // Attention reads each needed K/V token once per KV head: the routing kernel turns the per-query-
 // head selections of a GQA group into the union of chunks with a bitmask of the heads that attend
-// each of them; one CTA handles one part of one chunk for all those heads.  Partial (max, sum,
-// accumulator) triples go to a workspace and the last CTA of a (query, kv head) pair to finish -
-// found with an atomic ticket, nobody waits - merges them in a fixed order.
+// each of them, and a token serves all those heads.  Three kernels divide the work (the rule and its figures stand at
+// moba_decode_attend): clusters that merge through distributed shared memory for the smallest batches, a CTA per fixed part of
+// a chunk while that grid fits the GPU at once, equal shares of one list of stages beyond.  The last two leave partial (max, sum,
+// accumulator) triples in a workspace, and the CTA that finishes a (query, kv head) pair last - found with an atomic
+// ticket, nobody waits - merges them in a fixed order.
 #include "launch.cuh"
 #include "moba_b200.h"
 #include "prefill_common.cuh"
@@ -552,10 +554,11 @@ struct AttendArgs {
   const unsigned* u_mask;
   const int* u_count;
   int Hq, umax;
+  int ns, parts, part_tokens;  // fixed parts: slots per head, parts of a chunk and their tokens
   int* counters;   // [nq * Hkv], zero between launches
-  float* pm;       // [segments][G], see the streamed variant
+  float* pm;       // fixed parts: [nq*Hq*ns*parts]; streamed: [segments][G]
   float* pl;
-  float* pacc;     // [segments][G][D]
+  float* pacc;     // [.., D]
   __nv_bfloat16* out;
   float* lse;
   unsigned* status;
@@ -568,6 +571,8 @@ constexpr int kStageTokens = 64;  // tokens per pipeline stage: 16 per warp
 constexpr int stream_stages(int dp) { return dp <= 64 ? 4 : 2; }  // streamed variant: 64 KB of ring per CTA at D = 64 and 128, three CTAs per SM
 constexpr int cluster_stages(int dp) { return dp <= 64 ? 4 : 2; }  // cluster variant, per team
 constexpr int cluster_teams(int dp) { return dp <= 128 ? 2 : 1; }
+constexpr int kStages = 2;  // fixed parts, one team: two 32 KB stages (D <= 128) and 160 registers let three CTAs share an SM
+constexpr int deep_stages(int dp) { return dp <= 64 ? 4 : dp <= 128 ? 2 : 3; }  // fixed parts, per team (two teams up to D = 128)
 constexpr int kClusterList = 576;  // union entries a cluster CTA keeps in shared memory: 32 heads of 16 picks each, the own chunk
 
 // Shared-memory K/V stage: row = one token, DP bf16 values; the 16-byte units of a row are
@@ -619,6 +624,18 @@ struct StageCursor {
   }
 };
 
+// Row base (element offset of the K/V row of kv head g, or -1) of the token at offset r of logical page pg.  The
+// lookup goes through the page table; it is issued one stage ahead of the copy that needs it.  No branch depends
+// on the table entry, so several lookups can be in flight; a bad entry is recorded in `bad` and reported later.
+__device__ __forceinline__ long long attend_row_base(const CacheView& cv, int sid, int g, int pg, int r, bool exists,
+                                                     bool& bad) {
+  // an ordinary cached load (a page serves many tokens): not the read-only path, which a dependent launch must avoid
+  const int physical = exists ? cv.table[(long long)sid * cv.width + pg] : 0;
+  const bool wrong = physical < 0 || physical >= cv.num_pages;
+  bad |= wrong;
+  return exists && !wrong ? (((long long)physical * cv.page + r) * cv.Hkv + g) * cv.D : -1;
+}
+
 // Copies the K and V rows of one stage with cp.async.  Consecutive threads copy consecutive 16-byte
 // units of a row, so every 32-byte sector fetched from L2 is used in full; rows that do not exist
 // and head-dim padding are zero-filled.
@@ -661,12 +678,396 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// ---- pieces of the merge that are needed only when a head has more partials than fit in shared memory; they
+// are functions of their own so that the common path stays short.
+struct MergeTail {
+  const int* selected;  // null: dense, slot == chunk
+  const float *pm, *pl, *pacc;
+  int parts, cur, cur_parts, D;
+  __device__ __forceinline__ bool valid(long long hbase, int j) const {
+    const int sl = j / parts, pt = j - sl * parts;
+    const int c = selected ? __ldcg(selected + hbase + sl) : sl;
+    return c >= 0 && pt < (c == cur ? cur_parts : parts);
+  }
+};
 // a select, not a branch: stale values where the weight is zero never count and the load stays unconditional
 __device__ __forceinline__ void merge_add(float4& v, const float4& x, float w) {
   const bool use = w != 0.f;
   v.x = fmaf(use ? x.x : 0.f, w, v.x); v.y = fmaf(use ? x.y : 0.f, w, v.y);
   v.z = fmaf(use ? x.z : 0.f, w, v.z); v.w = fmaf(use ? x.w : 0.f, w, v.w);
 }
+__device__ __noinline__ float merge_tail_max(const MergeTail& t, long long hbase, int from, int total, float big) {
+  for (int j = from; j < total; j += 16)
+    if (t.valid(hbase, j)) big = fmaxf(big, __ldcg(t.pm + hbase * t.parts + j));
+  return big;
+}
+__device__ __noinline__ float merge_tail_den(const MergeTail& t, long long hbase, int from, int total, float big, float lsum) {
+  for (int j = from; j < total; j += 16)
+    if (t.valid(hbase, j))
+      lsum = fmaf(__ldcg(t.pl + hbase * t.parts + j), dec_exp2(__ldcg(t.pm + hbase * t.parts + j) - big), lsum);
+  return lsum;
+}
+// partials [from, to) whose weights are in shared memory but whose sums are not
+__device__ __noinline__ float4 merge_rest_acc(const MergeTail& t, long long hbase, int from, int to, int d, const float* wrow,
+                                              float4 v) {
+  const float4* src = reinterpret_cast<const float4*>(t.pacc + hbase * t.parts * t.D + d);
+#pragma unroll 8
+  for (int j = from; j < to; ++j) merge_add(v, __ldcg(src + (long long)j * (t.D >> 2)), wrow[j]);
+  return v;
+}
+// partials [from, total) with nothing in shared memory
+__device__ __noinline__ float4 merge_tail_acc(const MergeTail& t, long long hbase, int from, int total, int d, float big,
+                                              float4 v) {
+  const float4* src = reinterpret_cast<const float4*>(t.pacc + hbase * t.parts * t.D + d);
+  for (int j = from; j < total; ++j)
+    if (t.valid(hbase, j))
+      merge_add(v, __ldcg(src + (long long)j * (t.D >> 2)), dec_exp2(__ldcg(t.pm + hbase * t.parts + j) - big));
+  return v;
+}
+
+// ---- fixed parts -------------------------------------------------------------------------------------------------
+// Split-K paged attention for one (query row, kv head, union chunk, part), where that grid fits the GPU at once.  At most one
+// CTA per SM: two teams of four warps with a copy ring and a barrier of their own, each on half of the part's stages, because
+// with one warp per scheduler nothing hides the dependent chain of a stage (ldmatrix, mma, shuffles, exp2, mma); above that one team
+// with two stages and three CTAs per SM.  A CTA knows its part from its block index alone and starts at once, which is what
+// the streamed variant, whose CTAs first find their share, cannot do.
+template <int DP, int NS, int TEAMS, bool F16>
+__global__ void __launch_bounds__(128 * TEAMS, (TEAMS == 1 && DP <= 128 ? 3 : 1)) decode_attend_kernel(AttendArgs a) {
+  constexpr int NT = 128 * TEAMS, NW = 4 * TEAMS;  // threads and warps of the CTA
+  constexpr int KSTEPS = DP / 16;
+  constexpr int DT = DP / 8;  // 8-column output tiles
+  constexpr int STAGE_BYTES = 2 * kStageTokens * DP * 2;
+  extern __shared__ __align__(128) uint8_t s_pipe[];  // NS stages per team; reused for the cross-warp reduction
+  __shared__ int s_last, s_slot[kHeadBlock];
+  __shared__ long long s_rowbase_all[TEAMS][NS][kStageTokens];
+  dependents_may_start();   // e.g. the output projection, whose weight loads need nothing from here
+  wait_for_predecessor();   // routes, positions, the appended row
+  const CacheView& cv = a.cv;
+  const int D = cv.D, G = a.Hq / cv.Hkv;
+  const int rowg = blockIdx.z, row = rowg / cv.Hkv, g = rowg - row * cv.Hkv;
+  const int k = blockIdx.x, part = blockIdx.y;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int team = warp >> 2, wt = warp & 3, ltid = tid & 127;  // team, warp in the team, thread in the team
+  long long (*s_rowbase)[kStageTokens] = s_rowbase_all[team];
+  uint8_t* const t_pipe = s_pipe + (size_t)team * NS * STAGE_BYTES;
+  auto team_sync = [&]() {
+    if (TEAMS == 1) __syncthreads();
+    else asm volatile("bar.sync %0, 128;" ::"r"(team + 1) : "memory");
+  };
+  const int qr = lane >> 2, qc = lane & 3;  // fragment row within 8 and column pair
+  const int sid = a.ids[row], pos = a.positions[row];
+  const int visible = min(pos + 1, cv.lengths[sid]);  // tokens [0, visible) exist and are not in the future
+  const int cur = pos / cv.C;
+  const bool dense = a.selected == nullptr;
+  // the union entry of this CTA is read together with the count (k < umax always), not after the test on the count
+  const int listed = dense ? 0 : a.u_chunk[(long long)rowg * a.umax + k];
+  const unsigned listed_mask = dense ? 0u : a.u_mask[(long long)rowg * a.umax + k];
+  const int ucount = dense ? cur + 1 : a.u_count[rowg];
+  if (k >= ucount) return;
+  const int chunk = dense ? k : listed;
+  const unsigned mask = dense ? (G >= 32 ? 0xFFFFFFFFu : ((1u << G) - 1u)) : listed_mask;
+  const int limit = min((chunk + 1) * cv.C, visible);
+  const int t_begin = chunk * cv.C + part * a.part_tokens;
+  const int t_end = min(t_begin + a.part_tokens, limit);
+  if (t_begin >= t_end) return;
+  const int cur_parts = (visible - cur * cv.C + a.part_tokens - 1) / a.part_tokens;
+  const int expected = (ucount - 1) * a.parts + cur_parts;
+  const int all_tiles = (t_end - t_begin + kStageTokens - 1) / kStageTokens;
+  const int first_tile = team * ((all_tiles + TEAMS - 1) / TEAMS);           // this team's stages: [first_tile, first_tile + ntiles)
+  const int ntiles = max(0, min(all_tiles - first_tile, (all_tiles + TEAMS - 1) / TEAMS));
+  const int tt_begin = t_begin + first_tile * kStageTokens;                  // first token of the team
+
+  for (int hb = 0; hb < G; hb += kHeadBlock) {
+    const unsigned active = (mask >> hb) & 0xFFFFu;
+    if (!active) continue;
+    // row bases of the tokens of the stages about to be copied (ring of NS slots).  A thread looks up one token
+    // of every stage; from stage to stage the token advances by kStageTokens, so page and offset are stepped
+    // instead of divided anew.
+    int look_t = tt_begin + ltid, look_pg = 0, look_r = 0, step_pg = 0, step_r = 0;
+    bool look_bad = false;
+    if (ltid < kStageTokens) {
+      look_pg = look_t / cv.page; look_r = look_t - look_pg * cv.page;
+      step_pg = kStageTokens / cv.page; step_r = kStageTokens - step_pg * cv.page;
+    }
+    auto lookup = [&]() {
+      const long long base = attend_row_base(cv, sid, g, look_pg, look_r, look_t < t_end, look_bad);
+      look_t += kStageTokens; look_pg += step_pg; look_r += step_r;
+      if (look_r >= cv.page) { look_r -= cv.page; ++look_pg; }
+      return base;
+    };
+    long long first_base[NS];  // issued before the query loads below, stored after them
+    if (ltid < kStageTokens) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) first_base[s] = lookup();
+    }
+    // Q fragments (A operand): rows qr and qr+8 of the head block, all k-steps
+    uint32_t qf[KSTEPS][4];
+    {
+      const bool r0 = hb + qr < G && ((active >> qr) & 1u), r1 = hb + qr + 8 < G && ((active >> (qr + 8)) & 1u);
+      const __nv_bfloat16* q0 = a.q + ((long long)row * a.Hq + g * G + hb + qr) * D;
+      const __nv_bfloat16* q1 = q0 + 8 * D;
+#pragma unroll
+      for (int ks = 0; ks < KSTEPS; ++ks) {
+        const int c0 = ks * 16 + qc * 2, c1 = c0 + 8;
+        qf[ks][0] = (r0 && c0 < D) ? *reinterpret_cast<const uint32_t*>(q0 + c0) : 0u;
+        qf[ks][1] = (r1 && c0 < D) ? *reinterpret_cast<const uint32_t*>(q1 + c0) : 0u;
+        qf[ks][2] = (r0 && c1 < D) ? *reinterpret_cast<const uint32_t*>(q0 + c1) : 0u;
+        qf[ks][3] = (r1 && c1 < D) ? *reinterpret_cast<const uint32_t*>(q1 + c1) : 0u;
+      }
+    }
+    float o[DT][4];
+#pragma unroll
+    for (int dt = 0; dt < DT; ++dt) { o[dt][0] = o[dt][1] = o[dt][2] = o[dt][3] = 0.f; }
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;  // rows qr and qr+8; l: this thread's columns only
+
+    __syncthreads();  // the previous head block is done with shared memory
+    if (ltid < kStageTokens) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) s_rowbase[s][ltid] = first_base[s];
+    }
+    team_sync();
+#pragma unroll
+    for (int s = 0; s < NS - 1; ++s) {
+      if (s < ntiles) attend_load_stage<DP>(cv, t_pipe + s * STAGE_BYTES, s_rowbase[s], ltid);
+      cp_async_commit();
+    }
+    for (int i = 0; i < ntiles; ++i) {
+      cp_async_wait<NS - 2>();
+      team_sync();  // tile i has landed; every warp of the team finished tile i-1, whose buffer is refilled next
+      const int nx = i + NS - 1;
+      if (nx < ntiles) attend_load_stage<DP>(cv, t_pipe + (nx % NS) * STAGE_BYTES, s_rowbase[nx % NS], ltid);
+      cp_async_commit();
+      // look up the rows of tile nx+1 now, publish them after this tile's math (slot i % NS is free)
+      long long next_base = -1;
+      if (ltid < kStageTokens && nx + 1 < ntiles) next_base = lookup();
+      const int tok0 = wt * 16;                                   // this warp's tokens inside the stage
+      const int nvalid = t_end - (tt_begin + i * kStageTokens + tok0);  // tokens of the warp tile that exist
+      if (nvalid <= 0) {                                          // warp-uniform
+        if (ltid < kStageTokens) s_rowbase[i % NS][ltid] = next_base;
+        continue;
+      }
+      const uint32_t kbase = smem_u32(t_pipe + (i % NS) * STAGE_BYTES);
+      const uint32_t vbase = kbase + kStageTokens * DP * 2;
+      // ---- S = Q K^T for 16 tokens: two 8-token column tiles
+      float sc[2][4];
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) { sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f; }
+#pragma unroll
+      for (int ks = 0; ks < KSTEPS; ++ks) {
+        uint32_t b[4];
+        const int mat = lane >> 3, r = lane & 7;
+        ldmatrix_x4(kbase + kv_unit_offset<DP>(tok0 + (mat >> 1) * 8 + r, ks * 2 + (mat & 1)), b);
+        mma_16816<F16>(sc[0], qf[ks], b[0], b[1]);
+        mma_16816<F16>(sc[1], qf[ks], b[2], b[3]);
+      }
+      // ---- online softmax of rows qr / qr+8 (exp2 domain)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int col = nt * 8 + qc * 2 + (e & 1);
+          sc[nt][e] = col < nvalid ? sc[nt][e] * a.scale_log2 : -INFINITY;
+        }
+      }
+      float mx0 = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
+      float mx1 = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 1));
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 2));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 1));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 2));
+      const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);  // finite: column 0 of the warp tile always exists
+      const float al0 = dec_exp2(m0 - n0), al1 = dec_exp2(m1 - n1);
+      m0 = n0; m1 = n1;
+      uint32_t pf[4];
+      {
+        const float p00 = dec_exp2(sc[0][0] - n0), p01 = dec_exp2(sc[0][1] - n0), p02 = dec_exp2(sc[0][2] - n1), p03 = dec_exp2(sc[0][3] - n1);
+        const float p10 = dec_exp2(sc[1][0] - n0), p11 = dec_exp2(sc[1][1] - n0), p12 = dec_exp2(sc[1][2] - n1), p13 = dec_exp2(sc[1][3] - n1);
+        l0 = l0 * al0 + (p00 + p01) + (p10 + p11);
+        l1 = l1 * al1 + (p02 + p03) + (p12 + p13);
+        pf[0] = pack16<F16>(p00, p01); pf[1] = pack16<F16>(p02, p03);
+        pf[2] = pack16<F16>(p10, p11); pf[3] = pack16<F16>(p12, p13);
+      }
+      // ---- O = O * alpha + P V; the running maxima rarely move after the first tiles, and alpha == 1 needs no pass over O
+      const bool rescale = __any_sync(0xFFFFFFFFu, al0 != 1.f || al1 != 1.f);
+#pragma unroll
+      for (int dp = 0; dp < DT / 2; ++dp) {
+        uint32_t b[4];
+        const int mat = lane >> 3, r = lane & 7;
+        ldmatrix_x4_trans(vbase + kv_unit_offset<DP>(tok0 + (mat & 1) * 8 + r, dp * 2 + (mat >> 1)), b);
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2) {
+          float (&acc)[4] = o[dp * 2 + h2];
+          if (rescale) { acc[0] *= al0; acc[1] *= al0; acc[2] *= al1; acc[3] *= al1; }
+          mma_16816<F16>(acc, pf, b[h2 * 2], b[h2 * 2 + 1]);
+        }
+      }
+      if (ltid < kStageTokens) s_rowbase[i % NS][ltid] = next_base;
+    }
+    if (look_bad) atomicOr(a.status, kErrBadIndex);
+    // ---- combine the warps, then write one partial per active head
+    cp_async_wait<0>();
+    l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 1); l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 2);
+    l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 1); l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 2);
+    __syncthreads();
+    float* s_o = reinterpret_cast<float*>(s_pipe);                   // [NW warps][16 rows][DP]
+    float* s_ml = s_o + NW * 16 * DP;                                 // [NW warps][16 rows][2]
+#pragma unroll
+    for (int dt = 0; dt < DT; ++dt) {
+      float* w0 = s_o + ((size_t)warp * 16 + qr) * DP + dt * 8 + qc * 2;
+      float* w1 = w0 + 8 * DP;
+      w0[0] = o[dt][0]; w0[1] = o[dt][1]; w1[0] = o[dt][2]; w1[1] = o[dt][3];
+    }
+    if (qc == 0) {
+      s_ml[((size_t)warp * 16 + qr) * 2] = m0; s_ml[((size_t)warp * 16 + qr) * 2 + 1] = l0;
+      s_ml[((size_t)warp * 16 + qr + 8) * 2] = m1; s_ml[((size_t)warp * 16 + qr + 8) * 2 + 1] = l1;
+    }
+    // slot of this chunk in each head's route (all candidate slots are read before any is compared)
+    const int nh = min(kHeadBlock, G - hb);
+    if (tid < kHeadBlock) {
+      int slot = -1;
+      if (tid < nh && ((active >> tid) & 1u)) {
+        if (dense) {
+          slot = chunk;
+        } else {
+          const int* sel = a.selected + ((long long)row * a.Hq + g * G + hb + tid) * a.ns;
+#pragma unroll 4
+          for (int s2 = a.ns - 1; s2 >= 0; --s2)
+            if (__ldcg(sel + s2) == chunk) slot = s2;
+        }
+      }
+      s_slot[tid] = slot;
+    }
+    __syncthreads();
+    // every thread takes two dimensions of one head
+    const int d2n = D >> 1;
+    for (int item = tid; item < nh * d2n; item += NT) {
+      const int hh = item / d2n, d = (item - hh * d2n) * 2;
+      const int slot = s_slot[hh];
+      if (slot < 0) continue;
+      const int h = g * G + hb + hh;
+      const long long pidx = (((long long)row * a.Hq + h) * a.ns + slot) * a.parts + part;
+      float mw[NW], big = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) { mw[w] = s_ml[((size_t)w * 16 + hh) * 2]; big = fmaxf(big, mw[w]); }
+      float lsum = 0.f, v0 = 0.f, v1 = 0.f;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const float wgt = mw[w] == -INFINITY ? 0.f : dec_exp2(mw[w] - big);  // a warp that saw no token adds nothing
+        lsum += s_ml[((size_t)w * 16 + hh) * 2 + 1] * wgt;
+        const float2 x = *reinterpret_cast<const float2*>(s_o + ((size_t)w * 16 + hh) * DP + d);
+        v0 += x.x * wgt; v1 += x.y * wgt;
+      }
+      *reinterpret_cast<float2*>(a.pacc + pidx * D + d) = make_float2(v0, v1);
+      if (d == 0) { a.pm[pidx] = big; a.pl[pidx] = lsum; }
+    }
+  }
+
+  // ---- ticket: the last CTA of this (query, kv head) merges every partial of the group's heads
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    const int ticket = atomicAdd(&a.counters[rowg], 1);
+    s_last = ticket == expected - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // The partials of a head are (slot, part) pairs, j = slot * parts + part, and lie one after the other.  All
+  // threads first start asynchronous copies of the partial sums into shared memory, as many partials per head as
+  // fit, and read the maxima and denominators of every head's partials, all with accesses that do not depend on
+  // each other: one trip to L2 for the whole merge.  One warp per head then finds the maximum, the weights and the
+  // denominator; finally every thread takes four dimensions of one head and sums over the partials.  What does not
+  // fit in shared memory is read from global memory in the same fixed order, so the result is bit-repeatable.
+  const int nslots = dense ? cur + 1 : a.ns;
+  const int total = nslots * a.parts;
+  const int pipe_floats = TEAMS * NS * STAGE_BYTES / 4;
+  const int cap = min(min(1024, (total + 3) & ~3), (pipe_floats / (2 * G)) & ~3);  // maxima / weights kept per head
+  const int tc = min(total, cap);
+  const int pb = min(tc, (pipe_floats - 2 * G * cap) / (G * D));                   // partial sums kept per head
+  float* s_w = reinterpret_cast<float*>(s_pipe);  // [G][cap] maxima, then weights
+  float* s_l = s_w + G * cap;                       // [G][cap] denominators
+  float* s_acc = s_l + G * cap;                     // [G][pb][D] partial sums
+  __shared__ float s_big[32], s_inv[32];
+  const int d4n = D >> 2;  // the head dimension is a multiple of 8
+  const long long gbase = ((long long)row * a.Hq + g * G) * a.ns;  // first slot of the group's first head
+  for (int hl = 0; hl < G; ++hl) {
+    const float* src = a.pacc + (gbase + (long long)hl * a.ns) * a.parts * D;
+    const uint32_t dst = smem_u32(s_acc + (size_t)hl * pb * D);
+    for (int u = tid; u < pb * d4n; u += NT) cp_async16(dst + u * 16, src + u * 4, true);
+  }
+  cp_async_commit();
+  // This code runs once per launch in one CTA per group, from a cold instruction cache: it is kept short (little
+  // unrolling; the rarely needed paths sit in functions of their own) because fetching it costs more than running it.
+  const MergeTail tail{a.selected, a.pm, a.pl, a.pacc, a.parts, cur, cur_parts, D};
+#pragma unroll 2
+  for (int idx = tid; idx < G * tc; idx += NT) {
+    const int hl = idx / tc, j = idx - hl * tc;
+    const long long hbase = gbase + (long long)hl * a.ns;
+    const float m = __ldcg(a.pm + hbase * a.parts + j), l = __ldcg(a.pl + hbase * a.parts + j);
+    const bool ok = tail.valid(hbase, j);
+    s_w[hl * cap + j] = ok ? m : -INFINITY;
+    s_l[hl * cap + j] = ok ? l : 0.f;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  // half a warp per head
+  const int sub = lane & 15;
+#pragma unroll 1
+  for (int hl = warp * 2 + (lane >> 4); hl < ((G + 2 * NW - 1) / (2 * NW)) * (2 * NW); hl += 2 * NW) {
+    const bool live = hl < G;  // the shuffles below need every lane
+    const int hc = live ? hl : 0;
+    const int h = g * G + hc;
+    const long long hbase = gbase + (long long)hc * a.ns;
+    float big = -INFINITY;
+    if (live) {
+#pragma unroll 1
+      for (int j = sub; j < tc; j += 16) big = fmaxf(big, s_w[hc * cap + j]);
+      if (total > cap) big = merge_tail_max(tail, hbase, cap + sub, total, big);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xFFFFFFFFu, big, o));
+    float lsum = 0.f;
+    if (live) {
+#pragma unroll 1
+      for (int j = sub; j < tc; j += 16) {
+        const float m = s_w[hc * cap + j];
+        const float w = m == -INFINITY ? 0.f : dec_exp2(m - big);
+        s_w[hc * cap + j] = w;
+        lsum = fmaf(s_l[hc * cap + j], w, lsum);
+      }
+      if (total > cap) lsum = merge_tail_den(tail, hbase, cap + sub, total, big, lsum);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xFFFFFFFFu, lsum, o);
+    if (live && sub == 0) {
+      s_big[hc] = big;
+      s_inv[hc] = 1.f / lsum;
+      a.lse[(long long)row * a.Hq + h] = (big + log2f(lsum)) * 0.6931471805599453f;
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int item = tid; item < G * d4n; item += NT) {
+    const int hl = item / d4n, d = (item - hl * d4n) * 4;
+    const int h = g * G + hl;
+    const long long hbase = gbase + (long long)hl * a.ns;
+    const float* wrow = s_w + hl * cap;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4* sacc = reinterpret_cast<const float4*>(s_acc + (size_t)hl * pb * D + d);
+#pragma unroll 4
+    for (int j = 0; j < pb; ++j) merge_add(v, sacc[(size_t)j * d4n], wrow[j]);
+    if (tc > pb) v = merge_rest_acc(tail, hbase, pb, tc, d, wrow, v);
+    if (total > cap) v = merge_tail_acc(tail, hbase, cap, total, d, s_big[hl], v);
+    const float inv = s_inv[hl];
+    uint2 pk;
+    pk.x = pack16<F16>(v.x * inv, v.y * inv);
+    pk.y = pack16<F16>(v.z * inv, v.w * inv);
+    *reinterpret_cast<uint2*>(a.out + ((long long)row * a.Hq + h) * D + d) = pk;
+  }
+  __syncthreads();
+  if (tid == 0) a.counters[rowg] = 0;  // ready for the next launch (graph replay included)
+}
+
 // What a thread holds of the attention of its rows: rows qr and qr + 8 of the head block, l over its own columns only.
 template <int DP>
 struct AttendState {
@@ -1261,14 +1662,24 @@ extern "C" int moba_decode_route(const moba_cache_desc* c, const void* q, const 
   return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;
 }
 
+static int attend_part_tokens(const moba_cache_desc* c) {
+  return c->chunk_size >= 2048 ? 1024 : c->chunk_size >= 512 ? 512 : c->chunk_size;
+}
+static int attend_parts(const moba_cache_desc* c) {
+  const int part_tokens = attend_part_tokens(c);
+  return (c->chunk_size + part_tokens - 1) / part_tokens;
+}
+
 // A share below four stages would be mostly its start and its partials (2, 4, 8 and 16 within 1 % at the sizes above).
 constexpr int kStreamLeast = 4;
-constexpr int kClusterMost = 17;
+constexpr int kClusterMost = 11;
 constexpr int kStreamCtas = 3 * 148;  // streamed variant: what a B200 holds at once (one per SM above head dimension 128)
 
-// Partials of a launch, per head of a group: one for every segment.
-static size_t attend_partials(const moba_cache_desc* c, int rows, int hq) {
-  return ((size_t)kStreamCtas + (size_t)rows * c->hkv) * (hq / c->hkv);
+// Partials of a launch: with fixed parts a slot per (head, list entry, part), streamed one per head of a group and segment.
+static size_t attend_partials(const moba_cache_desc* c, int rows, int hq, int slots) {
+  const size_t fixed = (size_t)rows * hq * slots * attend_parts(c);
+  const size_t streamed = ((size_t)kStreamCtas + (size_t)rows * c->hkv) * (hq / c->hkv);
+  return fixed > streamed ? fixed : streamed;
 }
 static size_t attend_workspace(const moba_cache_desc* c, int rows, int hq, size_t partials) {
   return align256((size_t)rows * c->hkv * 4) + 2 * align256(partials * 4) + align256(partials * c->dim * 4);
@@ -1276,7 +1687,7 @@ static size_t attend_workspace(const moba_cache_desc* c, int rows, int hq, size_
 
 extern "C" size_t moba_decode_attend_workspace_bytes(const moba_cache_desc* c, int rows, int hq, int slots) {
   if (validate_cache(c) != MOBA_OK || rows < 1 || hq < 1 || slots < 1) return 0;
-  return attend_workspace(c, rows, hq, attend_partials(c, rows, hq));
+  return attend_workspace(c, rows, hq, attend_partials(c, rows, hq, slots));
 }
 
 extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const int32_t* ids, const int32_t* positions,
@@ -1295,8 +1706,10 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   a.q = static_cast<const __nv_bfloat16*>(q);
   a.ids = ids; a.positions = positions; a.selected = selected;
   a.u_chunk = u_chunk; a.u_mask = u_mask; a.u_count = u_count;
-  a.Hq = hq; a.umax = umax;
-  const size_t n = attend_partials(c, rows, hq);
+  a.Hq = hq; a.ns = slots; a.umax = selected ? umax : slots;
+  a.parts = attend_parts(c);
+  a.part_tokens = attend_part_tokens(c);
+  const size_t n = attend_partials(c, rows, hq, slots);
   char* p = static_cast<char*>(workspace);
   a.counters = reinterpret_cast<int*>(p); p += align256((size_t)rows * c->hkv * 4);
   a.pm = reinterpret_cast<float*>(p); p += align256(n * 4);
@@ -1313,13 +1726,22 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   a.rowgs = rows * c->hkv;
   a.spc = selected ? (c->chunk_size + kStageTokens - 1) / kStageTokens : 1;
   a.min_stages = kStreamLeast;
-  // Clusters while every pair can have one (16 CTAs for up to four pairs, 8 for up to 16) and a CTA's share, at the cache's
-  // capacity, stays below kClusterMost stages; from there on the whole GPU shares the list.
-  // Steps in us, cluster against streamed: one request, 14/2 heads, D = 64, dense, 1K 10.3 / 16.5, 16K 16.5 / 22.7, 32K 24.7 / 24.8; one
-  // request, 32/8 heads, D = 128, dense, 4K 14.5 / 20.6, 8K 20.6 / 22.7, 16K 30.9 / 27.4.
+  // Which variant, in us of a captured step (cluster / fixed parts / streamed), one request and heads 14/2 at D = 64 unless said:
+  //   clusters while every pair can have one (16 CTAs for up to four pairs, 8 for up to eight) and a CTA's share, at the
+  //   cache's capacity, stays below kClusterMost stages: dense 1K 10.3 / 12.4 / 16.5, 8K 12.4 / 14.4 / 18.6, but 16K 16.5 / 14.5 / 22.7;
+  //   heads 32/8, D = 128, dense 4K 14.5 / 16.5 / 20.6, but 8K 20.6 / 16.5 / 22.7; with 16 pairs 18.5 / 16.5 / 22.7 at 1K already;
+  //   fixed parts while their grid, at capacity, fits the GPU at once: heads 32/8, D = 128, dense 16K (264 CTAs) - / 24.7 / 27.4,
+  //   eight requests, 12/2, D = 128, routed 16K (304 CTAs) - / 29.9 / 36.8; beyond one wave the streamed variant: the first
+  //   at 32K (520 CTAs) - / 49.4 / 41.4, eight requests dense 16K (528 CTAs) - / 52.7 / 44.6.  A routed grid is a bound that
+  //   heads with picks in common and short contexts stay below, so there the line is two waves: 21 requests up to 5.5K, 8/2, D = 128
+  //   (546 CTAs) - / 36.7 / 38.9, 18 requests of 32K, 6/1, D = 32 (774 CTAs) - / 37.9 / 38.9, 42 requests of 53K, 28/4, D = 128
+  //   (1344 CTAs) - / 96.7 / 93.2.
   const long long most = selected ? (long long)umax * a.spc : ((long long)slots * c->chunk_size + kStageTokens - 1) / kStageTokens;
-  const int cl = a.rowgs <= 4 ? 16 : a.rowgs <= 16 ? 8 : 0;
+  const int cl = a.rowgs <= 4 ? 16 : a.rowgs <= 8 ? 8 : 0;
   const bool cluster = cl > 0 && most <= (long long)cl * kClusterMost && (!selected || umax <= kClusterList);
+  const dim3 grid(a.umax, a.parts, rows * c->hkv);
+  const long long ctas = (long long)grid.x * grid.y * grid.z;
+  const bool deep = ctas <= kStreamCtas / 3, fixed = ctas <= (dp <= 128 ? kStreamCtas : kStreamCtas / 3) * (selected ? 2 : 1);
   prof_begin(kProfDecodeAttend, st);
 #define MOBA_LAUNCH_CLUSTER(L, CL)                                                                                       \
   do {                                                                                                                  \
@@ -1332,11 +1754,22 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
     if (e == cudaSuccess)                                                                                               \
       e = launch_dependent_cluster(8u, kernel, dim3(CL, a.rowgs), dim3(128 * cluster_teams(L)), CL, smem, st, a);       \
   } while (0)
+#define MOBA_LAUNCH_FIXED(L, NS, T)                                                                                      \
+  do {                                                                                                                  \
+    constexpr size_t ring = (size_t)(T) * (NS) * 2 * kStageTokens * L * 2, red = (size_t)4 * (T) * 16 * (L + 2) * 4;    \
+    constexpr size_t smem = ring > red ? ring : red;                                                                    \
+    const auto kernel = half ? decode_attend_kernel<L, NS, T, true> : decode_attend_kernel<L, NS, T, false>;            \
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
+    if (e == cudaSuccess) e = launch_dependent(8u, kernel, grid, dim3(128 * (T)), smem, st, a);                         \
+  } while (0)
 #define MOBA_LAUNCH_ATTEND(L)                                                                                            \
   do {                                                                                                                  \
     if (cluster) {                                                                                                      \
       if (cl == 16) MOBA_LAUNCH_CLUSTER(L, 16);                                                                         \
       else MOBA_LAUNCH_CLUSTER(L, 8);                                                                                   \
+    } else if (fixed) {                                                                                                 \
+      if (deep) MOBA_LAUNCH_FIXED(L, deep_stages(L), (L <= 128 ? 2 : 1));                                                \
+      else MOBA_LAUNCH_FIXED(L, kStages, 1);                                                                            \
     } else {                                                                                                            \
       constexpr int NS = stream_stages(L);                                                                              \
       constexpr size_t pipe = (size_t)NS * 2 * kStageTokens * L * 2, red = (size_t)4 * 16 * (L + 2) * 4;                \
@@ -1353,6 +1786,7 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   else MOBA_LAUNCH_ATTEND(256);
 #undef MOBA_LAUNCH_ATTEND
 #undef MOBA_LAUNCH_CLUSTER
+#undef MOBA_LAUNCH_FIXED
   prof_end(kProfDecodeAttend, st);
   if (e != cudaSuccess) return MOBA_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;

@@ -420,6 +420,7 @@ def test_one_finite_check_for_all_inputs(dtype, layout):
     cache._finite.require(named)
 
 
+@pytest.mark.parametrize("repeat", [1, 8])      # a grid of fixed parts that fits the GPU at once, one that does not
 @pytest.mark.parametrize("mode", ["moba", "dense"])
 @pytest.mark.parametrize("hq,hkv,dim,chunk,page,dtype", [
     (4, 2, 64, 100, 7, torch.bfloat16),      # the last stage of a chunk is part of one
@@ -428,8 +429,8 @@ def test_one_finite_check_for_all_inputs(dtype, layout):
     (5, 5, 128, 192, 16, torch.float16),
     (2, 1, 256, 70, 3, torch.bfloat16),      # one CTA per SM
 ])
-def test_streamed_attend_divides_uneven_work(mode, hq, hkv, dim, chunk, page, dtype):
-    """Grids above one CTA per SM take shares of one list of stages: contexts from one token to many chunks, shares that
+def test_attend_divides_uneven_work(repeat, mode, hq, hkv, dim, chunk, page, dtype):
+    """Fixed parts, or, streamed, equal shares of one list of stages: contexts from one token to many chunks, shares that
     begin and end inside a chunk, several requests in a share and several shares in a request, repeatable bits."""
     from moba_opt import PagedKVCache
     lens = [1, 63, 64, 65, 900, 2, chunk, chunk + 1, 700, 1, 333, 1024, 5, 640, 129, 77, 2 * chunk, 511]
@@ -437,8 +438,8 @@ def test_streamed_attend_divides_uneven_work(mode, hq, hkv, dim, chunk, page, dt
     cu = np.concatenate(([0], np.cumsum(lens))).tolist()
     k, v = rand((cu[-1], hkv, dim), 71, dtype), rand((cu[-1], hkv, dim), 72, dtype)
     cache.append_prefill(k, v, sequence_ids=list(range(len(lens))), cu_seqlens=cu)
-    ids = list(range(len(lens))) + [4, 11, 11, 8]                      # several queries of a request, some not at its end
-    positions = [n - 1 for n in lens] + [450, 1000, 63, 0]
+    ids = (list(range(len(lens))) + [4, 11, 11, 8]) * repeat           # several queries of a request, some not at its end
+    positions = ([n - 1 for n in lens] + [450, 1000, 63, 0]) * repeat
     q = rand((len(ids), hq, dim), 73, dtype)
     result = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
     check(cache, result, q)
@@ -451,8 +452,8 @@ def test_streamed_attend_divides_uneven_work(mode, hq, hkv, dim, chunk, page, dt
     ((1,), 4, 1, 64, 100, 7, torch.bfloat16),             # fewer stages than CTAs in the cluster
     ((1000,), 14, 2, 64, 100, 16, torch.bfloat16),        # the last stage of a chunk is part of one
     ((63, 64, 65), 32, 1, 32, 64, 16, torch.float16),     # two head blocks, a stage is a chunk
-    ((640, 5, 129, 333), 6, 3, 96, 130, 48, torch.bfloat16),   # twelve pairs: clusters of eight
-    ((511, 700), 5, 5, 128, 192, 16, torch.float16),
+    ((640, 5, 129), 6, 2, 96, 130, 48, torch.bfloat16),   # six pairs: clusters of eight
+    ((511, 700), 4, 4, 128, 192, 16, torch.float16),
     ((900, 71), 2, 1, 256, 70, 3, torch.bfloat16),        # one team per CTA
 ])
 def test_cluster_attend_divides_a_request(lens, mode, hq, hkv, dim, chunk, page, dtype):
