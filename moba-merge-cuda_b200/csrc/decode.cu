@@ -1362,7 +1362,10 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
 // partly empty, and the merge of a long context had a partial per chunk.  Here the stages (64 tokens) of every (row, kv head) pair - of its
 // union of chunks, or of its whole context in dense mode - laid end to end are one list, and each of the CTAs that fit the
 // GPU at once takes an equal, consecutive share of it.  Eight requests of 16K-32K tokens, dense, 28/4 heads, D = 128:
-// 98.7 -> 78 us (4.1 -> 5.1 TB/s), step 111 -> 88 us; 64 requests of 4K-64K, routed, 12/2 heads, D = 128: step 264 -> 239 us.
+// 98.7 -> 80 us (4.1 -> 5.0 TB/s), step 111 -> 96 us; 64 requests of 4K-64K, routed, 12/2 heads, D = 128: step 265 -> 251 us.
+// (The first form of the kernel measured 78 us and steps of 94 and 243 us; sharing its loop with the cluster variant cost the rest.
+// The merge through the copy ring, a batch of partials at a time, was slower than reading them where they lie: one request of 32K,
+// 14/2 heads, dense, 39 against 25 us.)
 // A share may begin and end anywhere; what a CTA holds of one pair is a segment, with one partial per head in slot
 // (CTA + pair), which no other segment has, and the slots of a pair are consecutive.  The division depends on the
 // positions alone, so a result is bit-repeatable.
