@@ -14,6 +14,7 @@
 // two "lanes" that share one stream of K/V tiles and are served by specialised warps:
 //   warps 0-3   softmax of lane 0 (a thread owns a query row)      warp 8   issues every tcgen05.mma
 //   warps 4-7   softmax of lane 1                                   warp 9   issues the bulk copies
+//                                                                   warp 10  decodes the work items ahead of the others
 // Per key tile and lane: S = Q K^T (accumulator in TMEM) -> the row is read with tcgen05.ld, masked,
 // exponentiated in the exp2 domain against a running maximum that is only raised when it grew by more
 // than 2^8 (the rescale of O in TMEM is then done by the row's own thread), P is written back into
