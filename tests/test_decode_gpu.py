@@ -493,3 +493,35 @@ def test_append_reads_strided_views(layout):
         closed = caches[0].lengths[sid] // 64
         assert torch.equal(caches[0]._means[sid, :closed], caches[1]._means[sid, :closed])
     assert_payload(caches[0], 0, k[:130], v[:130])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("requests,queries,hq,hkv,dim,length,mode", [
+    (12, 1, 16, 4, 128, 6100, "dense"),      # streamed: 576 parts of 512 tokens do not fit the GPU at once
+    (12, 3, 16, 4, 64, 6100, "moba"),        # streamed: 36 rows x 4 heads, up to 12 of 12 chunks in a union
+    (1, 1, 14, 2, 64, 6100, "dense"),        # a cluster per pair
+    (2, 1, 8, 4, 128, 2900, "dense"),
+    (1, 2, 14, 2, 64, 6100, "moba"),
+])
+def test_probabilities_keep_more_than_16_bits(requests, queries, hq, hkv, dim, length, mode, dtype):
+    """Where a warp's run of tokens is longer than a fixed part, P is multiplied in two 16-bit pieces.  Each p is then off by at
+    most 2^-16 (2^-22) of itself and the sums by FP32 rounding, against 2^-9 (2^-12) for the rounding of the output: what
+    is left is the error of the oracle's own result rounded once, within 2 % (5 % in half precision, where the FP32
+    parts - scores of magnitude up to 6 off by 2^-21, exp2 by 2^-22 - are closer to it).  With P rounded once it is 20 to 30 % more."""
+    from moba_opt import PagedKVCache
+    cache = PagedKVCache(requests, length, hkv, dim, page_size=48, chunk_size=512, dtype=dtype)
+    lens = [length - 37 * i for i in range(requests)]
+    cu = np.concatenate(([0], np.cumsum(lens))).tolist()
+    k, v = rand((cu[-1], hkv, dim), 301, dtype), rand((cu[-1], hkv, dim), 302, dtype)
+    cache.append_prefill(k, v, sequence_ids=list(range(requests)), cu_seqlens=cu)
+    ids = [i for i in range(requests) for _ in range(queries)]
+    positions = [lens[i] - 1 - 500 * j for i in range(requests) for j in range(queries)]
+    q = rand((len(ids), hq, dim), 303, dtype)
+    result = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
+    check(cache, result, q)
+    keys, values = zip(*[[torch_to_f64(t) for t in cache.materialize(i)] for i in range(requests)])
+    sel = None if result.selected_blocks is None else result.selected_blocks.cpu().numpy()
+    want, _ = mo.decode_attend(torch_to_f64(q), keys, values, ids, positions, 512, sel)
+    rounded = torch_to_f64(torch.from_numpy(want).to(dtype))
+    error, least = np.linalg.norm(torch_to_f64(result.output) - want), np.linalg.norm(rounded - want)
+    assert error <= (1.02 if dtype == torch.bfloat16 else 1.05) * least, f"{error / least:.4f}"
