@@ -1068,7 +1068,9 @@ __global__ void __launch_bounds__(128 * TEAMS, (TEAMS == 1 && DP <= 128 ? 3 : 1)
   if (tid == 0) a.counters[rowg] = 0;  // ready for the next launch (graph replay included)
 }
 
-// What a thread holds of the attention of its rows: rows qr and qr + 8 of the head block, l over its own columns only.
+// What a thread holds of the attention of its rows, l over its own columns only.  WIDE (groups of more than eight heads): rows qr and
+// qr + 8 of the head block are two heads.  Otherwise row qr is a head and row qr + 8 the same one again, for the second
+// part of its P; o[.][2] and o[.][3] are to be added to o[.][0] and o[.][1].
 template <int DP>
 struct AttendState {
   float o[DP / 8][4];
@@ -1079,9 +1081,11 @@ struct AttendState {
 // not enough here: the error of a row is that of its largest probabilities, a token that raises the running maximum has p = 1
 // without any, and the longer a warp's run of tokens the fewer of those there are.  Against 64 bits the outputs of long dense
 // contexts were up to 1.13 times as far off as with fixed parts, which start a maximum anew every 512 tokens; with both
-// values what is left is the rounding of the output (2.1e-3 -> 1.7e-3 relative in bf16).  It costs 1 to 2 % of a step (streamed,
-// 64 requests: 245 -> 249 us).  `main` is taken a little below
-// p, so that `rest` is not zero where p is a 16-bit value: an infinite V then stays infinite instead of becoming 0 x Inf.
+// values what is left is the rounding of the output (2.1e-3 -> 1.7e-3 relative in bf16).  Groups of up to eight heads leave
+// half of the rows of a product unused, and the second values go there, at no cost; wider groups take a second product (for
+// groups of six that cost 4 % of a step: 64 requests 251 -> 260 us).  `main` is taken a
+// little below p, so that `rest` is not zero where p is a 16-bit value: an infinite V then stays infinite instead of becoming
+// 0 x Inf.
 template <bool F16>
 __device__ __forceinline__ void split_p(float p0, float p1, uint32_t& main, uint32_t& rest) {
   constexpr float below = F16 ? 1.f - 0x1p-11f : 1.f - 0x1p-8f;
@@ -1090,12 +1094,28 @@ __device__ __forceinline__ void split_p(float p0, float p1, uint32_t& main, uint
   rest = pack16<F16>(p0 - m.x, p1 - m.y);
 }
 
+// Online softmax of one row of two 8-token score tiles (exp2 domain): raises the row's running maximum, rescales and extends its
+// sum, and leaves the factor for O and the four probabilities.
+__device__ __forceinline__ void attend_softmax(const float (&s)[4], float& m, float& l, float& alpha, float (&p)[4]) {
+  float mx = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+  mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+  const float n = fmaxf(m, mx);
+  // a head that has attended nothing so far keeps -inf; its exponentials are taken against 0 and are 0
+  const float base = n == -INFINITY ? 0.f : n;
+  alpha = m == n ? 1.f : dec_exp2(m - base);
+  m = n;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) p[i] = dec_exp2(s[i] - base);
+  l = l * alpha + (p[0] + p[1]) + (p[2] + p[3]);
+}
+
 // Paged attention of one head block over `ntiles` consecutive stages, by a team of four warps.  The query heads of
 // the GQA group are the 16 rows of m16n8k16 tensor-core tiles (unused rows are zero), so a K/V token read from HBM
 // serves every head at no extra cost.  Each warp takes 16 tokens of every stage and keeps its own running (max, sum, O).
 //   ring      NS stages            rowbase [NS][64]   nv, mask [2 NS]: a slot is rewritten NS stages ahead, while the slots
 //                                                     before it are still read
-template <int DP, int NS, bool F16, class Sync>
+template <int DP, int NS, bool F16, bool WIDE, class Sync>
 __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& look, int ntiles, int sid, int row, int g, int hb, int ltid,
                                               uint8_t* ring, long long (*s_rowbase)[kStageTokens], int* s_nv, unsigned* s_mask,
                                               Sync team_sync, AttendState<DP>& st) {
@@ -1118,7 +1138,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
   }
   uint32_t qf[KSTEPS][4];  // A operand: rows qr and qr + 8, all k-steps
   {
-    const bool r0 = hb + qr < G, r1 = hb + qr + 8 < G;
+    const bool r0 = hb + qr < G, r1 = WIDE && hb + qr + 8 < G;
     const __nv_bfloat16* q0 = a.q + ((long long)row * a.Hq + g * G + hb + qr) * D;
     const __nv_bfloat16* q1 = q0 + 8 * D;
 #pragma unroll
@@ -1162,7 +1182,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
     const int nvalid = s_nv[i % META] - tok0;
     const unsigned heads = s_mask[i % META] >> hb;
     if (nvalid > 0 && (heads & 0xFFFFu)) {  // warp-uniform
-      const bool on0 = (heads >> qr) & 1u, on1 = (heads >> (qr + 8)) & 1u;
+      const bool on0 = (heads >> qr) & 1u, on1 = WIDE ? (heads >> (qr + 8)) & 1u : on0;
       const uint32_t kbase = smem_u32(ring + (i % NS) * STAGE_BYTES);
       const uint32_t vbase = kbase + kStageTokens * DP * 2;
       // ---- S = Q K^T for 16 tokens: two 8-token column tiles
@@ -1177,34 +1197,23 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
         mma_16816<F16>(sc[0], qf[ks], b[0], b[1]);
         mma_16816<F16>(sc[1], qf[ks], b[2], b[3]);
       }
-      // ---- online softmax of rows qr / qr+8 (exp2 domain)
+      // ---- softmax; tokens that do not exist and heads that are off have P = 0
+      float s0[4], s1[4], p0[4], p1[4], al0, al1;
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int col = nt * 8 + qc * 2 + (e & 1);
-          sc[nt][e] = col < nvalid && (e < 2 ? on0 : on1) ? sc[nt][e] * a.scale_log2 : -INFINITY;
-        }
+      for (int e = 0; e < 4; ++e) {
+        const bool col = (e >> 1) * 8 + qc * 2 + (e & 1) < nvalid;
+        s0[e] = col && on0 ? sc[e >> 1][e & 1] * a.scale_log2 : -INFINITY;
+        s1[e] = col && on1 ? sc[e >> 1][2 + (e & 1)] * a.scale_log2 : -INFINITY;
       }
-      float mx0 = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
-      float mx1 = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 1));
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 2));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 1));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 2));
-      const float n0 = fmaxf(st.m0, mx0), n1 = fmaxf(st.m1, mx1);
-      // a head that has attended nothing so far keeps -inf; its exponentials are taken against 0 and are 0
-      const float b0 = n0 == -INFINITY ? 0.f : n0, b1 = n1 == -INFINITY ? 0.f : n1;
-      const float al0 = st.m0 == n0 ? 1.f : dec_exp2(st.m0 - b0), al1 = st.m1 == n1 ? 1.f : dec_exp2(st.m1 - b1);
-      st.m0 = n0; st.m1 = n1;
-      uint32_t pf[4], pr[4];  // P and what its rounding left, see split_p
-      {
-        const float p00 = dec_exp2(sc[0][0] - b0), p01 = dec_exp2(sc[0][1] - b0), p02 = dec_exp2(sc[0][2] - b1), p03 = dec_exp2(sc[0][3] - b1);
-        const float p10 = dec_exp2(sc[1][0] - b0), p11 = dec_exp2(sc[1][1] - b0), p12 = dec_exp2(sc[1][2] - b1), p13 = dec_exp2(sc[1][3] - b1);
-        st.l0 = st.l0 * al0 + (p00 + p01) + (p10 + p11);
-        st.l1 = st.l1 * al1 + (p02 + p03) + (p12 + p13);
-        split_p<F16>(p00, p01, pf[0], pr[0]); split_p<F16>(p02, p03, pf[1], pr[1]);
-        split_p<F16>(p10, p11, pf[2], pr[2]); split_p<F16>(p12, p13, pf[3], pr[3]);
+      uint32_t pf[4], pr[4];  // A operand: P, and WIDE what its rounding left
+      attend_softmax(s0, st.m0, st.l0, al0, p0);
+      if (WIDE) {
+        attend_softmax(s1, st.m1, st.l1, al1, p1);
+        split_p<F16>(p0[0], p0[1], pf[0], pr[0]); split_p<F16>(p1[0], p1[1], pf[1], pr[1]);
+        split_p<F16>(p0[2], p0[3], pf[2], pr[2]); split_p<F16>(p1[2], p1[3], pf[3], pr[3]);
+      } else {
+        al1 = al0;
+        split_p<F16>(p0[0], p0[1], pf[0], pf[1]); split_p<F16>(p0[2], p0[3], pf[2], pf[3]);
       }
       // ---- O = O * alpha + P V; the running maxima rarely move after the first tiles, and alpha == 1 needs no pass over O
       const bool rescale = __any_sync(0xFFFFFFFFu, al0 != 1.f || al1 != 1.f);
@@ -1218,7 +1227,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
           float (&acc)[4] = st.o[dp * 2 + h2];
           if (rescale) { acc[0] *= al0; acc[1] *= al0; acc[2] *= al1; acc[3] *= al1; }
           mma_16816<F16>(acc, pf, b[h2 * 2], b[h2 * 2 + 1]);
-          mma_16816<F16>(acc, pr, b[h2 * 2], b[h2 * 2 + 1]);
+          if (WIDE) mma_16816<F16>(acc, pr, b[h2 * 2], b[h2 * 2 + 1]);
         }
       }
     }
@@ -1231,25 +1240,33 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
   cp_async_wait<0>();
 }
 
-// Combines the NW warps of a CTA through shared memory (s_o: NW * 16 * (DP + 2) floats) and hands every pair of
-// dimensions of every head of the block to sink(head in block, dimension, max, sum, v0, v1); heads nobody attended
-// come with -inf, 0 and zeros.
-template <int DP, int NW, class Sink>
-__device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, int nh, int D, Sink sink) {
+// Where the sums of a head block go: head h of it to m[h], l[h] and o[h * D ...]; -inf, 0 and zeros for a head nobody attended.
+struct AttendSums { float *m, *l, *o; };
+
+// Combines the NW warps of a CTA through shared memory (s_o: NW * 16 * (DP + 2) floats).
+template <int DP, int NW, bool WIDE>
+__device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, int nh, int D, const AttendSums& to) {
+  constexpr int ROWS = WIDE ? 16 : 8;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, qr = lane >> 2, qc = lane & 3;
   st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 1); st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 2);
-  st.l1 += __shfl_xor_sync(0xFFFFFFFFu, st.l1, 1); st.l1 += __shfl_xor_sync(0xFFFFFFFFu, st.l1, 2);
+  if (WIDE) { st.l1 += __shfl_xor_sync(0xFFFFFFFFu, st.l1, 1); st.l1 += __shfl_xor_sync(0xFFFFFFFFu, st.l1, 2); }
   __syncthreads();
-  float* s_ml = s_o + NW * 16 * DP;  // [NW warps][16 rows][2]
+  float* s_ml = s_o + NW * ROWS * DP;  // [NW warps][ROWS][2]
 #pragma unroll
   for (int dt = 0; dt < DP / 8; ++dt) {
-    float* w0 = s_o + ((size_t)warp * 16 + qr) * DP + dt * 8 + qc * 2;
-    float* w1 = w0 + 8 * DP;
-    w0[0] = st.o[dt][0]; w0[1] = st.o[dt][1]; w1[0] = st.o[dt][2]; w1[1] = st.o[dt][3];
+    const float (&acc)[4] = st.o[dt];
+    float* w0 = s_o + ((size_t)warp * ROWS + qr) * DP + dt * 8 + qc * 2;
+    if (WIDE) {
+      float* w1 = w0 + 8 * DP;
+      w0[0] = acc[0]; w0[1] = acc[1]; w1[0] = acc[2]; w1[1] = acc[3];
+    } else {
+      w0[0] = acc[0] + acc[2]; w0[1] = acc[1] + acc[3];
+    }
   }
   if (qc == 0) {
-    s_ml[((size_t)warp * 16 + qr) * 2] = st.m0; s_ml[((size_t)warp * 16 + qr) * 2 + 1] = st.l0;
-    s_ml[((size_t)warp * 16 + qr + 8) * 2] = st.m1; s_ml[((size_t)warp * 16 + qr + 8) * 2 + 1] = st.l1;
+    float* ml = s_ml + ((size_t)warp * ROWS + qr) * 2;
+    ml[0] = st.m0; ml[1] = st.l0;
+    if (WIDE) { ml[16] = st.m1; ml[17] = st.l1; }
   }
   __syncthreads();
   const int d2n = D >> 1;
@@ -1257,16 +1274,17 @@ __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, 
     const int hh = item / d2n, d = (item - hh * d2n) * 2;
     float mw[NW], big = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) { mw[w] = s_ml[((size_t)w * 16 + hh) * 2]; big = fmaxf(big, mw[w]); }
+    for (int w = 0; w < NW; ++w) { mw[w] = s_ml[((size_t)w * ROWS + hh) * 2]; big = fmaxf(big, mw[w]); }
     float lsum = 0.f, v0 = 0.f, v1 = 0.f;
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
       const float wgt = mw[w] == -INFINITY ? 0.f : dec_exp2(mw[w] - big);  // a warp that saw no token of the head adds nothing
-      lsum += s_ml[((size_t)w * 16 + hh) * 2 + 1] * wgt;
-      const float2 x = *reinterpret_cast<const float2*>(s_o + ((size_t)w * 16 + hh) * DP + d);
+      lsum += s_ml[((size_t)w * ROWS + hh) * 2 + 1] * wgt;
+      const float2 x = *reinterpret_cast<const float2*>(s_o + ((size_t)w * ROWS + hh) * DP + d);
       v0 += x.x * wgt; v1 += x.y * wgt;
     }
-    sink(hh, d, big, lsum, v0, v1);
+    *reinterpret_cast<float2*>(to.o + (size_t)hh * D + d) = make_float2(v0, v1);
+    if (d == 0) { to.m[hh] = big; to.l[hh] = lsum; }
   }
 }
 
@@ -1279,7 +1297,7 @@ __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, 
 // request of 4096 tokens, 14/2 heads, D = 64: step 18.6 us streamed, 11.5 us this way (dense); layers of a 2000-token
 // session 10 -> 6 us.
 // grid (CL, pairs), cluster (CL, 1, 1)
-template <int DP, int CL, bool F16>
+template <int DP, int CL, bool WIDE, bool F16>
 __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_cluster_kernel(AttendArgs a) {
   constexpr int NS = cluster_stages(DP), TEAMS = cluster_teams(DP), NT = 128 * TEAMS, NW = 4 * TEAMS;
   constexpr int STAGE_BYTES = 2 * kStageTokens * DP * 2;
@@ -1328,13 +1346,10 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
   AttendState<DP> st;
   for (int hb = 0; hb < G; hb += kHeadBlock) {
     look.start(first);
-    attend_stages<DP, NS, F16>(a, look, ntiles, sid, row, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
-                               s_nv[team], s_mask[team], team_sync, st);
-    attend_combine<DP, NW>(st, reinterpret_cast<float*>(s_pipe), min(kHeadBlock, G - hb), D,
-                           [&](int hh, int d, float big, float lsum, float v0, float v1) {
-                             *reinterpret_cast<float2*>(s_sum + (size_t)(hb + hh) * D + d) = make_float2(v0, v1);
-                             if (d == 0) { s_m[hb + hh] = big; s_l[hb + hh] = lsum; }
-                           });
+    attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
+                                     s_nv[team], s_mask[team], team_sync, st);
+    attend_combine<DP, NW, WIDE>(st, reinterpret_cast<float*>(s_pipe), min(kHeadBlock, G - hb), D,
+                                 AttendSums{s_m + hb, s_l + hb, s_sum + (size_t)hb * D});
   }
   // CL neighbouring lanes, one per CTA of the cluster, take four dimensions of a head; the items are divided over the CTAs
   cluster_barrier();
@@ -1399,7 +1414,7 @@ struct StreamShare {
   }
 };
 
-template <int DP, int NS, bool F16>
+template <int DP, int NS, bool WIDE, bool F16>
 __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_kernel(AttendArgs a) {
   constexpr int STAGE_BYTES = 2 * kStageTokens * DP * 2;
   extern __shared__ __align__(128) uint8_t s_pipe[];
@@ -1471,14 +1486,11 @@ __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_k
     look.visible = visible;
     AttendState<DP> st;
     for (int hb = 0; hb < G; hb += kHeadBlock) {
+      const long long pidx = (long long)slot * G + hb;
       look.start(j0);
-      attend_stages<DP, NS, F16>(a, look, ntiles, sid, row, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); }, st);
-      attend_combine<DP, 4>(st, reinterpret_cast<float*>(s_pipe), min(kHeadBlock, G - hb), D,
-                            [&](int hh, int d, float big, float lsum, float v0, float v1) {
-                              const long long pidx = (long long)slot * G + hb + hh;
-                              *reinterpret_cast<float2*>(a.pacc + pidx * D + d) = make_float2(v0, v1);
-                              if (d == 0) { a.pm[pidx] = big; a.pl[pidx] = lsum; }
-                            });
+      attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); }, st);
+      attend_combine<DP, 4, WIDE>(st, reinterpret_cast<float*>(s_pipe), min(kHeadBlock, G - hb), D,
+                                  AttendSums{a.pm + pidx, a.pl + pidx, a.pacc + pidx * D});
     }
 
     // ticket: the CTA that finishes a pair last merges its partials (slots c0 + rowg .. c1 + rowg, in this order)
@@ -1741,7 +1753,7 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   const int dp = c->dim <= 32 ? 32 : c->dim <= 64 ? 64 : c->dim <= 128 ? 128 : 256;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaSuccess;
-  const bool half = (c->flags & MOBA_CACHE_FP16) != 0;
+  const bool half = (c->flags & MOBA_CACHE_FP16) != 0, wide = hq / c->hkv > 8;
   a.rowgs = rows * c->hkv;
   a.spc = selected ? (c->chunk_size + kStageTokens - 1) / kStageTokens : 1;
   a.min_stages = kStreamLeast;
@@ -1767,7 +1779,8 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
     constexpr size_t ring = (size_t)cluster_teams(L) * cluster_stages(L) * 2 * kStageTokens * L * 2;                    \
     constexpr size_t red = (size_t)4 * cluster_teams(L) * 16 * (L + 2) * 4;                                             \
     const size_t smem = (ring > red ? ring : red) + (size_t)(hq / c->hkv) * c->dim * 4;                                 \
-    const auto kernel = half ? decode_attend_cluster_kernel<L, CL, true> : decode_attend_cluster_kernel<L, CL, false>;  \
+    const auto kernel = wide ? (half ? decode_attend_cluster_kernel<L, CL, true, true> : decode_attend_cluster_kernel<L, CL, true, false>)    \
+                             : (half ? decode_attend_cluster_kernel<L, CL, false, true> : decode_attend_cluster_kernel<L, CL, false, false>); \
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
     if (e == cudaSuccess && CL > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); \
     if (e == cudaSuccess)                                                                                               \
@@ -1793,7 +1806,8 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
       constexpr int NS = stream_stages(L);                                                                              \
       constexpr size_t pipe = (size_t)NS * 2 * kStageTokens * L * 2, red = (size_t)4 * 16 * (L + 2) * 4;                \
       constexpr size_t smem = pipe > red ? pipe : red;                                                                  \
-      const auto kernel = half ? decode_attend_stream_kernel<L, NS, true> : decode_attend_stream_kernel<L, NS, false>;  \
+      const auto kernel = wide ? (half ? decode_attend_stream_kernel<L, NS, true, true> : decode_attend_stream_kernel<L, NS, true, false>)    \
+                               : (half ? decode_attend_stream_kernel<L, NS, false, true> : decode_attend_stream_kernel<L, NS, false, false>); \
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                         \
       if (e == cudaSuccess)                                                                                             \
         e = launch_dependent(8u, kernel, dim3(L <= 128 ? kStreamCtas : kStreamCtas / 3), dim3(128), smem, st, a);       \
