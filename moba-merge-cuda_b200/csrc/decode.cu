@@ -1115,10 +1115,11 @@ __device__ __forceinline__ void attend_softmax(const float (&s)[4], float& m, fl
 // serves every head at no extra cost.  Each warp takes 16 tokens of every stage and keeps its own running (max, sum, O).
 //   ring      NS stages            rowbase [NS][64]   nv, mask [2 NS]: a slot is rewritten NS stages ahead, while the slots
 //                                                     before it are still read
+//   which     heads of the block that count: stages that none of them attends are passed over (see attend_spoiled)
 template <int DP, int NS, bool F16, bool WIDE, class Sync>
 __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& look, int ntiles, int sid, int row, int g, int hb, int ltid,
                                               uint8_t* ring, long long (*s_rowbase)[kStageTokens], int* s_nv, unsigned* s_mask,
-                                              Sync team_sync, AttendState<DP>& st) {
+                                              Sync team_sync, unsigned which, AttendState<DP>& st) {
   constexpr int KSTEPS = DP / 16;
   constexpr int DT = DP / 8;  // 8-column output tiles
   constexpr int STAGE_BYTES = 2 * kStageTokens * DP * 2;
@@ -1181,7 +1182,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
     const int tok0 = wt * 16;
     const int nvalid = s_nv[i % META] - tok0;
     const unsigned heads = s_mask[i % META] >> hb;
-    if (nvalid > 0 && (heads & 0xFFFFu)) {  // warp-uniform
+    if (nvalid > 0 && (heads & which)) {  // warp-uniform
       const bool on0 = (heads >> qr) & 1u, on1 = WIDE ? (heads >> (qr + 8)) & 1u : on0;
       const uint32_t kbase = smem_u32(ring + (i % NS) * STAGE_BYTES);
       const uint32_t vbase = kbase + kStageTokens * DP * 2;
@@ -1243,9 +1244,9 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
 // Where the sums of a head block go: head h of it to m[h], l[h] and o[h * D ...]; -inf, 0 and zeros for a head nobody attended.
 struct AttendSums { float *m, *l, *o; };
 
-// Combines the NW warps of a CTA through shared memory (s_o: NW * 16 * (DP + 2) floats).
+// Combines the NW warps of a CTA through shared memory (s_o: NW * 16 * (DP + 2) floats), for heads h0 to h1 - 1 of the block.
 template <int DP, int NW, bool WIDE>
-__device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, int nh, int D, const AttendSums& to) {
+__device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, int h0, int h1, int D, const AttendSums& to) {
   constexpr int ROWS = WIDE ? 16 : 8;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, qr = lane >> 2, qc = lane & 3;
   st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 1); st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 2);
@@ -1270,8 +1271,8 @@ __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, 
   }
   __syncthreads();
   const int d2n = D >> 1;
-  for (int item = tid; item < nh * d2n; item += 32 * NW) {
-    const int hh = item / d2n, d = (item - hh * d2n) * 2;
+  for (int item = tid; item < (h1 - h0) * d2n; item += 32 * NW) {
+    const int at = item / d2n, hh = h0 + at, d = (item - at * d2n) * 2;
     float mw[NW], big = -INFINITY;
 #pragma unroll
     for (int w = 0; w < NW; ++w) { mw[w] = s_ml[((size_t)w * ROWS + hh) * 2]; big = fmaxf(big, mw[w]); }
@@ -1286,6 +1287,21 @@ __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, 
     *reinterpret_cast<float2*>(to.o + (size_t)hh * D + d) = make_float2(v0, v1);
     if (d == 0) { to.m[hh] = big; to.l[hh] = lsum; }
   }
+}
+
+// A head that is off in a stage has P = 0 there, but 0 x Inf of a V that it did not select is NaN, and that stays in its sum.
+// Such a V gets into a cache only with the finite check switched off, so nothing is spent on it in the stages (dropping the products
+// of heads that are off one by one cost 10 % of a step: 64 requests, 12/2 heads, D = 128, 249 -> 274 us): where a sum
+// comes out not finite the CTA runs its stages again, once per head and without those the head does not attend.
+template <int DP>
+__device__ __forceinline__ bool attend_spoiled(const AttendState<DP>& st) {
+  float zero = 0.f;
+#pragma unroll
+  for (int dt = 0; dt < DP / 8; ++dt) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) zero = fmaf(st.o[dt][e], 0.f, zero);
+  }
+  return __syncthreads_or(zero != 0.f);  // NaN
 }
 
 // ---- cluster variant ---------------------------------------------------------------------------------------------
@@ -1345,11 +1361,18 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
   };
   AttendState<DP> st;
   for (int hb = 0; hb < G; hb += kHeadBlock) {
-    look.start(first);
-    attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
-                                     s_nv[team], s_mask[team], team_sync, st);
-    attend_combine<DP, NW, WIDE>(st, reinterpret_cast<float*>(s_pipe), min(kHeadBlock, G - hb), D,
-                                 AttendSums{s_m + hb, s_l + hb, s_sum + (size_t)hb * D});
+    const int nh = min(kHeadBlock, G - hb);
+    int head = -1;  // all together, see attend_spoiled
+    do {
+      look.start(first);
+      attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
+                                       s_nv[team], s_mask[team], team_sync, head < 0 ? 0xFFFFu : 1u << head, st);
+      const bool again = head < 0 && !dense && attend_spoiled(st);
+      if (!again)
+        attend_combine<DP, NW, WIDE>(st, reinterpret_cast<float*>(s_pipe), max(head, 0), head < 0 ? nh : head + 1, D,
+                                     AttendSums{s_m + hb, s_l + hb, s_sum + (size_t)hb * D});
+      if (again || head >= 0) ++head;
+    } while (head >= 0 && head < nh);
   }
   // CL neighbouring lanes, one per CTA of the cluster, take four dimensions of a head; the items are divided over the CTAs
   cluster_barrier();
@@ -1486,11 +1509,19 @@ __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_k
     look.visible = visible;
     AttendState<DP> st;
     for (int hb = 0; hb < G; hb += kHeadBlock) {
+      const int nh = min(kHeadBlock, G - hb);
       const long long pidx = (long long)slot * G + hb;
-      look.start(j0);
-      attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); }, st);
-      attend_combine<DP, 4, WIDE>(st, reinterpret_cast<float*>(s_pipe), min(kHeadBlock, G - hb), D,
-                                  AttendSums{a.pm + pidx, a.pl + pidx, a.pacc + pidx * D});
+      int head = -1;  // all together, see attend_spoiled
+      do {
+        look.start(j0);
+        attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); },
+                                         head < 0 ? 0xFFFFu : 1u << head, st);
+        const bool again = head < 0 && !dense && attend_spoiled(st);
+        if (!again)
+          attend_combine<DP, 4, WIDE>(st, reinterpret_cast<float*>(s_pipe), max(head, 0), head < 0 ? nh : head + 1, D,
+                                      AttendSums{a.pm + pidx, a.pl + pidx, a.pacc + pidx * D});
+        if (again || head >= 0) ++head;
+      } while (head >= 0 && head < nh);
     }
 
     // ticket: the CTA that finishes a pair last merges its partials (slots c0 + rowg .. c1 + rowg, in this order)

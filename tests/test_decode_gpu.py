@@ -525,3 +525,44 @@ def test_probabilities_keep_more_than_16_bits(requests, queries, hq, hkv, dim, l
     rounded = torch_to_f64(torch.from_numpy(want).to(dtype))
     error, least = np.linalg.norm(torch_to_f64(result.output) - want), np.linalg.norm(rounded - want)
     assert error <= (1.02 if dtype == torch.bfloat16 else 1.05) * least, f"{error / least:.4f}"
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("rows,hq,hkv,dim,dtype", [
+    (1, 8, 2, 64, torch.bfloat16),       # a cluster per pair
+    (2, 6, 1, 128, torch.float16),
+    (20, 8, 2, 64, torch.bfloat16),      # fixed parts
+    (4, 40, 2, 128, torch.bfloat16),     # two head blocks
+    (20, 40, 2, 128, torch.bfloat16),    # fixed parts, two head blocks
+    (120, 8, 2, 64, torch.float16),      # streamed
+    (60, 40, 2, 96, torch.bfloat16),     # streamed, two head blocks
+])
+def test_values_of_a_chunk_reach_only_the_heads_that_selected_it(rows, hq, hkv, dim, dtype, bad):
+    """A V that is not finite (a caller may switch the check off) spoils the heads that attend its chunk; the others keep
+    their bits, whichever kernel runs."""
+    from moba_opt import PagedKVCache
+    chunk, chunks, poisoned = 100, 6, 2
+    length = chunks * chunk + 41
+    k, v = rand((length, hkv, dim), 311, dtype), rand((length, hkv, dim), 312, dtype)
+    k[:, :, :chunks] = 0
+    for c in range(chunks):
+        k[c * chunk:(c + 1) * chunk, :, c] = 8                     # chunk c is the best match of a query along axis c
+    q = rand((rows, hq, dim), 313, dtype)
+    for h in range(hq):
+        q[:, h, h % chunks] = 40
+    caches = []
+    for value in (1.0, bad):
+        vv = v.clone()
+        vv[poisoned * chunk + 33, :, 5] = value
+        vv[poisoned * chunk + 99, :, dim - 1] = value
+        cache = PagedKVCache(2, length, hkv, dim, page_size=7, chunk_size=chunk, dtype=dtype)
+        cache.check_finite = False
+        cache.append(torch.cat((k, k)), torch.cat((vv, vv)), sequence_ids=[0, 1], cu_seqlens=[0, length, 2 * length])
+        caches.append(cache.attend(q, sequence_ids=[i % 2 for i in range(rows)], topk=2))
+    good, spoiled = caches
+    reads = (good.selected_blocks == poisoned).any(-1)
+    assert torch.equal(good.selected_blocks, spoiled.selected_blocks) and reads.any() and not reads.all()
+    assert torch.equal(good.output[~reads], spoiled.output[~reads]) and torch.equal(good.lse, spoiled.lse)
+    assert not spoiled.output[reads][:, 5].isfinite().any() and bool(good.output.isfinite().all())
+    if bad == bad:                                                 # an infinity stays one, of its sign
+        assert (spoiled.output[reads][:, 5] == bad).all()
