@@ -1809,10 +1809,12 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   do {                                                                                                                  \
     constexpr size_t ring = (size_t)cluster_teams(L) * cluster_stages(L) * 2 * kStageTokens * L * 2;                    \
     constexpr size_t red = (size_t)4 * cluster_teams(L) * 16 * (L + 2) * 4;                                             \
+    /* the limit belongs to the function, not to the launch: one value for all groups, so that no thread lowers another's */ \
+    constexpr size_t most_smem = (ring > red ? ring : red) + (size_t)32 * L * 4;                                        \
     const size_t smem = (ring > red ? ring : red) + (size_t)(hq / c->hkv) * c->dim * 4;                                 \
     const auto kernel = wide ? (half ? decode_attend_cluster_kernel<L, CL, true, true> : decode_attend_cluster_kernel<L, CL, true, false>)    \
                              : (half ? decode_attend_cluster_kernel<L, CL, false, true> : decode_attend_cluster_kernel<L, CL, false, false>); \
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most_smem);                      \
     if (e == cudaSuccess && CL > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); \
     if (e == cudaSuccess)                                                                                               \
       e = launch_dependent_cluster(8u, kernel, dim3(CL, a.rowgs), dim3(128 * cluster_teams(L)), CL, smem, st, a);       \

@@ -566,3 +566,41 @@ def test_values_of_a_chunk_reach_only_the_heads_that_selected_it(rows, hq, hkv, 
     assert not spoiled.output[reads][:, 5].isfinite().any() and bool(good.output.isfinite().all())
     if bad == bad:                                                 # an infinity stays one, of its sign
         assert (spoiled.output[reads][:, 5] == bad).all()
+
+
+def _two_threads(calls, times=20000):
+    """Runs each (entry point, arguments) `times` times in a thread of its own, both at once: how many of each failed."""
+    import threading
+    failed, start = [0] * len(calls), threading.Barrier(len(calls))
+
+    def loop(i):
+        entry, args = calls[i]
+        start.wait()
+        for _ in range(times):
+            failed[i] += entry(*args) != 0
+    threads = [threading.Thread(target=loop, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    return failed
+
+
+def test_threads_with_groups_of_different_size():
+    """The cluster kernel's shared memory grows with the group; the limit that a launch sets belongs to the function, so a
+    cache with small groups in one thread must not lower it under a launch of another."""
+    import ctypes
+    from moba_opt import PagedKVCache
+    calls, keep = [], []
+    for group in (32, 9):
+        cache = PagedKVCache(1, 512, 1, 128, chunk_size=64)
+        cache.append(rand((300, 1, 128), 321), rand((300, 1, 128), 322), sequence_ids=[0], cu_seqlens=[0, 300])
+        p = cache.prepare_decode([0], group, mode="dense", check_finite=False)
+        p.launch("attend")
+        desc = cache._desc()
+        calls.append((p._lib.moba_decode_attend, (
+            ctypes.byref(desc), p.q.data_ptr(), p.gpu_ids.data_ptr(), p.positions.data_ptr(), 1, group, None, p._slots, None, None, None, 1,
+            p._workspace.data_ptr(), p._ws_bytes, p.output.data_ptr(), p.lse.data_ptr(), cache._status.data_ptr(), p._stream())))
+        keep.append((p, desc))
+    assert _two_threads(calls) == [0, 0]
