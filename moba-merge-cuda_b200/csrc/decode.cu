@@ -1712,9 +1712,10 @@ extern "C" int moba_decode_route(const moba_cache_desc* c, const void* q, const 
   if (G > 32 || remote > 16) return MOBA_ERR_UNSUPPORTED;
   const size_t smem = ((((size_t)G * width + width + 1 + (size_t)G * c->dim + 3) & ~(size_t)3)) * 4 +
                       (size_t)kRouteTile * ((c->dim / 8) | 1) * 16;
-  if (smem > 200 * 1024) return MOBA_ERR_UNSUPPORTED;
+  constexpr int most_smem = 200 * 1024;  // the limit belongs to the function: one value, so that no thread lowers another's
+  if (smem > most_smem) return MOBA_ERR_UNSUPPORTED;
   const auto kernel = (c->flags & MOBA_CACHE_FP16) ? decode_route_kernel<true> : decode_route_kernel<false>;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem) != cudaSuccess)
     return MOBA_ERR_CUDA;
   const int umax = moba_decode_union_capacity(hq, c->hkv, remote, width);
   if (launch_dependent(4u, kernel, dim3(rows, c->hkv), dim3(kRouteThreads), smem, (cudaStream_t)stream, make_cache_view(*c),

@@ -19,6 +19,7 @@
 namespace moba {
 
 constexpr int kCandBatch = 32;   // candidate means staged in shared memory per pass
+constexpr int kMostChunks = 4096;  // per sequence
 constexpr int kMeanRows = 256;   // tokens per CTA of the mean pass
 
 // --------------------------------------------------------------------------- 1. chunk means
@@ -388,7 +389,7 @@ int validate_desc(const moba_prefill_desc* d) {
   if (d->chunk_size < 1 || d->remote_k < 0 || d->num_chunks < 1 || d->num_qtiles < 1) return MOBA_ERR_INVALID;
   if (d->remote_k > 16 || d->dim > 128) return MOBA_ERR_UNSUPPORTED;  // prefill kernels: head_dim up to 128
   if ((long long)d->total_tokens * d->hq * (d->remote_k > 0 ? d->remote_k : 1) >= (1ll << 31)) return MOBA_ERR_UNSUPPORTED;
-  if (d->max_chunks_per_seq > 4096) return MOBA_ERR_UNSUPPORTED;
+  if (d->max_chunks_per_seq > kMostChunks) return MOBA_ERR_UNSUPPORTED;
   if (!d->cu_seqlens || !d->chunk_start || !d->chunk_seq || !d->chunk_local || !d->qtile_chunk || !d->qtile_tok0 ||
       !d->qtile_local || !d->self_pairs || d->num_self_pairs < 1 || d->num_self_pairs > d->num_qtiles)
     return MOBA_ERR_INVALID;
@@ -400,7 +401,9 @@ static cudaError_t launch_gate_as(const PrefillView& pv, const __nv_bfloat16* q,
                                   int max_chunks_per_seq, cudaStream_t st) {
   constexpr int DP = DD * LPR;
   const size_t smem = (size_t)kCandBatch * DP * 4 + (size_t)kTile * (DP * 2 + 16) + (size_t)max_chunks_per_seq * 4 + 16;
-  cudaError_t e = cudaFuncSetAttribute(gate_topk_kernel<RT, DD, LPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit belongs to the function: one value for all batches, so that no thread lowers another's
+  constexpr size_t most_smem = (size_t)kCandBatch * DP * 4 + (size_t)kTile * (DP * 2 + 16) + (size_t)kMostChunks * 4 + 16;
+  cudaError_t e = cudaFuncSetAttribute(gate_topk_kernel<RT, DD, LPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most_smem);
   if (e != cudaSuccess) return e;
   gate_topk_kernel<RT, DD, LPR><<<dim3(pv.n_qtiles, pv.Hq), 32 * LPR, smem, st>>>(pv, q, means, sel, cnt);
   return cudaGetLastError();

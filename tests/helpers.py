@@ -65,3 +65,24 @@ def config1_inputs():
     q, k, v = [torch.randn(2048, 8, 64, generator=rng).bfloat16() for _ in range(3)]
     g = torch.randn(2048, 8, 64, generator=rng).bfloat16()
     return q, k, v, g
+
+
+def two_threads(calls, times=20000):
+    """Runs each (entry point, arguments) `times` times in a thread of its own, both at once: how many of each failed."""
+    import threading
+
+    import torch
+    failed, start = [0] * len(calls), threading.Barrier(len(calls))
+
+    def loop(i):
+        entry, args = calls[i]
+        start.wait()
+        for _ in range(times):
+            failed[i] += entry(*args) != 0
+    threads = [threading.Thread(target=loop, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    return failed

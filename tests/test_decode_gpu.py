@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import DECODE_GOLDENS, bits_to_torch, load, torch_to_f64
+from helpers import DECODE_GOLDENS, bits_to_torch, load, torch_to_f64, two_threads
 from oracle import moba_oracle as mo
 
 pytestmark = pytest.mark.gpu
@@ -568,25 +568,6 @@ def test_values_of_a_chunk_reach_only_the_heads_that_selected_it(rows, hq, hkv, 
         assert (spoiled.output[reads][:, 5] == bad).all()
 
 
-def _two_threads(calls, times=20000):
-    """Runs each (entry point, arguments) `times` times in a thread of its own, both at once: how many of each failed."""
-    import threading
-    failed, start = [0] * len(calls), threading.Barrier(len(calls))
-
-    def loop(i):
-        entry, args = calls[i]
-        start.wait()
-        for _ in range(times):
-            failed[i] += entry(*args) != 0
-    threads = [threading.Thread(target=loop, args=(i,)) for i in range(len(calls))]
-    for t in threads:
-        t.start()
-    for t in threads:
-        t.join()
-    torch.cuda.synchronize()
-    return failed
-
-
 def test_threads_with_groups_of_different_size():
     """The cluster kernel's shared memory grows with the group; the limit that a launch sets belongs to the function, so a
     cache with small groups in one thread must not lower it under a launch of another."""
@@ -603,4 +584,23 @@ def test_threads_with_groups_of_different_size():
             ctypes.byref(desc), p.q.data_ptr(), p.gpu_ids.data_ptr(), p.positions.data_ptr(), 1, group, None, p._slots, None, None, None, 1,
             p._workspace.data_ptr(), p._ws_bytes, p.output.data_ptr(), p.lse.data_ptr(), cache._status.data_ptr(), p._stream())))
         keep.append((p, desc))
-    assert _two_threads(calls) == [0, 0]
+    assert two_threads(calls) == [0, 0]
+
+
+def test_threads_with_caches_of_different_width():
+    """The same for routing, whose shared memory grows with the number of chunks a query may be routed to."""
+    import ctypes
+    from moba_opt import PagedKVCache
+    calls, keep = [], []
+    for width in (600, 400):
+        cache = PagedKVCache(1, width * 16 + 1, 1, 64, chunk_size=16)
+        cache.append(rand((300, 1, 64), 331), rand((300, 1, 64), 332), sequence_ids=[0], cu_seqlens=[0, 300])
+        p = cache.prepare_decode([0], 32, check_finite=False)
+        assert p.width == width
+        p.launch("attend")
+        desc = cache._desc()
+        calls.append((p._lib.moba_decode_route, (
+            ctypes.byref(desc), p.q.data_ptr(), p.gpu_ids.data_ptr(), p.positions.data_ptr(), 1, 32, p.remote, p.width, p.scores.data_ptr(),
+            p.selected.data_ptr(), p._u_chunk.data_ptr(), p._u_mask.data_ptr(), p._u_count.data_ptr(), p._stream())))
+        keep.append((p, desc))
+    assert two_threads(calls) == [0, 0]

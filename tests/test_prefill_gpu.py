@@ -12,7 +12,7 @@ import pytest
 import torch
 
 from helpers import (PREFILL_GOLDENS, ROUTE_GOLDENS, bits_to_torch, config1_inputs, cu_from_lens, load, rel_rms,
-                     torch_to_f64, unpack_selected)
+                     torch_to_f64, two_threads, unpack_selected)
 from oracle import moba_oracle as mo
 
 pytestmark = pytest.mark.gpu
@@ -363,3 +363,18 @@ def test_remembered_offsets_follow_in_place_changes_of_cu_seqlens():
     assert torch.equal(moba_opt.run_impl("opt_gqa_cuda", q, k, v, cu, 64, cfg),
                        moba_opt.run_impl("opt_gqa_cuda", q, k, v, fresh, 64, cfg))
     assert not torch.equal(first, moba_opt.run_impl("opt_gqa_cuda", q, k, v, fresh, 64, cfg))
+
+
+def test_threads_with_batches_of_different_chunk_counts():
+    """The gate's shared memory grows with the chunks of a sequence; the limit that a launch sets belongs to the function, so a
+    batch with fewer chunks in one thread must not lower it under a launch of another."""
+    import moba_opt.grouped_attention as ga
+    device, calls, keep = torch.device("cuda", torch.cuda.current_device()), [], []
+    for chunk in (1, 50):
+        q, k = (torch.randn(400, h, 128, device=device).bfloat16() for h in (2, 1))
+        call = ga.get_plan((0, 400), chunk, device).call(q, k, k, 2)
+        state, scratch = (torch.empty(n, dtype=torch.uint8, device=device) for n in (call.state_bytes, call.route_bytes))
+        calls.append((ga._ext.lib().moba_prefill_route, (call.ref, q.data_ptr(), k.data_ptr(), state.data_ptr(), scratch.data_ptr(),
+                                                         call.route_bytes, ga._stream(device))))
+        keep.append((q, k, call, state, scratch))
+    assert two_threads(calls, 4000) == [0, 0]
