@@ -224,6 +224,11 @@ int moba_decode_attend(const moba_cache_desc* c, const void* q, const int32_t* i
                        const int32_t* selected, int slots, const int32_t* u_chunk, const uint32_t* u_mask,
                        const int32_t* u_count, int umax, void* workspace, size_t workspace_bytes, void* out, float* lse,
                        unsigned* status, void* stream);
+/* The kernel that moba_decode_attend takes for a call of this shape (routed: selected != null): one of the values below, or
+ * minus a MOBA_ERR_* code.  sms, most_cluster: SMs of the device and the largest cluster that it can hold; sms = 0 and most_cluster = -1 ask
+ * the current device. */
+enum { MOBA_ATTEND_FIXED_DEEP = 1, MOBA_ATTEND_FIXED = 2, MOBA_ATTEND_STREAMED = 3, MOBA_ATTEND_CLUSTER_8 = 8, MOBA_ATTEND_CLUSTER_16 = 16 };
+int moba_decode_attend_variant(const moba_cache_desc* c, int rows, int hq, int routed, int slots, int umax, int sms, int most_cluster);
 
 /* ---------------------------------------------------------------------------------------------
  * Standalone merge operator: replaces merge_forward of the reference (src/moba_opt/ops/bindings.cpp:6-22,

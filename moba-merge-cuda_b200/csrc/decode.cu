@@ -10,10 +10,12 @@
 // Attention reads each needed K/V token once per KV head: the routing kernel turns the per-query-
 // head selections of a GQA group into the union of chunks with a bitmask of the heads that attend
 // each of them, and a token serves all those heads.  Three kernels divide the work (the rule and its figures stand at
-// moba_decode_attend): clusters that merge through distributed shared memory for the smallest batches, a CTA per fixed part of
+// attend_variant): clusters that merge through distributed shared memory for the smallest batches, a CTA per fixed part of
 // a chunk while that grid fits the GPU at once, equal shares of one list of stages beyond.  The last two leave partial (max, sum,
 // accumulator) triples in a workspace, and the CTA that finishes a (query, kv head) pair last - found with an atomic
 // ticket, nobody waits - merges them in a fixed order.
+#include <atomic>
+
 #include "launch.cuh"
 #include "moba_b200.h"
 #include "prefill_common.cuh"
@@ -1736,16 +1738,109 @@ static int attend_parts(const moba_cache_desc* c) {
 // A share below four stages would be mostly its start and its partials (2, 4, 8 and 16 within 1 % at the sizes above).
 constexpr int kStreamLeast = 4;
 constexpr int kClusterMost = 11;
-constexpr int kStreamCtas = 3 * 148;  // streamed variant: what a B200 holds at once (one per SM above head dimension 128)
+// What the GPU holds of the one-team kernels at once: three CTAs per SM, one above head dimension 128.
+static int attend_wave(int dim, int sms) { return dim <= 128 ? 3 * sms : sms; }
 
 // Partials of a launch: with fixed parts a slot per (head, list entry, part), streamed one per head of a group and segment.
 static size_t attend_partials(const moba_cache_desc* c, int rows, int hq, int slots) {
   const size_t fixed = (size_t)rows * hq * slots * attend_parts(c);
-  const size_t streamed = ((size_t)kStreamCtas + (size_t)rows * c->hkv) * (hq / c->hkv);
+  const size_t streamed = ((size_t)attend_wave(1, device_sms()) + (size_t)rows * c->hkv) * (hq / c->hkv);
   return fixed > streamed ? fixed : streamed;
 }
 static size_t attend_workspace(const moba_cache_desc* c, int rows, int hq, size_t partials) {
   return align256((size_t)rows * c->hkv * 4) + 2 * align256(partials * 4) + align256(partials * c->dim * 4);
+}
+
+template <int DP>
+struct ClusterSmem {
+  static constexpr size_t ring = (size_t)cluster_teams(DP) * cluster_stages(DP) * 2 * kStageTokens * DP * 2;
+  static constexpr size_t red = (size_t)4 * cluster_teams(DP) * 16 * (DP + 2) * 4;
+  static constexpr size_t fixed = ring > red ? ring : red;  // behind it the sums of a group: [G][D]
+  // the limit belongs to the function, not to the launch: one value for all groups, so that no thread lowers another's
+  static constexpr size_t most = fixed + (size_t)32 * DP * 4;
+};
+template <int DP, int CL>
+static auto cluster_kernel(bool wide, bool half) {
+  return wide ? (half ? decode_attend_cluster_kernel<DP, CL, true, true> : decode_attend_cluster_kernel<DP, CL, true, false>)
+              : (half ? decode_attend_cluster_kernel<DP, CL, false, true> : decode_attend_cluster_kernel<DP, CL, false, false>);
+}
+template <int DP, int CL>
+static cudaError_t cluster_attributes(bool wide, bool half) {
+  const auto kernel = cluster_kernel<DP, CL>(wide, half);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ClusterSmem<DP>::most);
+  if (e == cudaSuccess && CL > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+// Whether the current device can hold a cluster of CL CTAs at all: 16 is more than the portable size, and a partition of a GPU
+// may have fewer SMs side by side.  Asked once per device and kernel.
+template <int DP, int CL>
+static bool cluster_fits(bool wide, bool half) {
+  static std::atomic<signed char> known[2][2][64];  // 0 not asked yet, 1 yes, -1 no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  std::atomic<signed char>& answer = known[wide][half][dev];
+  if (answer.load(std::memory_order_relaxed) == 0) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CL);
+    cfg.blockDim = dim3(128 * cluster_teams(DP));
+    cfg.dynamicSmemBytes = ClusterSmem<DP>::most;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const bool yes = cluster_attributes<DP, CL>(wide, half) == cudaSuccess &&
+                     cudaOccupancyMaxActiveClusters(&clusters, cluster_kernel<DP, CL>(wide, half), &cfg) == cudaSuccess && clusters > 0;
+    if (!yes) cudaGetLastError();  // an answer, not an error of the call
+    answer.store(yes ? 1 : -1, std::memory_order_relaxed);
+  }
+  return answer.load(std::memory_order_relaxed) > 0;
+}
+static bool device_holds_cluster(int dim, int cl, bool wide, bool half) {
+  if (dim <= 32) return cl == 16 ? cluster_fits<32, 16>(wide, half) : cluster_fits<32, 8>(wide, half);
+  if (dim <= 64) return cl == 16 ? cluster_fits<64, 16>(wide, half) : cluster_fits<64, 8>(wide, half);
+  if (dim <= 128) return cl == 16 ? cluster_fits<128, 16>(wide, half) : cluster_fits<128, 8>(wide, half);
+  return cl == 16 ? cluster_fits<256, 16>(wide, half) : cluster_fits<256, 8>(wide, half);
+}
+
+// Which variant, in us of a captured step (cluster / fixed parts / streamed), one request and heads 14/2 at D = 64 unless said:
+//   clusters while every pair can have one (16 CTAs for up to four pairs, 8 for up to eight) and a CTA's share, at the
+//   cache's capacity, stays below kClusterMost stages: dense 1K 10.3 / 12.4 / 16.5, 8K 12.4 / 14.4 / 18.6, but 16K 16.5 / 14.5 / 22.7;
+//   heads 32/8, D = 128, dense 4K 14.5 / 16.5 / 20.6, but 8K 20.6 / 16.5 / 22.7; with 16 pairs 18.5 / 16.5 / 22.7 at 1K already;
+//   where the device cannot hold 16 CTAs side by side, 8 take their place;
+//   fixed parts while their grid, at capacity, fits the GPU at once: heads 32/8, D = 128, dense 16K (264 CTAs) - / 24.7 / 27.4,
+//   eight requests, 12/2, D = 128, routed 16K (304 CTAs) - / 29.9 / 36.8; beyond one wave the streamed variant: the first
+//   at 32K (520 CTAs) - / 49.4 / 41.4, eight requests dense 16K (528 CTAs) - / 52.7 / 44.6.  A routed grid is a bound that
+//   heads with picks in common and short contexts stay below, so there the line is two waves: 21 requests up to 5.5K, 8/2, D = 128
+//   (546 CTAs) - / 36.7 / 38.9, 18 requests of 32K, 6/1, D = 32 (774 CTAs) - / 37.9 / 38.9, 42 requests of 53K, 28/4, D = 128
+//   (1344 CTAs) - / 96.7 / 93.2.
+// holds(cl): whether the device can hold a cluster of cl CTAs.
+template <class Holds>
+static int attend_variant(const moba_cache_desc* c, int rows, bool routed, int slots, int umax, int sms, Holds holds) {
+  const long long pairs = (long long)rows * c->hkv;
+  const int spc = (c->chunk_size + kStageTokens - 1) / kStageTokens;
+  const long long most = routed ? (long long)umax * spc : ((long long)slots * c->chunk_size + kStageTokens - 1) / kStageTokens;
+  if (!routed || umax <= kClusterList) {
+    if (pairs <= 4 && most <= 16 * kClusterMost && holds(16)) return MOBA_ATTEND_CLUSTER_16;
+    if (pairs <= 8 && most <= 8 * kClusterMost && holds(8)) return MOBA_ATTEND_CLUSTER_8;
+  }
+  const long long ctas = (long long)(routed ? umax : slots) * attend_parts(c) * pairs;
+  if (ctas <= sms) return MOBA_ATTEND_FIXED_DEEP;
+  return ctas <= (long long)attend_wave(c->dim, sms) * (routed ? 2 : 1) ? MOBA_ATTEND_FIXED : MOBA_ATTEND_STREAMED;
+}
+
+extern "C" int moba_decode_attend_variant(const moba_cache_desc* c, int rows, int hq, int routed, int slots, int umax, int sms,
+                                          int most_cluster) {
+  const int rc = validate_cache(c);
+  if (rc != MOBA_OK) return -rc;
+  if (rows < 1 || hq < 1 || hq % c->hkv || slots < 1 || (routed && umax < 1)) return -MOBA_ERR_INVALID;
+  if (hq / c->hkv > 32) return -MOBA_ERR_UNSUPPORTED;
+  const bool wide = hq / c->hkv > 8, half = (c->flags & MOBA_CACHE_FP16) != 0;
+  return attend_variant(c, rows, routed != 0, slots, umax, sms > 0 ? sms : device_sms(), [&](int cl) {
+    return most_cluster >= 0 ? cl <= most_cluster : device_holds_cluster(c->dim, cl, wide, half);
+  });
 }
 
 extern "C" size_t moba_decode_attend_workspace_bytes(const moba_cache_desc* c, int rows, int hq, int slots) {
@@ -1789,36 +1884,16 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   a.rowgs = rows * c->hkv;
   a.spc = selected ? (c->chunk_size + kStageTokens - 1) / kStageTokens : 1;
   a.min_stages = kStreamLeast;
-  // Which variant, in us of a captured step (cluster / fixed parts / streamed), one request and heads 14/2 at D = 64 unless said:
-  //   clusters while every pair can have one (16 CTAs for up to four pairs, 8 for up to eight) and a CTA's share, at the
-  //   cache's capacity, stays below kClusterMost stages: dense 1K 10.3 / 12.4 / 16.5, 8K 12.4 / 14.4 / 18.6, but 16K 16.5 / 14.5 / 22.7;
-  //   heads 32/8, D = 128, dense 4K 14.5 / 16.5 / 20.6, but 8K 20.6 / 16.5 / 22.7; with 16 pairs 18.5 / 16.5 / 22.7 at 1K already;
-  //   fixed parts while their grid, at capacity, fits the GPU at once: heads 32/8, D = 128, dense 16K (264 CTAs) - / 24.7 / 27.4,
-  //   eight requests, 12/2, D = 128, routed 16K (304 CTAs) - / 29.9 / 36.8; beyond one wave the streamed variant: the first
-  //   at 32K (520 CTAs) - / 49.4 / 41.4, eight requests dense 16K (528 CTAs) - / 52.7 / 44.6.  A routed grid is a bound that
-  //   heads with picks in common and short contexts stay below, so there the line is two waves: 21 requests up to 5.5K, 8/2, D = 128
-  //   (546 CTAs) - / 36.7 / 38.9, 18 requests of 32K, 6/1, D = 32 (774 CTAs) - / 37.9 / 38.9, 42 requests of 53K, 28/4, D = 128
-  //   (1344 CTAs) - / 96.7 / 93.2.
-  const long long most = selected ? (long long)umax * a.spc : ((long long)slots * c->chunk_size + kStageTokens - 1) / kStageTokens;
-  const int cl = a.rowgs <= 4 ? 16 : a.rowgs <= 8 ? 8 : 0;
-  const bool cluster = cl > 0 && most <= (long long)cl * kClusterMost && (!selected || umax <= kClusterList);
+  const int variant = moba_decode_attend_variant(c, rows, hq, selected != nullptr, slots, umax, 0, -1);
+  if (variant < 0) return -variant;
   const dim3 grid(a.umax, a.parts, rows * c->hkv);
-  const long long ctas = (long long)grid.x * grid.y * grid.z;
-  const bool deep = ctas <= kStreamCtas / 3, fixed = ctas <= (dp <= 128 ? kStreamCtas : kStreamCtas / 3) * (selected ? 2 : 1);
   prof_begin(kProfDecodeAttend, st);
 #define MOBA_LAUNCH_CLUSTER(L, CL)                                                                                       \
   do {                                                                                                                  \
-    constexpr size_t ring = (size_t)cluster_teams(L) * cluster_stages(L) * 2 * kStageTokens * L * 2;                    \
-    constexpr size_t red = (size_t)4 * cluster_teams(L) * 16 * (L + 2) * 4;                                             \
-    /* the limit belongs to the function, not to the launch: one value for all groups, so that no thread lowers another's */ \
-    constexpr size_t most_smem = (ring > red ? ring : red) + (size_t)32 * L * 4;                                        \
-    const size_t smem = (ring > red ? ring : red) + (size_t)(hq / c->hkv) * c->dim * 4;                                 \
-    const auto kernel = wide ? (half ? decode_attend_cluster_kernel<L, CL, true, true> : decode_attend_cluster_kernel<L, CL, true, false>)    \
-                             : (half ? decode_attend_cluster_kernel<L, CL, false, true> : decode_attend_cluster_kernel<L, CL, false, false>); \
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most_smem);                      \
-    if (e == cudaSuccess && CL > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); \
+    const size_t smem = ClusterSmem<L>::fixed + (size_t)(hq / c->hkv) * c->dim * 4;                                     \
+    e = cluster_attributes<L, CL>(wide, half);                                                                          \
     if (e == cudaSuccess)                                                                                               \
-      e = launch_dependent_cluster(8u, kernel, dim3(CL, a.rowgs), dim3(128 * cluster_teams(L)), CL, smem, st, a);       \
+      e = launch_dependent_cluster(8u, cluster_kernel<L, CL>(wide, half), dim3(CL, a.rowgs), dim3(128 * cluster_teams(L)), CL, smem, st, a); \
   } while (0)
 #define MOBA_LAUNCH_FIXED(L, NS, T)                                                                                      \
   do {                                                                                                                  \
@@ -1830,13 +1905,11 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   } while (0)
 #define MOBA_LAUNCH_ATTEND(L)                                                                                            \
   do {                                                                                                                  \
-    if (cluster) {                                                                                                      \
-      if (cl == 16) MOBA_LAUNCH_CLUSTER(L, 16);                                                                         \
-      else MOBA_LAUNCH_CLUSTER(L, 8);                                                                                   \
-    } else if (fixed) {                                                                                                 \
-      if (deep) MOBA_LAUNCH_FIXED(L, deep_stages(L), (L <= 128 ? 2 : 1));                                                \
-      else MOBA_LAUNCH_FIXED(L, kStages, 1);                                                                            \
-    } else {                                                                                                            \
+    if (variant == MOBA_ATTEND_CLUSTER_16) MOBA_LAUNCH_CLUSTER(L, 16);                                                  \
+    else if (variant == MOBA_ATTEND_CLUSTER_8) MOBA_LAUNCH_CLUSTER(L, 8);                                               \
+    else if (variant == MOBA_ATTEND_FIXED_DEEP) MOBA_LAUNCH_FIXED(L, deep_stages(L), (L <= 128 ? 2 : 1));               \
+    else if (variant == MOBA_ATTEND_FIXED) MOBA_LAUNCH_FIXED(L, kStages, 1);                                            \
+    else {                                                                                                              \
       constexpr int NS = stream_stages(L);                                                                              \
       constexpr size_t pipe = (size_t)NS * 2 * kStageTokens * L * 2, red = (size_t)4 * 16 * (L + 2) * 4;                \
       constexpr size_t smem = pipe > red ? pipe : red;                                                                  \
@@ -1844,7 +1917,7 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
                                : (half ? decode_attend_stream_kernel<L, NS, false, true> : decode_attend_stream_kernel<L, NS, false, false>); \
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                         \
       if (e == cudaSuccess)                                                                                             \
-        e = launch_dependent(8u, kernel, dim3(L <= 128 ? kStreamCtas : kStreamCtas / 3), dim3(128), smem, st, a);       \
+        e = launch_dependent(8u, kernel, dim3(attend_wave(L, device_sms())), dim3(128), smem, st, a);                     \
     }                                                                                                                   \
   } while (0)
   if (dp == 32) MOBA_LAUNCH_ATTEND(32);

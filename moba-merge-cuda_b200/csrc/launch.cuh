@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 namespace moba {
 
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
@@ -39,6 +41,19 @@ inline cudaError_t launch_dependent(unsigned kind, void (*kernel)(KArgs...), dim
   cfg.attrs = attr;
   cfg.numAttrs = (dependent_launch_mask() & kind) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// SMs of the current device; a full B200's where none answers (sizes asked for without a GPU).
+inline int device_sms() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 // The same for a grid of clusters of `cluster` CTAs along x.

@@ -64,6 +64,7 @@ _DECODE_ABI = {
     "moba_decode_union_capacity": (_I, [_I, _I, _I, _I]),
     "moba_decode_route": (_I, [_P, _VP, _VP, _VP, _I, _I, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP]),
     "moba_decode_attend_workspace_bytes": (_SZ, [_P, _I, _I, _I]),
+    "moba_decode_attend_variant": (_I, [_P, _I, _I, _I, _I, _I, _I, _I]),
     "moba_check_finite": (_I, [ctypes.POINTER(FiniteInput), _I, _I, _I, _VP, _VP]),
     "moba_decode_attend": (_I, [_P, _VP, _VP, _VP, _I, _I, _VP, _I, _VP, _VP, _VP, _I, _VP, _SZ, _VP, _VP, _VP, _VP]),
 }

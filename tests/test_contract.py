@@ -104,3 +104,26 @@ def test_both_16_bit_formats_pass_the_input_check():
     import torch
     from moba_opt import baseline_adapter as ba
     assert ba.SUPPORTED_DTYPES == (torch.bfloat16, torch.float16)      # as src/moba_opt/baseline_adapter.py:13
+
+
+@pytest.mark.parametrize("requests,hq,hk,dim,capacity,chunk,routed,sms,most_cluster,want", [
+    (1, 14, 2, 64, 4096, 512, False, 148, 16, 16),       # 64 stages of 64 tokens over 16 CTAs
+    (1, 14, 2, 64, 4096, 512, False, 148, 8, 8),         # a partition of a GPU that holds eight CTAs side by side, not 16
+    (1, 14, 2, 64, 4096, 512, False, 148, 0, 1),         # none at all: 16 fixed parts
+    (1, 14, 2, 64, 8192, 512, False, 148, 8, 1),         # 128 stages are too many for eight
+    (1, 14, 2, 64, 8192, 512, False, 18, 8, 2),          # 32 parts: more than 18 SMs, not more than three parts on each
+    (1, 14, 2, 64, 16384, 512, False, 18, 8, 3),         # 64 parts: more than that
+    (2, 14, 2, 64, 16384, 512, True, 18, 8, 2),          # routed: 22 entries a pair are 88 parts, within two waves
+    (2, 12, 4, 256, 16384, 512, False, 148, 16, 3),      # above head dimension 128 one part per SM
+    (64, 12, 2, 128, 65536, 2048, True, 148, 16, 3),
+])
+def test_attention_kernel_rule(requests, hq, hk, dim, capacity, chunk, routed, sms, most_cluster, want):
+    """Which decode attention kernel serves a shape, on a whole GPU and on a part of one: a cluster that the device cannot
+    hold is never chosen."""
+    from moba_opt.kv_cache import CacheDesc, decode_library
+    lib = decode_library()
+    chunks = -(-capacity // chunk)
+    desc = CacheDesc(requests, capacity, 16, 1, 1, chunk, chunks, hk, dim, 0, 1, 1, 1, 1, 1)
+    umax = lib.moba_decode_union_capacity(hq, hk, 3, chunks) if routed else 1
+    slots = 4 if routed else chunks
+    assert lib.moba_decode_attend_variant(ctypes.byref(desc), requests, hq, int(routed), slots, umax, sms, most_cluster) == want
