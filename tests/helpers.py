@@ -86,3 +86,21 @@ def two_threads(calls, times=20000):
         t.join()
     torch.cuda.synchronize()
     return failed
+
+
+# MOBA_ATTEND_* of the library's header: the decode attention kernels
+FIXED_DEEP, FIXED, STREAMED, CLUSTER_8, CLUSTER_16 = 1, 2, 3, 8, 16
+
+
+def attend_kernels(cache):
+    """A list that grows by the kernel of every attention that `cache` launches from now on, as the library answers for the
+    arguments of that launch."""
+    taken, launch = [], cache._launch
+
+    def recorded(name, *args):
+        if name == "moba_decode_attend":
+            desc, rows, hq, selected, slots, umax = args[0], args[4], args[5], args[6], args[7], args[11]
+            taken.append(cache._lib.moba_decode_attend_variant(desc, rows, hq, int(selected is not None), slots, umax, 0, -1))
+        return launch(name, *args)
+    cache._launch = recorded
+    return taken

@@ -7,7 +7,8 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import DECODE_GOLDENS, bits_to_torch, load, torch_to_f64, two_threads
+from helpers import (CLUSTER_8, CLUSTER_16, DECODE_GOLDENS, FIXED, FIXED_DEEP, STREAMED, attend_kernels, bits_to_torch, load, torch_to_f64,
+                     two_threads)
 from oracle import moba_oracle as mo
 
 pytestmark = pytest.mark.gpu
@@ -285,16 +286,49 @@ def test_chunk_size_extremes(chunk, dim, length, page):
     check(cache, cache.attend(q, sequence_ids=[0], mode="dense"), q)
 
 
-@pytest.mark.parametrize("hq,dim,chunk,length", [(32, 32, 4, 700), (8, 64, 1, 1100), (7, 64, 2, 300)])
-def test_dense_merge_over_more_partials_than_fit_in_shared_memory(hq, dim, chunk, length):
-    """The merge keeps the weights of a head's partials in shared memory up to a capacity that shrinks with the
-    group size; the partials beyond it take the recomputing path.  (32 heads, dim 32: capacity 128 of 176
-    partials; 8 heads, dim 64: 1024 of 1101; the last case stays inside the capacity.)"""
+@pytest.mark.parametrize("hq,dim,chunk,length,kernel", [
+    (32, 32, 4, 700, CLUSTER_16), (8, 64, 1, 1100, CLUSTER_16), (7, 64, 2, 300, CLUSTER_16),   # merged without partials in memory
+    (32, 32, 64, 12790, FIXED),          # weights of 64 of 200 partials fit, and no sums
+    (16, 64, 64, 19190, FIXED),          # 256 of 300
+    (32, 32, 128, 12790, FIXED_DEEP),    # the weights of all 100 partials, the sums of 9
+    (32, 32, 64, 66500, STREAMED),       # 260 shares of the one pair, weights of 256 would fit
+])
+def test_dense_merge_over_more_partials_than_fit_in_shared_memory(hq, dim, chunk, length, kernel):
+    """The merge keeps weights and sums of a head's partials in shared memory up to a capacity that shrinks with the group
+    size; the partials beyond it are read and weighted from memory.  A cluster keeps none."""
     from moba_opt import PagedKVCache
     cache = PagedKVCache(1, length + 1, 1, dim, page_size=16, chunk_size=chunk)
     cache.append(rand((length, 1, dim), 271), rand((length, 1, dim), 272), sequence_ids=[0], cu_seqlens=[0, length])
+    taken = attend_kernels(cache)
     q = rand((1, hq, dim), 273)
     check(cache, cache.attend(q, sequence_ids=[0], mode="dense"), q)
+    assert taken == [kernel]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("dim", [32, 64, 128, 256])
+@pytest.mark.parametrize("mode,chunk,topk,kernel", [
+    ("dense", 2048, 4, FIXED_DEEP),      # 12 pairs x 6 chunks x 2 parts of 1024 tokens: a ring wraps in each team
+    ("moba", 2048, 3, FIXED_DEEP),
+    ("dense", 512, 4, FIXED),            # 288 CTAs
+    ("moba", 512, 9, FIXED),
+])
+def test_fixed_parts(mode, chunk, topk, kernel, dim, dtype):
+    """A CTA per part of a chunk, whole parts and ragged last ones, with one team of warps and with two (above head dimension
+    128 always one, and a dense grid of more than one CTA per SM is streamed)."""
+    from moba_opt import PagedKVCache
+    lens = [12000, 5003, 70]
+    cache = PagedKVCache(3, 12288, 4, dim, page_size=48, chunk_size=chunk, dtype=dtype)
+    cu = np.concatenate(([0], np.cumsum(lens))).tolist()
+    k, v = rand((cu[-1], 4, dim), 275, dtype), rand((cu[-1], 4, dim), 276, dtype)
+    cache.append_prefill(k, v, sequence_ids=[0, 1, 2], cu_seqlens=cu)
+    taken = attend_kernels(cache)
+    q = rand((3, 8, dim), 277, dtype)
+    result = cache.attend(q, sequence_ids=[0, 1, 2], topk=topk, mode=mode)
+    check(cache, result, q)
+    again = cache.attend(q, sequence_ids=[0, 1, 2], topk=topk, mode=mode)
+    assert torch.equal(result.output, again.output) and torch.equal(result.lse, again.lse)
+    assert taken == [STREAMED if (dim, mode, kernel) == (256, "dense", FIXED) else kernel] * 2
 
 
 @pytest.mark.parametrize("page,chunk,dim,hk", [(16, 32, 64, 2), (7, 24, 40, 3), (48, 128, 128, 1), (3, 1, 8, 2), (16, 512, 64, 2)])
@@ -420,7 +454,43 @@ def test_one_finite_check_for_all_inputs(dtype, layout):
     cache._finite.require(named)
 
 
-@pytest.mark.parametrize("repeat", [1, 8])      # a grid of fixed parts that fits the GPU at once, one that does not
+def test_the_first_input_at_fault_is_reported():
+    """One finite check covers all inputs of a call, but a tensor's NaN comes before the faults of the tensors after it, and a
+    fault of shape before the NaN of a later one; nothing reaches the cache or the plan's positions."""
+    from moba_opt import PagedKVCache
+    cache = PagedKVCache(1, 64, 2, 16)
+    k, v, q = rand((3, 2, 16), 341), rand((3, 2, 16), 342), rand((3, 4, 16), 343)
+    cache.append(k, v, sequence_ids=[0], cu_seqlens=[0, 3])
+    before = [t.clone() for t in cache.materialize(0)]
+    nan = float("nan")
+    bad_k, bad_v, bad_q = torch.full_like(k, nan), torch.full_like(v, nan), torch.full_like(q, nan)
+    faults = [
+        (dict(q=q, k=bad_k, v=v[:, :1]), "k contains NaN/Inf"),
+        (dict(q=q, k=k[:, :1], v=bad_v), "k KV head count differs"),
+        (dict(q=q[:2], k=k, v=bad_v), "v contains NaN/Inf"),
+        (dict(q=bad_q, k=k, v=v[:2]), "v token count differs"),
+        (dict(q=bad_q, k=bad_k, v=bad_v), "k contains NaN/Inf"),
+        (dict(q=bad_q, k=k, v=v), "q contains NaN/Inf"),
+        (dict(q=q[:, :3], k=k, v=v), "multiple of Hkv"),
+    ]
+    for tensors, message in faults:
+        with pytest.raises(ValueError, match=message):
+            cache.append_and_attend(**tensors, sequence_ids=[0], cu_seqlens=[0, 3])
+    with pytest.raises(ValueError, match="k contains NaN/Inf"):
+        cache.append(bad_k, v[:, :1], sequence_ids=[0], cu_seqlens=[0, 3])
+    plan = cache.prepare_decode([0], 4, check_finite=True)
+    step = [t[:1].contiguous() for t in (q, k, v, bad_q, bad_k)]
+    for tensors, message in [((step[3], step[1][:, :1], step[2]), "q contains NaN/Inf"), ((step[0][:, :3], step[4], step[2]), "q must have fixed shape"),
+                             ((step[0], step[4], step[2][:, :1]), "k contains NaN/Inf")]:
+        with pytest.raises(ValueError, match=message):
+            plan.step(*tensors)
+    plan.close()
+    assert cache.lengths == (3,)
+    for got, want in zip(cache.materialize(0), before):
+        assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("repeat", [1, 8])      # 22 queries: fixed parts, but for three of the dense grids; 176: streamed
 @pytest.mark.parametrize("mode", ["moba", "dense"])
 @pytest.mark.parametrize("hq,hkv,dim,chunk,page,dtype", [
     (4, 2, 64, 100, 7, torch.bfloat16),      # the last stage of a chunk is part of one
@@ -441,10 +511,12 @@ def test_attend_divides_uneven_work(repeat, mode, hq, hkv, dim, chunk, page, dty
     ids = (list(range(len(lens))) + [4, 11, 11, 8]) * repeat           # several queries of a request, some not at its end
     positions = ([n - 1 for n in lens] + [450, 1000, 63, 0]) * repeat
     q = rand((len(ids), hq, dim), 73, dtype)
+    taken = attend_kernels(cache)
     result = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
     check(cache, result, q)
     again = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
     assert torch.equal(result.output, again.output) and torch.equal(result.lse, again.lse)
+    assert taken == [FIXED if repeat == 1 and (mode == "moba" or dim in (32, 96)) else STREAMED] * 2
 
 
 @pytest.mark.parametrize("mode", ["moba", "dense"])
@@ -464,10 +536,12 @@ def test_cluster_attend_divides_a_request(lens, mode, hq, hkv, dim, chunk, page,
     k, v = rand((cu[-1], hkv, dim), 81, dtype), rand((cu[-1], hkv, dim), 82, dtype)
     cache.append_prefill(k, v, sequence_ids=list(range(len(lens))), cu_seqlens=cu)
     q = rand((len(lens), hq, dim), 83, dtype)
+    taken = attend_kernels(cache)
     result = cache.attend(q, sequence_ids=list(range(len(lens))), topk=4, mode=mode)
     check(cache, result, q)
     again = cache.attend(q, sequence_ids=list(range(len(lens))), topk=4, mode=mode)
     assert torch.equal(result.output, again.output) and torch.equal(result.lse, again.lse)
+    assert taken == [CLUSTER_16 if len(lens) * hkv <= 4 else CLUSTER_8] * 2
 
 
 @pytest.mark.parametrize("layout", ["fused", "heads_first", "expanded", "unaligned"])
@@ -517,8 +591,10 @@ def test_probabilities_keep_more_than_16_bits(requests, queries, hq, hkv, dim, l
     ids = [i for i in range(requests) for _ in range(queries)]
     positions = [lens[i] - 1 - 500 * j for i in range(requests) for j in range(queries)]
     q = rand((len(ids), hq, dim), 303, dtype)
+    taken = attend_kernels(cache)
     result = cache.attend(q, sequence_ids=ids, positions=positions, topk=4, mode=mode)
     check(cache, result, q)
+    assert taken[0] in ((STREAMED,) if requests == 12 else (CLUSTER_8, CLUSTER_16))
     keys, values = zip(*[[torch_to_f64(t) for t in cache.materialize(i)] for i in range(requests)])
     sel = None if result.selected_blocks is None else result.selected_blocks.cpu().numpy()
     want, _ = mo.decode_attend(torch_to_f64(q), keys, values, ids, positions, 512, sel)
@@ -528,16 +604,16 @@ def test_probabilities_keep_more_than_16_bits(requests, queries, hq, hkv, dim, l
 
 
 @pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
-@pytest.mark.parametrize("rows,hq,hkv,dim,dtype", [
-    (1, 8, 2, 64, torch.bfloat16),       # a cluster per pair
-    (2, 6, 1, 128, torch.float16),
-    (20, 8, 2, 64, torch.bfloat16),      # fixed parts
-    (4, 40, 2, 128, torch.bfloat16),     # two head blocks
-    (20, 40, 2, 128, torch.bfloat16),    # fixed parts, two head blocks
-    (120, 8, 2, 64, torch.float16),      # streamed
-    (60, 40, 2, 96, torch.bfloat16),     # streamed, two head blocks
+@pytest.mark.parametrize("rows,hq,hkv,dim,dtype,kernel", [
+    (1, 8, 2, 64, torch.bfloat16, CLUSTER_16),
+    (2, 6, 1, 128, torch.float16, CLUSTER_16),
+    (20, 8, 2, 64, torch.bfloat16, FIXED),
+    (4, 40, 2, 128, torch.bfloat16, CLUSTER_8),      # two head blocks
+    (20, 40, 2, 128, torch.bfloat16, FIXED),
+    (120, 8, 2, 64, torch.float16, STREAMED),
+    (80, 40, 2, 96, torch.bfloat16, STREAMED),       # two head blocks
 ])
-def test_values_of_a_chunk_reach_only_the_heads_that_selected_it(rows, hq, hkv, dim, dtype, bad):
+def test_values_of_a_chunk_reach_only_the_heads_that_selected_it(rows, hq, hkv, dim, dtype, kernel, bad):
     """A V that is not finite (a caller may switch the check off) spoils the heads that attend its chunk; the others keep
     their bits, whichever kernel runs."""
     from moba_opt import PagedKVCache
@@ -558,7 +634,9 @@ def test_values_of_a_chunk_reach_only_the_heads_that_selected_it(rows, hq, hkv, 
         cache = PagedKVCache(2, length, hkv, dim, page_size=7, chunk_size=chunk, dtype=dtype)
         cache.check_finite = False
         cache.append(torch.cat((k, k)), torch.cat((vv, vv)), sequence_ids=[0, 1], cu_seqlens=[0, length, 2 * length])
+        taken = attend_kernels(cache)
         caches.append(cache.attend(q, sequence_ids=[i % 2 for i in range(rows)], topk=2))
+        assert taken == [kernel]
     good, spoiled = caches
     reads = (good.selected_blocks == poisoned).any(-1)
     assert torch.equal(good.selected_blocks, spoiled.selected_blocks) and reads.any() and not reads.all()
