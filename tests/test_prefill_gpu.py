@@ -242,6 +242,40 @@ def test_backward_divided_over_a_cluster(lens, hq, hkv, dim, chunk, topk):
     assert torch.equal(grads[1], again[1]) and torch.equal(grads[2], again[2])
 
 
+_RAGGED = (1500, 1300, 1200, 1000)
+
+
+@pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk,blocks", [
+    (_RAGGED, 16, 8, 64, 200, 3, 400),   # one CTA per key block; a chunk's second block has 72 keys
+    (_RAGGED, 8, 8, 32, 130, 4, 616),    # two keys in a chunk's second block, padded head dimension
+    (_RAGGED, 16, 8, 128, 200, 3, 400),
+    (_RAGGED, 8, 8, 96, 130, 4, 616),
+    ((1184,), 2, 1, 64, 16, 5, 74),      # the last batch whose blocks take clusters of four, the first of two
+    ((1200,), 2, 1, 128, 16, 5, 75),
+    ((1184,), 4, 4, 128, 16, 5, 296),    # the last of two, the first of one
+    ((1584,), 3, 3, 64, 16, 5, 297),
+])
+@pytest.mark.parametrize("dtype,deterministic", [(torch.bfloat16, False), (torch.float16, False), (torch.bfloat16, True)],
+                         ids=["bf16", "fp16", "deterministic"])
+def test_backward_on_both_sides_of_the_cluster_rule(lens, hq, hkv, dim, chunk, topk, blocks, dtype, deterministic):
+    """The undivided kernels of ordinary training batches, and the block counts at which the division changes."""
+    from moba_opt.grouped_attention import get_plan
+    rng = torch.Generator().manual_seed(98)
+    total = sum(lens)
+    q, k, v = [torch.randn(total, h, dim, generator=rng).to(dtype) for h in (hq, hkv, hkv)]
+    do = torch.randn(total, hq, dim, generator=rng).to(dtype)
+    cu = cu_from_lens(lens)
+    assert get_plan(tuple(int(x) for x in cu), chunk, torch.device("cuda", 0)).num_qtiles * hkv == blocks
+    flags = dict(deterministic_backward=True) if deterministic else {}
+    _, _, captured, grads = _run(q, k, v, cu, chunk, topk, d_out=do, **flags)
+    qf, kf, vf, dof = (torch_to_f64(t) for t in (q, k, v, do))
+    r = mo.route_prefill(qf, kf, cu, chunk, topk)
+    sel = mo.sel_from_selected(captured["selected"].numpy(), r["filtered"], r["sel"].shape[-1])
+    ref = mo.attention_fixed_route(qf, kf, vf, cu, sel, chunk, d_out=dof)
+    for key, got in zip(("dq", "dk", "dv"), grads):
+        _check_close(key, torch_to_f64(got), ref[key])
+
+
 @pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk", [((1500, 800), 4, 2, 64, 256, 3), ((1024,), 8, 2, 128, 128, 5)])
 def test_deterministic_backward_is_bit_repeatable(lens, hq, hkv, dim, chunk, topk):
     """deterministic_backward=True (the counterpart of deterministic=True in the reference's two backward calls,
