@@ -123,6 +123,9 @@ size_t moba_prefill_bwd_scratch_bytes(const moba_prefill_desc* d);
 int moba_prefill_bwd(const moba_prefill_desc* d, const void* q, const void* k, const void* v, const void* out,
                      const float* lse, const void* dout, const void* route_state, void* scratch, size_t scratch_bytes,
                      void* dq, void* dk, void* dv, unsigned* status, void* stream);
+/* Over how many CTAs moba_prefill_bwd divides a key block of this shape (1, 2 or 4; minus a MOBA_ERR_* code) on a device of `sms`
+ * SMs; 0: the current device. */
+int moba_prefill_bwd_split(const moba_prefill_desc* d, int sms);
 
 /* ---------------------------------------------------------------------------------------------
  * Decode: paged KV cache, block routing and attention for single-token queries.

@@ -8,6 +8,9 @@
 // reductions of the copy engine), dq = dq_acc rounded to the input format.  With MOBA_BWD_DETERMINISTIC the accumulator
 // is 64-bit fixed point and the reductions are integer, which makes dQ bit-repeatable like everything else (the
 // reference asks FlashAttention for the same: deterministic=True in both backward calls, mixed_attention.py:185,220).
+#include <math.h>
+
+#include "launch.cuh"
 #include "prefill_bwd.cuh"
 
 namespace moba {
@@ -82,6 +85,52 @@ extern "C" size_t moba_prefill_bwd_scratch_bytes(const moba_prefill_desc* d) {
   return bytes;
 }
 
+// How many CTAs a key block's query tiles are divided over.  Few blocks leave SMs idle and last as long as the heaviest one, a
+// block of the earliest chunk, which most later rows attend; but every CTA has its own start and end, and a second wave of
+// them repeats both.  So the time is estimated in query tiles and the division with the smallest estimate taken, a smaller
+// one only where it is 10 % better:
+//   the heaviest block's share and its overhead, or the work of an SM, the overhead of its waves, and the uneven end of the last one.
+// Overhead: 3 tiles, 3 more for a cluster.  Four are tried up to half a block per SM and two up to two per SM.  Backward in us
+// with 1 / 2 / 4 CTAs per block, 148 SMs, chunk 512, topk 4; > marks the choice:
+//   14/2 heads, D = 64     24 blocks 147 / 89 / >58    72: 315 / 179 / >132    80: 331 / >187    296: 588 / >478
+//    6/1 heads, D = 128    24 blocks 428 / 227 / >131  72: 684 / 369 / >220    148: 904 / >499   296: 1172 / >744
+//    8/8 heads, D = 64     48 blocks 27 / >25 / 37     72: 32 / >29 / 49       128: >45 / 51     296: >94 / 105
+//    8/8 heads, D = 128    72 blocks 50 / >41 / 68     96: 62 / >60            160: >88 / 101    296: >176 / 180
+// With the block count alone as the rule, groups of one head took up to 1.55 (D = 128: 1.97) times as long as undivided.  Of 408 shapes
+// (eight head shapes, chunks of 128 to 2048, topk 2 to 8) the worst is now 1.11 times as long as undivided and on average within
+// 0.4 % of the best of the three.
+static int bwd_split(const moba_prefill_desc& d, int sms) {
+  const double blocks = (double)d.num_qtiles * d.hkv, group = d.hq / d.hkv;
+  const int most = 2 * blocks <= sms ? 4 : blocks <= 2.0 * sms ? 2 : 1;
+  if (most == 1) return 1;
+  // expected tiles: a row attends min(j, R) of the j chunks before its own, any of them as likely as another
+  const int longest = d.max_tiles_per_seq * kTile, chunk = d.chunk_size < longest ? d.chunk_size : longest;
+  const double chunk_tiles = chunk / (double)kTile;
+  const int chunk_blocks = (chunk + kTile - 1) / kTile;
+  double first = 0.0, picks = 0.0;
+  for (int j = 1; j < d.max_chunks_per_seq; ++j) first += d.remote_k < j ? (double)d.remote_k / j : 1.0;
+  const int chunks = d.num_chunks > d.num_seqs ? d.num_chunks / d.num_seqs : 1;
+  for (int j = 1; j < chunks; ++j) picks += d.remote_k < j ? d.remote_k : j;
+  const double heaviest = group * (chunk_blocks + chunk_tiles * first);
+  const double work = d.hkv * group * (d.num_chunks * chunk_blocks * (chunk_blocks + 1) / 2.0 +
+                                       d.total_tokens / (double)kTile * picks / chunks * chunk_blocks);
+  int best = 0;
+  double least = 0.0;
+  for (int s = most; s >= 1; s >>= 1) {
+    const double overhead = s > 1 ? 6.0 : 3.0;
+    const double share = heaviest / s + overhead;
+    const double even = work / sms + ceil(blocks * s / sms) * overhead + (blocks * s > sms ? work / blocks / s : 0.0);
+    const double time = share > even ? share : even;
+    if (best == 0 || time < 0.9 * least) { best = s; least = time; }
+  }
+  return best;
+}
+
+extern "C" int moba_prefill_bwd_split(const moba_prefill_desc* d, int sms) {
+  const int rc = validate_desc(d);
+  return rc != MOBA_OK ? -rc : bwd_split(*d, sms > 0 ? sms : device_sms());
+}
+
 extern "C" int moba_prefill_bwd(const moba_prefill_desc* d, const void* q, const void* k, const void* v, const void* out,
                                 const float* lse, const void* dout, const void* route_state, void* scratch,
                                 size_t scratch_bytes, void* dq, void* dk, void* dv, unsigned* status, void* stream) {
@@ -151,7 +200,8 @@ extern "C" int moba_prefill_bwd(const moba_prefill_desc* d, const void* q, const
     a.lsepack = lsepack; a.deltapack = deltapack;
   }
   prof_begin(kProfBwdMain, st);
-  cudaError_t e = d->dim > 64 ? launch_bwd_ws128(a, st) : launch_bwd_ws(a, st);
+  const int split = bwd_split(*d, device_sms());
+  cudaError_t e = d->dim > 64 ? launch_bwd_ws128(a, split, st) : launch_bwd_ws(a, split, st);
   prof_end(kProfBwdMain, st);
   if (e != cudaSuccess) return MOBA_ERR_CUDA;
   const long long n8 = rows * d->dim / 8;

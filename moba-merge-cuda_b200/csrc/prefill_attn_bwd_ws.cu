@@ -504,14 +504,8 @@ static cudaError_t launch_bwd_ws_as(const BwdArgs& a, cudaStream_t st) {
   return launch_clusters(kernel, dim3(a.pv.n_qtiles * SPLIT, a.pv.Hkv), dim3(kWsThreads), SPLIT, smem, st, a);
 }
 
-cudaError_t launch_bwd_ws(const BwdArgs& a, cudaStream_t st) {
-  // A key block per SM or fewer leaves SMs without work, and up to two per SM the earliest chunks, attended by several times
-  // the rows of an average one, still set the time; beyond that the blocks, heaviest first, even out by themselves.  Whole
-  // training pass, 8681 tokens, 6/1 heads, D = 64, 68 blocks: 380 -> 240 us; 1647 tokens, D = 128, 26 blocks: host-bound either way.
-  const long long blocks = (long long)a.pv.n_qtiles * a.pv.Hkv;
-  if (blocks <= kSplit4Blocks) return launch_bwd_ws_as<4>(a, st);
-  if (blocks <= kSplit2Blocks) return launch_bwd_ws_as<2>(a, st);
-  return launch_bwd_ws_as<1>(a, st);
+cudaError_t launch_bwd_ws(const BwdArgs& a, int split, cudaStream_t st) {
+  return split == 4 ? launch_bwd_ws_as<4>(a, st) : split == 2 ? launch_bwd_ws_as<2>(a, st) : launch_bwd_ws_as<1>(a, st);
 }
 
 }  // namespace moba

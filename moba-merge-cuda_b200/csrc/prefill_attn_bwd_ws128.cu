@@ -457,11 +457,8 @@ static cudaError_t launch_bwd_ws128_as(const BwdArgs& a, cudaStream_t st) {
   return launch_clusters(kernel, dim3(a.pv.n_qtiles * SPLIT, a.pv.Hkv), dim3(kThreads), SPLIT, smem, st, a);
 }
 
-cudaError_t launch_bwd_ws128(const BwdArgs& a, cudaStream_t st) {
-  const long long blocks = (long long)a.pv.n_qtiles * a.pv.Hkv;
-  if (blocks <= kSplit4Blocks) return launch_bwd_ws128_as<4>(a, st);
-  if (blocks <= kSplit2Blocks) return launch_bwd_ws128_as<2>(a, st);
-  return launch_bwd_ws128_as<1>(a, st);
+cudaError_t launch_bwd_ws128(const BwdArgs& a, int split, cudaStream_t st) {
+  return split == 4 ? launch_bwd_ws128_as<4>(a, st) : split == 2 ? launch_bwd_ws128_as<2>(a, st) : launch_bwd_ws128_as<1>(a, st);
 }
 
 }  // namespace moba

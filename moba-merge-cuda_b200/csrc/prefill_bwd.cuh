@@ -78,9 +78,9 @@ inline cudaError_t launch_clusters(Kernel kernel, dim3 grid, dim3 block, unsigne
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
-constexpr int kSplit4Blocks = 74, kSplit2Blocks = 296;
-cudaError_t launch_bwd_ws128(const BwdArgs& a, cudaStream_t st);  // 64 < head_dim <= 128
-cudaError_t launch_bwd_ws(const BwdArgs& a, cudaStream_t st);
+// split: CTAs that the query tiles of a key block are divided over, 1, 2 or 4
+cudaError_t launch_bwd_ws128(const BwdArgs& a, int split, cudaStream_t st);  // 64 < head_dim <= 128
+cudaError_t launch_bwd_ws(const BwdArgs& a, int split, cudaStream_t st);
 // Packs dO, LSE and delta of every query tile (rows as listed in a.rowpack).
 cudaError_t launch_bwd_pack(const BwdArgs& a, long long tiles, void* dopack, float* lsepack, float* deltapack, cudaStream_t st);
 

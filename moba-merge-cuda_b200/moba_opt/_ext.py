@@ -44,6 +44,7 @@ def lib():
         L.moba_prefill_route_static_capacity.restype = c_sz
         L.moba_prefill_route_static_capacity.argtypes = []
         L.moba_prefill_fwd.argtypes = [P, c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp]
+        L.moba_prefill_bwd_split.argtypes = [P, ctypes.c_int]
         L.moba_prefill_bwd.argtypes = [P, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp, c_vp]
         L.moba_merge_scratch_bytes.restype = c_sz
         L.moba_merge_scratch_bytes.argtypes = [ctypes.c_longlong, ctypes.c_int]

@@ -127,3 +127,25 @@ def test_attention_kernel_rule(requests, hq, hk, dim, capacity, chunk, routed, s
     umax = lib.moba_decode_union_capacity(hq, hk, 3, chunks) if routed else 1
     slots = 4 if routed else chunks
     assert lib.moba_decode_attend_variant(ctypes.byref(desc), requests, hq, int(routed), slots, umax, sms, most_cluster) == want
+
+
+@pytest.mark.parametrize("lens,hq,hk,chunk,topk,sms,want", [
+    ((4608,), 14, 2, 512, 4, 148, 4),                # 72 key blocks that half a chip cannot fill, the heaviest 77 tiles and more
+    ((5120,), 14, 2, 512, 4, 148, 2),
+    ((18944,), 14, 2, 512, 4, 148, 2),               # 296
+    ((20480,), 14, 2, 512, 4, 148, 1),
+    ((768,), 8, 8, 512, 4, 148, 2),                  # 48 light blocks: four CTAs each would make two waves
+    ((2048,), 8, 8, 256, 3, 148, 1),
+    ((4608,), 14, 2, 512, 4, 74, 2),                 # half the device
+    ((4608,), 14, 2, 512, 4, 18, 1),
+    ((300, 150, 7), 4, 2, 4096, 1, 148, 4),          # dense
+])
+def test_backward_division_rule(lens, hq, hk, chunk, topk, sms, want):
+    import torch
+    from itertools import accumulate
+    from moba_opt import _ext
+    from moba_opt.grouped_attention import PrefillPlan
+    plan = PrefillPlan([0, *accumulate(lens)], min(chunk, max(lens)), "cpu")
+    q, k = (torch.empty(sum(lens), h, 64, dtype=torch.bfloat16) for h in (hq, hk))
+    call = plan.call(q, k, k, min(topk - 1, plan.num_routable))
+    assert _ext.lib().moba_prefill_bwd_split(call.ref, sms) == want

@@ -214,20 +214,37 @@ def test_gradients_against_oracle_on_seeded_inputs(lens, hq, hkv, dim, chunk, to
         _check_close(key, torch_to_f64(got), ref[key])
 
 
-@pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk", [
-    ((7,), 1, 1, 64, 64, 3),             # one query tile for a cluster of four
-    ((40, 130), 1, 1, 128, 64, 2),
-    ((129, 257), 3, 1, 128, 128, 3),     # shares of unequal size
-    ((1100, 1200), 8, 8, 64, 200, 3),    # clusters of two
-    ((1250,), 10, 10, 96, 256, 3),
+def _split(q, k, v, cu, chunk, topk):
+    """Over how many CTAs the backward divides a key block of this batch."""
+    import moba_opt.grouped_attention as ga
+    cu = tuple(int(x) for x in cu)
+    plan = ga.get_plan(cu, chunk, torch.device("cuda", 0))
+    remote_k = min(topk - 1, plan.num_routable)
+    if remote_k == 0:
+        plan = ga.get_plan(cu, max(b - a for a, b in zip(cu, cu[1:])), torch.device("cuda", 0))
+    return ga._ext.lib().moba_prefill_bwd_split(plan.call(q, k, v, remote_k).ref, 0)
+
+
+@pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk,split", [
+    ((7,), 1, 1, 64, 64, 3, 1),             # one query tile
+    ((40, 130), 1, 1, 128, 64, 2, 1),
+    ((7,), 32, 1, 64, 64, 3, 4),            # 32 of them
+    ((40, 130), 16, 1, 128, 64, 2, 4),
+    ((129, 257), 3, 1, 128, 128, 3, 4),     # shares of unequal size
+    ((129, 257), 6, 1, 64, 128, 3, 4),
+    ((1100, 1200), 8, 8, 64, 200, 3, 1),    # as few blocks, but too little in each
+    ((1250,), 10, 10, 96, 256, 3, 1),
+    ((1100, 1200), 16, 4, 64, 200, 3, 2),
+    ((1100, 1200), 16, 4, 96, 200, 3, 2),
 ])
-def test_backward_divided_over_a_cluster(lens, hq, hkv, dim, chunk, topk):
+def test_backward_divided_over_a_cluster(lens, hq, hkv, dim, chunk, topk, split):
     """Few key blocks: the query tiles of a block over the CTAs of a cluster; dK and dV stay bit-repeatable."""
     rng = torch.Generator().manual_seed(99)
     total = sum(lens)
     q, k, v = [torch.randn(total, h, dim, generator=rng).bfloat16() for h in (hq, hkv, hkv)]
     do = torch.randn(total, hq, dim, generator=rng).bfloat16()
     cu = cu_from_lens(lens)
+    assert _split(q, k, v, cu, chunk, topk) == split
     out, lse, captured, grads = _run(q, k, v, cu, chunk, topk, d_out=do)
     qf, kf, vf, dof = (torch_to_f64(t) for t in (q, k, v, do))
     if max(lens) <= chunk:
@@ -245,27 +262,28 @@ def test_backward_divided_over_a_cluster(lens, hq, hkv, dim, chunk, topk):
 _RAGGED = (1500, 1300, 1200, 1000)
 
 
-@pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk,blocks", [
-    (_RAGGED, 16, 8, 64, 200, 3, 400),   # one CTA per key block; a chunk's second block has 72 keys
-    (_RAGGED, 8, 8, 32, 130, 4, 616),    # two keys in a chunk's second block, padded head dimension
-    (_RAGGED, 16, 8, 128, 200, 3, 400),
-    (_RAGGED, 8, 8, 96, 130, 4, 616),
-    ((1184,), 2, 1, 64, 16, 5, 74),      # the last batch whose blocks take clusters of four, the first of two
-    ((1200,), 2, 1, 128, 16, 5, 75),
-    ((1184,), 4, 4, 128, 16, 5, 296),    # the last of two, the first of one
-    ((1584,), 3, 3, 64, 16, 5, 297),
+@pytest.mark.parametrize("lens,hq,hkv,dim,chunk,topk,split", [
+    (_RAGGED, 16, 8, 64, 200, 3, 1),     # one CTA per key block, 400 of them; a chunk's second block has 72 keys
+    (_RAGGED, 8, 8, 32, 130, 4, 1),      # two keys in a chunk's second block, padded head dimension
+    (_RAGGED, 16, 8, 128, 200, 3, 1),
+    (_RAGGED, 8, 8, 96, 130, 4, 1),
+    ((1100, 1200), 16, 4, 64, 200, 3, 2),
+    ((1100, 1200), 16, 4, 96, 200, 3, 2),
+    ((1500, 800), 8, 2, 64, 256, 3, 4),
+    ((1250,), 12, 4, 32, 256, 3, 4),
+    ((1024,), 8, 2, 128, 128, 5, 4),
+    ((1250,), 12, 4, 96, 256, 3, 4),
 ])
 @pytest.mark.parametrize("dtype,deterministic", [(torch.bfloat16, False), (torch.float16, False), (torch.bfloat16, True)],
                          ids=["bf16", "fp16", "deterministic"])
-def test_backward_on_both_sides_of_the_cluster_rule(lens, hq, hkv, dim, chunk, topk, blocks, dtype, deterministic):
-    """The undivided kernels of ordinary training batches, and the block counts at which the division changes."""
-    from moba_opt.grouped_attention import get_plan
+def test_backward_undivided_and_divided(lens, hq, hkv, dim, chunk, topk, split, dtype, deterministic):
+    """The undivided kernels of ordinary training batches and the divided ones, in both formats and with fixed-point dQ."""
     rng = torch.Generator().manual_seed(98)
     total = sum(lens)
     q, k, v = [torch.randn(total, h, dim, generator=rng).to(dtype) for h in (hq, hkv, hkv)]
     do = torch.randn(total, hq, dim, generator=rng).to(dtype)
     cu = cu_from_lens(lens)
-    assert get_plan(tuple(int(x) for x in cu), chunk, torch.device("cuda", 0)).num_qtiles * hkv == blocks
+    assert _split(q, k, v, cu, chunk, topk) == split
     flags = dict(deterministic_backward=True) if deterministic else {}
     _, _, captured, grads = _run(q, k, v, cu, chunk, topk, d_out=do, **flags)
     qf, kf, vf, dof = (torch_to_f64(t) for t in (q, k, v, do))
