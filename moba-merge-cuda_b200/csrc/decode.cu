@@ -14,6 +14,8 @@
 // a chunk while that grid fits the GPU at once, equal shares of one list of stages beyond.  The last two leave partial (max, sum,
 // accumulator) triples in a workspace, and the CTA that finishes a (query, kv head) pair last - found with an atomic
 // ticket, nobody waits - merges them in a fixed order.
+#include <limits.h>
+
 #include <atomic>
 
 #include "launch.cuh"
@@ -565,7 +567,8 @@ struct AttendArgs {
   float* lse;
   unsigned* status;
   float scale_log2;
-  int rowgs, spc, min_stages;  // streamed variant: (row, kv head) pairs, stages of a whole chunk, least stages per CTA
+  int step_pg, step_r;         // a stage in pages and tokens
+  int rowgs, spc;              // streamed variant: (row, kv head) pairs, stages of a whole chunk
 };
 
 constexpr int kHeadBlock = 16;    // query heads of a group processed together (MMA M dimension)
@@ -598,6 +601,7 @@ struct StageCursor {
   int nv;                 // of the stage looked up last: its tokens, from its first one
   unsigned heads;         // and the heads that attend it
   bool bad;
+  int at, pg, r;          // first token of that stage, page and offset in it of this thread's token
   __device__ __forceinline__ void fetch() {
     if (!chunks) { chunk = entry; return; }
     if (entry < entries) { chunk = chunks[entry]; mask = masks[entry]; }
@@ -607,22 +611,32 @@ struct StageCursor {
     off = stage - entry * spc;
     bad = false;
     nv = 0; heads = 0u;
+    at = INT_MIN;
     fetch();
   }
   // Element offset of the K/V row (kv head g) of token `lane_token` of the next stage, or -1.  No branch depends on the
   // table entry, so several lookups can be in flight; the table is read through the ordinary cached path (a page serves many
-  // tokens), not the read-only one, which a dependent launch must avoid.
-  __device__ __forceinline__ long long next(const CacheView& cv, int sid, int g, int lane_token) {
+  // tokens), not the read-only one, which a dependent launch must avoid.  From a stage to the one behind it page and offset
+  // are stepped; only the first one of a run of chunks divides (with a division in every stage: 64 requests 263 -> 260 us).
+  __device__ __forceinline__ long long next(const AttendArgs& a, int sid, int g, int lane_token) {
+    const CacheView& cv = a.cv;
     const int t0 = chunk * span + off * kStageTokens, t = t0 + lane_token;
     const int limit = min((chunk + 1) * span, visible);
-    const int pg = t / cv.page;
+    if (t0 == at + kStageTokens) {
+      pg += a.step_pg; r += a.step_r;
+      if (r >= cv.page) { r -= cv.page; ++pg; }
+    } else {
+      pg = t / cv.page;
+      r = t - pg * cv.page;
+    }
+    at = t0;
     const int physical = t <= pos && pg < cv.width ? cv.table[(long long)sid * cv.width + pg] : 0;
     const bool exists = t < limit, wrong = exists && (physical < 0 || physical >= cv.num_pages);
     bad |= wrong;
     nv = limit - t0;
     heads = mask;
     if (++off == spc) { off = 0; ++entry; fetch(); }
-    return exists && !wrong ? (((long long)physical * cv.page + (t - pg * cv.page)) * cv.Hkv + g) * cv.D : -1;
+    return exists && !wrong ? (((long long)physical * cv.page + r) * cv.Hkv + g) * cv.D : -1;
   }
 };
 
@@ -1135,7 +1149,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
   if (ltid < kStageTokens) {
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      first_base[s] = s < ntiles ? look.next(cv, sid, g, ltid) : -1;
+      first_base[s] = s < ntiles ? look.next(a, sid, g, ltid) : -1;
       first_nv[s] = look.nv; first_heads[s] = look.heads;
     }
   }
@@ -1180,7 +1194,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
     // look up the rows of tile nx+1 now, publish them after this tile's math (ring slot i % NS is free)
     long long next_base = -1;
     const bool more = ltid < kStageTokens && nx + 1 < ntiles;
-    if (more) next_base = look.next(cv, sid, g, ltid);
+    if (more) next_base = look.next(a, sid, g, ltid);
     const int tok0 = wt * 16;
     const int nvalid = s_nv[i % META] - tok0;
     const unsigned heads = s_mask[i % META] >> hb;
@@ -1418,13 +1432,18 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
 // partly empty, and the merge of a long context had a partial per chunk.  Here the stages (64 tokens) of every (row, kv head) pair - of its
 // union of chunks, or of its whole context in dense mode - laid end to end are one list, and each of the CTAs that fit the
 // GPU at once takes an equal, consecutive share of it.  Eight requests of 16K-32K tokens, dense, 28/4 heads, D = 128:
-// 98.7 -> 80 us (4.1 -> 5.0 TB/s), step 111 -> 96 us; 64 requests of 4K-64K, routed, 12/2 heads, D = 128: step 265 -> 251 us.
-// (The first form of the kernel measured 78 us and steps of 94 and 243 us; sharing its loop with the cluster variant cost the rest.
-// The merge through the copy ring, a batch of partials at a time, was slower than reading them where they lie: one request of 32K,
-// 14/2 heads, dense, 39 against 25 us.)
+// step 111 -> 95 us; 64 requests of 4K-64K, routed, 12/2 heads, D = 128: step 265 -> 250 us.
+// (With a loop of its own, without the cluster variant's, the steps were 94 and 243 us.  The merge through the copy ring, a batch of
+// partials at a time, was slower than reading them where they lie: one request of 32K, 14/2 heads, dense, 39 against 25 us; so was dividing
+// its loads over the warps by partial, with twice as many in flight and more code: 41 against 34 us, eight requests of 9K in a cache for 64K.)
 // A share may begin and end anywhere; what a CTA holds of one pair is a segment, with one partial per head in slot
 // (CTA + pair), which no other segment has, and the slots of a pair are consecutive.  The division depends on the
 // positions alone, so a result is bit-repeatable.
+// A share has at least kStreamLeast stages, or an eighth of an average pair where that is less: shorter ones are mostly their
+// start and their partials (dense, four requests of 9000 tokens, 14/2 heads: 24.8 us with four, 28.0 with two), but where pairs are
+// short, longer ones begin and end in several pairs, one after the other (eight requests of 300 tokens in a cache for 65536: 18.5 us with
+// four, 13.5 with one; fixed parts 16.4).
+constexpr int kStreamLeast = 4;
 struct StreamShare {
   int total, ctas, base, rem;
   __device__ __forceinline__ StreamShare(int stages, int grid, int least) : total(stages) {
@@ -1478,7 +1497,8 @@ __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_k
   __syncthreads();
   int before = incl - mine;
   for (int w = 0; w < warp; ++w) before += s_sum[w];
-  const StreamShare share(s_sum[0] + s_sum[1] + s_sum[2] + s_sum[3], gridDim.x, a.min_stages);
+  const int total = s_sum[0] + s_sum[1] + s_sum[2] + s_sum[3];
+  const StreamShare share(total, gridDim.x, min(kStreamLeast, max(1, total / (8 * a.rowgs))));
   if ((int)blockIdx.x >= share.ctas) return;
   int at = share.first(blockIdx.x);
   const int end = share.first(blockIdx.x + 1);
@@ -1540,11 +1560,16 @@ __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_k
     float* s_w = reinterpret_cast<float*>(s_pipe);          // [G][np] weights, where they fit
     const bool kept = (size_t)np * G * 4 <= (size_t)NS * STAGE_BYTES;
     for (int hl = warp; hl < G; hl += 4) {
-      float big = -INFINITY, lsum = 0.f;
-      for (int j = lane; j < np; j += 32) big = fmaxf(big, __ldcg(a.pm + first + (long long)j * G + hl));
+      const float m0 = lane < np ? __ldcg(a.pm + first + (long long)lane * G + hl) : -INFINITY;
+      const float l0 = lane < np ? __ldcg(a.pl + first + (long long)lane * G + hl) : 0.f;
+      float big = m0;
+      for (int j = lane + 32; j < np; j += 32) big = fmaxf(big, __ldcg(a.pm + first + (long long)j * G + hl));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xFFFFFFFFu, big, o));
-      for (int j = lane; j < np; j += 32) {
+      const float w0 = m0 == -INFINITY ? 0.f : dec_exp2(m0 - big);
+      float lsum = l0 * w0;
+      if (kept && lane < np) s_w[hl * np + lane] = w0;
+      for (int j = lane + 32; j < np; j += 32) {
         const float m = __ldcg(a.pm + first + (long long)j * G + hl);
         const float w = m == -INFINITY ? 0.f : dec_exp2(m - big);
         lsum = fmaf(__ldcg(a.pl + first + (long long)j * G + hl), w, lsum);
@@ -1566,8 +1591,15 @@ __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_k
       const float* src = a.pacc + (first + hl) * D + d;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (kept) {
-#pragma unroll 8
-        for (int j = 0; j < np; ++j) merge_add(v, __ldcg(reinterpret_cast<const float4*>(src + (long long)j * G * D)), s_w[hl * np + j]);
+#pragma unroll 1
+        for (int j0 = 0; j0 < np; j0 += 8) {
+          float4 x[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)  // no remainder loop: its loads would wait for each other
+            x[i] = __ldcg(reinterpret_cast<const float4*>(src + (long long)min(j0 + i, np - 1) * G * D));
+#pragma unroll
+          for (int i = 0; i < 8; ++i) merge_add(v, x[i], j0 + i < np ? s_w[hl * np + j0 + i] : 0.f);
+        }
       } else {
         const float big = s_big[hl];
         for (int j = 0; j < np; ++j) {
@@ -1735,8 +1767,6 @@ static int attend_parts(const moba_cache_desc* c) {
   return (c->chunk_size + part_tokens - 1) / part_tokens;
 }
 
-// A share below four stages would be mostly its start and its partials (2, 4, 8 and 16 within 1 % at the sizes above).
-constexpr int kStreamLeast = 4;
 constexpr int kClusterMost = 11;
 // What the GPU holds of the one-team kernels at once: three CTAs per SM, one above head dimension 128.
 static int attend_wave(int dim, int sms) { return dim <= 128 ? 3 * sms : sms; }
@@ -1883,7 +1913,8 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   const bool half = (c->flags & MOBA_CACHE_FP16) != 0, wide = hq / c->hkv > 8;
   a.rowgs = rows * c->hkv;
   a.spc = selected ? (c->chunk_size + kStageTokens - 1) / kStageTokens : 1;
-  a.min_stages = kStreamLeast;
+  a.step_pg = kStageTokens / c->page_size;
+  a.step_r = kStageTokens - a.step_pg * c->page_size;
   const int variant = moba_decode_attend_variant(c, rows, hq, selected != nullptr, slots, umax, 0, -1);
   if (variant < 0) return -variant;
   const dim3 grid(a.umax, a.parts, rows * c->hkv);

@@ -544,6 +544,42 @@ def test_cluster_attend_divides_a_request(lens, mode, hq, hkv, dim, chunk, page,
     assert taken == [CLUSTER_16 if len(lens) * hkv <= 4 else CLUSTER_8] * 2
 
 
+@pytest.mark.parametrize("mode,chunk", [("dense", 512), ("moba", 512), ("moba", 100)])
+@pytest.mark.parametrize("rows,kernel", [(1, CLUSTER_16), (160, STREAMED)])
+def test_lookups_step_over_pages_of_any_size(rows, kernel, mode, chunk):
+    """From a stage of 64 tokens to the next the page is stepped, not divided for: any page size gives the same bits."""
+    from moba_opt import PagedKVCache
+    length = 3001
+    k, v, q = rand((length, 2, 64), 361), rand((length, 2, 64), 362), rand((rows, 32, 64), 363)
+    first = None
+    for page in (1, 3, 48, 63, 64, 65, 200, 4096):
+        cache = PagedKVCache(1, 4096, 2, 64, page_size=page, chunk_size=chunk)
+        cache.append_prefill(k, v, sequence_ids=[0], cu_seqlens=[0, length])
+        taken = attend_kernels(cache)
+        result = cache.attend(q, sequence_ids=[0] * rows, positions=[length - 1 - 7 * i for i in range(rows)], topk=4, mode=mode)
+        assert taken == [kernel]
+        if first is None:
+            first = result
+            check(cache, result, q)
+        assert torch.equal(first.output, result.output) and torch.equal(first.lse, result.lse)
+
+
+@pytest.mark.parametrize("requests,length", [(200, 40), (64, 300), (64, 330), (30, 700)])
+def test_streamed_shares_of_short_requests(requests, length):
+    """Requests of a few stages in a cache for many more: a share is an eighth of an average pair, down to one stage."""
+    from moba_opt import PagedKVCache
+    cache = PagedKVCache(requests, 16384, 2, 64, page_size=16, num_pages=requests * 64, chunk_size=512)
+    lens = [length - i % 7 for i in range(requests)]
+    cu = np.concatenate(([0], np.cumsum(lens))).tolist()
+    cache.append_prefill(rand((cu[-1], 2, 64), 371), rand((cu[-1], 2, 64), 372), sequence_ids=list(range(requests)), cu_seqlens=cu)
+    taken = attend_kernels(cache)
+    q = rand((requests, 14, 64), 373)
+    result = cache.attend(q, sequence_ids=list(range(requests)), mode="dense")
+    check(cache, result, q)
+    again = cache.attend(q, sequence_ids=list(range(requests)), mode="dense")
+    assert torch.equal(result.output, again.output) and taken == [STREAMED] * 2
+
+
 @pytest.mark.parametrize("layout", ["fused", "heads_first", "expanded", "unaligned"])
 def test_append_reads_strided_views(layout):
     """Views of a fused projection, a transposed layout, one head for all and rows off the 16-byte grid give the cache that
