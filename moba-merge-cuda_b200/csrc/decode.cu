@@ -1844,8 +1844,11 @@ static bool device_holds_cluster(int dim, int cl, bool wide, bool half) {
 //   eight requests, 12/2, D = 128, routed 16K (304 CTAs) - / 29.9 / 36.8; beyond one wave the streamed variant: the first
 //   at 32K (520 CTAs) - / 49.4 / 41.4, eight requests dense 16K (528 CTAs) - / 52.7 / 44.6.  A routed grid is a bound that
 //   heads with picks in common and short contexts stay below, so there the line is two waves: 21 requests up to 5.5K, 8/2, D = 128
-//   (546 CTAs) - / 36.7 / 38.9, 18 requests of 32K, 6/1, D = 32 (774 CTAs) - / 37.9 / 38.9, 42 requests of 53K, 28/4, D = 128
-//   (1344 CTAs) - / 96.7 / 93.2.
+//   (546 CTAs) - / 36.7 / 38.9, 18 requests of 32K, 6/1, D = 32 (774 CTAs) - / 37.9 / 38.9.  With few pairs the streamed kernel merges
+//   many shares of each, and the line is two and a half: 11 requests, 28/4, D = 128, chunk 512, 16K (44 pairs, 968 CTAs) - / 57.1 / 59.4,
+//   but 14 of them (56 pairs, 1232 CTAs) - / 71.8 / 67.9.
+// Contexts far below the capacity that the rule goes by are the streamed kernel's worst case: with 5K of 16K tokens the first of these takes
+// 38.8 / 44.1, the second 52.3 / 49.2; dense, eight requests, 12/2, D = 128, cache for 64K: 9K tokens 31.7 / 33.9, 2K 26.9 / 22.0, 300 19.8 / 15.8.
 // holds(cl): whether the device can hold a cluster of cl CTAs.
 template <class Holds>
 static int attend_variant(const moba_cache_desc* c, int rows, bool routed, int slots, int umax, int sms, Holds holds) {
@@ -1858,7 +1861,8 @@ static int attend_variant(const moba_cache_desc* c, int rows, bool routed, int s
   }
   const long long ctas = (long long)(routed ? umax : slots) * attend_parts(c) * pairs;
   if (ctas <= sms) return MOBA_ATTEND_FIXED_DEEP;
-  return ctas <= (long long)attend_wave(c->dim, sms) * (routed ? 2 : 1) ? MOBA_ATTEND_FIXED : MOBA_ATTEND_STREAMED;
+  const long long wave = attend_wave(c->dim, sms);
+  return 2 * ctas <= wave * (!routed ? 2 : 10 * pairs <= wave ? 5 : 4) ? MOBA_ATTEND_FIXED : MOBA_ATTEND_STREAMED;
 }
 
 extern "C" int moba_decode_attend_variant(const moba_cache_desc* c, int rows, int hq, int routed, int slots, int umax, int sms,

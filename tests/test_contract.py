@@ -116,6 +116,8 @@ def test_both_16_bit_formats_pass_the_input_check():
     (2, 14, 2, 64, 16384, 512, True, 18, 8, 2),          # routed: 22 entries a pair are 88 parts, within two waves
     (2, 12, 4, 256, 16384, 512, False, 148, 16, 3),      # above head dimension 128 one part per SM
     (64, 12, 2, 128, 65536, 2048, True, 148, 16, 3),
+    (11, 28, 4, 128, 16384, 512, True, 148, 16, 2),      # 44 pairs, 968 parts: few pairs, two and a half waves
+    (14, 28, 4, 128, 16384, 512, True, 148, 16, 3),      # 56 pairs: two
 ])
 def test_attention_kernel_rule(requests, hq, hk, dim, capacity, chunk, routed, sms, most_cluster, want):
     """Which decode attention kernel serves a shape, on a whole GPU and on a part of one: a cluster that the device cannot
