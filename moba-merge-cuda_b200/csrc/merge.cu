@@ -293,7 +293,7 @@ template <typename T, int LPR>
 void launch_rows_as(const T* so, const float* self_lse, const T* ro, const float* remote_lse, const int* counts, const int* slots,
                     long long rows, int dim, int kmax, T* o, float* lse, cudaStream_t st) {
   // A warp takes 32 rows where that still gives every SM a few warps; below that its groups take one row each.
-  const int rpw = rows >= 32ll * 148 * 4 ? 32 : 32 / LPR;
+  const int rpw = rows >= 32ll * 4 * device_sms() ? 32 : 32 / LPR;
   const long long per_cta = 4ll * rpw;
   auto go = [&](auto kernel) {
     launch_dependent(32u, kernel, dim3((unsigned)((rows + per_cta - 1) / per_cta)), dim3(128), 0, st, so, self_lse, ro, remote_lse, counts,

@@ -95,7 +95,7 @@ extern "C" size_t moba_prefill_bwd_scratch_bytes(const moba_prefill_desc* d) {
 //   14/2 heads, D = 64     24 blocks 147 / 89 / >58    72: 315 / 179 / >132    80: 331 / >187    296: 588 / >478
 //    6/1 heads, D = 128    24 blocks 428 / 227 / >131  72: 684 / 369 / >220    148: 904 / >499   296: 1172 / >744
 //    8/8 heads, D = 64     48 blocks 27 / >25 / 37     72: 32 / >29 / 49       128: >45 / 51     296: >94 / 105
-//    8/8 heads, D = 128    72 blocks 50 / >41 / 68     96: 62 / >60            160: >88 / 101    296: >176 / 180
+//    8/8 heads, D = 128    72 blocks 50 / >41 / 68     96: >62 / 60              160: >88 / 101    296: >176 / 180
 // With the block count alone as the rule, groups of one head took up to 1.55 (D = 128: 1.97) times as long as undivided.  Of 408 shapes
 // (eight head shapes, chunks of 128 to 2048, topk 2 to 8) the worst is now 1.11 times as long as undivided and on average within
 // 0.4 % of the best of the three.
