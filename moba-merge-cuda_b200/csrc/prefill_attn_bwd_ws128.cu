@@ -17,9 +17,10 @@ namespace moba {
 
 namespace {
 
-constexpr int kThreads = 512;  // 8 compute warps, MMA warp, producer warp (+2 idle), 4 dQ drain warps
+constexpr int kThreads = 512;  // 8 compute warps, MMA warp, producer warp, 2 warps that help the drain, 4 dQ drain warps
 constexpr int kRing = 3;       // (Q, dO) half tiles in flight; the dQ staging takes the room of a fourth
 constexpr int kQRows = 64;     // query rows per step
+constexpr int kAskDrain = 11, kAskHelp = (kQRows - 4 * kAskDrain) / 2;  // staged dQ rows a drain warp / warp 10 or 11 asks for
 
 struct Smem128 {
   uint64_t st_full, p_ready, ka_ready, dpt_full, ds_ready, dq_done, dq_free, kv_ready;
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
     mbar_init(&cb.dq_done, 1);
     mbar_init(&cb.dq_free, 4);
     mbar_init(&cb.kv_ready, 1);
-    for (int i = 0; i < kRing; ++i) { mbar_init(&cb.qdo_full[i], 1); mbar_init(&cb.qdo_free[i], 5); }
+    for (int i = 0; i < kRing; ++i) { mbar_init(&cb.qdo_full[i], 1); mbar_init(&cb.qdo_free[i], 7); }
     mbar_fence_init();
   }
   if (warp == 0) tmem_alloc(&cb.tmem_slot, TMEM_COLS);
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
   const uint32_t tmem = cb.tmem_slot;
   bool alive = true;
 
+  auto drain_sync = [&]() { asm volatile("bar.sync 1, 192;" ::: "memory"); };  // warps 10-15
   if (warp >= 12) {
     // ================================================================== dQ drain (warps 12-15)
     // dQ^T has the head dimension on the lanes: a warp owns 32 consecutive dimensions, every thread the
@@ -106,11 +108,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
     float* rows = reinterpret_cast<float*>(sStage);                  // [64 queries][128 dimensions]
     const bool fixed = a.dq_fixed != nullptr;
     const uint32_t tlane = tmem + (uint32_t(quad * 32) << 16);
-    auto drain_sync = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+    const int ask_row = quad * kAskDrain + lane;                     // staged row this thread asks the copy engine to add (lanes < kAskDrain)
     for (int it = 0; it < n_iter; ++it) {
       const int slot = it % kRing;
       alive = warp_wait(&cb.qdo_full[slot], (it / kRing) & 1, a.status, alive);
-      const int th0 = cb.rowth[slot][lane], th1 = cb.rowth[slot][32 + lane];
+      const int th = lane < kAskDrain ? cb.rowth[slot][ask_row] : -1;
       warp_arrive(&cb.qdo_free[slot]);
       alive = warp_wait(&cb.dq_done, it & 1, a.status, alive);
       tc_fence_after_sync();
@@ -123,10 +125,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
       if (!fixed) {
         // Ordinary mode: the step's dQ goes to shared memory as 64 query rows (a thread writes its dimension of every
         // row, lanes on consecutive floats), and the copy engine adds each row to its place in the FP32 accumulator:
-        // one 512-byte reduction per row issued by warps 12 and 13, carried by the engine's own path to the L2 cache
-        // instead of the load/store pipe.  The four warps meet twice per step: before writing (the engine has read
-        // the previous step's rows) and before the rows are handed over.
-        if (quad < 2) bulk_wait_group_read();
+        // one 512-byte reduction per row, carried by the engine's own path to the L2 cache instead of the load/store pipe.
+        // The warps meet twice per step: before writing (the engine has read the previous step's rows) and before
+        // the rows are handed over.  A warp needs 62 cycles to ask for one row, whatever its size (one lane after the
+        // other), so six ask, warps 10 and 11 among them: with two warps asking for 32 rows each, 2040 of the 3070
+        // cycles of a step went there and the products waited for the drain.  A step takes 2100 to 2400 cycles now; at
+        // full size the clock falls with it (power cap), so training steps went 41.5 -> 38.0 ms (131072 tokens, 4/1 heads,
+        // chunk 4096, topk 12) and 3.48 -> 3.26 ms (4 x 8192 tokens, 12/2 heads, chunk 512, topk 8).
+        bulk_wait_group_read();
         drain_sync();
         const int dcol = quad * 32 + lane;
 #pragma unroll
@@ -136,11 +142,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
         }
         fence_async_smem();
         drain_sync();
-        if (quad < 2) {
-          const int th = quad == 0 ? th0 : th1;
-          if (th >= 0 && alive) bulk_reduce_add_f32(a.dq_acc + (long long)th * D, rows + (quad * 32 + lane) * 128, (uint32_t)D * 4u);
-          bulk_commit_group();
-        }
+        if (th >= 0 && alive) bulk_reduce_add_f32(a.dq_acc + (long long)th * D, rows + ask_row * 128, (uint32_t)D * 4u);
+        bulk_commit_group();
         continue;
       }
       // Deterministic mode: the same hand-over with 64-bit fixed-point values (32 fractional bits), whose integer sums
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
       unsigned long long* rows64 = reinterpret_cast<unsigned long long*>(sStage);   // [64 queries][64 dimensions]
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        if (quad < 2) bulk_wait_group_read();
+        bulk_wait_group_read();
         drain_sync();
         if ((quad >> 1) == r) {
           const int dl = (quad & 1) * 32 + lane;   // dimension inside the round
@@ -162,12 +165,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
           fence_async_smem();
         }
         drain_sync();
-        if (quad < 2) {
-          const int th = quad == 0 ? th0 : th1;
-          if (th >= 0 && alive && r * 64 < D)
-            bulk_reduce_add_u64(a.dq_fixed + (long long)th * D + r * 64, rows64 + (quad * 32 + lane) * 64, (uint32_t)min(64, D - r * 64) * 8u);
-          bulk_commit_group();
-        }
+        if (th >= 0 && alive && r * 64 < D)
+          bulk_reduce_add_u64(a.dq_fixed + (long long)th * D + r * 64, rows64 + ask_row * 64, (uint32_t)min(64, D - r * 64) * 8u);
+        bulk_commit_group();
       }
     }
     bulk_wait_group();   // the engine has finished with this CTA's shared memory and its reductions are performed
@@ -214,6 +214,27 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
           bulk_load(cb.delta_s[b], a.deltapack + moff, kQRows * 4, &cb.qdo_full[b]);
         }
       }
+    } else if (warp >= 10) {
+      // ================================================================== dQ reductions beside the drain warps' own
+      const bool fixed = a.dq_fixed != nullptr;
+      const int ask_row = 4 * kAskDrain + (warp - 10) * kAskHelp + lane;
+      for (int it = 0; it < n_iter; ++it) {
+        const int slot = it % kRing;
+        alive = warp_wait(&cb.qdo_full[slot], (it / kRing) & 1, a.status, alive);
+        const int th = lane < kAskHelp ? cb.rowth[slot][ask_row] : -1;
+        warp_arrive(&cb.qdo_free[slot]);
+        for (int r = 0; r < (fixed ? 2 : 1); ++r) {   // the rounds of the deterministic mode, as in the drain warps
+          bulk_wait_group_read();
+          drain_sync();
+          drain_sync();
+          if (th >= 0 && alive) {
+            if (!fixed) bulk_reduce_add_f32(a.dq_acc + (long long)th * D, sStage + ask_row * 512, (uint32_t)D * 4u);
+            else if (r * 64 < D) bulk_reduce_add_u64(a.dq_fixed + (long long)th * D + r * 64, sStage + ask_row * 512, (uint32_t)min(64, D - r * 64) * 8u);
+          }
+          bulk_commit_group();
+        }
+      }
+      bulk_wait_group();
     } else if (warp == 8) {
       // ================================================================== MMA issue
       // Fixed order per step n:  dV(n) | S^T(n+1) | dK(n) | dP^T(n+1) | dQ^T(n): P^T lives in the columns of S^T, dS^T in
@@ -314,10 +335,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
       tc_fence_before_sync();
       warp_arrive(&cb.ka_ready);
     }
+    // tiles until the next one on the causal diagonal: the tile of the key block itself, first of each head's own-chunk tiles
+    int to_diag = jt0 <= n_remote ? n_remote - jt0 : (n_self - (jt0 - n_remote) % n_self) % n_self;
     for (int it = 0; it < n_iter; ++it) {
-      const int ms = it % kRing, jt = jt0 + (it >> 1), sub = it & 1;
+      const int ms = it % kRing, sub = it & 1;
       // queries below qmin (index inside the 128-row tile) are masked for this key
-      const bool diag = jt >= n_remote && ((jt - n_remote) % n_self) == 0;
+      const bool diag = to_diag == 0;
+      if (sub) to_diag = diag ? n_self - 1 : to_diag - 1;
       const int qmin = r >= nkeys ? kTile : (diag ? r : 0);
       const int q0 = sub * kQRows + half * 32;  // first query of this thread's columns
       const bool unmasked = __all_sync(0xFFFFFFFFu, qmin <= q0);
