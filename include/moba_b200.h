@@ -227,6 +227,14 @@ int moba_decode_attend(const moba_cache_desc* c, const void* q, const int32_t* i
                        const int32_t* selected, int slots, const int32_t* u_chunk, const uint32_t* u_mask,
                        const int32_t* u_count, int umax, void* workspace, size_t workspace_bytes, void* out, float* lse,
                        unsigned* status, void* stream);
+/* moba_decode_step_begin, moba_decode_route (selected != null) and moba_decode_attend of one appended token per row, with their
+ * arguments and results: one launch where the attention takes a cluster per (row, kv head) and the head dimension is at most 128
+ * (u_chunk, u_mask and u_count are then left as they are), the two or three of them otherwise. */
+int moba_decode_step(const moba_cache_desc* c, const int32_t* ids, int32_t* positions, const int32_t* delta, int rows, int hq,
+                     const void* qkv, const void* cosv, const void* sinv, void* q, void* k, void* v, int remote, int width,
+                     float* scores, int32_t* selected, int slots, int32_t* u_chunk, uint32_t* u_mask, int32_t* u_count, int umax,
+                     void* workspace, size_t workspace_bytes, void* out, float* lse, unsigned* status, void* stream);
+
 /* The kernel that moba_decode_attend takes for a call of this shape (routed: selected != null): one of the values below, or
  * minus a MOBA_ERR_* code.  sms, most_cluster: SMs of the device and the largest cluster that it can hold; sms = 0 and most_cluster = -1 ask
  * the current device. */

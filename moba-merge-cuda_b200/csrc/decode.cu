@@ -283,6 +283,24 @@ __global__ void __launch_bounds__(256) stage_inputs_kernel(uint4* dq, const uint
   else if (i < nq + nk + nv) dv[i - nq - nk] = sv[i - nq - nk];
 }
 
+// Rotary embedding (rotate-half) of eight dimensions c * 8 .. of a head: own and the unit half a head away, cos and sin of
+// the own unit; rounding to bf16 where the Hugging Face implementation does.
+__device__ __forceinline__ uint4 rope_unit(const uint4& own, const uint4& oth, const uint4& cs, const uint4& sn, bool low) {
+  const uint32_t xw[4] = {own.x, own.y, own.z, own.w}, ow[4] = {oth.x, oth.y, oth.z, oth.w};
+  const uint32_t cw[4] = {cs.x, cs.y, cs.z, cs.w}, sw[4] = {sn.x, sn.y, sn.z, sn.w};
+  uint32_t out[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float lo = __bfloat162float(__float2bfloat16_rn(bf_lo(xw[i]) * bf_lo(cw[i]))) +
+                     __bfloat162float(__float2bfloat16_rn((low ? -bf_lo(ow[i]) : bf_lo(ow[i])) * bf_lo(sw[i])));
+    const float hi = __bfloat162float(__float2bfloat16_rn(bf_hi(xw[i]) * bf_hi(cw[i]))) +
+                     __bfloat162float(__float2bfloat16_rn((low ? -bf_hi(ow[i]) : bf_hi(ow[i])) * bf_hi(sw[i])));
+    const __nv_bfloat162 pk = __floats2bfloat162_rn(lo, hi);
+    out[i] = *reinterpret_cast<const uint32_t*>(&pk);
+  }
+  return make_uint4(out[0], out[1], out[2], out[3]);
+}
+
 // --------------------------------------------------------------------------- first launch of an appending decode step
 // Metadata, append and the predicated chunk mean of one request per CTA, and, when the caller hands over the fused
 // q/k/v projection instead of separate k and v, the rotary embedding and the split as well: what were four
@@ -347,19 +365,7 @@ __global__ void __launch_bounds__(256) decode_step_begin_kernel(CacheView cv, co
       const uint4 oth = *reinterpret_cast<const uint4*>(src + h * D + (low ? c + (upr >> 1) : c - (upr >> 1)) * 8);
       const uint4 cs = *reinterpret_cast<const uint4*>(cosv + (long long)row * D + c * 8);
       const uint4 sn = *reinterpret_cast<const uint4*>(sinv + (long long)row * D + c * 8);
-      const uint32_t xw[4] = {own.x, own.y, own.z, own.w}, ow[4] = {oth.x, oth.y, oth.z, oth.w};
-      const uint32_t cw[4] = {cs.x, cs.y, cs.z, cs.w}, sw[4] = {sn.x, sn.y, sn.z, sn.w};
-      uint32_t out[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float lo = __bfloat162float(__float2bfloat16_rn(bf_lo(xw[i]) * bf_lo(cw[i]))) +
-                         __bfloat162float(__float2bfloat16_rn((low ? -bf_lo(ow[i]) : bf_lo(ow[i])) * bf_lo(sw[i])));
-        const float hi = __bfloat162float(__float2bfloat16_rn(bf_hi(xw[i]) * bf_hi(cw[i]))) +
-                         __bfloat162float(__float2bfloat16_rn((low ? -bf_hi(ow[i]) : bf_hi(ow[i])) * bf_hi(sw[i])));
-        const __nv_bfloat162 pk = __floats2bfloat162_rn(lo, hi);
-        out[i] = *reinterpret_cast<const uint32_t*>(&pk);
-      }
-      const uint4 res = make_uint4(out[0], out[1], out[2], out[3]);
+      const uint4 res = rope_unit(own, oth, cs, sn, low);
       if (h < Hq) {
         *reinterpret_cast<uint4*>(q + ((long long)row * Hq + h) * D + c * 8) = res;
       } else {
@@ -408,28 +414,18 @@ __global__ void __launch_bounds__(256) decode_step_begin_kernel(CacheView cv, co
 constexpr int kRouteTile = 64;      // chunk means staged in shared memory per round of decode_route_kernel
 constexpr int kRouteThreads = 256;  // eight warps: a group of up to eight heads is ranked in one round
 
-// --------------------------------------------------------------------------- routing (K12, K13, K17, K18)
-// One CTA (kRouteThreads threads) per (query row, kv head).  scores[row, h, c] = q . mean[c] in FP32 for the
-// chunks completed before the query's own chunk, -inf elsewhere; top-`remote` per head in descending
-// score order with the lowest chunk winning exact ties; selected[row, h, :] = (own chunk, picks...,
-// -1 padding); and the group's union list (chunk ascending, bitmask of heads) for the attention kernel.
+// Scores and picks of one (query row, kv head) by kRouteThreads threads, see decode_route_kernel: q, scores (or null) and selected (or
+// null) of the group's first head.  s_dyn: route_floats(G, width, D) floats and a tile of means; the heads that picked a
+// chunk are left in route_mask(s_dyn).
+__host__ __device__ __forceinline__ size_t route_floats(int G, int width, int D) { return ((size_t)G * width + width + 1 + (size_t)G * D + 3) & ~(size_t)3; }
+__host__ __device__ __forceinline__ size_t route_bytes(int G, int width, int D) { return route_floats(G, width, D) * 4 + (size_t)kRouteTile * ((D / 8) | 1) * 16; }
+__device__ __forceinline__ unsigned* route_mask(float* s_dyn, int G, int width) { return reinterpret_cast<unsigned*>(s_dyn + G * width); }
 template <bool F16>
-__global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView cv, const __nv_bfloat16* q, const int* ids, const int* positions,
-                                                           int Hq, int remote, int width, float* scores, int* selected, int* u_chunk,
-                                                           unsigned* u_mask, int* u_count, int umax) {
-  // As in decode_step_begin_kernel: no __restrict__, no read-only loads - positions, the query and the chunk means
-  // come from kernels this grid may overlap with until the wait below.
-  extern __shared__ float s_dyn[];
-  dependents_may_start();
-  wait_for_predecessor();  // positions, the query, a chunk mean the step's first launch may just have written
-  const int G = Hq / cv.Hkv;
+__device__ __forceinline__ void route_group(const CacheView& cv, float* s_dyn, const __nv_bfloat16* qsrc, int sid, int g, int G, int cur, int nlegal,
+                                            int remote, int width, float* scores, int* selected) {
   float* s_scores = s_dyn;                                            // [G][width]
-  unsigned* s_mask = reinterpret_cast<unsigned*>(s_dyn + G * width);  // [width + 1]
-  const int row = blockIdx.x, g = blockIdx.y;
+  unsigned* s_mask = route_mask(s_dyn, G, width);                     // [width + 1]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int sid = ids[row], pos = positions[row];
-  const int cur = pos / cv.C;
-  const int nlegal = min(min(cur, width), cv.max_chunks);
   const int upr = cv.D >> 3;
 
   for (int i = tid; i <= width; i += kRouteThreads) s_mask[i] = 0u;
@@ -438,7 +434,6 @@ __global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView c
   float* s_q = reinterpret_cast<float*>(s_mask + width + 1);  // [G][D]
   // the query loads are issued here and stored after the first tile of means has been requested, so that the two
   // trips to L2 overlap (a store to shared memory would make the warp wait for its load first)
-  const __nv_bfloat16* qsrc = q + ((long long)row * Hq + g * G) * cv.D;
   float qreg[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -457,7 +452,7 @@ __global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView c
   // depend on each other (one trip to L2 per tile); the (head, chunk) pairs are then scored from there.  Rows are
   // padded to an odd number of 16-byte units so that threads on consecutive chunks hit different banks.
   const int ustride = upr | 1;
-  uint4* s_tile = reinterpret_cast<uint4*>(s_dyn + ((G * width + width + 1 + G * cv.D + 3) & ~3));
+  uint4* s_tile = reinterpret_cast<uint4*>(s_dyn + route_floats(G, width, cv.D));
   for (int c0 = 0; c0 < nlegal; c0 += kRouteTile) {
     const int nt = min(kRouteTile, nlegal - c0);
 #pragma unroll 4
@@ -484,21 +479,21 @@ __global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView c
       }
       const float sc = (a0 + a1) + (a2 + a3);
       s_scores[hl * width + c0 + cl] = sc;
-      if (scores) scores[((long long)row * Hq + g * G + hl) * width + c0 + cl] = sc;
+      if (scores) scores[(long long)hl * width + c0 + cl] = sc;
     }
     __syncthreads();
   }
   for (int pair = tid; pair < G * (width - nlegal); pair += kRouteThreads) {  // not a candidate
     const int hl = pair / (width - nlegal), c = nlegal + pair - hl * (width - nlegal);
     s_scores[hl * width + c] = -INFINITY;
-    if (scores) scores[((long long)row * Hq + g * G + hl) * width + c] = -INFINITY;
+    if (scores) scores[(long long)hl * width + c] = -INFINITY;
   }
   __syncthreads();
   // top-k: one warp per head, `remote` rounds of (max value, lowest index among equals)
   for (int hl = warp; hl < G; hl += kRouteThreads / 32) {
     float* sc = s_scores + hl * width;
-    int* out = selected + ((long long)row * Hq + g * G + hl) * (remote + 1);
-    if (lane == 0) out[0] = cur;
+    int* out = selected ? selected + hl * (remote + 1) : nullptr;
+    if (out && lane == 0) out[0] = cur;
     for (int r = 0; r < remote; ++r) {
       float best = -INFINITY;
       int idx = 0x7FFFFFFF;
@@ -514,7 +509,7 @@ __global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView c
       }
       const bool found = best > -INFINITY && idx != 0x7FFFFFFF;
       if (lane == 0) {
-        out[1 + r] = found ? idx : -1;
+        if (out) out[1 + r] = found ? idx : -1;
         if (found) {
           sc[idx] = -INFINITY;
           atomicOr(&s_mask[idx], 1u << hl);
@@ -524,6 +519,32 @@ __global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView c
     }
   }
   __syncthreads();
+}
+
+// --------------------------------------------------------------------------- routing (K12, K13, K17, K18)
+// One CTA (kRouteThreads threads) per (query row, kv head).  scores[row, h, c] = q . mean[c] in FP32 for the
+// chunks completed before the query's own chunk, -inf elsewhere; top-`remote` per head in descending
+// score order with the lowest chunk winning exact ties; selected[row, h, :] = (own chunk, picks...,
+// -1 padding); and the group's union list (chunk ascending, bitmask of heads) for the attention kernel.
+template <bool F16>
+__global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView cv, const __nv_bfloat16* q, const int* ids, const int* positions,
+                                                           int Hq, int remote, int width, float* scores, int* selected, int* u_chunk,
+                                                           unsigned* u_mask, int* u_count, int umax) {
+  // As in decode_step_begin_kernel: no __restrict__, no read-only loads - positions, the query and the chunk means
+  // come from kernels this grid may overlap with until the wait below.
+  extern __shared__ float s_dyn[];
+  dependents_may_start();
+  wait_for_predecessor();  // positions, the query, a chunk mean the step's first launch may just have written
+  const int G = Hq / cv.Hkv;
+  const int row = blockIdx.x, g = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sid = ids[row], pos = positions[row];
+  const int cur = pos / cv.C;
+  const int nlegal = min(min(cur, width), cv.max_chunks);
+  const long long first = (long long)row * Hq + g * G;  // the group's first head
+  route_group<F16>(cv, s_dyn, q + first * cv.D, sid, g, G, cur, nlegal, remote, width, scores ? scores + first * width : nullptr,
+                   selected + first * (remote + 1));
+  const unsigned* s_mask = route_mask(s_dyn, G, width);
   // union list: routed chunks ascending, the own chunk (all heads) last
   if (warp == 0) {
     const long long base = ((long long)row * cv.Hkv + g) * umax;
@@ -1129,11 +1150,12 @@ __device__ __forceinline__ void attend_softmax(const float (&s)[4], float& m, fl
 // Paged attention of one head block over `ntiles` consecutive stages, by a team of four warps.  The query heads of
 // the GQA group are the 16 rows of m16n8k16 tensor-core tiles (unused rows are zero), so a K/V token read from HBM
 // serves every head at no extra cost.  Each warp takes 16 tokens of every stage and keeps its own running (max, sum, O).
+//   q         the group's query rows, D values each
 //   ring      NS stages            rowbase [NS][64]   nv, mask [2 NS]: a slot is rewritten NS stages ahead, while the slots
 //                                                     before it are still read
 //   which     heads of the block that count: stages that none of them attends are passed over (see attend_spoiled)
 template <int DP, int NS, bool F16, bool WIDE, class Sync>
-__device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& look, int ntiles, int sid, int row, int g, int hb, int ltid,
+__device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& look, int ntiles, int sid, const __nv_bfloat16* q, int g, int hb, int ltid,
                                               uint8_t* ring, long long (*s_rowbase)[kStageTokens], int* s_nv, unsigned* s_mask,
                                               Sync team_sync, unsigned which, AttendState<DP>& st) {
   constexpr int KSTEPS = DP / 16;
@@ -1156,7 +1178,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
   uint32_t qf[KSTEPS][4];  // A operand: rows qr and qr + 8, all k-steps
   {
     const bool r0 = hb + qr < G, r1 = WIDE && hb + qr + 8 < G;
-    const __nv_bfloat16* q0 = a.q + ((long long)row * a.Hq + g * G + hb + qr) * D;
+    const __nv_bfloat16* q0 = q + (hb + qr) * D;
     const __nv_bfloat16* q1 = q0 + 8 * D;
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
@@ -1260,9 +1282,13 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
 // Where the sums of a head block go: head h of it to m[h], l[h] and o[h * D ...]; -inf, 0 and zeros for a head nobody attended.
 struct AttendSums { float *m, *l, *o; };
 
+// A token beside the stages: its score for every head of the block (exp2 domain; null: there is none) and its V row.
+struct AttendExtra { const float* score; const __nv_bfloat16* v; };
+
 // Combines the NW warps of a CTA through shared memory (s_o: NW * 16 * (DP + 2) floats), for heads h0 to h1 - 1 of the block.
 template <int DP, int NW, bool WIDE>
-__device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, int h0, int h1, int D, const AttendSums& to) {
+__device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, int h0, int h1, int D, const AttendSums& to,
+                                               const AttendExtra& extra = AttendExtra{nullptr, nullptr}, bool f16 = false) {
   constexpr int ROWS = WIDE ? 16 : 8;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, qr = lane >> 2, qc = lane & 3;
   st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 1); st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 2);
@@ -1293,6 +1319,13 @@ __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, 
 #pragma unroll
     for (int w = 0; w < NW; ++w) { mw[w] = s_ml[((size_t)w * ROWS + hh) * 2]; big = fmaxf(big, mw[w]); }
     float lsum = 0.f, v0 = 0.f, v1 = 0.f;
+    if (extra.score) {
+      const float m = extra.score[hh];
+      big = fmaxf(big, m);
+      const float2 x = unpack16(*reinterpret_cast<const uint32_t*>(extra.v + d), f16);
+      lsum = dec_exp2(m - big);
+      v0 = x.x * lsum; v1 = x.y * lsum;
+    }
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
       const float wgt = mw[w] == -INFINITY ? 0.f : dec_exp2(mw[w] - big);  // a warp that saw no token of the head adds nothing
@@ -1328,12 +1361,32 @@ __device__ __forceinline__ bool attend_spoiled(const AttendState<DP>& st) {
 // memory, a fence, a ticket and the last CTA reading all of them back.  One
 // request of 4096 tokens, 14/2 heads, D = 64: step 18.6 us streamed, 11.5 us this way (dense); layers of a 2000-token
 // session 10 -> 6 us.
+//
+// STEP: the whole decode step in this launch, metadata, append (with the rotary embedding and the split of a fused projection where the
+// caller hands that over), routing and attention, which are otherwise two or three launches in a row, each waiting for the last: one request
+// of 16384 tokens took 2.5 + 4.3 + 10.4 us of them, a sparse layer of a 2000-token session 4.8 + 6.5 + 7.7.  Every CTA does what its
+// pair needs before the stages for itself (rotary embedding and routing of one group: a few thousand multiply-adds, and means that
+// lie in L2), so nothing waits for another CTA.  The new token is not read back through the cache: its score and V
+// row enter where CTA 0 combines its warps.  The length is advanced by the row's last cluster to have read it, found with a ticket.
+// One launch: 14.0 us instead of 17.2 (the step as a caller sees it 23.4 -> 22.6, where the host is the limit), layers 9.9 and 13.4 instead
+// of 12.2 and 19 (session step 292 -> 267 us).
 // grid (CL, pairs), cluster (CL, 1, 1)
-template <int DP, int CL, bool WIDE, bool F16>
-__global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_cluster_kernel(AttendArgs a) {
+struct StepArgs {
+  const int* delta;
+  int* positions;
+  const __nv_bfloat16 *qkv, *cosv, *sinv;  // fused projection and rotary table, or null: q, k, v hold the new token already
+  __nv_bfloat16 *q, *k, *v;
+  int b, remote, width;
+  float* scores;
+  int* selected;   // null: dense
+};
+
+template <int DP, int CL, bool WIDE, bool F16, bool STEP>
+__global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_cluster_kernel(AttendArgs a, StepArgs step) {
   constexpr int NS = cluster_stages(DP), TEAMS = cluster_teams(DP), NT = 128 * TEAMS, NW = 4 * TEAMS;
   constexpr int STAGE_BYTES = 2 * kStageTokens * DP * 2;
   constexpr int PIPE = TEAMS * NS * STAGE_BYTES > NW * 16 * (DP + 2) * 4 ? TEAMS * NS * STAGE_BYTES : NW * 16 * (DP + 2) * 4;
+  static_assert(!STEP || NT == kRouteThreads, "routing and chunk means are written for 256 threads");
   extern __shared__ __align__(128) uint8_t s_pipe[];  // the teams' rings, reused to combine the warps; then [G][D] sums of the CTA
   __shared__ long long s_rowbase[TEAMS][NS][kStageTokens];
   __shared__ int s_nv[TEAMS][2 * NS];
@@ -1341,25 +1394,114 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
   __shared__ int s_list[kClusterList];
   __shared__ unsigned s_heads[kClusterList];
   __shared__ float s_m[32], s_l[32];
+  __shared__ __align__(16) __nv_bfloat16 s_new[STEP ? 34 * DP : 8];  // the group's query rows, the new K row, the new V row
+  __shared__ float s_score[32];                                      // of the new token
+  __shared__ int s_count;
   dependents_may_start();   // e.g. the output projection, whose weight loads need nothing from here
   wait_for_predecessor();   // routes, positions, the appended row
   const CacheView& cv = a.cv;
   const int D = cv.D, G = a.Hq / cv.Hkv;
   const int rank = blockIdx.x, rowg = blockIdx.y, row = rowg / cv.Hkv, g = rowg - row * cv.Hkv;
   const int tid = threadIdx.x, team = tid >> 7, ltid = tid & 127;
-  const bool dense = a.selected == nullptr;
+  const bool dense = STEP ? step.selected == nullptr : a.selected == nullptr;
   float* s_sum = reinterpret_cast<float*>(s_pipe + PIPE);
-  // one trip: position, sequence, the whole list and its length
-  const int pos = a.positions[row], sid = a.ids[row];
-  const int listed = dense ? 1 : a.u_count[rowg];
-  if (!dense) {
-    for (int i = tid; i < a.umax; i += NT) {
-      s_list[i] = a.u_chunk[(long long)rowg * a.umax + i];
-      s_heads[i] = a.u_mask[(long long)rowg * a.umax + i];
+  const __nv_bfloat16* q = a.q + ((long long)row * a.Hq + g * G) * D;
+  const int sid = a.ids[row];
+  int pos, listed;
+  if (!STEP) {
+    // one trip: position, sequence, the whole list and its length
+    pos = a.positions[row];
+    listed = dense ? 1 : a.u_count[rowg];
+    if (!dense) {
+      for (int i = tid; i < a.umax; i += NT) {
+        s_list[i] = a.u_chunk[(long long)rowg * a.umax + i];
+        s_heads[i] = a.u_mask[(long long)rowg * a.umax + i];
+      }
+      __syncthreads();
     }
+  } else {
+    pos = cv.lengths[sid];
+    const int upr = D >> 3;
+    for (int i = tid; i < (G + 2) * upr; i += NT) {
+      const int hl = i / upr, c = i - hl * upr;
+      // head of the projection, and place in q, k or v
+      const int h = hl < G ? g * G + hl : hl == G ? a.Hq + g : a.Hq + cv.Hkv + g;
+      __nv_bfloat16* own = (hl < G ? step.q + ((long long)row * a.Hq + h) * D : (hl == G ? step.k : step.v) + ((long long)row * cv.Hkv + g) * D) + c * 8;
+      uint4 w;
+      if (step.qkv) {
+        const __nv_bfloat16* src = step.qkv + ((long long)row * (a.Hq + 2 * cv.Hkv) + h) * D;
+        w = *reinterpret_cast<const uint4*>(src + c * 8);
+        if (hl <= G) {
+          const bool low = c < (upr >> 1);
+          w = rope_unit(w, *reinterpret_cast<const uint4*>(src + (low ? c + (upr >> 1) : c - (upr >> 1)) * 8),
+                        *reinterpret_cast<const uint4*>(step.cosv + (long long)row * D + c * 8),
+                        *reinterpret_cast<const uint4*>(step.sinv + (long long)row * D + c * 8), low);
+        }
+        if (rank == 0) *reinterpret_cast<uint4*>(own) = w;
+      } else {
+        w = *reinterpret_cast<const uint4*>(own);
+      }
+      *reinterpret_cast<uint4*>(s_new + hl * D + c * 8) = w;
+    }
+    q = s_new;
     __syncthreads();
+    if (rank == 0) {
+      // append; the page may have been opened by this step's delta
+      const int logical = step.delta[row], opened = step.delta[step.b + row], page = pos / cv.page;
+      if (g == 0 && tid == 0 && logical >= 0 && logical < cv.width) cv.table[(long long)sid * cv.width + logical] = opened;
+      const int physical = page >= cv.width ? -1 : page == logical ? opened : cv.table[(long long)sid * cv.width + page];
+      if (physical < 0 || physical >= cv.num_pages) {
+        if (tid == 0) atomicOr(a.status, kErrBadIndex);
+      } else if (tid < 2 * upr) {
+        const long long dst = (((long long)physical * cv.page + (pos - page * cv.page)) * cv.Hkv + g) * D + (tid % upr) * 8;
+        *reinterpret_cast<uint4*>((tid < upr ? cv.kc : cv.vc) + dst) = *reinterpret_cast<const uint4*>(s_new + G * D + tid * 8);
+      }
+      for (int hl = tid >> 5; hl < G; hl += NW) {  // scores of the new token, a warp per head
+        float dot = 0.f;
+        for (int d = (tid & 31) * 2; d < D; d += 64) {
+          const float2 x = unpack16<F16>(*reinterpret_cast<const uint32_t*>(s_new + hl * D + d));
+          const float2 y = unpack16<F16>(*reinterpret_cast<const uint32_t*>(s_new + G * D + d));
+          dot = fmaf(x.x, y.x, fmaf(x.y, y.y, dot));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xFFFFFFFFu, dot, o);
+        if ((tid & 31) == 0) s_score[hl] = dot * a.scale_log2;
+      }
+    }
+    listed = 1;
+    if (!dense) {
+      const int cur = pos / cv.C, nlegal = min(min(cur, step.width), cv.max_chunks);
+      float* s_dyn = reinterpret_cast<float*>(s_pipe);
+      const long long first = (long long)row * a.Hq + g * G;
+      route_group<F16>(cv, s_dyn, s_new, sid, g, G, cur, nlegal, step.remote, step.width, rank == 0 && step.scores ? step.scores + first * step.width : nullptr,
+                       rank == 0 ? step.selected + first * (step.remote + 1) : nullptr);
+      const unsigned* picked = route_mask(s_dyn, G, step.width);
+      if (tid < 32) {  // routed chunks ascending, the own chunk (all heads) last
+        int count = 0;
+        for (int c0 = 0; c0 < nlegal; c0 += 32) {
+          const int c = c0 + tid;
+          const unsigned m = c < nlegal ? picked[c] : 0u;
+          const unsigned bal = __ballot_sync(0xFFFFFFFFu, m != 0u);
+          if (m) {
+            const int at = count + __popc(bal & ((1u << tid) - 1u));
+            if (at < a.umax - 1) { s_list[at] = c; s_heads[at] = m; }
+          }
+          count += __popc(bal);
+        }
+        if (tid == 0) {
+          count = min(count, a.umax - 1);
+          s_list[count] = cur;
+          s_heads[count] = G >= 32 ? 0xFFFFFFFFu : ((1u << G) - 1u);
+          s_count = count + 1;
+        }
+      }
+      __syncthreads();
+      listed = s_count;
+    }
   }
-  const int own = dense ? pos + 1 : pos + 1 - pos / cv.C * cv.C;
+  // STEP: the stages end before the new token
+  const int tokens = STEP ? pos : pos + 1;
+  const int own = dense ? tokens : tokens - pos / cv.C * cv.C;
   const int stages = (listed - 1) * a.spc + (own + kStageTokens - 1) / kStageTokens;
   const int lo = (int)((long long)stages * rank / CL), hi = (int)((long long)stages * (rank + 1) / CL);
   const int half = (hi - lo + TEAMS - 1) / TEAMS;
@@ -1367,10 +1509,10 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
   StageCursor look;
   look.chunks = dense ? nullptr : s_list;
   look.masks = s_heads;
-  look.entries = a.umax; look.spc = a.spc; look.span = dense ? kStageTokens : cv.C;
+  look.entries = STEP ? listed : a.umax; look.spc = a.spc; look.span = dense ? kStageTokens : cv.C;
   look.mask = G >= 32 ? 0xFFFFFFFFu : ((1u << G) - 1u);
   look.pos = pos;
-  look.visible = min(pos + 1, cv.lengths[sid]);
+  look.visible = STEP ? pos : min(pos + 1, cv.lengths[sid]);
   auto team_sync = [&]() {
     if (TEAMS == 1) __syncthreads();
     else asm volatile("bar.sync %0, 128;" ::"r"(team + 1) : "memory");
@@ -1381,17 +1523,26 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
     int head = -1;  // all together, see attend_spoiled
     do {
       look.start(first);
-      attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
+      attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, q, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
                                        s_nv[team], s_mask[team], team_sync, head < 0 ? 0xFFFFu : 1u << head, st);
       const bool again = head < 0 && !dense && attend_spoiled(st);
       if (!again)
         attend_combine<DP, NW, WIDE>(st, reinterpret_cast<float*>(s_pipe), max(head, 0), head < 0 ? nh : head + 1, D,
-                                     AttendSums{s_m + hb, s_l + hb, s_sum + (size_t)hb * D});
+                                     AttendSums{s_m + hb, s_l + hb, s_sum + (size_t)hb * D},
+                                     STEP && rank == 0 ? AttendExtra{s_score + hb, s_new + (G + 1) * D} : AttendExtra{nullptr, nullptr}, F16);
       if (again || head >= 0) ++head;
     } while (head >= 0 && head < nh);
   }
   // CL neighbouring lanes, one per CTA of the cluster, take four dimensions of a head; the items are divided over the CTAs
   cluster_barrier();
+  if (STEP && rank == 0 && tid == 0) {  // every CTA of the cluster has read the length
+    __threadfence();
+    if (atomicAdd(&a.counters[row * cv.Hkv], 1) == cv.Hkv - 1) {
+      step.positions[row] = pos;
+      cv.lengths[sid] = pos + 1;
+      a.counters[row * cv.Hkv] = 0;     // ready for the next launch (graph replay included)
+    }
+  }
   const int d4n = D >> 2, items = G * d4n, per = (items + CL - 1) / CL;
   const int peer = tid % CL;
   const uint32_t pm = peer_smem(s_m, peer), pl = peer_smem(s_l, peer), ps = peer_smem(s_sum, peer);
@@ -1424,6 +1575,13 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
     }
   }
   cluster_barrier();  // no CTA leaves while another may still read its sums
+  if (STEP && rank == 0 && (pos + 1) % cv.C == 0 && pos / cv.C < cv.max_chunks) {
+    // the new token, which this CTA appended, completes its chunk
+    const int logical = step.delta[row];
+    if (tid == 0 && logical >= 0 && logical < cv.width) cv.table[(long long)sid * cv.width + logical] = step.delta[step.b + row];
+    __syncthreads();
+    chunk_mean_cta(cv, sid, pos / cv.C, g, reinterpret_cast<float*>(s_pipe), a.status);
+  }
 }
 
 // ---- streamed variant -------------------------------------------------------------------------------------------
@@ -1536,7 +1694,7 @@ __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_k
       int head = -1;  // all together, see attend_spoiled
       do {
         look.start(j0);
-        attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, row, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); },
+        attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, a.q + ((long long)row * a.Hq + g * G) * D, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); },
                                          head < 0 ? 0xFFFFu : 1u << head, st);
         const bool again = head < 0 && !dense && attend_spoiled(st);
         if (!again)
@@ -1744,8 +1902,7 @@ extern "C" int moba_decode_route(const moba_cache_desc* c, const void* q, const 
     return MOBA_ERR_INVALID;
   const int G = hq / c->hkv;
   if (G > 32 || remote > 16) return MOBA_ERR_UNSUPPORTED;
-  const size_t smem = ((((size_t)G * width + width + 1 + (size_t)G * c->dim + 3) & ~(size_t)3)) * 4 +
-                      (size_t)kRouteTile * ((c->dim / 8) | 1) * 16;
+  const size_t smem = route_bytes(G, width, c->dim);
   constexpr int most_smem = 200 * 1024;  // the limit belongs to the function: one value, so that no thread lowers another's
   if (smem > most_smem) return MOBA_ERR_UNSUPPORTED;
   const auto kernel = (c->flags & MOBA_CACHE_FP16) ? decode_route_kernel<true> : decode_route_kernel<false>;
@@ -1789,14 +1946,14 @@ struct ClusterSmem {
   // the limit belongs to the function, not to the launch: one value for all groups, so that no thread lowers another's
   static constexpr size_t most = fixed + (size_t)32 * DP * 4;
 };
-template <int DP, int CL>
+template <int DP, int CL, bool STEP = false>
 static auto cluster_kernel(bool wide, bool half) {
-  return wide ? (half ? decode_attend_cluster_kernel<DP, CL, true, true> : decode_attend_cluster_kernel<DP, CL, true, false>)
-              : (half ? decode_attend_cluster_kernel<DP, CL, false, true> : decode_attend_cluster_kernel<DP, CL, false, false>);
+  return wide ? (half ? decode_attend_cluster_kernel<DP, CL, true, true, STEP> : decode_attend_cluster_kernel<DP, CL, true, false, STEP>)
+              : (half ? decode_attend_cluster_kernel<DP, CL, false, true, STEP> : decode_attend_cluster_kernel<DP, CL, false, false, STEP>);
 }
-template <int DP, int CL>
+template <int DP, int CL, bool STEP = false>
 static cudaError_t cluster_attributes(bool wide, bool half) {
-  const auto kernel = cluster_kernel<DP, CL>(wide, half);
+  const auto kernel = cluster_kernel<DP, CL, STEP>(wide, half);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ClusterSmem<DP>::most);
   if (e == cudaSuccess && CL > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   return e;
@@ -1882,17 +2039,9 @@ extern "C" size_t moba_decode_attend_workspace_bytes(const moba_cache_desc* c, i
   return attend_workspace(c, rows, hq, attend_partials(c, rows, hq, slots));
 }
 
-extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const int32_t* ids, const int32_t* positions,
-                                  int rows, int hq, const int32_t* selected, int slots, const int32_t* u_chunk,
-                                  const uint32_t* u_mask, const int32_t* u_count, int umax, void* workspace,
-                                  size_t workspace_bytes, void* out, float* lse, unsigned* status, void* stream) {
-  int rc = validate_cache(c);
-  if (rc != MOBA_OK) return rc;
-  if (!q || !ids || !positions || !workspace || !out || !lse || !status || rows < 1 || hq < 1 || hq % c->hkv || slots < 1)
-    return MOBA_ERR_INVALID;
-  if (selected && (!u_chunk || !u_mask || !u_count || umax < 1)) return MOBA_ERR_INVALID;
-  if (hq / c->hkv > 32) return MOBA_ERR_UNSUPPORTED;
-  if (workspace_bytes < moba_decode_attend_workspace_bytes(c, rows, hq, slots)) return MOBA_ERR_WORKSPACE;
+static AttendArgs attend_args(const moba_cache_desc* c, const void* q, const int32_t* ids, const int32_t* positions, int rows, int hq,
+                              const int32_t* selected, int slots, const int32_t* u_chunk, const uint32_t* u_mask, const int32_t* u_count,
+                              int umax, void* workspace, void* out, float* lse, unsigned* status) {
   AttendArgs a;
   a.cv = make_cache_view(*c);
   a.q = static_cast<const __nv_bfloat16*>(q);
@@ -1911,14 +2060,29 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
   a.lse = lse;
   a.status = status;
   a.scale_log2 = (float)(1.4426950408889634 / sqrt((double)c->dim));
-  const int dp = c->dim <= 32 ? 32 : c->dim <= 64 ? 64 : c->dim <= 128 ? 128 : 256;
-  cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaSuccess;
-  const bool half = (c->flags & MOBA_CACHE_FP16) != 0, wide = hq / c->hkv > 8;
   a.rowgs = rows * c->hkv;
   a.spc = selected ? (c->chunk_size + kStageTokens - 1) / kStageTokens : 1;
   a.step_pg = kStageTokens / c->page_size;
   a.step_r = kStageTokens - a.step_pg * c->page_size;
+  return a;
+}
+
+extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const int32_t* ids, const int32_t* positions,
+                                  int rows, int hq, const int32_t* selected, int slots, const int32_t* u_chunk,
+                                  const uint32_t* u_mask, const int32_t* u_count, int umax, void* workspace,
+                                  size_t workspace_bytes, void* out, float* lse, unsigned* status, void* stream) {
+  int rc = validate_cache(c);
+  if (rc != MOBA_OK) return rc;
+  if (!q || !ids || !positions || !workspace || !out || !lse || !status || rows < 1 || hq < 1 || hq % c->hkv || slots < 1)
+    return MOBA_ERR_INVALID;
+  if (selected && (!u_chunk || !u_mask || !u_count || umax < 1)) return MOBA_ERR_INVALID;
+  if (hq / c->hkv > 32) return MOBA_ERR_UNSUPPORTED;
+  if (workspace_bytes < moba_decode_attend_workspace_bytes(c, rows, hq, slots)) return MOBA_ERR_WORKSPACE;
+  const AttendArgs a = attend_args(c, q, ids, positions, rows, hq, selected, slots, u_chunk, u_mask, u_count, umax, workspace, out, lse, status);
+  const int dp = c->dim <= 32 ? 32 : c->dim <= 64 ? 64 : c->dim <= 128 ? 128 : 256;
+  cudaStream_t st = (cudaStream_t)stream;
+  cudaError_t e = cudaSuccess;
+  const bool half = (c->flags & MOBA_CACHE_FP16) != 0, wide = hq / c->hkv > 8;
   const int variant = moba_decode_attend_variant(c, rows, hq, selected != nullptr, slots, umax, 0, -1);
   if (variant < 0) return -variant;
   const dim3 grid(a.umax, a.parts, rows * c->hkv);
@@ -1928,7 +2092,7 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
     const size_t smem = ClusterSmem<L>::fixed + (size_t)(hq / c->hkv) * c->dim * 4;                                     \
     e = cluster_attributes<L, CL>(wide, half);                                                                          \
     if (e == cudaSuccess)                                                                                               \
-      e = launch_dependent_cluster(8u, cluster_kernel<L, CL>(wide, half), dim3(CL, a.rowgs), dim3(128 * cluster_teams(L)), CL, smem, st, a); \
+      e = launch_dependent_cluster(8u, cluster_kernel<L, CL>(wide, half), dim3(CL, a.rowgs), dim3(128 * cluster_teams(L)), CL, smem, st, a, StepArgs{}); \
   } while (0)
 #define MOBA_LAUNCH_FIXED(L, NS, T)                                                                                      \
   do {                                                                                                                  \
@@ -1962,6 +2126,72 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
 #undef MOBA_LAUNCH_ATTEND
 #undef MOBA_LAUNCH_CLUSTER
 #undef MOBA_LAUNCH_FIXED
+  prof_end(kProfDecodeAttend, st);
+  if (e != cudaSuccess) return MOBA_ERR_CUDA;
+  return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;
+}
+
+// A step in one launch: where its attention takes a cluster per pair, the head dimension is at most 128 (256 threads a CTA), the routing
+// of a group fits the memory that the stages' ring takes later, and rows can be read 16 bytes at a time.
+static bool step_fits_cluster(const moba_cache_desc* c, int hq, int variant, bool routed, int width, const void* qkv, uintptr_t addresses) {
+  if ((variant != MOBA_ATTEND_CLUSTER_16 && variant != MOBA_ATTEND_CLUSTER_8) || c->dim > 128 || (addresses & 15)) return false;
+  if (qkv && c->dim % 16) return false;
+  const size_t ring = c->dim <= 32 ? ClusterSmem<32>::ring : c->dim <= 64 ? ClusterSmem<64>::ring : ClusterSmem<128>::ring;
+  return !routed || route_bytes(hq / c->hkv, width, c->dim) <= ring;
+}
+
+extern "C" int moba_decode_step(const moba_cache_desc* c, const int32_t* ids, int32_t* positions, const int32_t* delta, int rows, int hq,
+                                const void* qkv, const void* cosv, const void* sinv, void* q, void* k, void* v, int remote, int width,
+                                float* scores, int32_t* selected, int slots, int32_t* u_chunk, uint32_t* u_mask, int32_t* u_count, int umax,
+                                void* workspace, size_t workspace_bytes, void* out, float* lse, unsigned* status, void* stream) {
+  int rc = validate_cache(c);
+  if (rc != MOBA_OK) return rc;
+  if (!ids || !positions || !delta || !q || !k || !v || !workspace || !out || !lse || !status || rows < 1 || hq < 1 || hq % c->hkv || slots < 1)
+    return MOBA_ERR_INVALID;
+  if (selected && (!u_chunk || !u_mask || !u_count || umax < 1 || remote < 0 || width < 1)) return MOBA_ERR_INVALID;
+  if (qkv && (!cosv || !sinv || (c->dim & 1))) return MOBA_ERR_INVALID;
+  if (hq / c->hkv > 32 || (selected && remote > 16) || (qkv && (c->flags & MOBA_CACHE_FP16))) return MOBA_ERR_UNSUPPORTED;
+  if (workspace_bytes < moba_decode_attend_workspace_bytes(c, rows, hq, slots)) return MOBA_ERR_WORKSPACE;
+  const int variant = moba_decode_attend_variant(c, rows, hq, selected != nullptr, slots, umax, 0, -1);
+  if (variant < 0) return -variant;
+  const uintptr_t addresses = (uintptr_t)qkv | (uintptr_t)cosv | (uintptr_t)sinv | (uintptr_t)q | (uintptr_t)k | (uintptr_t)v |
+                              (uintptr_t)c->k_cache | (uintptr_t)c->v_cache;
+  if (!step_fits_cluster(c, hq, variant, selected != nullptr, width, qkv, addresses)) {
+    rc = moba_decode_step_begin(c, ids, positions, delta, rows, hq, qkv, cosv, sinv, q, k, v, status, stream);
+    if (rc == MOBA_OK && selected)
+      rc = moba_decode_route(c, q, ids, positions, rows, hq, remote, width, scores, selected, u_chunk, u_mask, u_count, stream);
+    if (rc == MOBA_OK)
+      rc = moba_decode_attend(c, q, ids, positions, rows, hq, selected, slots, u_chunk, u_mask, u_count, umax, workspace, workspace_bytes, out,
+                              lse, status, stream);
+    return rc;
+  }
+  const AttendArgs a = attend_args(c, q, ids, positions, rows, hq, selected, slots, u_chunk, u_mask, u_count, umax, workspace, out, lse, status);
+  StepArgs s;
+  s.delta = delta; s.positions = positions;
+  s.qkv = static_cast<const __nv_bfloat16*>(qkv); s.cosv = static_cast<const __nv_bfloat16*>(cosv); s.sinv = static_cast<const __nv_bfloat16*>(sinv);
+  s.q = static_cast<__nv_bfloat16*>(q); s.k = static_cast<__nv_bfloat16*>(k); s.v = static_cast<__nv_bfloat16*>(v);
+  s.b = rows; s.remote = remote; s.width = width; s.scores = scores; s.selected = selected;
+  cudaStream_t st = (cudaStream_t)stream;
+  cudaError_t e = cudaSuccess;
+  const bool half = (c->flags & MOBA_CACHE_FP16) != 0, wide = hq / c->hkv > 8;
+  prof_begin(kProfDecodeAttend, st);
+#define MOBA_LAUNCH_STEP(L, CL)                                                                                          \
+  do {                                                                                                                  \
+    const size_t smem = ClusterSmem<L>::fixed + (size_t)(hq / c->hkv) * c->dim * 4;                                     \
+    e = cluster_attributes<L, CL, true>(wide, half);                                                                    \
+    if (e == cudaSuccess)                                                                                               \
+      e = launch_dependent_cluster(8u, cluster_kernel<L, CL, true>(wide, half), dim3(CL, a.rowgs), dim3(128 * cluster_teams(L)), CL, smem, st, a, s); \
+  } while (0)
+#define MOBA_LAUNCH_STEP_OF(L)                                       \
+  do {                                                               \
+    if (variant == MOBA_ATTEND_CLUSTER_16) MOBA_LAUNCH_STEP(L, 16);  \
+    else MOBA_LAUNCH_STEP(L, 8);                                     \
+  } while (0)
+  if (c->dim <= 32) MOBA_LAUNCH_STEP_OF(32);
+  else if (c->dim <= 64) MOBA_LAUNCH_STEP_OF(64);
+  else MOBA_LAUNCH_STEP_OF(128);
+#undef MOBA_LAUNCH_STEP_OF
+#undef MOBA_LAUNCH_STEP
   prof_end(kProfDecodeAttend, st);
   if (e != cudaSuccess) return MOBA_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;

@@ -58,6 +58,8 @@ _DECODE_ABI = {
     "moba_decode_append": (_I, [_P, _VP, _VP, _VP, _VP, _I, _VP, _VP]),
     "moba_decode_means": (_I, [_P, _VP, _VP, _I, _I, _VP, _VP]),
     "moba_decode_step_begin": (_I, [_P, _VP, _VP, _VP, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP]),
+    "moba_decode_step": (_I, [_P, _VP, _VP, _VP, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _VP, _VP, _I, _VP, _VP, _VP, _I, _VP, _SZ, _VP, _VP,
+                              _VP, _VP]),
     "moba_decode_stage_inputs": (_I, [_VP, _VP, _SZ, _VP, _VP, _SZ, _VP, _VP, _SZ, _VP]),
     "moba_prefill_to_cache": (_I, [_P, _VP, _VP, _VP, _VP, _VP, _I, _I, _VP, _VP]),
     "moba_prefill_to_cache_strided": (_I, [_P, _VP, _I64, _I64, _VP, _I64, _I64, _VP, _VP, _VP, _I, _I, _VP, _VP]),

@@ -8,8 +8,9 @@ persistent buffers and are overwritten by the next call.
 
 How a step runs here: the host plans the pages (a few integer operations) and, only when some
 sequence opens a new page, sends a 2 x b int32 delta from a ring of pinned buffers; the device work is
-three launches whose shapes were fixed at preparation - `moba_decode_step_begin` (metadata, append and
-predicated chunk mean in one kernel), `moba_decode_route`, `moba_decode_attend` - two for dense plans.
+`moba_decode_step`, whose launches have shapes that were fixed at preparation: one where every (request, kv head) pair has a
+cluster of CTAs, otherwise `moba_decode_step_begin` (metadata, append and predicated chunk mean in one kernel),
+`moba_decode_route` (not for dense plans) and `moba_decode_attend`.
 Fixed shapes, fixed addresses and positions read from device memory are what make the step capturable.
 
 Besides the reference's methods there is a small driver interface for callers that run several plans
@@ -249,20 +250,21 @@ class PreparedDecode:
         status = c._status.data_ptr()
         ids, pos = self.gpu_ids.data_ptr(), self.positions.data_ptr()
         union = (self._u_chunk.data_ptr(), self._u_mask.data_ptr(), self._u_count.data_ptr())
+        selected = None if self.dense else self.selected.data_ptr()
+        work = (self._workspace.data_ptr(), self._ws_bytes, self.output.data_ptr(), self.lse.data_ptr(), status, st)
         if kind == "step":
             qkv, cos, sin = (None, None, None) if projected is None else (t.data_ptr() for t in projected)
-            buffers = (self.q.data_ptr(), self.k.data_ptr(), self.v.data_ptr())
-            _ext.check(lib.moba_decode_step_begin(ctypes.byref(d), ids, pos, self.delta.data_ptr(), b, h, qkv, cos, sin,
-                                                  *buffers, status, st), "moba_decode_step_begin")
-        else:
-            _ext.check(lib.moba_decode_metadata(ctypes.byref(d), ids, pos, self.delta.data_ptr(), b, 0, st), "moba_decode_metadata")
+            _ext.check(lib.moba_decode_step(ctypes.byref(d), ids, pos, self.delta.data_ptr(), b, h, qkv, cos, sin, self.q.data_ptr(),
+                                            self.k.data_ptr(), self.v.data_ptr(), self.remote, self.width,
+                                            None if self.dense else self.scores.data_ptr(), selected, self._slots, *union, self._umax, *work),
+                       "moba_decode_step")
+            return
+        _ext.check(lib.moba_decode_metadata(ctypes.byref(d), ids, pos, self.delta.data_ptr(), b, 0, st), "moba_decode_metadata")
         if not self.dense:
             _ext.check(lib.moba_decode_route(ctypes.byref(d), self.q.data_ptr(), ids, pos, b, h, self.remote, self.width,
-                                             self.scores.data_ptr(), self.selected.data_ptr(), *union, st), "moba_decode_route")
-        _ext.check(lib.moba_decode_attend(ctypes.byref(d), self.q.data_ptr(), ids, pos, b, h,
-                                          None if self.dense else self.selected.data_ptr(), self._slots, *union, self._umax,
-                                          self._workspace.data_ptr(), self._ws_bytes, self.output.data_ptr(),
-                                          self.lse.data_ptr(), status, st), "moba_decode_attend")
+                                             self.scores.data_ptr(), selected, *union, st), "moba_decode_route")
+        _ext.check(lib.moba_decode_attend(ctypes.byref(d), self.q.data_ptr(), ids, pos, b, h, selected, self._slots, *union, self._umax,
+                                          *work), "moba_decode_attend")
 
     def replay(self, kind):
         self._graphs[kind].replay()

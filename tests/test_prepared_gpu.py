@@ -225,3 +225,68 @@ def test_combined_api_rejects_nonfinite_before_append(bad_name):
     with pytest.raises(ValueError, match="NaN/Inf"):
         cache.append_and_attend(**tensors, sequence_ids=[0])
     assert cache.lengths == (0,)
+
+
+@pytest.mark.parametrize("requests,hq,hk,dim,chunk,page,mode,dtype,start", [
+    (1, 14, 2, 64, 32, 16, "moba", torch.bfloat16, 61),     # pages and chunks end together
+    (1, 14, 2, 64, 32, 16, "dense", torch.bfloat16, 61),
+    (4, 6, 1, 128, 24, 7, "moba", torch.float16, 70),       # a page across a chunk's end
+    (2, 40, 2, 96, 16, 1, "moba", torch.bfloat16, 45),      # two head blocks; every token opens a page
+    (2, 4, 4, 32, 20, 5, "moba", torch.float16, 18),        # eight CTAs a pair; no candidate at first
+    (3, 8, 1, 8, 16, 16, "dense", torch.bfloat16, 1),
+])
+def test_step_in_one_launch_equals_its_three_launches(requests, hq, hk, dim, chunk, page, mode, dtype, start):
+    """A small batch's step is one launch; the entry points it stands for, called one after the other, leave the same routes, scores,
+    cache, means and lengths.  The new token's product is exact in one and split in two 16-bit pieces in the other, so outputs may
+    round to neighbouring values: one unit in the last place, 2^-7 of the value in bf16 and 2^-10 in half precision."""
+    import ctypes
+    from moba_opt import PagedKVCache
+    gen = torch.Generator().manual_seed(dim + chunk)
+    rnd = lambda *shape: torch.randn(*shape, generator=gen).to("cuda", dtype)
+    steps = 2 * chunk + 3
+    plans, caches = [], []
+    lens = [start + 3 * i for i in range(requests)]
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    k0, v0 = rnd(cu[-1], hk, dim), rnd(cu[-1], hk, dim)
+    for _ in range(2):
+        cache = PagedKVCache(requests, max(lens) + steps, hk, dim, page_size=page, chunk_size=chunk, dtype=dtype)
+        cache.append(k0, v0, sequence_ids=list(range(requests)), cu_seqlens=cu)
+        caches.append(cache)
+        plans.append(cache.prepare_decode(list(range(requests)), hq, topk=3, mode=mode, check_finite=False))
+    one, three = plans
+    lib, desc = one._lib, caches[0]._desc()
+    assert lib.moba_decode_attend_variant(ctypes.byref(desc), requests, hq, int(mode == "moba"), one._slots, one._umax, 0, -1) in (8, 16)
+
+    def launch(kind, projected=None):
+        p, d, st = three, caches[1]._desc(), three._stream()
+        ids, pos = p.gpu_ids.data_ptr(), p.positions.data_ptr()
+        union = (p._u_chunk.data_ptr(), p._u_mask.data_ptr(), p._u_count.data_ptr())
+        status, b = caches[1]._status.data_ptr(), requests
+        assert lib.moba_decode_step_begin(ctypes.byref(d), ids, pos, p.delta.data_ptr(), b, hq, None, None, None, p.q.data_ptr(), p.k.data_ptr(),
+                                          p.v.data_ptr(), status, st) == 0
+        selected = None if p.dense else p.selected.data_ptr()
+        if not p.dense:
+            assert lib.moba_decode_route(ctypes.byref(d), p.q.data_ptr(), ids, pos, b, hq, p.remote, p.width, p.scores.data_ptr(), selected,
+                                         *union, st) == 0
+        assert lib.moba_decode_attend(ctypes.byref(d), p.q.data_ptr(), ids, pos, b, hq, selected, p._slots, *union, p._umax,
+                                      p._workspace.data_ptr(), p._ws_bytes, p.output.data_ptr(), p.lse.data_ptr(), status, st) == 0
+    three.launch = launch
+    for _ in range(steps):
+        q, k, v = rnd(requests, hq, dim), rnd(requests, hk, dim), rnd(requests, hk, dim)
+        a, b = one.step(q, k, v), three.step(q, k, v)
+        torch.testing.assert_close(a.output.float(), b.output.float(), rtol=2.0 ** (-7 if dtype == torch.bfloat16 else -10), atol=2e-5)
+        torch.testing.assert_close(a.lse, b.lse, rtol=1e-5, atol=1e-5)
+        assert torch.equal(one.positions, three.positions)
+        if mode == "moba":
+            assert torch.equal(a.selected_blocks, b.selected_blocks) and torch.equal(one.scores, three.scores)
+    for t in ("_table", "_lengths"):
+        assert torch.equal(getattr(caches[0], t), getattr(caches[1], t))
+    for p in plans:
+        p.close()
+    for sid in range(requests):
+        for x, y in zip(caches[0].materialize(sid), caches[1].materialize(sid)):
+            assert torch.equal(x, y)
+        closed = caches[0].lengths[sid] // chunk
+        assert torch.equal(caches[0]._means[sid, :closed], caches[1]._means[sid, :closed])
