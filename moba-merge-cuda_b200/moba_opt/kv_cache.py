@@ -24,13 +24,13 @@ import ctypes
 import enum
 import threading
 from dataclasses import dataclass
+from typing import NamedTuple
 
-import numpy as np
 import torch
 
 from . import _ext
 from .cache_layout import PageAllocator, positive_int
-from .grouped_attention import _status_word
+from .grouped_attention import _current, _status_word
 
 MAX_CHUNK = 8192
 MAX_TOPK = 17
@@ -83,6 +83,12 @@ def decode_library():
             fn.restype, fn.argtypes = restype, argtypes
         lib._decode_abi_bound = True
     return lib
+
+
+def current_stream_handle(device_index):
+    """The current CUDA stream of the device as an integer handle (the cheapest route torch offers; a call asks more than once)."""
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(device_index) if raw is not None else torch.cuda.current_stream(device_index).cuda_stream
 
 
 def _rows_of_16_bytes(t):
@@ -161,8 +167,7 @@ class CacheLife(enum.Enum):
     BROKEN = "broken"      # a launch failed: contents undefined
 
 
-@dataclass(frozen=True)
-class TensorRule:
+class TensorRule(NamedTuple):
     """What a q / k / v argument has to satisfy besides being finite; `check` raises ValueError with the reference's wording."""
     name: str
     heads: object = None        # exact head count, or None
@@ -186,70 +191,84 @@ class TensorRule:
             raise ValueError(f"{n} token count differs")
 
 
+def _nothing():
+    pass
+
+
 class FiniteCheck:
     """NaN/Inf check of the q, k, v of a call: one launch over all of them that writes into pinned words, one wait for
     the stream.  The owner serialises calls (the cache's lock)."""
 
     def __init__(self, lib, device, words):
         self._lib, self._device, self._words = lib, device, words    # at least three pinned int32
-        self._flags = self._words.numpy()
+        self._flags, self._address = self._words.numpy(), self._words.data_ptr()
 
     def require(self, named):
         """`named`: up to three (name, [N,H,D] 16-bit tensor of the cache's device); raises ValueError for the first that
         is not finite."""
-        if not named:
-            return
+        if named:
+            self.start(named)()
+
+    def start(self, named):
+        """Enqueues the check and returns a function that waits for its answer and raises as `require` does: the host has
+        work of its own (planning, staging) while the kernel runs.  One check at a time."""
         args = (FiniteInput * 3)()
         for a, (_, t) in zip(args, named):
             a.data, a.tokens, a.heads = t.data_ptr(), t.shape[0], t.shape[1]
             a.stride_t, a.stride_h = t.stride(0), t.stride(1)
         self._flags[:] = 0
-        stream = torch.cuda.current_stream(self._device)
+        stream = torch.cuda.current_stream(self._device.index)
         _ext.check(self._lib.moba_check_finite(args, len(named), named[0][1].shape[2], 1 if named[0][1].dtype == torch.float16 else 0,
-                                               self._words.data_ptr(), stream.cuda_stream), "moba_check_finite")
-        stream.synchronize()
-        for flag, (name, _) in zip(self._flags.tolist(), named):
-            if flag:
-                raise ValueError(f"{name} contains NaN/Inf")
+                                               self._address, stream.cuda_stream), "moba_check_finite")
+
+        def answer():
+            stream.synchronize()
+            for flag, (name, _) in zip(self._flags.tolist(), named):
+                if flag:
+                    raise ValueError(f"{name} contains NaN/Inf")
+        return answer
 
 
 class HostStaging:
     """Small int32 vectors of a call, sent to the device as one block: the vectors are laid out back to back in a
-    pinned buffer, copied with one asynchronous transfer and returned as views of one device tensor.  A few pinned
-    buffers are used in turn, so the host waits only if the copy that last used a buffer is still in flight."""
+    pinned buffer and copied with one asynchronous transfer.  A few pinned buffers are used in turn, so the host waits
+    only if the copy that last used a buffer is still in flight."""
 
     def __init__(self, device, slots=4, words=4096):
         self.device = device
         block = torch.zeros(slots * words + 4, dtype=torch.int32, pin_memory=True)   # one allocation: pinning is slow
         self._pinned = list(block[:slots * words].split(words))
+        self._host = [t.numpy() for t in self._pinned]
         self.spare = block[slots * words:]         # for whoever needs a word both sides can reach (FiniteCheck)
         self._busy = [None] * slots
         self._next = 0
 
     def send(self, *vectors):
-        arrays = [np.ascontiguousarray(v, dtype=np.int32).reshape(-1) for v in vectors]
-        sizes = [a.size for a in arrays]
-        total = sum(sizes)
-        if total == 0:
-            empty = torch.empty(0, dtype=torch.int32, device=self.device)
-            return tuple(empty for _ in arrays)
+        """(device block, address of every vector in it); the block has to be kept until the launches that read it are
+        enqueued."""
+        total = sum(map(len, vectors))
         slot = self._next
         self._next = (slot + 1) % len(self._pinned)
-        if self._busy[slot] is not None:
-            self._busy[slot].synchronize()
+        busy = self._busy[slot]
+        if busy is None:
+            busy = self._busy[slot] = torch.cuda.Event()
+        else:
+            busy.synchronize()
         if self._pinned[slot].numel() < total:
             self._pinned[slot] = torch.empty(max(total, 2 * self._pinned[slot].numel()), dtype=torch.int32, pin_memory=True)
-        host = self._pinned[slot].numpy()
-        at = 0
-        for a in arrays:
-            host[at:at + a.size] = a
-            at += a.size
+            self._host[slot] = self._pinned[slot].numpy()
+        host = self._host[slot]
+        offsets, at = [], 0
+        for v in vectors:
+            offsets.append(at)
+            if len(v):
+                host[at:at + len(v)] = v
+            at += len(v)
         dev = torch.empty(total, dtype=torch.int32, device=self.device)
         dev.copy_(self._pinned[slot][:total], non_blocking=True)
-        done = torch.cuda.Event()
-        done.record()
-        self._busy[slot] = done
-        return dev.split(sizes)
+        busy.record()
+        base = dev.data_ptr()
+        return dev, [base + 4 * at for at in offsets]
 
 
 # ----------------------------------------------------------------------------------------- the cache
@@ -298,6 +317,7 @@ class PagedKVCache:
             self._status = _status_word(self.device)
             self._staging = HostStaging(self.device)
             self._finite = FiniteCheck(self._lib, self.device, self._staging.spare)
+            self._pools = frozenset(t.untyped_storage().data_ptr() for t in (self.k_cache, self.v_cache))
             self._attend_buffers = {}         # (rows, Hq, slots, umax) -> union lists + split-K workspace, kept between calls
 
     # ------------------------------------------------------------------ views of the CPU layout
@@ -308,7 +328,8 @@ class PagedKVCache:
     @property
     def page_table(self):
         """Immutable CPU snapshot of the logical->physical page map."""
-        return self._owner.page_table if self._owner is not None else self._layout.tables
+        with self._lock:
+            return self._owner.page_table if self._owner is not None else self._layout.tables
 
     # ------------------------------------------------------------------ plumbing shared with PreparedDecode
     def _desc(self):
@@ -322,7 +343,7 @@ class PagedKVCache:
     def _launch(self, name, *args):
         """One C-ABI call on the cache's stream; a refused launch leaves the cache contents undefined."""
         with _ext.nvtx(name):
-            status = getattr(self._lib, name)(*args, ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream))
+            status = getattr(self._lib, name)(*args, self._stream)    # the current stream, or `_guard` had refused
         if status != 0:
             self._life = CacheLife.BROKEN
         _ext.check(status, name)
@@ -336,12 +357,11 @@ class PagedKVCache:
             raise ValueError("prepared decode owns cache; close it before ordinary cache operations")
         if torch.cuda.is_current_stream_capturing():
             raise ValueError("CUDA Graph capture is unsupported for this cache API")
-        if torch.cuda.current_stream(self.device).cuda_stream != self._stream:
+        if current_stream_handle(self.device.index) != self._stream:
             raise ValueError("cross-stream cache access is unsupported")
 
     def _refuse_pool_aliases(self, *tensors):
-        pools = {self.k_cache.untyped_storage().data_ptr(), self.v_cache.untyped_storage().data_ptr()}
-        if any(t.untyped_storage().data_ptr() in pools for t in tensors):
+        if any(t.untyped_storage().data_ptr() in self._pools for t in tensors):
             raise ValueError("append inputs must not alias KV cache storage; clone first")
 
     def _routable(self, lengths):
@@ -367,52 +387,67 @@ class PagedKVCache:
                               stable_routes=stable_routes)
 
     def _check_inputs(self, check_finite, **tensors):
-        """The contracts of the tensors given, in the order given; a tensor's NaN/Inf fault comes before the faults of the
-        tensors after it, as when they are checked one after the other."""
+        """The contracts of the tensors given, in the order given; returns a function that waits for the answer of their
+        NaN/Inf check (to be called before anything is modified, and whatever else the call finds wrong: a tensor's NaN/Inf
+        fault comes before the faults of the tensors after it and of the other arguments, as when they are checked one
+        after the other)."""
         check_finite = check_finite and self.check_finite
         tokens, seen = None, []
         try:
             for name, t in tensors.items():
-                TensorRule(name, heads=None if name == "q" else self.num_kv_heads, tokens=tokens).check(self, t)
+                TensorRule(name, None if name == "q" else self.num_kv_heads, tokens).check(self, t)
                 tokens = t.shape[0]
                 seen.append((name, t))
-        finally:
+        except Exception:
             if check_finite:
                 self._finite.require(seen)
+            raise
+        return self._finite.start(seen) if check_finite else _nothing
 
-    def _store(self, k, v, ids, counts, extra=()):
-        """Plans the append on the CPU, sends the changed table entries, the new lengths, the segment description and
-        the caller's `extra` vectors in one block, applies the edits and stores the tokens with their chunk means.
-        Returns (plan, first position of every segment, device views of `extra`); the CPU layout is committed once
-        both launches were accepted."""
+    def _plan_store(self, ids, counts, extra=()):
+        """Plans an append on the CPU and sends the changed table entries, the new lengths, the segment description and
+        the caller's `extra` vectors in one block; changes nothing."""
         lay = self._layout
         starts = [lay.lengths[s] for s in ids]
         plan = lay.plan_append(ids, counts, tokens=False)
-        cu = np.zeros(len(ids) + 1, dtype=np.int32)
-        np.cumsum(counts, out=cu[1:])
-        edits = np.asarray(plan.page_edits, dtype=np.int32).reshape(-1, 3)
+        cu = [0]
+        for n in counts:
+            cu.append(cu[-1] + n)
+        edits = [x for edit in plan.page_edits for x in edit]
         sent = self._staging.send(edits, ids, [plan.lengths[s] for s in ids], starts, cu, *extra)
-        d_edits, d_ids, d_lengths, d_starts, d_cu = sent[:5]
-        desc = self._desc()
-        self._launch("moba_cache_update", ctypes.byref(desc), d_edits.data_ptr() if len(edits) else None, len(edits),
-                     d_ids.data_ptr(), d_lengths.data_ptr(), len(ids), 0)
+        return plan, starts, sent
+
+    def _store(self, k, v, ids, counts, planned, desc):
+        """Applies the edits of `_plan_store` and stores the tokens with their chunk means; the CPU layout is committed once
+        both launches were accepted."""
+        plan, starts, (_, at) = planned
+        d_edits, d_ids, d_lengths, d_starts, d_cu = at[:5]
+        n_edits = len(plan.page_edits)
+        self._launch("moba_cache_update", desc, d_edits if n_edits else None, n_edits, d_ids, d_lengths, len(ids), 0)
         c = self.chunk_size
         touched = max((first + n - 1) // c - first // c + 1 for first, n in zip(starts, counts))
         k, v = _rows_of_16_bytes(k), _rows_of_16_bytes(v)
-        self._launch("moba_prefill_to_cache_strided", ctypes.byref(desc), k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0),
-                     v.stride(1), d_ids.data_ptr(), d_starts.data_ptr(), d_cu.data_ptr(), len(ids), touched, self._status.data_ptr())
-        lay.commit(plan)
+        self._launch("moba_prefill_to_cache_strided", desc, k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0),
+                     v.stride(1), d_ids, d_starts, d_cu, len(ids), touched, self._status.data_ptr())
+        self._layout.commit(plan)
         self._candidate_count = self._routable(plan.lengths)
-        return plan, starts, sent[5:]
+
+    def _append(self, k, v, sequence_ids, cu_seqlens, check_finite):
+        finite = self._check_inputs(check_finite, k=k, v=v)
+        try:                                      # beside the check
+            self._refuse_pool_aliases(k, v)
+            ids, counts = self._segments(k.shape[0], sequence_ids, cu_seqlens)
+            planned = self._plan_store(ids, counts)
+        finally:
+            finite()
+        self._store(k, v, ids, counts, planned, ctypes.byref(self._desc()))
+        return ids, counts, planned
 
     @torch.no_grad()
     def append(self, k, v, *, sequence_ids, cu_seqlens=None):
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, _current(self.device):
             self._guard()
-            self._check_inputs(True, k=k, v=v)
-            self._refuse_pool_aliases(k, v)
-            ids, counts = self._segments(k.shape[0], sequence_ids, cu_seqlens)
-            _, starts, _ = self._store(k, v, ids, counts)
+            ids, counts, (_, starts, _) = self._append(k, v, sequence_ids, cu_seqlens, True)
             return AppendResult(ids, starts, counts)
 
     @torch.no_grad()
@@ -421,17 +456,14 @@ class PagedKVCache:
         lengths of the given sequences instead of per-token positions.  `check_finite=False` leaves out the NaN/Inf
         check of k and v, which reads a flag back from the device and so makes the host wait for everything enqueued
         before (as `prepare_decode` offers for decode steps)."""
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, _current(self.device):
             self._guard()
-            self._check_inputs(check_finite, k=k, v=v)
-            self._refuse_pool_aliases(k, v)
-            ids, counts = self._segments(k.shape[0], sequence_ids, cu_seqlens)
-            plan, _, _ = self._store(k, v, ids, counts)
+            ids, _, (plan, _, _) = self._append(k, v, sequence_ids, cu_seqlens, check_finite)
             return tuple(plan.lengths[s] for s in ids)
 
     # ------------------------------------------------------------------ attend
     def _query_rows(self, q, sequence_ids, positions):
-        self._check_inputs(True, q=q)
+        self._check_inputs(True, q=q)()
         if q.shape[1] % self.num_kv_heads:
             raise ValueError("Hq must be a multiple of Hkv")
         ids = self._layout.validate_ids(_ints(sequence_ids, "sequence_ids"))
@@ -454,7 +486,7 @@ class PagedKVCache:
             if len(self._attend_buffers) >= 8:
                 self._attend_buffers.pop(next(iter(self._attend_buffers)))
             hk, dev = self.num_kv_heads, self.device
-            nbytes = self._lib.moba_decode_attend_workspace_bytes(ctypes.byref(desc), rows, hq, slots)
+            nbytes = self._lib.moba_decode_attend_workspace_bytes(desc, rows, hq, slots)
             found = dict(u_chunk=torch.empty((rows, hk, umax), dtype=torch.int32, device=dev),
                          u_mask=torch.empty((rows, hk, umax), dtype=torch.int32, device=dev),
                          u_count=torch.empty((rows, hk), dtype=torch.int32, device=dev),
@@ -462,12 +494,12 @@ class PagedKVCache:
             self._attend_buffers[key] = found
         return found
 
-    def _attend_rows(self, q, ids, pos, topk, dense, d_ids, d_pos):
+    def _attend_rows(self, q, ids, pos, topk, dense, d_ids, d_pos, desc):
         """Routing (unless dense) and attention for validated query rows whose sequence ids and positions are already on
         the device."""
         q = q.contiguous()
         rows, hq, _ = q.shape
-        desc, lib = self._desc(), self._lib
+        lib = self._lib
         out = torch.empty_like(q)
         lse = torch.empty((rows, hq), dtype=torch.float32, device=self.device)
         selected, remote = None, 0
@@ -484,41 +516,46 @@ class PagedKVCache:
         buf = self._attend_scratch(rows, hq, slots, umax, desc)
         union = (buf["u_chunk"].data_ptr(), buf["u_mask"].data_ptr(), buf["u_count"].data_ptr())
         if not dense:
-            self._launch("moba_decode_route", ctypes.byref(desc), q.data_ptr(), d_ids.data_ptr(), d_pos.data_ptr(), rows, hq, remote,
+            self._launch("moba_decode_route", desc, q.data_ptr(), d_ids, d_pos, rows, hq, remote,
                          width, None, selected.data_ptr(), *union)
-        self._launch("moba_decode_attend", ctypes.byref(desc), q.data_ptr(), d_ids.data_ptr(), d_pos.data_ptr(), rows, hq,
+        self._launch("moba_decode_attend", desc, q.data_ptr(), d_ids, d_pos, rows, hq,
                      None if dense else selected.data_ptr(), slots, *(union if not dense else (None, None, None)), umax,
                      buf["workspace"].data_ptr(), buf["nbytes"], out.data_ptr(), lse.data_ptr(), self._status.data_ptr())
         return DecodeResult(out, lse, selected, ids, pos)
 
     @torch.no_grad()
     def attend(self, q, *, sequence_ids, positions=None, topk=4, mode="moba"):
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, _current(self.device):
             self._guard()
             dense = wants_dense(mode, topk)
             ids, pos = self._query_rows(q, sequence_ids, positions)
-            d_ids, d_pos = self._staging.send(ids, pos)
-            return self._attend_rows(q, ids, pos, topk, dense, d_ids, d_pos)
+            block, (d_ids, d_pos) = self._staging.send(ids, pos)
+            return self._attend_rows(q, ids, pos, topk, dense, d_ids, d_pos, ctypes.byref(self._desc()))
 
     @torch.no_grad()
     def append_and_attend(self, q, k, v, *, sequence_ids, cu_seqlens=None, topk=4, mode="moba"):
         """Appends k, v and attends with one query per appended token (token i of a segment sees the cache up to and
         including itself)."""
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, _current(self.device):
             self._guard()
             dense = wants_dense(mode, topk)
-            self._check_inputs(True, k=k, v=v, q=q)
-            self._refuse_pool_aliases(q, k, v)
-            if q.shape[1] % self.num_kv_heads:
-                raise ValueError("Hq must be a multiple of Hkv")
-            if q.shape[0] * q.shape[1] >= 2 ** 31:
-                raise ValueError("query grid exceeds int32 capacity")
-            ids, counts = self._segments(k.shape[0], sequence_ids, cu_seqlens)
-            starts = [self._layout.lengths[s] for s in ids]
-            row_ids = np.repeat(np.asarray(ids, dtype=np.int32), counts)
-            row_pos = np.concatenate([np.arange(first, first + n, dtype=np.int32) for first, n in zip(starts, counts)])
-            _, _, (d_ids, d_pos) = self._store(k, v, ids, counts, extra=(row_ids, row_pos))
-            return self._attend_rows(q, tuple(row_ids.tolist()), tuple(row_pos.tolist()), topk, dense, d_ids, d_pos)
+            finite = self._check_inputs(True, k=k, v=v, q=q)
+            try:                                      # beside the check
+                self._refuse_pool_aliases(q, k, v)
+                if q.shape[1] % self.num_kv_heads:
+                    raise ValueError("Hq must be a multiple of Hkv")
+                if q.shape[0] * q.shape[1] >= 2 ** 31:
+                    raise ValueError("query grid exceeds int32 capacity")
+                ids, counts = self._segments(k.shape[0], sequence_ids, cu_seqlens)
+                lengths = self._layout.lengths
+                row_ids = tuple(s for s, n in zip(ids, counts) for _ in range(n))
+                row_pos = tuple(p for s, n in zip(ids, counts) for p in range(lengths[s], lengths[s] + n))
+                planned = self._plan_store(ids, counts, extra=(row_ids, row_pos))
+            finally:
+                finite()
+            desc = ctypes.byref(self._desc())
+            self._store(k, v, ids, counts, planned, desc)
+            return self._attend_rows(q, row_ids, row_pos, topk, dense, *planned[2][1][5:], desc)
 
     # ------------------------------------------------------------------ reset / read-back
     @torch.no_grad()
@@ -526,13 +563,11 @@ class PagedKVCache:
         with self._lock, torch.cuda.device(self.device):
             self._guard()
             ids = tuple(range(self._layout.batch_size)) if sequence_ids is None else _ints(sequence_ids, "sequence_ids")
-            staged = self._layout.clone()      # a copy first: a failure while staging publishes nothing
-            staged.reset(ids)
-            d_ids, d_zero = self._staging.send(ids, [0] * len(ids))
-            desc = self._desc()
-            self._launch("moba_cache_update", ctypes.byref(desc), None, 0, d_ids.data_ptr(), d_zero.data_ptr(), len(ids), 1)
-            self._layout = staged
-            self._candidate_count = self._routable(staged.lengths)
+            ids = self._layout.validate_ids(ids, unique=True)
+            block, (d_ids, d_zero) = self._staging.send(ids, (0,) * len(ids))
+            self._launch("moba_cache_update", ctypes.byref(self._desc()), None, 0, d_ids, d_zero, len(ids), 1)
+            self._layout.reset(ids)            # last: a failure while staging publishes nothing
+            self._candidate_count = self._routable(self._layout.lengths)
 
     @torch.no_grad()
     def materialize(self, sequence_id):

@@ -25,13 +25,7 @@ import torch
 
 from . import _ext
 from .cache_layout import IncrementalLayout, positive_int
-from .kv_cache import CacheLife, DecodeResult, _ints, wants_dense
-
-
-def current_stream_handle(device_index):
-    """The current CUDA stream of the device as an integer handle (the cheapest route torch offers; a step asks twice)."""
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return raw(device_index) if raw is not None else torch.cuda.current_stream(device_index).cuda_stream
+from .kv_cache import CacheLife, DecodeResult, _ints, current_stream_handle, wants_dense
 
 
 def _storage_address(t):
