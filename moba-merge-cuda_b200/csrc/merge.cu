@@ -20,12 +20,22 @@
 namespace moba {
 namespace {
 
+// Clears the counters.  A kernel, not a memset, so that the ticket pass can be a dependent launch behind it, its mapping read by
+// then (229376 rows, 619 thousand contributions: 36.9 -> 33.8 us a merge).
+__global__ void __launch_bounds__(256) merge_clear_kernel(int* counts, long long P) {
+  dependents_may_start();
+  const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
+  if (i + 4 <= P && !(reinterpret_cast<uintptr_t>(counts) & 15)) *reinterpret_cast<int4*>(counts + i) = make_int4(0, 0, 0, 0);
+  else for (long long j = i; j < min(i + 4, P); ++j) counts[j] = 0;
+}
+
 __global__ void __launch_bounds__(256) merge_ticket_kernel(const int64_t* __restrict__ mapping, long long M, long long P, int kmax,
-                                                           int* __restrict__ counts, int* __restrict__ slots, unsigned* status) {
-  dependents_may_start();   // the row kernel's self rows do not depend on the lists
+                                                           int* counts, int* slots, unsigned* status) {
   const long long m = (long long)blockIdx.x * 256 + threadIdx.x;
+  const long long p = m < M ? mapping[m] : 0;   // an input of the call, read beside the clearing
+  wait_for_predecessor();                       // the counters are clear, and whoever used this scratch before is done
+  dependents_may_start();                       // the row kernel's self rows do not depend on the lists
   if (m >= M) return;
-  const long long p = mapping[m];
   if (p < 0 || p >= P) { atomicOr(status, kErrBadIndex); return; }
   const int slot = atomicAdd(counts + p, 1);
   if (slot < kmax) slots[p * kmax + slot] = (int)m;
@@ -349,9 +359,10 @@ extern "C" int moba_merge_forward(const void* self_out, const float* self_lse, c
   cudaStream_t st = (cudaStream_t)stream;
   int* counts = static_cast<int*>(scratch);
   int* slots = reinterpret_cast<int*>(static_cast<char*>(scratch) + align256m((size_t)rows * 4));
-  if (cudaMemsetAsync(counts, 0, (size_t)rows * 4, st) != cudaSuccess) return MOBA_ERR_CUDA;
+  merge_clear_kernel<<<(unsigned)((rows + 1023) / 1024), 256, 0, st>>>(counts, rows);
   if (remote_rows > 0)
-    merge_ticket_kernel<<<(unsigned)((remote_rows + 255) / 256), 256, 0, st>>>(mapping, remote_rows, rows, kmax, counts, slots, status);
+    launch_dependent(32u, merge_ticket_kernel, dim3((unsigned)((remote_rows + 255) / 256)), dim3(256), 0, st, mapping, remote_rows, rows, kmax, counts, slots,
+                     status);
   if (dtype == 0)
     launch_rows<__nv_bfloat16>(self_out, self_lse, remote_out, remote_lse, counts, slots, rows, dim, kmax, out, lse, st);
   else if (dtype == 2)
