@@ -56,6 +56,20 @@ inline int device_sms() {
   return n;
 }
 
+// The limit of a kernel's dynamic shared memory, which belongs to the function: one value per kernel, set once per device (a call
+// of the runtime costs a small prefill as much as a tenth of a launch, and it has four such kernels).
+template <auto KERNEL>
+inline cudaError_t shared_memory_limit(int bytes) {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 64 && done[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+  e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev < 64) done[dev].store(true, std::memory_order_relaxed);
+  return e;
+}
+
 // The same for a grid of clusters of `cluster` CTAs along x.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent_cluster(unsigned kind, void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster, size_t smem,

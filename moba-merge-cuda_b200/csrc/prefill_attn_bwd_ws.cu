@@ -17,6 +17,7 @@
 //                per row into the FP32 accumulator by the copy engine, behind the next tile's math
 // Tensor memory: S^T 0-127 (P^T as packed 16-bit over the first columns of each thread's range), dP^T 128-255 (dS^T
 // likewise), dV 256-319, dK 320-383, dQ 384-447, K 448-479 and V 480-511 as stationary A operands.
+#include "launch.cuh"
 #include "prefill_bwd.cuh"
 
 namespace moba {
@@ -499,7 +500,7 @@ template <int SPLIT>
 static cudaError_t launch_bwd_ws_as(const BwdArgs& a, cudaStream_t st) {
   const size_t smem = 8192 + (size_t)kTile * 64 * 2 * (1 + 2 * kWsRing) + (size_t)kTile * kStageRow + (size_t)kTile * kTile * 2;
   const auto kernel = a.pv.fp16 ? attn_bwd_ws_kernel<true, SPLIT> : attn_bwd_ws_kernel<false, SPLIT>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = a.pv.fp16 ? shared_memory_limit<attn_bwd_ws_kernel<true, SPLIT>>((int)smem) : shared_memory_limit<attn_bwd_ws_kernel<false, SPLIT>>((int)smem);
   if (e != cudaSuccess) return e;
   return launch_clusters(kernel, dim3(a.pv.n_qtiles * SPLIT, a.pv.Hkv), dim3(kWsThreads), SPLIT, smem, st, a);
 }

@@ -11,6 +11,7 @@
 // thread's own range), dV 128-255, dK 256-383, dQ^T 384-447, K 448-511 as a stationary A operand.
 // Shared memory: K and V images (32 KB each), a 3-slot ring of (Q, dO) half tiles (64 rows x 128 columns
 // each, 16 KB), the dS^T tile (128 key rows x 64 query columns, 16 KB), the dQ rows of a step (32 KB).
+#include "launch.cuh"
 #include "prefill_bwd.cuh"
 
 namespace moba {
@@ -476,7 +477,7 @@ template <int SPLIT>
 static cudaError_t launch_bwd_ws128_as(const BwdArgs& a, cudaStream_t st) {
   const size_t smem = 4096 + 2 * (size_t)kTile * 128 * 2 + (size_t)kRing * 2 * kQRows * 128 * 2 + (size_t)kTile * kQRows * 2 + (size_t)kQRows * 128 * 4;
   const auto kernel = a.pv.fp16 ? attn_bwd_ws128_kernel<true, SPLIT> : attn_bwd_ws128_kernel<false, SPLIT>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = a.pv.fp16 ? shared_memory_limit<attn_bwd_ws128_kernel<true, SPLIT>>((int)smem) : shared_memory_limit<attn_bwd_ws128_kernel<false, SPLIT>>((int)smem);
   if (e != cudaSuccess) return e;
   return launch_clusters(kernel, dim3(a.pv.n_qtiles * SPLIT, a.pv.Hkv), dim3(kThreads), SPLIT, smem, st, a);
 }

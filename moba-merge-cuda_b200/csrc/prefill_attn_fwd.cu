@@ -20,6 +20,7 @@
 // than 2^8 (the rescale of O in TMEM is then done by the row's own thread), P is written back into
 // tensor memory over S as packed bf16 -> O += P V with P read from TMEM.  While one lane does its
 // softmax the tensor pipe works for the other, and the copy engine runs K/V tiles ahead of both.
+#include "launch.cuh"
 #include "prefill_common.cuh"
 #include "sm100.cuh"
 
@@ -675,7 +676,7 @@ static int sm_count() {
 template <int DPAD, bool SELF, bool F16>
 static cudaError_t launch_fwd_as(const FwdArgs& a, long long items, cudaStream_t st) {
   const int smem = FwdCfg<DPAD, SELF>::SMEM;
-  cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<DPAD, SELF, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = shared_memory_limit<attn_fwd_kernel<DPAD, SELF, F16>>(smem);
   if (e != cudaSuccess) return e;
   const int sms = sm_count();
   if (sms <= 0) return cudaErrorUnknown;

@@ -430,3 +430,17 @@ def test_threads_with_batches_of_different_chunk_counts():
                                                          call.route_bytes, ga._stream(device))))
         keep.append((q, k, call, state, scratch))
     assert two_threads(calls, 4000) == [0, 0]
+
+
+@pytest.mark.parametrize("chunk", [256, 257, 2048, 2049])    # one slice of 256 tokens, two, eight (a cluster), nine (counters)
+def test_chunk_means_over_any_number_of_slices(chunk):
+    """Selection against the oracle's FP64 gate where the mean of a chunk is one CTA's, a cluster's and the last arriving CTA's."""
+    gen = torch.Generator().manual_seed(chunk)
+    lens, hq, hkv, dim = (4 * chunk + 33, 2 * chunk), 4, 2, 64
+    q, k, v = (torch.randn(sum(lens), h, dim, generator=gen).bfloat16() for h in (hq, hkv, hkv))
+    cu = cu_from_lens(lens)
+    _, _, captured, _ = _run(q, k, v, cu, chunk, 3)
+    r = mo.route_prefill(torch_to_f64(q), torch_to_f64(k), cu, chunk, 3)
+    differs = (captured["selected"].numpy() != r["selected"]).any(axis=0).T
+    # the bound of test_forward_against_oracle_on_seeded_inputs: 64 products, each off by an FP32 rounding of its scale
+    assert (r["margin"][differs] <= (64 * np.finfo(np.float32).eps * r["scale"])[differs]).all() and differs.mean() < 1e-3
