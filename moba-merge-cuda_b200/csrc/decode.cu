@@ -414,15 +414,15 @@ __global__ void __launch_bounds__(256) decode_step_begin_kernel(CacheView cv, co
 constexpr int kRouteTile = 64;      // chunk means staged in shared memory per round of decode_route_kernel
 constexpr int kRouteThreads = 256;  // eight warps: a group of up to eight heads is ranked in one round
 
-// Scores and picks of one (query row, kv head) by kRouteThreads threads, see decode_route_kernel: q, scores (or null) and selected (or
-// null) of the group's first head.  s_dyn: route_floats(G, width, D) floats and a tile of means; the heads that picked a
+// Scores and picks of one (query row, kv head) by kRouteThreads threads, see decode_route_kernel.  HELD: the group's query rows are at `held`, and
+// selected may be null; otherwise they are those of `row` in q.  s_dyn: route_floats(G, width, D) floats and a tile of means; the heads that picked a
 // chunk are left in route_mask(s_dyn).
 __host__ __device__ __forceinline__ size_t route_floats(int G, int width, int D) { return ((size_t)G * width + width + 1 + (size_t)G * D + 3) & ~(size_t)3; }
 __host__ __device__ __forceinline__ size_t route_bytes(int G, int width, int D) { return route_floats(G, width, D) * 4 + (size_t)kRouteTile * ((D / 8) | 1) * 16; }
 __device__ __forceinline__ unsigned* route_mask(float* s_dyn, int G, int width) { return reinterpret_cast<unsigned*>(s_dyn + G * width); }
-template <bool F16>
-__device__ __forceinline__ void route_group(const CacheView& cv, float* s_dyn, const __nv_bfloat16* qsrc, int sid, int g, int G, int cur, int nlegal,
-                                            int remote, int width, float* scores, int* selected) {
+template <bool F16, bool HELD>
+__device__ __forceinline__ void route_group(const CacheView& cv, float* s_dyn, const __nv_bfloat16* q, const __nv_bfloat16* held, int row, int Hq, int sid,
+                                            int g, int G, int cur, int nlegal, int remote, int width, float* scores, int* selected) {
   float* s_scores = s_dyn;                                            // [G][width]
   unsigned* s_mask = route_mask(s_dyn, G, width);                     // [width + 1]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -434,6 +434,7 @@ __device__ __forceinline__ void route_group(const CacheView& cv, float* s_dyn, c
   float* s_q = reinterpret_cast<float*>(s_mask + width + 1);  // [G][D]
   // the query loads are issued here and stored after the first tile of means has been requested, so that the two
   // trips to L2 overlap (a store to shared memory would make the warp wait for its load first)
+  const __nv_bfloat16* qsrc = HELD ? held : q + ((long long)row * Hq + g * G) * cv.D;
   float qreg[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -479,21 +480,22 @@ __device__ __forceinline__ void route_group(const CacheView& cv, float* s_dyn, c
       }
       const float sc = (a0 + a1) + (a2 + a3);
       s_scores[hl * width + c0 + cl] = sc;
-      if (scores) scores[(long long)hl * width + c0 + cl] = sc;
+      if (scores) scores[((long long)row * Hq + g * G + hl) * width + c0 + cl] = sc;
     }
     __syncthreads();
   }
   for (int pair = tid; pair < G * (width - nlegal); pair += kRouteThreads) {  // not a candidate
     const int hl = pair / (width - nlegal), c = nlegal + pair - hl * (width - nlegal);
     s_scores[hl * width + c] = -INFINITY;
-    if (scores) scores[(long long)hl * width + c] = -INFINITY;
+    if (scores) scores[((long long)row * Hq + g * G + hl) * width + c] = -INFINITY;
   }
   __syncthreads();
   // top-k: one warp per head, `remote` rounds of (max value, lowest index among equals)
   for (int hl = warp; hl < G; hl += kRouteThreads / 32) {
     float* sc = s_scores + hl * width;
-    int* out = selected ? selected + hl * (remote + 1) : nullptr;
-    if (out && lane == 0) out[0] = cur;
+    int* out = selected + ((long long)row * Hq + g * G + hl) * (remote + 1);
+    const bool keep = !HELD || selected != nullptr;
+    if (keep && lane == 0) out[0] = cur;
     for (int r = 0; r < remote; ++r) {
       float best = -INFINITY;
       int idx = 0x7FFFFFFF;
@@ -509,7 +511,7 @@ __device__ __forceinline__ void route_group(const CacheView& cv, float* s_dyn, c
       }
       const bool found = best > -INFINITY && idx != 0x7FFFFFFF;
       if (lane == 0) {
-        if (out) out[1 + r] = found ? idx : -1;
+        if (keep) out[1 + r] = found ? idx : -1;
         if (found) {
           sc[idx] = -INFINITY;
           atomicOr(&s_mask[idx], 1u << hl);
@@ -541,9 +543,7 @@ __global__ void __launch_bounds__(kRouteThreads) decode_route_kernel(CacheView c
   const int sid = ids[row], pos = positions[row];
   const int cur = pos / cv.C;
   const int nlegal = min(min(cur, width), cv.max_chunks);
-  const long long first = (long long)row * Hq + g * G;  // the group's first head
-  route_group<F16>(cv, s_dyn, q + first * cv.D, sid, g, G, cur, nlegal, remote, width, scores ? scores + first * width : nullptr,
-                   selected + first * (remote + 1));
+  route_group<F16, false>(cv, s_dyn, q, nullptr, row, Hq, sid, g, G, cur, nlegal, remote, width, scores, selected);
   const unsigned* s_mask = route_mask(s_dyn, G, width);
   // union list: routed chunks ascending, the own chunk (all heads) last
   if (warp == 0) {
@@ -1150,12 +1150,12 @@ __device__ __forceinline__ void attend_softmax(const float (&s)[4], float& m, fl
 // Paged attention of one head block over `ntiles` consecutive stages, by a team of four warps.  The query heads of
 // the GQA group are the 16 rows of m16n8k16 tensor-core tiles (unused rows are zero), so a K/V token read from HBM
 // serves every head at no extra cost.  Each warp takes 16 tokens of every stage and keeps its own running (max, sum, O).
-//   q         the group's query rows, D values each
+//   held      the group's query rows, D values each, where the caller has them (HELD), else they are those of `row` in a.q
 //   ring      NS stages            rowbase [NS][64]   nv, mask [2 NS]: a slot is rewritten NS stages ahead, while the slots
 //                                                     before it are still read
 //   which     heads of the block that count: stages that none of them attends are passed over (see attend_spoiled)
-template <int DP, int NS, bool F16, bool WIDE, class Sync>
-__device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& look, int ntiles, int sid, const __nv_bfloat16* q, int g, int hb, int ltid,
+template <int DP, int NS, bool F16, bool WIDE, bool HELD, class Sync>
+__device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& look, int ntiles, int sid, int row, const __nv_bfloat16* held, int g, int hb, int ltid,
                                               uint8_t* ring, long long (*s_rowbase)[kStageTokens], int* s_nv, unsigned* s_mask,
                                               Sync team_sync, unsigned which, AttendState<DP>& st) {
   constexpr int KSTEPS = DP / 16;
@@ -1178,7 +1178,7 @@ __device__ __forceinline__ void attend_stages(const AttendArgs& a, StageCursor& 
   uint32_t qf[KSTEPS][4];  // A operand: rows qr and qr + 8, all k-steps
   {
     const bool r0 = hb + qr < G, r1 = WIDE && hb + qr + 8 < G;
-    const __nv_bfloat16* q0 = q + (hb + qr) * D;
+    const __nv_bfloat16* q0 = HELD ? held + (hb + qr) * D : a.q + ((long long)row * a.Hq + g * G + hb + qr) * D;
     const __nv_bfloat16* q1 = q0 + 8 * D;
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
@@ -1286,9 +1286,9 @@ struct AttendSums { float *m, *l, *o; };
 struct AttendExtra { const float* score; const __nv_bfloat16* v; };
 
 // Combines the NW warps of a CTA through shared memory (s_o: NW * 16 * (DP + 2) floats), for heads h0 to h1 - 1 of the block.
-template <int DP, int NW, bool WIDE>
+template <int DP, int NW, bool WIDE, bool EXTRA, bool F16>
 __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, int h0, int h1, int D, const AttendSums& to,
-                                               const AttendExtra& extra = AttendExtra{nullptr, nullptr}, bool f16 = false) {
+                                               const AttendExtra& extra) {
   constexpr int ROWS = WIDE ? 16 : 8;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, qr = lane >> 2, qc = lane & 3;
   st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 1); st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 2);
@@ -1319,10 +1319,10 @@ __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, 
 #pragma unroll
     for (int w = 0; w < NW; ++w) { mw[w] = s_ml[((size_t)w * ROWS + hh) * 2]; big = fmaxf(big, mw[w]); }
     float lsum = 0.f, v0 = 0.f, v1 = 0.f;
-    if (extra.score) {
+    if (EXTRA && extra.score) {
       const float m = extra.score[hh];
       big = fmaxf(big, m);
-      const float2 x = unpack16(*reinterpret_cast<const uint32_t*>(extra.v + d), f16);
+      const float2 x = unpack16<F16>(*reinterpret_cast<const uint32_t*>(extra.v + d));
       lsum = dec_exp2(m - big);
       v0 = x.x * lsum; v1 = x.y * lsum;
     }
@@ -1405,7 +1405,6 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
   const int tid = threadIdx.x, team = tid >> 7, ltid = tid & 127;
   const bool dense = STEP ? step.selected == nullptr : a.selected == nullptr;
   float* s_sum = reinterpret_cast<float*>(s_pipe + PIPE);
-  const __nv_bfloat16* q = a.q + ((long long)row * a.Hq + g * G) * D;
   const int sid = a.ids[row];
   int pos, listed;
   if (!STEP) {
@@ -1443,7 +1442,6 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
       }
       *reinterpret_cast<uint4*>(s_new + hl * D + c * 8) = w;
     }
-    q = s_new;
     __syncthreads();
     if (rank == 0) {
       // append; the page may have been opened by this step's delta
@@ -1472,9 +1470,8 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
     if (!dense) {
       const int cur = pos / cv.C, nlegal = min(min(cur, step.width), cv.max_chunks);
       float* s_dyn = reinterpret_cast<float*>(s_pipe);
-      const long long first = (long long)row * a.Hq + g * G;
-      route_group<F16>(cv, s_dyn, s_new, sid, g, G, cur, nlegal, step.remote, step.width, rank == 0 && step.scores ? step.scores + first * step.width : nullptr,
-                       rank == 0 ? step.selected + first * (step.remote + 1) : nullptr);
+      route_group<F16, true>(cv, s_dyn, nullptr, s_new, row, a.Hq, sid, g, G, cur, nlegal, step.remote, step.width, rank == 0 ? step.scores : nullptr,
+                             rank == 0 ? step.selected : nullptr);
       const unsigned* picked = route_mask(s_dyn, G, step.width);
       if (tid < 32) {  // routed chunks ascending, the own chunk (all heads) last
         int count = 0;
@@ -1523,13 +1520,13 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
     int head = -1;  // all together, see attend_spoiled
     do {
       look.start(first);
-      attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, q, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
+      attend_stages<DP, NS, F16, WIDE, STEP>(a, look, ntiles, sid, row, s_new, g, hb, ltid, s_pipe + (size_t)team * NS * STAGE_BYTES, s_rowbase[team],
                                        s_nv[team], s_mask[team], team_sync, head < 0 ? 0xFFFFu : 1u << head, st);
       const bool again = head < 0 && !dense && attend_spoiled(st);
       if (!again)
-        attend_combine<DP, NW, WIDE>(st, reinterpret_cast<float*>(s_pipe), max(head, 0), head < 0 ? nh : head + 1, D,
+        attend_combine<DP, NW, WIDE, STEP, F16>(st, reinterpret_cast<float*>(s_pipe), max(head, 0), head < 0 ? nh : head + 1, D,
                                      AttendSums{s_m + hb, s_l + hb, s_sum + (size_t)hb * D},
-                                     STEP && rank == 0 ? AttendExtra{s_score + hb, s_new + (G + 1) * D} : AttendExtra{nullptr, nullptr}, F16);
+                                     STEP && rank == 0 ? AttendExtra{s_score + hb, s_new + (G + 1) * D} : AttendExtra{nullptr, nullptr});
       if (again || head >= 0) ++head;
     } while (head >= 0 && head < nh);
   }
@@ -1694,12 +1691,12 @@ __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) decode_attend_stream_k
       int head = -1;  // all together, see attend_spoiled
       do {
         look.start(j0);
-        attend_stages<DP, NS, F16, WIDE>(a, look, ntiles, sid, a.q + ((long long)row * a.Hq + g * G) * D, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); },
+        attend_stages<DP, NS, F16, WIDE, false>(a, look, ntiles, sid, row, nullptr, g, hb, tid, s_pipe, s_rowbase, s_nv, s_mask, [] { __syncthreads(); },
                                          head < 0 ? 0xFFFFu : 1u << head, st);
         const bool again = head < 0 && !dense && attend_spoiled(st);
         if (!again)
-          attend_combine<DP, 4, WIDE>(st, reinterpret_cast<float*>(s_pipe), max(head, 0), head < 0 ? nh : head + 1, D,
-                                      AttendSums{a.pm + pidx, a.pl + pidx, a.pacc + pidx * D});
+          attend_combine<DP, 4, WIDE, false, F16>(st, reinterpret_cast<float*>(s_pipe), max(head, 0), head < 0 ? nh : head + 1, D,
+                                                  AttendSums{a.pm + pidx, a.pl + pidx, a.pacc + pidx * D}, AttendExtra{nullptr, nullptr});
         if (again || head >= 0) ++head;
       } while (head >= 0 && head < nh);
     }
