@@ -258,11 +258,11 @@ class FullQwen2Session:
             p.launch("step")
 
     def _compute_step_fused(self):
-        """The same step in six launches per dense layer and seven per MoBA layer: every projection is one
-        `moba_decode_linear` (the weight read once, all loads in flight), with the residual add + RMSNorm in front of
-        the q/k/v and the gate/up projections and SiLU * up behind the latter inside the same launch; rotary embedding
-        and split of q/k/v run inside the first launch of the attention step (metadata + append + chunk mean), then
-        routing (MoBA layers) and the attention kernel."""
+        """The same step in five launches per layer: every projection is one `moba_decode_linear` (the weight read once, all
+        loads in flight), with the residual add + RMSNorm in front of the q/k/v and the gate/up projections and SiLU * up
+        behind the latter inside the same launch; rotary embedding and split of q/k/v, metadata, append, chunk mean, routing (MoBA
+        layers) and attention are `moba_decode_step`, one launch while every KV head has a cluster of CTAs, else two or
+        three."""
         import ctypes
         lib, body, cfg = self._lib, self.model.model, self.model.config
         st = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
