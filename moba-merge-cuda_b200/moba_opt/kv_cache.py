@@ -328,8 +328,8 @@ class PagedKVCache:
     @property
     def page_table(self):
         """Immutable CPU snapshot of the logical->physical page map."""
-        with self._lock:
-            return self._owner.page_table if self._owner is not None else self._layout.tables
+        owner = self._owner
+        return owner.page_table if owner is not None else self._layout.tables
 
     # ------------------------------------------------------------------ plumbing shared with PreparedDecode
     def _desc(self):

@@ -2,9 +2,14 @@
 reference's tests pin (tests/test_cache_layout.py:13-68, tests/test_prepared_layout.py:6-30):
 atomic planning, stale plans, LIFO page reuse, page math for non-dividing sizes, and equivalence of
 the incremental lease with the transactional allocator."""
+import copy
+import pickle
+import random
+from dataclasses import FrozenInstanceError, replace
+
 import pytest
 
-from moba_opt.cache_layout import IncrementalLayout, PageAllocator
+from moba_opt.cache_layout import AppendPlan, IncrementalLayout, PageAllocator
 
 
 def snapshot(a):
@@ -133,19 +138,98 @@ def test_plan_without_token_lists_is_the_same_plan(page):
     assert a.lengths == (13, 1, 14)
 
 
-def test_a_plan_shows_the_next_state_until_the_allocator_moves_on():
-    """A plan holds what an append changes; its tables and pool are the next state's before and after the commit, and are
-    refused once another call has changed the allocator."""
+class EagerAllocator:
+    """The allocator's contract in its plainest form: every plan and every state is a copy of everything."""
+
+    def __init__(self, sequences, width, page, pages):
+        self.page = page
+        self.tables, self.lengths = ((-1,) * width,) * sequences, (0,) * sequences
+        self.free_pages = tuple(range(pages - 1, -1, -1))
+
+    def append(self, ids, counts):
+        tables, lengths, pool = [list(row) for row in self.tables], list(self.lengths), list(self.free_pages)
+        for sid, n in zip(ids, counts):
+            for logical in range(-(-lengths[sid] // self.page), -(-(lengths[sid] + n) // self.page)):
+                tables[sid][logical] = pool.pop()
+            lengths[sid] += n
+        return tuple(map(tuple, tables)), tuple(lengths), tuple(pool)
+
+    def reset(self, ids):
+        tables, lengths, pool = list(self.tables), list(self.lengths), list(self.free_pages)
+        for sid in ids:
+            pool += [p for p in tables[sid] if p >= 0]
+            tables[sid], lengths[sid] = (-1,) * len(tables[sid]), 0
+        return tuple(tables), tuple(lengths), tuple(pool)
+
+
+def shown(x):
+    return x.tables, x.lengths, x.free_pages
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_plans_are_snapshots_whatever_the_allocator_does_next(seed):
+    """Plans hold what an append changes and build tables and pool late; what they show, and what the allocator shows, is what copies
+    made at once would: read before or after the commit, after later commits, resets and leases, or never."""
+    rng = random.Random(seed)
+    a, plain = PageAllocator(3, 40, 3, 30, 4), EagerAllocator(3, 14, 3, 30)
+    kept = [(a.tables, plain.tables)]
+    for _ in range(60):
+        ids = rng.sample(range(3), rng.randint(1, 3))
+        step = rng.randrange(4)
+        if step == 0:
+            a.reset(ids)
+            plain.tables, plain.lengths, plain.free_pages = plain.reset(ids)
+        elif step == 1 and max(a.lengths) < 40 and len(a.free_pages) >= 3:
+            lease = IncrementalLayout(a, ids)
+            lease.commit(lease.plan())
+            lease.publish(a)
+            plain.tables, plain.lengths, plain.free_pages = plain.append(ids, [1] * len(ids))
+        else:
+            counts = [rng.randint(1, 9) for _ in ids]
+            try:
+                plan, other = a.plan_append(ids, counts), a.plan_append(ids[:1], counts[:1], tokens=False)
+            except ValueError:
+                continue
+            want, unused = plain.append(ids, counts), plain.append(ids[:1], counts[:1])
+            if rng.random() < 0.3:
+                assert shown(plan) == want
+            if rng.random() < 0.5:
+                kept.append((other, unused))
+            if rng.random() < 0.7:
+                a.commit(plan)
+                plain.tables, plain.lengths, plain.free_pages = want
+            kept.append((plan, want))
+        assert shown(a) == shown(plain)
+        kept.append((a.tables, plain.tables))
+        if len(kept) > 12:
+            got, want = kept.pop(rng.randrange(len(kept)))
+            assert (shown(got) if isinstance(got, AppendPlan) else got) == want
+    for got, want in kept:
+        assert (shown(got) if isinstance(got, AppendPlan) else got) == want
+
+
+def test_plans_and_allocators_are_values():
+    """A plan is a frozen dataclass of its fields, and commit takes any plan of the present version; clones, copies and pickles of an
+    allocator stand for themselves, and a snapshot that nothing has changed is not built again."""
     a = PageAllocator(2, 20, 3, 14, 4)
     a.commit(a.plan_append([1], [4]))
-    first, second = a.plan_append([0, 1], [7, 3]), a.plan_append([0], [2])
-    want = (first.tables, first.free_pages)
-    assert want[0][0][:3] == (2, 3, 4) and want[0][1][:3] == (0, 1, 5) and len(want[1]) == 8
-    a.commit(first)
-    assert (a.tables, a.free_pages) == want == (first.tables, first.free_pages)
-    for stale in (lambda: a.commit(second), lambda: second.tables, lambda: second.free_pages, lambda: a.reset([0]) or first.tables):
-        with pytest.raises(RuntimeError, match="stale"):
-            stale()
-    other = PageAllocator(2, 20, 3, 14, 4)
-    with pytest.raises(RuntimeError, match="stale"):      # a plan of another allocator
-        other.commit(PageAllocator(2, 20, 3, 14, 4).plan_append([0], [1]))
+    plan, same, first = (a.plan_append([0, 1], [7, 3]) for _ in range(3))
+    assert plan == same and hash(plan) == hash(same) and repr(plan) == repr(same) and "tables=((2, 3, 4" in repr(plan)
+    with pytest.raises(FrozenInstanceError):
+        plan.lengths = ()
+    whole = AppendPlan(plan.version, plan.tables, plan.lengths, plan.free_pages, plan.token_sequences, plan.token_positions,
+                       plan.completed_chunks, plan.page_edits)
+    assert whole == plan == copy.copy(same) == pickle.loads(pickle.dumps(first)) == replace(first, page_edits=first.page_edits)
+    twins = [a.clone(), copy.copy(a), copy.deepcopy(a), pickle.loads(pickle.dumps(a))]
+    before = snapshot(a)
+    for twin, made in zip(twins, (whole, plan, a.plan_append([0, 1], [7, 3]), twins[3].plan_append([0, 1], [7, 3]))):
+        assert snapshot(twin) == before
+        twin.commit(made)                                  # another allocator's plan among them
+        assert shown(twin) == shown(plan) and snapshot(a) == before
+        twin.reset([0])
+        assert snapshot(a) == before
+    assert a.tables is a.tables
+    a.commit(a.plan_append([0], [1]))
+    assert a.tables is a.tables and a.tables[1] is before[0][1]     # the row that did not change
+    with pytest.raises(RuntimeError, match="stale"):
+        a.commit(plan)
