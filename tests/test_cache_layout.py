@@ -233,3 +233,21 @@ def test_plans_and_allocators_are_values():
     assert a.tables is a.tables and a.tables[1] is before[0][1]     # the row that did not change
     with pytest.raises(RuntimeError, match="stale"):
         a.commit(plan)
+
+
+def test_a_plan_shows_the_next_state_until_the_allocator_moves_on():
+    """A plan holds what an append changes; its tables and pool are the next state's before and after the commit, and are
+    refused once another call has changed the allocator."""
+    a = PageAllocator(2, 20, 3, 14, 4)
+    a.commit(a.plan_append([1], [4]))
+    first, second = a.plan_append([0, 1], [7, 3]), a.plan_append([0], [2])
+    want = (first.tables, first.free_pages)
+    assert want[0][0][:3] == (2, 3, 4) and want[0][1][:3] == (0, 1, 5) and len(want[1]) == 8
+    a.commit(first)
+    assert (a.tables, a.free_pages) == want == (first.tables, first.free_pages)
+    for stale in (lambda: a.commit(second), lambda: second.tables, lambda: second.free_pages, lambda: a.reset([0]) or first.tables):
+        with pytest.raises(RuntimeError, match="stale"):
+            stale()
+    other = PageAllocator(2, 20, 3, 14, 4)
+    with pytest.raises(RuntimeError, match="stale"):      # a plan of another allocator
+        other.commit(PageAllocator(2, 20, 3, 14, 4).plan_append([0], [1]))
