@@ -229,7 +229,9 @@ int moba_decode_attend(const moba_cache_desc* c, const void* q, const int32_t* i
                        unsigned* status, void* stream);
 /* moba_decode_step_begin, moba_decode_route (selected != null) and moba_decode_attend of one appended token per row, with their
  * arguments and results: one launch where the attention takes a cluster per (row, kv head) and the head dimension is at most 128
- * (u_chunk, u_mask and u_count are then left as they are), the two or three of them otherwise. */
+ * (u_chunk, u_mask and u_count are then left as they are), the two or three of them otherwise. The workspace's counters are used either
+ * way: zero before the first call, left at zero.  A token without a page in the table is reported in status, not stored, and counts as a row
+ * of zeros; its chunk's mean is not written. */
 int moba_decode_step(const moba_cache_desc* c, const int32_t* ids, int32_t* positions, const int32_t* delta, int rows, int hq,
                      const void* qkv, const void* cosv, const void* sinv, void* q, void* k, void* v, int remote, int width,
                      float* scores, int32_t* selected, int slots, int32_t* u_chunk, uint32_t* u_mask, int32_t* u_count, int umax,

@@ -161,8 +161,8 @@ __device__ __forceinline__ void chunk_mean_cta(const CacheView& cv, int sid, int
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (ri < rpi) {
     for (int w = ri; w < cv.C; w += rpi) {
-      const int t = chunk * cv.C + w;
-      const int physical = cv.table[(long long)sid * cv.width + t / cv.page];
+      const int t = chunk * cv.C + w, page = t / cv.page;
+      const int physical = page < cv.width ? cv.table[(long long)sid * cv.width + page] : -1;  // the last chunk may end behind the table
       if (physical < 0 || physical >= cv.num_pages) {
         if (status) atomicOr(status, kErrBadIndex);
         continue;
@@ -1367,7 +1367,8 @@ __device__ __forceinline__ bool attend_spoiled(const AttendState<DP>& st) {
 // of 16384 tokens took 2.5 + 4.3 + 10.4 us of them, a sparse layer of a 2000-token session 4.8 + 6.5 + 7.7.  Every CTA does what its
 // pair needs before the stages for itself (rotary embedding and routing of one group: a few thousand multiply-adds, and means that
 // lie in L2), so nothing waits for another CTA.  The new token is not read back through the cache: its score and V
-// row enter where CTA 0 combines its warps.  The length is advanced by the row's last cluster to have read it, found with a ticket.
+// row enter where CTA 0 combines its warps.  One that has no page is reported, not stored, counts as the row of zeros that the stages
+// read where a page is missing, and completes no mean: what the separate launches leave.  The length is advanced by the row's last cluster to have read it, found with a ticket.
 // One launch: 14.0 us instead of 17.2 (the step as a caller sees it 23.4 -> 22.6, where the host is the limit), layers 9.9 and 13.4 instead
 // of 12.2 and 19 (session step 292 -> 267 us).
 // grid (CL, pairs), cluster (CL, 1, 1)
@@ -1407,6 +1408,7 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
   float* s_sum = reinterpret_cast<float*>(s_pipe + PIPE);
   const int sid = a.ids[row];
   int pos, listed;
+  bool stored = true;   // the new token has a place in the cache (STEP, CTA 0)
   if (!STEP) {
     // one trip: position, sequence, the whole list and its length
     pos = a.positions[row];
@@ -1443,13 +1445,16 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
       *reinterpret_cast<uint4*>(s_new + hl * D + c * 8) = w;
     }
     __syncthreads();
+    stored = false;
     if (rank == 0) {
       // append; the page may have been opened by this step's delta
       const int logical = step.delta[row], opened = step.delta[step.b + row], page = pos / cv.page;
       if (g == 0 && tid == 0 && logical >= 0 && logical < cv.width) cv.table[(long long)sid * cv.width + logical] = opened;
       const int physical = page >= cv.width ? -1 : page == logical ? opened : cv.table[(long long)sid * cv.width + page];
-      if (physical < 0 || physical >= cv.num_pages) {
+      stored = physical >= 0 && physical < cv.num_pages;  // the same for every thread
+      if (!stored) {
         if (tid == 0) atomicOr(a.status, kErrBadIndex);
+        if (tid < upr) *reinterpret_cast<uint4*>(s_new + (G + 1) * D + tid * 8) = make_uint4(0u, 0u, 0u, 0u);  // V; read behind barriers
       } else if (tid < 2 * upr) {
         const long long dst = (((long long)physical * cv.page + (pos - page * cv.page)) * cv.Hkv + g) * D + (tid % upr) * 8;
         *reinterpret_cast<uint4*>((tid < upr ? cv.kc : cv.vc) + dst) = *reinterpret_cast<const uint4*>(s_new + G * D + tid * 8);
@@ -1463,7 +1468,7 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xFFFFFFFFu, dot, o);
-        if ((tid & 31) == 0) s_score[hl] = dot * a.scale_log2;
+        if ((tid & 31) == 0) s_score[hl] = stored ? dot * a.scale_log2 : 0.f;
       }
     }
     listed = 1;
@@ -1572,7 +1577,7 @@ __global__ void __launch_bounds__(128 * cluster_teams(DP), 1) decode_attend_clus
     }
   }
   cluster_barrier();  // no CTA leaves while another may still read its sums
-  if (STEP && rank == 0 && (pos + 1) % cv.C == 0 && pos / cv.C < cv.max_chunks) {
+  if (STEP && rank == 0 && stored && (pos + 1) % cv.C == 0 && pos / cv.C < cv.max_chunks) {
     // the new token, which this CTA appended, completes its chunk
     const int logical = step.delta[row];
     if (tid == 0 && logical >= 0 && logical < cv.width) cv.table[(long long)sid * cv.width + logical] = step.delta[step.b + row];

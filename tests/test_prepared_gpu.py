@@ -290,3 +290,74 @@ def test_step_in_one_launch_equals_its_three_launches(requests, hq, hk, dim, chu
             assert torch.equal(x, y)
         closed = caches[0].lengths[sid] // chunk
         assert torch.equal(caches[0]._means[sid, :closed], caches[1]._means[sid, :closed])
+
+
+def twin_plans(lens, hq, hk, dim, chunk, page, mode, dtype, room, seed, k0=None, v0=None):
+    """Two plans over equal caches: the first one's step is `moba_decode_step`, the second one's the entry points that it stands for."""
+    import ctypes
+    from moba_opt import PagedKVCache
+    gen = torch.Generator().manual_seed(seed)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    k0, v0 = (torch.randn(cu[-1], hk, dim, generator=gen).to("cuda", dtype) if t is None else t for t in (k0, v0))
+    plans, ids = [], list(range(len(lens)))
+    for _ in range(2):
+        cache = PagedKVCache(len(lens), max(lens) + room, hk, dim, page_size=page, chunk_size=chunk, dtype=dtype)
+        cache.append_prefill(k0, v0, sequence_ids=ids, cu_seqlens=cu, check_finite=False)
+        plans.append(cache.prepare_decode(ids, hq, topk=3, mode=mode, check_finite=False))
+    one, p = plans
+
+    def launch(kind, projected=None):
+        lib, d, st, rows = p._lib, p.cache._desc(), p._stream(), len(lens)
+        seqs, pos, status = p.gpu_ids.data_ptr(), p.positions.data_ptr(), p.cache._status.data_ptr()
+        union = (p._u_chunk.data_ptr(), p._u_mask.data_ptr(), p._u_count.data_ptr())
+        qkv, cos, sin = (None, None, None) if projected is None else (t.data_ptr() for t in projected)
+        assert lib.moba_decode_step_begin(ctypes.byref(d), seqs, pos, p.delta.data_ptr(), rows, hq, qkv, cos, sin, p.q.data_ptr(), p.k.data_ptr(),
+                                          p.v.data_ptr(), status, st) == 0
+        selected = None if p.dense else p.selected.data_ptr()
+        if not p.dense:
+            assert lib.moba_decode_route(ctypes.byref(d), p.q.data_ptr(), seqs, pos, rows, hq, p.remote, p.width, p.scores.data_ptr(), selected,
+                                         *union, st) == 0
+        assert lib.moba_decode_attend(ctypes.byref(d), p.q.data_ptr(), seqs, pos, rows, hq, selected, p._slots, *union, p._umax,
+                                      p._workspace.data_ptr(), p._ws_bytes, p.output.data_ptr(), p.lse.data_ptr(), status, st) == 0
+    p.launch = launch
+    return one, p
+
+
+@pytest.mark.parametrize("lens,hq,hk,dim,chunk,page,mode,dtype", [
+    ((63, 94), 14, 2, 64, 32, 16, "moba", torch.bfloat16),     # one row completes its chunk, the other does not
+    ((63,), 14, 2, 64, 32, 16, "dense", torch.bfloat16),
+    ((71, 95, 72), 6, 1, 128, 24, 7, "moba", torch.float16),   # pages across a chunk's end
+    ((31, 47), 8, 4, 32, 16, 5, "moba", torch.float16),        # eight CTAs a pair
+])
+def test_a_new_token_without_a_page(lens, hq, hk, dim, chunk, page, mode, dtype):
+    """The page of a row's new token is not mapped (a caller of the C entries without the planner): one launch and the separate ones
+    report it, leave the chunk's mean and the pool alone, and give the same routes, positions, lengths and outputs."""
+    import moba_opt.grouped_attention as ga
+    plans = twin_plans(lens, hq, hk, dim, chunk, page, mode, dtype, 2 * chunk, 41 + dim)
+    results = []
+    for p in plans:
+        c = p.cache
+        ga.check_status()
+        for sid, n in enumerate(lens):
+            assert n % page, "the page exists already"
+            c._table[sid, n // page] = -1
+        c._means[:, :, :] = 3.0
+        bits = [t.view(torch.int16) for t in (c.k_cache, c.v_cache)]     # unused pages may hold anything, NaN among it
+        pools = [t.clone() for t in bits]
+        gen = torch.Generator().manual_seed(5)
+        q, k, v = (torch.randn(len(lens), h, dim, generator=gen).to("cuda", dtype) for h in (hq, hk, hk))
+        p.stage_inputs(((q, p.q), (k, p.k), (v, p.v)))
+        p.launch("step")
+        with pytest.raises(RuntimeError, match="status bits"):
+            ga.check_status()
+        assert torch.equal(pools[0], bits[0]) and torch.equal(pools[1], bits[1])
+        assert bool((c._means == 3.0).all())
+        results.append([t.clone() for t in (c._table, c._lengths, p.positions, p.output, p.lse)] + ([] if p.dense else [p.selected.clone()]))
+    one, separate = results
+    for i in (0, 1, 2, 5)[:len(one) - 2]:
+        assert torch.equal(one[i], separate[i])
+    # the bounds of test_step_in_one_launch_equals_its_three_launches: neighbouring 16-bit values
+    torch.testing.assert_close(one[3].float(), separate[3].float(), rtol=2.0 ** (-7 if dtype == torch.bfloat16 else -10), atol=2e-5)
+    torch.testing.assert_close(one[4], separate[4], rtol=1e-5, atol=1e-5)
