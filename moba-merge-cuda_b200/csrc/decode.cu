@@ -1323,7 +1323,7 @@ __device__ __forceinline__ void attend_combine(AttendState<DP>& st, float* s_o, 
       const float m = extra.score[hh];
       big = fmaxf(big, m);
       const float2 x = unpack16<F16>(*reinterpret_cast<const uint32_t*>(extra.v + d));
-      lsum = dec_exp2(m - big);
+      lsum = m == -INFINITY ? 0.f : dec_exp2(m - big);  // a product beyond FP32; nothing else may be here yet
       v0 = x.x * lsum; v1 = x.y * lsum;
     }
 #pragma unroll

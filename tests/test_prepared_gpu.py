@@ -361,3 +361,21 @@ def test_a_new_token_without_a_page(lens, hq, hk, dim, chunk, page, mode, dtype)
     # the bounds of test_step_in_one_launch_equals_its_three_launches: neighbouring 16-bit values
     torch.testing.assert_close(one[3].float(), separate[3].float(), rtol=2.0 ** (-7 if dtype == torch.bfloat16 else -10), atol=2e-5)
     torch.testing.assert_close(one[4], separate[4], rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("mode", ["moba", "dense"])
+@pytest.mark.parametrize("length", [40, 1500])       # less than a stage for each CTA of a cluster, and more
+def test_a_new_token_whose_product_overflows(mode, length):
+    """q . k of the new token is -inf in FP32: it has no weight, in one launch as in the separate ones."""
+    hq, hk, dim = 4, 2, 64
+    results = []
+    for p in twin_plans((length,), hq, hk, dim, 512 if length > 512 else 32, 16, mode, torch.bfloat16, 8, 77):
+        gen = torch.Generator().manual_seed(9)
+        q, k, v = (torch.randn(1, h, dim, generator=gen).to("cuda", torch.bfloat16) for h in (hq, hk, hk))
+        q[:, :, 0], k[:, :, 0] = 2.0 ** 70, -(2.0 ** 70)
+        r = p.step(q, k, v)
+        results.append((r.output.clone(), r.lse.clone()))
+    (out, lse), (want, want_lse) = results
+    assert bool(want.isfinite().all()) and bool(want_lse.isfinite().all())
+    assert torch.equal(out, want)                    # scores of 2^70: all the weight is on one token
+    torch.testing.assert_close(lse, want_lse, rtol=1e-5, atol=0)
