@@ -1961,8 +1961,8 @@ static cudaError_t cluster_attributes(bool wide, bool half) {
   return e;
 }
 // Whether the current device can hold a cluster of CL CTAs at all: 16 is more than the portable size, and a partition of a GPU
-// may have fewer SMs side by side.  Asked once per device and kernel.
-template <int DP, int CL>
+// may have fewer SMs side by side.  Asked once per device and kernel (a whole step's has up to 8.8 KB more shared memory than the attention's).
+template <int DP, int CL, bool STEP = false>
 static bool cluster_fits(bool wide, bool half) {
   static std::atomic<signed char> known[2][2][64];  // 0 not asked yet, 1 yes, -1 no
   int dev = 0;
@@ -1980,8 +1980,8 @@ static bool cluster_fits(bool wide, bool half) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    const bool yes = cluster_attributes<DP, CL>(wide, half) == cudaSuccess &&
-                     cudaOccupancyMaxActiveClusters(&clusters, cluster_kernel<DP, CL>(wide, half), &cfg) == cudaSuccess && clusters > 0;
+    const bool yes = cluster_attributes<DP, CL, STEP>(wide, half) == cudaSuccess &&
+                     cudaOccupancyMaxActiveClusters(&clusters, cluster_kernel<DP, CL, STEP>(wide, half), &cfg) == cudaSuccess && clusters > 0;
     if (!yes) cudaGetLastError();  // an answer, not an error of the call
     answer.store(yes ? 1 : -1, std::memory_order_relaxed);
   }
@@ -1992,6 +1992,11 @@ static bool device_holds_cluster(int dim, int cl, bool wide, bool half) {
   if (dim <= 64) return cl == 16 ? cluster_fits<64, 16>(wide, half) : cluster_fits<64, 8>(wide, half);
   if (dim <= 128) return cl == 16 ? cluster_fits<128, 16>(wide, half) : cluster_fits<128, 8>(wide, half);
   return cl == 16 ? cluster_fits<256, 16>(wide, half) : cluster_fits<256, 8>(wide, half);
+}
+static bool device_holds_step(int dim, int cl, bool wide, bool half) {  // dim <= 128
+  if (dim <= 32) return cl == 16 ? cluster_fits<32, 16, true>(wide, half) : cluster_fits<32, 8, true>(wide, half);
+  if (dim <= 64) return cl == 16 ? cluster_fits<64, 16, true>(wide, half) : cluster_fits<64, 8, true>(wide, half);
+  return cl == 16 ? cluster_fits<128, 16, true>(wide, half) : cluster_fits<128, 8, true>(wide, half);
 }
 
 // Which variant, in us of a captured step (cluster / fixed parts / streamed), one request and heads 14/2 at D = 64 unless said:
@@ -2134,12 +2139,13 @@ extern "C" int moba_decode_attend(const moba_cache_desc* c, const void* q, const
 }
 
 // A step in one launch: where its attention takes a cluster per pair, the head dimension is at most 128 (256 threads a CTA), the routing
-// of a group fits the memory that the stages' ring takes later, and rows can be read 16 bytes at a time.
+// of a group fits the memory that the stages' ring takes later, rows can be read 16 bytes at a time, and the device holds a cluster of it.
 static bool step_fits_cluster(const moba_cache_desc* c, int hq, int variant, bool routed, int width, const void* qkv, uintptr_t addresses) {
   if ((variant != MOBA_ATTEND_CLUSTER_16 && variant != MOBA_ATTEND_CLUSTER_8) || c->dim > 128 || (addresses & 15)) return false;
   if (qkv && c->dim % 16) return false;
   const size_t ring = c->dim <= 32 ? ClusterSmem<32>::ring : c->dim <= 64 ? ClusterSmem<64>::ring : ClusterSmem<128>::ring;
-  return !routed || route_bytes(hq / c->hkv, width, c->dim) <= ring;
+  return (!routed || route_bytes(hq / c->hkv, width, c->dim) <= ring) &&
+         device_holds_step(c->dim, variant == MOBA_ATTEND_CLUSTER_16 ? 16 : 8, hq / c->hkv > 8, (c->flags & MOBA_CACHE_FP16) != 0);
 }
 
 extern "C" int moba_decode_step(const moba_cache_desc* c, const int32_t* ids, int32_t* positions, const int32_t* delta, int rows, int hq,
