@@ -379,3 +379,102 @@ def test_a_new_token_whose_product_overflows(mode, length):
     assert bool(want.isfinite().all()) and bool(want_lse.isfinite().all())
     assert torch.equal(out, want)                    # scores of 2^70: all the weight is on one token
     torch.testing.assert_close(lse, want_lse, rtol=1e-5, atol=0)
+
+
+def projected_step(p, qkv, cos, sin):
+    """One step from the fused projection, as a model session drives it; returns whether it was one launch (plans that route)."""
+    plan = p.plan_step()
+    p.send_delta(plan)
+    p._u_count.fill_(-7)                       # the one-launch form leaves the union lists alone
+    p.launch("step", (qkv, cos, sin))
+    p.commit_step(plan)
+    return p.dense or bool((p._u_count == -7).all())
+
+
+@pytest.mark.parametrize("lens,hq,hk,dim,chunk,page,mode,offset,one_launch", [
+    ((61, 94, 33), 14, 2, 64, 32, 16, "moba", 0, True),
+    ((20, 47), 8, 2, 32, 16, 5, "dense", 0, True),
+    ((70, 95), 6, 1, 96, 24, 7, "moba", 0, True),
+    ((63, 40, 55, 90), 8, 2, 128, 32, 16, "moba", 0, True),
+    ((63, 40), 20, 2, 128, 32, 16, "dense", 0, True),      # two head blocks
+    ((45, 61), 4, 2, 24, 16, 8, "moba", 0, False),         # half a head is not whole 16-byte units
+    ((61, 94), 14, 2, 64, 32, 16, "moba", 4, False),       # a projection 8 bytes off
+])
+def test_step_from_a_projection_equals_its_three_launches(lens, hq, hk, dim, chunk, page, mode, offset, one_launch):
+    """Rotary embedding and split of several rows inside the one launch, or in front of the separate ones where it cannot be taken."""
+    dtype, rows, width = torch.bfloat16, len(lens), (hq + 2 * hk) * dim
+    one, separate = twin_plans(lens, hq, hk, dim, chunk, page, mode, dtype, 2 * chunk, 13 + dim)
+    gen = torch.Generator().manual_seed(dim + hq)
+    for _ in range(chunk + 3):
+        flat = torch.randn(rows * width + offset, generator=gen).to("cuda", dtype)
+        qkv = flat[offset:].view(rows, width)
+        angle = torch.rand(rows, dim, generator=gen) * 6.3
+        cos, sin = angle.cos().to("cuda", dtype), angle.sin().to("cuda", dtype)
+        took = projected_step(one, qkv, cos, sin)
+        projected_step(separate, qkv, cos, sin)
+        assert mode == "dense" or took == one_launch
+        for name in ("q", "k", "v", "positions"):
+            assert torch.equal(getattr(one, name), getattr(separate, name)), name
+        if mode == "moba":
+            assert torch.equal(one.selected, separate.selected) and torch.equal(one.scores, separate.scores)
+        # the bounds of test_step_in_one_launch_equals_its_three_launches
+        torch.testing.assert_close(one.output.float(), separate.output.float(), rtol=2.0 ** -7, atol=2e-5)
+        torch.testing.assert_close(one.lse, separate.lse, rtol=1e-5, atol=1e-5)
+    a, b = one.cache, separate.cache
+    assert torch.equal(a._table, b._table) and torch.equal(a._lengths, b._lengths)
+    for p in (one, separate):
+        p.close()
+    for sid in range(rows):
+        for x, y in zip(a.materialize(sid), b.materialize(sid)):
+            assert torch.equal(x, y)
+        closed = a.lengths[sid] // chunk
+        assert closed and torch.equal(a._means[sid, :closed], b._means[sid, :closed])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("rows,hq,hk,dim,dtype", [
+    (1, 8, 2, 64, torch.bfloat16),
+    (2, 6, 1, 128, torch.float16),
+    (4, 40, 2, 128, torch.bfloat16),                       # eight CTAs a pair, two head blocks
+    (3, 4, 1, 32, torch.bfloat16),
+])
+def test_a_step_over_values_that_are_not_finite(rows, hq, hk, dim, dtype, bad):
+    """Such a V (of a caller that switched the check off) reaches the heads that attend its chunk and no other one, cached or new,
+    in the one-launch step as in the separate ones; every other value keeps its bits."""
+    chunk, chunks, poisoned = 100, 6, 2
+    length = chunks * chunk + 41
+    gen = torch.Generator().manual_seed(411)
+    rnd = lambda *shape: torch.randn(*shape, generator=gen).to("cuda", dtype)
+    k, v = rnd(length, hk, dim), rnd(length, hk, dim)
+    k[:, :, :chunks] = 0
+    for c in range(chunks):
+        k[c * chunk:(c + 1) * chunk, :, c] = 8             # chunk c is the best match of a query along axis c
+    turns = [(rnd(rows, hq, dim), rnd(rows, hk, dim), rnd(rows, hk, dim)) for _ in range(3)]
+    for q, _, _ in turns:
+        for h in range(hq):
+            q[:, h, h % chunks] = 40
+    seen = {}
+    for value in (1.0, bad):
+        vv = v.clone()
+        vv[poisoned * chunk + 33, :, 5] = value
+        one, separate = twin_plans((length,) * rows, hq, hk, dim, chunk, 7, "moba", dtype, 8, 0, k.repeat(rows, 1, 1), vv.repeat(rows, 1, 1))
+        seen[value] = []
+        for turn, (q, kn, vn) in enumerate(turns):
+            vn = vn.clone()
+            if turn == 1:
+                vn[:, :, 7] = value                        # the new token's
+            a, b = one.step(q, kn, vn), separate.step(q, kn, vn)
+            assert torch.equal(a.selected_blocks, b.selected_blocks) and torch.equal(a.output.isfinite(), b.output.isfinite())
+            seen[value].append((a.output.clone(), a.lse.clone(), a.selected_blocks.clone()))
+    for turn, ((good, lse, picks), (spoiled, lse_spoiled, _)) in enumerate(zip(seen[1.0], seen[bad])):
+        reads = (picks == poisoned).any(-1)
+        assert reads.any() and not reads.all()
+        assert bool(good.isfinite().all()) and torch.equal(lse, lse_spoiled)
+        wrong = torch.zeros_like(good, dtype=torch.bool)
+        wrong[..., 5] |= reads
+        if turn > 0:
+            wrong[..., 7] = True
+        assert torch.equal(spoiled.isfinite(), ~wrong)
+        assert torch.equal(good[~wrong], spoiled[~wrong])
+        if bad == bad:                                     # an infinity stays one, of its sign
+            assert (spoiled[wrong] == bad).all()
