@@ -203,14 +203,11 @@ __device__ __forceinline__ float dot8(const uint4& w, const uint4& x, float acc)
   return acc;
 }
 
-// Threads of a CTA.  Nine warps where a warp holds a gate/up pair: 4 CTAs an SM hold 5328 pairs then, 4736 with eight, and the few
-// CTAs of a second wave fetch their weights only when the first have left (ffn 4864: 608 CTAs on 592 places).
-constexpr int linear_threads(int tpr, bool pair) { return pair && tpr == 32 ? 288 : 256; }
-
-template <int TPR, bool PAIR>
-__global__ void __launch_bounds__(linear_threads(TPR, PAIR), 4) decode_linear_kernel(LinearArgs a) {
+// NT: threads of a CTA, 256 or 288 (see moba_decode_linear); the norm is the first 256 threads' either way.
+template <int TPR, bool PAIR, int NT>
+__global__ void __launch_bounds__(NT, 4) decode_linear_kernel(LinearArgs a) {
   constexpr int CH = PAIR ? 4 : 8;     // 16-byte loads per thread and weight row
-  constexpr int GROUPS = linear_threads(TPR, PAIR) / TPR;    // outputs per CTA and pass
+  constexpr int GROUPS = NT / TPR;     // outputs per CTA and pass
   extern __shared__ __align__(16) uint8_t s_raw[];
   __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(s_raw);
   __shared__ float s_part[8], s_red[2][8];
@@ -250,8 +247,8 @@ __global__ void __launch_bounds__(linear_threads(TPR, PAIR), 4) decode_linear_ke
   if (a.h_in) {
     float sum = 0.f;
     // The first 1024 elements are all requested before any is used: with a store to shared memory behind every load each of the
-    // four cost a trip to L2 of its own, in every projection of the step (eight layers, hidden 896: with the nine warps above
-    // 267 -> 254 us a step).
+    // four cost a trip to L2 of its own, in every projection of the step (eight layers, hidden 896, ffn 4864: with nine warps for
+    // gate/up 267 -> 254 us a step).
     __nv_bfloat16 hv[4], dv[4];
     if (tid < 256) {
 #pragma unroll
@@ -294,7 +291,7 @@ __global__ void __launch_bounds__(linear_threads(TPR, PAIR), 4) decode_linear_ke
         s_x[i] = __float2bfloat16_rn(__bfloat162float(a.norm_w[i]) * bf(__bfloat162float(s_x[i]) * r));
     }
   } else {
-    for (int c = tid; c < chunks; c += linear_threads(TPR, PAIR))
+    for (int c = tid; c < chunks; c += NT)
       reinterpret_cast<uint4*>(s_x)[c] = __ldcg(reinterpret_cast<const uint4*>(a.x) + c);  // not the read-only path: see above
   }
   __syncthreads();
@@ -479,6 +476,33 @@ extern "C" int moba_silu_mul(const void* gate_up, long long rows, int ffn, void*
   return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;
 }
 
+// CTAs that the device holds at once; 0 where it cannot be asked.
+template <int TPR, bool PAIR, int NT>
+static long long linear_resident(size_t smem, int sms) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_linear_kernel<TPR, PAIR, NT>, NT, smem) != cudaSuccess) return 0;
+  return (long long)per_sm * sms;
+}
+
+template <int TPR, bool PAIR, int NT = 256>
+static int launch_linear(const LinearArgs& a, size_t smem, int sms, cudaStream_t st) {
+  const long long groups = NT / TPR, units = (a.N + groups - 1) / groups, resident = linear_resident<TPR, PAIR, NT>(smem, sms);
+  if (resident < 1) return MOBA_ERR_CUDA;
+  const long long passes = units > 4 * resident ? (units + resident - 1) / resident : 1;  // a short tail is cheaper
+  return launch_dependent(1u, decode_linear_kernel<TPR, PAIR, NT>, dim3((unsigned)((units + passes - 1) / passes)), dim3(NT), smem, st, a) ==
+                 cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;
+}
+
+// Gate/up projection with a pair per warp.  Nine warps a CTA hold more pairs on the GPU at once than eight (5328 and 4736 with 4 CTAs on each
+// of 148 SMs), and the few CTAs of a second wave would fetch their weights only when the first have left; but where that is not
+// at stake nine are slower, with fewer registers and a barrier over more warps.  So nine exactly where they save the second wave.  us a launch, eight
+// / nine, hidden 896: ffn 2560 3.76 / 4.32, 3072 4.07 / 4.48, 4096 4.59 / 5.22, 4736 5.27 / 5.56, 4864 6.48 / 5.71, 5328 6.91 / 6.09,
+// 5632 7.20 / 7.66, 8192 8.50 / 9.84; hidden 512 4096 3.58 / 3.68, 4864 5.10 / 3.98; hidden 1024 4096 4.99 / 5.35, 4864 7.02 / 6.09.
+static int launch_linear_pairs(const LinearArgs& a, size_t smem, int sms, cudaStream_t st) {
+  const bool nine = (a.N + 7) / 8 > linear_resident<32, true, 256>(smem, sms) && (a.N + 8) / 9 <= linear_resident<32, true, 288>(smem, sms);
+  return nine ? launch_linear<32, true, 288>(a, smem, sms, st) : launch_linear<32, true>(a, smem, sms, st);
+}
+
 extern "C" int moba_decode_linear(const void* x, const void* h_in, const void* delta, const void* norm_weight, float eps, void* h_out,
                                   const void* weight, const void* bias, int k, int n, int epilogue, void* y, void* stream) {
   if (!weight || !y || k < 8 || (k & 7) || n < 1 || (epilogue != 0 && epilogue != 1)) return MOBA_ERR_INVALID;
@@ -505,28 +529,12 @@ extern "C" int moba_decode_linear(const void* x, const void* h_in, const void* d
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return MOBA_ERR_CUDA;
-#define MOBA_LAUNCH_LINEAR_P(T, P)                                                                                  \
-  do {                                                                                                              \
-    int per_sm = 0;                                                                                                 \
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_linear_kernel<T, P>, linear_threads(T, P), smem) != cudaSuccess || per_sm < 1) \
-      return MOBA_ERR_CUDA;                                                                                         \
-    const long long groups = linear_threads(T, P) / T, units = (n + groups - 1) / groups, resident = (long long)per_sm * sms;                      \
-    const long long passes = units > 4 * resident ? (units + resident - 1) / resident : 1; /* a short tail is cheaper */ \
-    if (launch_dependent(1u, decode_linear_kernel<T, P>, dim3((unsigned)((units + passes - 1) / passes)), dim3(linear_threads(T, P)), smem, st, \
-                         a) != cudaSuccess)                                                                         \
-      return MOBA_ERR_CUDA;                                                                                         \
-  } while (0)
-#define MOBA_LAUNCH_LINEAR(T)                                                                                       \
-  do {                                                                                                              \
-    if (pair) MOBA_LAUNCH_LINEAR_P(T, true);                                                                        \
-    else MOBA_LAUNCH_LINEAR_P(T, false);                                                                            \
-  } while (0)
-  if (tpr == 32) MOBA_LAUNCH_LINEAR(32);
-  else if (tpr == 64) MOBA_LAUNCH_LINEAR(64);
-  else if (tpr == 128) MOBA_LAUNCH_LINEAR(128);
-  else MOBA_LAUNCH_LINEAR(256);
-#undef MOBA_LAUNCH_LINEAR_P
-#undef MOBA_LAUNCH_LINEAR
+  int rc = MOBA_OK;
+  if (tpr == 32) rc = pair ? launch_linear_pairs(a, smem, sms, st) : launch_linear<32, false>(a, smem, sms, st);
+  else if (tpr == 64) rc = pair ? launch_linear<64, true>(a, smem, sms, st) : launch_linear<64, false>(a, smem, sms, st);
+  else if (tpr == 128) rc = pair ? launch_linear<128, true>(a, smem, sms, st) : launch_linear<128, false>(a, smem, sms, st);
+  else rc = pair ? launch_linear<256, true>(a, smem, sms, st) : launch_linear<256, false>(a, smem, sms, st);
+  if (rc != MOBA_OK) return rc;
   return cudaGetLastError() == cudaSuccess ? MOBA_OK : MOBA_ERR_CUDA;
 }
 

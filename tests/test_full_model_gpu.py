@@ -192,6 +192,32 @@ def test_decode_linear_gate_up_epilogue(k, ffn):
     assert _rel_l2(y, want) <= 8e-3
 
 
+@pytest.mark.parametrize("k,ffn", [(8, 33), (896, 4736), (896, 4737), (1024, 5000), (512, 5328), (1024, 5329), (1032, 77),
+                                   (64, 19500)])   # both sides of what eight and nine warps hold at once, of 32 lanes a pair, of one pass
+@pytest.mark.parametrize("delta", [False, True])
+def test_decode_linear_gate_up_behind_the_norm(k, ffn, delta):
+    """Residual add, RMSNorm and gate/up projection in one launch, with eight and with nine warps a CTA, against the module arithmetic."""
+    import ctypes
+    from moba_opt import _ext
+    lib = _ext.lib()
+    g = torch.Generator().manual_seed(k * 7 + ffn)
+    w = (torch.randn(2 * ffn, k, generator=g) * k ** -0.5).cuda().bfloat16()
+    h, d = (torch.randn(k, generator=g).cuda().bfloat16() for _ in range(2))
+    nw = (1 + 0.1 * torch.randn(k, generator=g)).cuda().bfloat16()
+    y, h_out = torch.empty(ffn, device="cuda", dtype=torch.bfloat16), torch.empty(k, device="cuda", dtype=torch.bfloat16)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.moba_decode_linear(None, h.data_ptr(), d.data_ptr() if delta else None, nw.data_ptr(), 1e-6, h_out.data_ptr(), w.data_ptr(), None,
+                                  k, ffn, 1, y.data_ptr(), st) == 0
+    res = h + d if delta else h
+    assert torch.equal(h_out, res)
+    f = res.float()
+    x = nw * (f * torch.rsqrt(f.pow(2).mean() + 1e-6)).bfloat16()
+    gu = w.double() @ x.double()
+    want = torch.nn.functional.silu(gu[:ffn]) * gu[ffn:]
+    # the bound of test_decode_linear_gate_up_epilogue: gate, up, silu and product rounded to bf16, 2^-9 each
+    assert _rel_l2(y, want) <= 8e-3
+
+
 def test_decode_linear_contract():
     import ctypes
     from moba_opt import _ext
