@@ -251,3 +251,15 @@ def test_a_plan_shows_the_next_state_until_the_allocator_moves_on():
     other = PageAllocator(2, 20, 3, 14, 4)
     with pytest.raises(RuntimeError, match="stale"):      # a plan of another allocator
         other.commit(PageAllocator(2, 20, 3, 14, 4).plan_append([0], [1]))
+
+
+@pytest.mark.parametrize("ids,counts", [((2,), (1,)), ((0, 2), (3, 5)), ((1, 0, 2), (20, 40, 4)), ((1, 0, 2), (20, 40, 5)), ((1,), (700,))])
+def test_rows_of_an_append_in_both_forms(ids, counts):
+    """Up to 64 tokens and more: the ids and positions that a full plan lists."""
+    from moba_opt.kv_cache import token_rows
+    a = PageAllocator(3, 1000, 7, 500, 16)
+    a.commit(a.plan_append([0, 2], [11, 30]))
+    plan = a.plan_append(ids, counts)
+    rows = token_rows(ids, counts, a.lengths)
+    assert all(isinstance(r, tuple) == (sum(counts) <= 64) for r in rows)
+    assert [tuple(int(x) for x in r) for r in rows] == [plan.token_sequences, plan.token_positions]
