@@ -329,7 +329,6 @@ class PagedKVCache:
             self._status = _status_word(self.device)
             self._staging = HostStaging(self.device)
             self._finite = FiniteCheck(self._lib, self.device, self._staging.spare)
-            self._pools = frozenset(t.untyped_storage().data_ptr() for t in (self.k_cache, self.v_cache))
             self._attend_buffers = {}         # (rows, Hq, slots, umax) -> union lists + split-K workspace, kept between calls
 
     # ------------------------------------------------------------------ views of the CPU layout
@@ -373,7 +372,8 @@ class PagedKVCache:
             raise ValueError("cross-stream cache access is unsupported")
 
     def _refuse_pool_aliases(self, *tensors):
-        if any(t.untyped_storage().data_ptr() in self._pools for t in tensors):
+        pools = {self.k_cache.untyped_storage().data_ptr(), self.v_cache.untyped_storage().data_ptr()}   # the present ones
+        if any(t.untyped_storage().data_ptr() in pools for t in tensors):
             raise ValueError("append inputs must not alias KV cache storage; clone first")
 
     def _routable(self, lengths):

@@ -718,3 +718,17 @@ def test_threads_with_caches_of_different_width():
             p.selected.data_ptr(), p._u_chunk.data_ptr(), p._u_mask.data_ptr(), p._u_count.data_ptr(), p._stream())))
         keep.append((p, desc))
     assert two_threads(calls) == [0, 0]
+
+
+def test_the_alias_check_looks_at_the_pools_in_use():
+    """Pools that a caller has put in the place of the first ones (offloaded and brought back, say) count, the first ones no longer."""
+    from moba_opt import PagedKVCache
+    cache = PagedKVCache(1, 8, 1, 8, page_size=3, chunk_size=4)
+    first = cache.k_cache.zero_()
+    cache.v_cache.zero_()
+    cache.k_cache = first.clone()
+    external = rand((1, 1, 8), 271)
+    with pytest.raises(ValueError, match="must not alias"):
+        cache.append(cache.k_cache.reshape(-1, 1, 8)[:1], external, sequence_ids=[0])
+    cache.append(first.reshape(-1, 1, 8)[:1], external, sequence_ids=[0])
+    assert cache.lengths == (1,)
