@@ -732,3 +732,22 @@ def test_the_alias_check_looks_at_the_pools_in_use():
         cache.append(cache.k_cache.reshape(-1, 1, 8)[:1], external, sequence_ids=[0])
     cache.append(first.reshape(-1, 1, 8)[:1], external, sequence_ids=[0])
     assert cache.lengths == (1,)
+
+
+@pytest.mark.parametrize("counts", [(30, 34), (30, 35), (1, 300)])    # ids and positions as integers, and as arrays
+def test_long_segments_in_one_call_equal_append_then_attend(counts):
+    from moba_opt import PagedKVCache
+    results, n, cu = [], sum(counts), [0, counts[0], sum(counts)]
+    first, q, k, v = rand((90, 2, 64), 601), rand((n, 8, 64), 602), rand((n, 2, 64), 603), rand((n, 2, 64), 604)
+    for combined in (True, False):
+        cache = PagedKVCache(2, 512, 2, 64, page_size=16, chunk_size=32)
+        cache.append(first, first, sequence_ids=[1, 0], cu_seqlens=[0, 50, 90])
+        if combined:
+            results.append(cache.append_and_attend(q, k, v, sequence_ids=[1, 0], cu_seqlens=cu, topk=3))
+        else:
+            cache.append(k, v, sequence_ids=[1, 0], cu_seqlens=cu)
+            ids = [1] * counts[0] + [0] * counts[1]
+            results.append(cache.attend(q, sequence_ids=ids, positions=[*range(50, 50 + counts[0]), *range(40, 40 + counts[1])], topk=3))
+    a, b = results
+    assert a.sequence_ids == b.sequence_ids and a.positions == b.positions and all(type(x) is int for x in a.positions)
+    assert torch.equal(a.output, b.output) and torch.equal(a.lse, b.lse) and torch.equal(a.selected_blocks, b.selected_blocks)
