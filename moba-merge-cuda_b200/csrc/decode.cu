@@ -1369,8 +1369,8 @@ __device__ __forceinline__ bool attend_spoiled(const AttendState<DP>& st) {
 // lie in L2), so nothing waits for another CTA.  The new token is not read back through the cache: its score and V
 // row enter where CTA 0 combines its warps.  One that has no page is reported, not stored, counts as the row of zeros that the stages
 // read where a page is missing, and completes no mean: what the separate launches leave.  The length is advanced by the row's last cluster to have read it, found with a ticket.
-// One launch: 14.0 us instead of 17.2 (the step as a caller sees it 23.4 -> 22.6, where the host is the limit), layers 9.9 and 13.4 instead
-// of 12.2 and 19 (session step 292 -> 267 us).
+// One launch: 14.0 us instead of 17.2 (a caller of one plan sees no difference beyond the runs' spread, 22 to 23 us either way: the host is the
+// limit there), layers 9.9 and 13.4 instead of 12.2 and 19 (session step 292 -> 267 us).
 // grid (CL, pairs), cluster (CL, 1, 1)
 struct StepArgs {
   const int* delta;

@@ -128,9 +128,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_ws128_kernel(BwdArgs a) 
         // row, lanes on consecutive floats), and the copy engine adds each row to its place in the FP32 accumulator:
         // one 512-byte reduction per row, carried by the engine's own path to the L2 cache instead of the load/store pipe.
         // The warps meet twice per step: before writing (the engine has read the previous step's rows) and before
-        // the rows are handed over.  A warp needs 62 cycles to ask for one row, whatever its size (one lane after the
-        // other), so six ask, warps 10 and 11 among them: with two warps asking for 32 rows each, 2040 of the 3070
-        // cycles of a step went there and the products waited for the drain.  A step takes 2100 to 2400 cycles now; at
+        // the rows are handed over.  A warp needs 63 cycles to ask for one row, whatever its size (one lane after the
+        // other), so six ask, warps 10 and 11 among them: with two warps asking for 32 rows each, 2010 of the 3050
+        // cycles of a step went there (clock stamps) and the products waited for the drain.  A step takes 2360 cycles now; at
         // full size the clock falls with it (power cap), so training steps went 41.5 -> 38.0 ms (131072 tokens, 4/1 heads,
         // chunk 4096, topk 12) and 3.48 -> 3.26 ms (4 x 8192 tokens, 12/2 heads, chunk 512, topk 8).
         bulk_wait_group_read();

@@ -28,8 +28,8 @@ constexpr int kMeanRows = 256;   // tokens per CTA of the mean pass
 // left zero).  Every sum has a fixed order - rows of a slice by (row mod rows-per-pass, then pass), slices
 // ascending - so the means are bit-repeatable whichever CTA happens to finish last.
 // CLUSTER: the slices of a chunk are the CTAs of a cluster, and the first one reads the others' sums from their shared memory: no
-// counters, so none to clear before the call (a launch less, 4 us of the host's and the GPU's time in a small call), and no trip
-// through global memory.  The same additions in the same order.
+// counters, so none to clear before the call (a launch less: 1 x 2048 tokens 67.5 -> 64.6 us together with shared-memory limits that are set once,
+// runs of one side 2.6 % apart), and no trip through global memory.  The same additions in the same order.
 template <bool CLUSTER>
 __global__ void __launch_bounds__(256) chunk_mean_kernel(PrefillView pv, const __nv_bfloat16* __restrict__ k, float* part,
                                                          float* __restrict__ means, int* tickets, int* scan_ticket, int round_bf16, int splits) {
